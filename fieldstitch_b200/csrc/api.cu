@@ -49,7 +49,7 @@ void DevBuf::release() {
 }
 
 size_t Workspace::bytes() const {
-    size_t t = dog.bytes + mag.bytes + ang.bytes + img.bytes + cand.bytes + refined.bytes + oriented.bytes +
+    size_t t = dog.bytes + grad.bytes + img.bytes + cand.bytes + refined.bytes + oriented.bytes +
                keys_a.bytes + keys_b.bytes + vals_a.bytes + vals_b.bytes + sort_tmp.bytes + counters.bytes +
                kx.bytes + ky.bytes + ksize.bytes + kangle.bytes + kresp.bytes + koct.bytes + klayer.bytes +
                spread.bytes + take.bytes;
@@ -58,7 +58,7 @@ size_t Workspace::bytes() const {
 }
 
 void Workspace::release() {
-    DevBuf* all[] = {&dog, &mag, &ang, &img, &cand, &refined, &oriented, &keys_a, &keys_b, &vals_a, &vals_b,
+    DevBuf* all[] = {&dog, &grad, &img, &cand, &refined, &oriented, &keys_a, &keys_b, &vals_a, &vals_b,
                      &sort_tmp, &counters, &kx, &ky, &ksize, &kangle, &kresp, &koct, &klayer,
                      &plane[0], &plane[1], &plane[2], &next_base, &spread, &take};
     for (DevBuf* b : all) b->release();
@@ -71,8 +71,7 @@ static int32_t prepare_workspace(Workspace& ws, int h, int w) {
     const size_t sum = (size_t)g.grad_off[g.n_oct] / 3;   // sum of octave pixels
     const size_t p0 = (size_t)g.R[0] * g.C[0];
     FSB_TRY(ws.dog.ensure(5 * sum * 4));
-    FSB_TRY(ws.mag.ensure(3 * sum * 4));
-    FSB_TRY(ws.ang.ensure(3 * sum * 4));
+    FSB_TRY(ws.grad.ensure(3 * sum * 8));
     for (auto& b : ws.plane) FSB_TRY(b.ensure(p0 * 4));
     if (g.n_oct > 1) FSB_TRY(ws.next_base.ensure(2 * (((size_t)g.R[1] * g.C[1] + 63) / 64 * 64) * 4));
     FSB_TRY(ws.img.ensure((size_t)h * w));
@@ -228,6 +227,13 @@ static int32_t detect_into(fsb_ctx* ctx, Workspace& ws, const uint8_t* img, int 
     }
     ctx->stage_end(ST_UPLOAD);
     return detect_dev(ctx, ws, ws.img.as<uint8_t>(), w, p, max_kp);
+}
+
+// one component of the gradient atlas: part 0 the magnitudes, 1 the angles
+__global__ void k_grad_part(const float2* __restrict__ g, long long n, int part, float* __restrict__ out) {
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
+        out[i] = part ? g[i].y : g[i].x;
 }
 
 // selected keypoints -> describe inputs (tx..tly) and optional interleaved xy / response outputs
@@ -700,9 +706,20 @@ int32_t fsb_state_atlas(fsb_state* st, int32_t which, float* out, int64_t n_floa
         return FSB_ERR_ARG;
     }
     FSB_TRY(use_device(st->ctx));
-    const DevBuf& b = which == 0 ? st->ws->dog : which == 1 ? st->ws->mag : st->ws->ang;
-    if (want) FSB_CUDA(cudaMemcpyAsync(out, b.p, (size_t)want * 4, cudaMemcpyDeviceToHost, st->ctx->stream));
-    FSB_CUDA(cudaStreamSynchronize(st->ctx->stream));
+    fsb_ctx* ctx = st->ctx;
+    if (!want) return FSB_OK;
+    const float* src = st->ws->dog.as<float>();
+    if (which != 0) {   // the magnitudes or the angles of the (magnitude, angle) atlas
+        FSB_TRY(ctx->s_misc.ensure((size_t)want * 4));
+        const long long nb = (want + 255) / 256;
+        k_grad_part<<<(unsigned)std::min<long long>(nb, 148 * 64), 256, 0, ctx->stream>>>(
+            st->ws->grad.as<float2>(), want, which - 1, ctx->s_misc.as<float>());
+        note_launch();
+        FSB_CUDA(cudaGetLastError());
+        src = ctx->s_misc.as<float>();
+    }
+    FSB_CUDA(cudaMemcpyAsync(out, src, (size_t)want * 4, cudaMemcpyDeviceToHost, ctx->stream));
+    FSB_CUDA(cudaStreamSynchronize(ctx->stream));
     return FSB_OK;
 }
 
@@ -943,7 +960,7 @@ int32_t sift_features_batch(fsb_ctx* ctx, int32_t n_img, const uint8_t* const* h
         key_put(key, d_rootsift[i]);
     }
     for (Workspace* ws : x.ws) {
-        const void* ptrs[] = {ws->dog.p, ws->mag.p, ws->ang.p, ws->plane[0].p, ws->plane[1].p, ws->plane[2].p,
+        const void* ptrs[] = {ws->dog.p, ws->grad.p, ws->plane[0].p, ws->plane[1].p, ws->plane[2].p,
                               ws->next_base.p, ws->cand.p, ws->refined.p, ws->oriented.p, ws->keys_a.p, ws->keys_b.p,
                               ws->vals_a.p, ws->sort_tmp.p, ws->counters.p, ws->kx.p, ws->ky.p, ws->ksize.p,
                               ws->kangle.p, ws->kresp.p, ws->koct.p, ws->klayer.p, ws->spread.p, ws->take.p};
@@ -1089,7 +1106,7 @@ int32_t fsb_pyramid_batch_d(fsb_ctx* ctx, int32_t n_img, const uint8_t* const* d
     for (int i = 0; i < n_img; ++i) key_put(key, d_imgs[i]);
     for (int c = 0; c < chains; ++c) {
         const Workspace* ws = x.ws[c];
-        const void* ptrs[] = {ws->dog.p, ws->mag.p, ws->ang.p, ws->plane[0].p, ws->plane[1].p, ws->plane[2].p,
+        const void* ptrs[] = {ws->dog.p, ws->grad.p, ws->plane[0].p, ws->plane[1].p, ws->plane[2].p,
                               ws->next_base.p, ws->counters.p};
         for (const void* q : ptrs) key_put(key, q);
     }

@@ -138,7 +138,7 @@ struct GuidedGraph {
 // Pyramid + detection workspace sized for one image geometry.
 struct Workspace {
     Geometry g{};
-    DevBuf dog, mag, ang;        // atlases
+    DevBuf dog, grad;            // atlases: DoG float32, gradient (magnitude, angle) float2
     DevBuf plane[3];             // gauss-layer scratch planes (octave-0 size)
     DevBuf next_base;            // two octave-1-sized halves: the next octave's base, alternating
     DevBuf img;                  // uploaded uint8 image
@@ -225,18 +225,18 @@ int32_t run_pyramid(Workspace& ws, const uint8_t* d_img, int img_stride, bool ex
                     cudaStream_t side = nullptr, cudaEvent_t* ev = nullptr);
 // octave.cu
 int32_t upload_octave_taps(const float* taps, int stride, const int* counts);
-int32_t launch_octave_fused(const float* L0, int R, int C, float* dog, float* mag, float* ang, float* down,
+int32_t launch_octave_fused(const float* L0, int R, int C, float* dog, float2* grad, float* down,
                             int down_cols, cudaStream_t s);
 int layer_tile_variants();
 int layer_tile_height(int variant);
-int32_t launch_layer_fast(int layer, const float* src, int R, int C, float* dst, float* dog, float* mag, float* ang,
+int32_t launch_layer_fast(int layer, const float* src, int R, int C, float* dst, float* dog, float2* grad,
                           float* down, int down_cols, int variant, int* err, cudaStream_t s);
 int32_t launch_base_fast(const uint8_t* img, int stride, int ih, int iw, float* dst, int variant, cudaStream_t s);
-int32_t launch_group_lower(const float* src, int R, int C, float* dog, float* mag, float* ang, float* l3, float* down,
+int32_t launch_group_lower(const float* src, int R, int C, float* dog, float2* grad, float* l3, float* down,
                            int down_cols, cudaStream_t s);
 int32_t launch_group_upper(const float* src, int R, int C, float* dog3, cudaStream_t s);
 // strip engine: the whole float32 octave in one launch (err: device word set when a TMA wait gives up)
-int32_t launch_octave_strip(const float* L0, int R, int C, float* dog, float* mag, float* ang, float* down,
+int32_t launch_octave_strip(const float* L0, int R, int C, float* dog, float2* grad, float* down,
                             int down_cols, int* err, cudaStream_t s);
 constexpr int PYR_ERR_WORD = 8;   // index of the pyramid's error word in Workspace::counters
 // autotune.cu: the fastest of n_variants launches of `run` for `key` (timed once per process and

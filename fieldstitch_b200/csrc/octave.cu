@@ -63,8 +63,7 @@ struct Args {
     const float* L0;              // octave base, pitch C
     int R, C, rows_per_cta;
     float* dog[5];                // DoG planes R x C
-    float* mag[3];                // gradient magnitude of layers 1..3
-    float* ang[3];                // gradient angle of layers 1..3
+    float2* grad[3];              // gradient (magnitude, angle) of layers 1..3
     float* down;                  // next octave base or null
     int down_cols;
 };
@@ -72,6 +71,25 @@ struct Args {
 // 16-byte alignment of a plane address: the atlases pack octaves back to back, so an octave's
 // planes can start off a 16-byte boundary even when its width is a multiple of 4
 __device__ __forceinline__ bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+__device__ __forceinline__ bool al32(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31) == 0; }
+
+// Four gradient pixels (magnitude, angle) to a 32-byte aligned address: one 32-byte store, so a lane
+// fills whole sectors (two 16-byte stores 32 bytes apart per lane would send each sector twice).
+__device__ __forceinline__ void st_grad4(float2* p, const float (&mg)[4], const float (&an)[4]) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(mg[0]), "f"(an[0]), "f"(mg[1]),
+                 "f"(an[1]), "f"(mg[2]), "f"(an[2]), "f"(mg[3]), "f"(an[3])
+                 : "memory");
+}
+// the first `left` of four gradient pixels; vec: all four and p's row may allow the wide store
+__device__ __forceinline__ void store_grad4(float2* p, const float (&mg)[4], const float (&an)[4], bool vec, int left) {
+    if (vec && al32(p)) {
+        st_grad4(p, mg, an);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (k < left) p[k] = make_float2(mg[k], an[k]);
+    }
+}
 
 __device__ __forceinline__ int mir(int p, int n) {
     if (n == 1) return 0;
@@ -317,17 +335,7 @@ __device__ __forceinline__ void epilogue(const float* prev, const float* cur, co
             }
         }
         fast_grad4(dx, dy, mg, an);
-        float* m = a.mag[I - 2] + at;
-        float* n = a.ang[I - 2] + at;
-        if (vec && al16(m) && al16(n)) {
-            *reinterpret_cast<float4*>(m) = make_float4(mg[0], mg[1], mg[2], mg[3]);
-            *reinterpret_cast<float4*>(n) = make_float4(an[0], an[1], an[2], an[3]);
-        } else {
-            for (int k = 0; k < 4 && xg + k < a.C; ++k) {
-                m[k] = mg[k];
-                n[k] = an[k];
-            }
-        }
+        store_grad4(a.grad[I - 2] + at, mg, an, vec, a.C - xg);
     }
     if (I == 4 && a.down && !(y & 1)) {
         float* o = a.down + (y >> 1) * a.down_cols + (xg >> 1);
@@ -460,8 +468,7 @@ struct LayerArgs {
     int R, C;
     float* dst;         // L_I or null
     float* dog;         // L_I - L_{I-1}
-    float* mag;         // gradient of L_{I-1} or null
-    float* ang;
+    float2* grad;       // gradient (magnitude, angle) of L_{I-1} or null
     float* down;        // L_{I-1}[::2, ::2] or null
     int down_cols;
     int* err;           // set to 1 when the tile's TMA copy does not complete in time
@@ -563,7 +570,7 @@ __device__ __forceinline__ void layer_compute(const LayerArgs& a, const float* _
     bool fast = (a.C & 3) == 0 && (long long)a.R * a.C < (1ll << 31) && x0 + LX <= a.C && y0 + LY <= a.R &&
                 (!a.dst || al16(a.dst));
     if (!BASE)
-        fast = fast && al16(a.dog) && (!a.mag || (al16(a.mag) && al16(a.ang))) && y0 >= 1 && y0 + LY <= a.R - 1 &&
+        fast = fast && al16(a.dog) && (!a.grad || al32(a.grad)) && y0 >= 1 && y0 + LY <= a.R - 1 &&
                x0 >= 1 && x0 + LX < a.C;
     if (fast) {
         for (int it = tid; it < (LY / 2) * (LX / 4); it += LNT) {
@@ -595,7 +602,7 @@ __device__ __forceinline__ void layer_compute(const LayerArgs& a, const float* _
                 const float4 pv = *reinterpret_cast<const float4*>(ctr);
                 *reinterpret_cast<float4*>(a.dog + at) = make_float4(lv.x - pv.x, lv.y - pv.y, lv.z - pv.z, lv.w - pv.w);
                 if (a.dst) *reinterpret_cast<float4*>(a.dst + at) = lv;
-                if (a.mag) {
+                if (a.grad) {
                     const float4 up = *reinterpret_cast<const float4*>(ctr - LIN_W);
                     const float4 dn = *reinterpret_cast<const float4*>(ctr + LIN_W);
                     const float lf = ctr[-1], rt = ctr[4];
@@ -605,8 +612,7 @@ __device__ __forceinline__ void layer_compute(const LayerArgs& a, const float* _
                                          __fsub_rn(up.w, dn.w)};
                     float mg[4], an[4];
                     fast_grad4(dx, dy, mg, an);
-                    *reinterpret_cast<float4*>(a.mag + at) = make_float4(mg[0], mg[1], mg[2], mg[3]);
-                    *reinterpret_cast<float4*>(a.ang + at) = make_float4(an[0], an[1], an[2], an[3]);
+                    st_grad4(a.grad + at, mg, an);
                 }
                 if (a.down && h == 0) {   // y is even: y0 and 2p are
                     float* o2 = a.down + (y >> 1) * a.down_cols + (x >> 1);
@@ -668,20 +674,10 @@ __device__ __forceinline__ void layer_compute(const LayerArgs& a, const float* _
                     if (a.dst) a.dst[at + k] = lv[k];
                 }
             }
-            if (a.mag) {
+            if (a.grad) {
                 float mg[4], an[4];
                 grad4<LIN_W>(ctr, yy, x, a.R, a.C, mg, an);
-                if (vec && al16(a.mag) && al16(a.ang)) {
-                    *reinterpret_cast<float4*>(a.mag + at) = make_float4(mg[0], mg[1], mg[2], mg[3]);
-                    *reinterpret_cast<float4*>(a.ang + at) = make_float4(an[0], an[1], an[2], an[3]);
-                } else {
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        if (x + k >= a.C) break;
-                        a.mag[at + k] = mg[k];
-                        a.ang[at + k] = an[k];
-                    }
-                }
+                store_grad4(a.grad + at, mg, an, vec, a.C - x);
             }
             if (a.down && !(yy & 1)) {
                 float* o2 = a.down + (size_t)(yy >> 1) * a.down_cols + (x >> 1);
@@ -968,8 +964,7 @@ struct GroupArgs {
     int R, C;
     int tiles_x, n_tiles;
     float* dog[3];      // DoG planes of the group's layers
-    float* mag[3];      // group 0: gradients of L1, L2, L3
-    float* ang[3];
+    float2* grad[3];    // group 0: gradients of L1, L2, L3
     float* dst;         // group 0: L3
     float* down;        // group 0: L3[::2, ::2] or null
     int down_cols;
@@ -1070,20 +1065,19 @@ __device__ __forceinline__ void g_store4(float* p, float4 v, bool vec, int left)
     }
 }
 
-// at image row yy, columns xx .. xx + 3: the DoG cur - prev and, with mag set, the gradient of
+// at image row yy, columns xx .. xx + 3: the DoG cur - prev and, with grad set, the gradient of
 // prev (prev points at prev(yy, xx) in a shared level of pitch P; the same arithmetic as k_layer)
 template <int P>
 __device__ __forceinline__ void g_dog_grad(const GroupArgs& a, int yy, int xx, const float* prev, float4 cur,
-                                           float* dog, float* mag, float* ang) {
+                                           float* dog, float2* grad) {
     const float4 pv = *reinterpret_cast<const float4*>(prev);
     const size_t at = (size_t)yy * a.C + xx;
     const bool vec = (a.C & 3) == 0;   // xx is a multiple of 4 below C
     g_store4(dog + at, make_float4(cur.x - pv.x, cur.y - pv.y, cur.z - pv.z, cur.w - pv.w), vec, a.C - xx);
-    if (mag) {
+    if (grad) {
         float mg[4], an[4];
         grad4<P>(prev, yy, xx, a.R, a.C, mg, an);
-        g_store4(mag + at, make_float4(mg[0], mg[1], mg[2], mg[3]), vec, a.C - xx);
-        g_store4(ang + at, make_float4(an[0], an[1], an[2], an[3]), vec, a.C - xx);
+        store_grad4(grad + at, mg, an, vec, a.C - xx);
     }
 }
 
@@ -1094,14 +1088,15 @@ struct GEpi {
     const GroupArgs& a;
     int y0, x0;
     const float* prev;
-    float *dog, *mag, *ang;
+    float* dog;
+    float2* grad;
     __device__ __forceinline__ void operator()(int ty, int tx, float4 top, float4 bot) const {
         if (tx < 0 || tx >= GX || x0 + tx >= a.C) return;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int t = ty + h;
             if (t < 0 || t >= GY || y0 + t >= a.R) continue;
-            g_dog_grad<P>(a, y0 + t, x0 + tx, prev + (PH + t) * P + PX + tx, h ? bot : top, dog, mag, ang);
+            g_dog_grad<P>(a, y0 + t, x0 + tx, prev + (PH + t) * P + PX + tx, h ? bot : top, dog, grad);
         }
     }
 };
@@ -1132,19 +1127,19 @@ __global__ void __launch_bounds__(GNT, 1) k_group(GroupArgs a) {
             g_vpass<1, LA>(b0, reinterpret_cast<float2*>(b1), vy + 2 * LA::HOUT, vx + 2 * LA::XOUT);  // L0 -> V1
             __syncthreads();
             g_hpass<1, LA>(reinterpret_cast<const float2*>(b1), b2,                               // V1 -> L1
-                           GEpi<LA::HIN, LA::XIN, LA::MIN>{a, y0, x0, b0, a.dog[0], nullptr, nullptr},
+                           GEpi<LA::HIN, LA::XIN, LA::MIN>{a, y0, x0, b0, a.dog[0], nullptr},
                            vy + 2 * LA::HOUT, vx + 2 * LA::XOUT);
             __syncthreads();
             g_vpass<2, LB>(b2, reinterpret_cast<float2*>(b0), vy + 2 * LB::HOUT, vx + 2 * LB::XOUT);  // L1 -> V2
             __syncthreads();
             g_hpass<2, LB>(reinterpret_cast<const float2*>(b0), b1,                               // V2 -> L2
-                           GEpi<LB::HIN, LB::XIN, LB::MIN>{a, y0, x0, b2, a.dog[1], a.mag[0], a.ang[0]},
+                           GEpi<LB::HIN, LB::XIN, LB::MIN>{a, y0, x0, b2, a.dog[1], a.grad[0]},
                            vy + 2 * LB::HOUT, vx + 2 * LB::XOUT);
             __syncthreads();
             g_vpass<3, LC>(b1, reinterpret_cast<float2*>(b0), vy + 2 * LC::HOUT, vx + 2 * LC::XOUT);  // L2 -> V3
             __syncthreads();
             g_hpass<3, LC>(reinterpret_cast<const float2*>(b0), b2,                               // V3 -> L3
-                           GEpi<LC::HIN, LC::XIN, LC::MIN>{a, y0, x0, b1, a.dog[2], a.mag[1], a.ang[1]},
+                           GEpi<LC::HIN, LC::XIN, LC::MIN>{a, y0, x0, b1, a.dog[2], a.grad[1]},
                            vy + 2 * LC::HOUT, vx + 2 * LC::XOUT);
             __syncthreads();
             // gradient of L3, L3 and L3[::2, ::2] on the tile
@@ -1158,8 +1153,7 @@ __global__ void __launch_bounds__(GNT, 1) k_group(GroupArgs a) {
                 grad4<LC::MOUT>(l3, yy, xx, a.R, a.C, mg, an);
                 const size_t at = (size_t)yy * a.C + xx;
                 const bool vec = (a.C & 3) == 0;
-                g_store4(a.mag[2] + at, make_float4(mg[0], mg[1], mg[2], mg[3]), vec, a.C - xx);
-                g_store4(a.ang[2] + at, make_float4(an[0], an[1], an[2], an[3]), vec, a.C - xx);
+                store_grad4(a.grad[2] + at, mg, an, vec, a.C - xx);
                 g_store4(a.dst + at, v, vec, a.C - xx);
                 if (a.down && !(yy & 1)) {
                     float* o2 = a.down + (size_t)(yy >> 1) * a.down_cols + (xx >> 1);
@@ -1172,13 +1166,13 @@ __global__ void __launch_bounds__(GNT, 1) k_group(GroupArgs a) {
             g_vpass<4, LA>(b0, reinterpret_cast<float2*>(b1), vy + 2 * LA::HOUT, vx + 2 * LA::XOUT);  // L3 -> V4
             __syncthreads();
             g_hpass<4, LA>(reinterpret_cast<const float2*>(b1), b2,                               // V4 -> L4
-                           GEpi<LA::HIN, LA::XIN, LA::MIN>{a, y0, x0, b0, a.dog[0], nullptr, nullptr},
+                           GEpi<LA::HIN, LA::XIN, LA::MIN>{a, y0, x0, b0, a.dog[0], nullptr},
                            vy + 2 * LA::HOUT, vx + 2 * LA::XOUT);
             __syncthreads();
             g_vpass<5, LB>(b2, reinterpret_cast<float2*>(b0), vy + 2 * LB::HOUT, vx + 2 * LB::XOUT);  // L4 -> V5
             __syncthreads();
             g_hpass<5, LB>(reinterpret_cast<const float2*>(b0), nullptr,                          // V5 -> L5
-                           GEpi<LB::HIN, LB::XIN, LB::MIN>{a, y0, x0, b2, a.dog[1], nullptr, nullptr},
+                           GEpi<LB::HIN, LB::XIN, LB::MIN>{a, y0, x0, b2, a.dog[1], nullptr},
                            vy + 2 * LB::HOUT, vx + 2 * LB::XOUT);
         }
     }
@@ -1255,8 +1249,7 @@ struct StripArgs {
     const float* L0;   // octave base, R x C, row pitch C
     int R, C, rows;    // rows: output rows per CTA
     float* dog[5];
-    float* mag[3];
-    float* ang[3];
+    float2* grad[3];
     float* down;       // L3[::2, ::2] (pitch down_cols) or null
     int down_cols;
     int* err;          // set to 1 when a TMA wait gives up
@@ -1383,8 +1376,7 @@ __device__ __forceinline__ void s_grad_item(const float* __restrict__ ring, cons
     float mg[4], an[4];
     fast_grad4(dxv, dyv, mg, an);
     const size_t at = (size_t)y * a.C + x;
-    s_store4(a.mag[I - 1] + at, make_float4(mg[0], mg[1], mg[2], mg[3]), k.vec, a.C - x);
-    s_store4(a.ang[I - 1] + at, make_float4(an[0], an[1], an[2], an[3]), k.vec, a.C - x);
+    store_grad4(a.grad[I - 1] + at, mg, an, k.vec, a.C - x);
     if (I == 3 && a.down && !(y & 1)) {
         float* o = a.down + (size_t)(y >> 1) * a.down_cols + (x >> 1);
         o[0] = c0.x;
@@ -1515,7 +1507,6 @@ __global__ void __launch_bounds__(TNT, 2) k_strip(const __grid_constant__ CUtens
     k.RB = V0 - 64;                // every row read is above RB
     k.vec = (a.C & 3) == 0;
     for (int i = 0; i < 5; ++i) k.vec = k.vec && al16(a.dog[i]);
-    for (int i = 0; i < 3; ++i) k.vec = k.vec && al16(a.mag[i]) && al16(a.ang[i]);
     const bool tma = use_tma != 0;
     const int T = (k.yz - k.ya + TE(0) + TLAG(5) - 3 + TSTEP - 1) / TSTEP;   // steps
     if (tma && threadIdx.x == 0) {
@@ -1564,9 +1555,9 @@ __global__ void __launch_bounds__(TNT, 2) k_strip(const __grid_constant__ CUtens
 }  // namespace
 
 // One float32 octave by the strip engine (one launch): from the base L0 (R x C, pitch C), the five
-// DoG planes at dog + k RC, gradients of L1..L3 at mag / ang + k RC, L3[::2, ::2] to down (pitch
+// DoG planes at dog + k RC, gradients of L1..L3 at grad + k RC, L3[::2, ::2] to down (pitch
 // down_cols; null for the last octave). err (device) is set when a TMA wait gives up.
-int32_t launch_octave_strip(const float* L0, int R, int C, float* dog, float* mag, float* ang, float* down,
+int32_t launch_octave_strip(const float* L0, int R, int C, float* dog, float2* grad, float* down,
                             int down_cols, int* err, cudaStream_t s) {
     static std::atomic<int> attr[64];
     FSB_TRY(smem_attr((const void*)k_strip, TSMEM, attr));
@@ -1576,10 +1567,7 @@ int32_t launch_octave_strip(const float* L0, int R, int C, float* dog, float* ma
     a.C = C;
     const long long RC = (long long)R * C;
     for (int i = 0; i < 5; ++i) a.dog[i] = dog + i * RC;
-    for (int i = 0; i < 3; ++i) {
-        a.mag[i] = mag + i * RC;
-        a.ang[i] = ang + i * RC;
-    }
+    for (int i = 0; i < 3; ++i) a.grad[i] = grad + i * RC;
     a.down = down;
     a.down_cols = down_cols;
     a.err = err;
@@ -1611,7 +1599,7 @@ int32_t launch_octave_strip(const float* L0, int R, int C, float* dog, float* ma
     return FSB_OK;
 }
 
-int32_t launch_octave_fused(const float* L0, int R, int C, float* dog, float* mag, float* ang, float* down,
+int32_t launch_octave_fused(const float* L0, int R, int C, float* dog, float2* grad, float* down,
                             int down_cols, cudaStream_t s) {
     static std::atomic<int> attr[64];
     FSB_TRY(smem_attr((const void*)k_octave, SMEM_BYTES, attr, 100));
@@ -1621,10 +1609,7 @@ int32_t launch_octave_fused(const float* L0, int R, int C, float* dog, float* ma
     a.C = C;
     const long long RC = (long long)R * C;
     for (int i = 0; i < 5; ++i) a.dog[i] = dog + i * RC;
-    for (int i = 0; i < 3; ++i) {
-        a.mag[i] = mag + i * RC;
-        a.ang[i] = ang + i * RC;
-    }
+    for (int i = 0; i < 3; ++i) a.grad[i] = grad + i * RC;
     a.down = down;
     a.down_cols = down_cols;
     // about two CTAs per SM over the whole octave
@@ -1650,7 +1635,7 @@ int layer_tile_height(int variant) { return kTileHeights[variant < 0 || variant 
 
 // One layer of the float32 pyramid by the tiled per-layer kernel: L_layer from src (R x C), tile
 // height layer_tile_height(variant).
-int32_t launch_layer_fast(int layer, const float* src, int R, int C, float* dst, float* dog, float* mag, float* ang,
+int32_t launch_layer_fast(int layer, const float* src, int R, int C, float* dst, float* dog, float2* grad,
                           float* down, int down_cols, int variant, int* err, cudaStream_t s) {
     LayerArgs a{};
     a.err = err;
@@ -1659,8 +1644,7 @@ int32_t launch_layer_fast(int layer, const float* src, int R, int C, float* dst,
     a.C = C;
     a.dst = dst;
     a.dog = dog;
-    a.mag = mag;
-    a.ang = ang;
+    a.grad = grad;
     a.down = down;
     a.down_cols = down_cols;
     switch (layer) {
@@ -1675,9 +1659,9 @@ int32_t launch_layer_fast(int layer, const float* src, int R, int C, float* dst,
 
 
 // Layers 1..3 of a float32 octave by the fused group kernel: from L0 (src, R x C), DoG planes
-// 0..2 at dog, dog + RC, dog + 2RC, gradients of L1..L3 at mag / ang (+ RC, + 2RC), L3 to l3 and
+// 0..2 at dog, dog + RC, dog + 2RC, gradients of L1..L3 at grad (+ RC, + 2RC), L3 to l3 and
 // L3[::2, ::2] to down (null: last octave). down must not alias src (other tiles still read it).
-int32_t launch_group_lower(const float* src, int R, int C, float* dog, float* mag, float* ang, float* l3, float* down,
+int32_t launch_group_lower(const float* src, int R, int C, float* dog, float2* grad, float* l3, float* down,
                            int down_cols, cudaStream_t s) {
     const long long RC = (long long)R * C;
     GroupArgs a{};
@@ -1686,8 +1670,7 @@ int32_t launch_group_lower(const float* src, int R, int C, float* dog, float* ma
     a.C = C;
     for (int k = 0; k < 3; ++k) {
         a.dog[k] = dog + k * RC;
-        a.mag[k] = mag + k * RC;
-        a.ang[k] = ang + k * RC;
+        a.grad[k] = grad + k * RC;
     }
     a.dst = l3;
     a.down = down;

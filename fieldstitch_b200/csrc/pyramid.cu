@@ -5,7 +5,8 @@
 //
 // Layout in HBM (per image):
 //   DoG atlas   float32 [octave][layer 0..4][R][C], octave o at Geometry::dog_off[o]
-//   MAG / ANG   float32 [octave][layer 1..3][R][C], octave o at Geometry::grad_off[o]
+//   GRAD        float2 (magnitude, angle) [octave][layer 1..3][R][C], octave o at Geometry::grad_off[o];
+//               one 8-byte load gives a sample of the orientation and descriptor windows
 //   planes      three octave-0-sized float32 scratch planes for gauss layers in flight
 //
 // One launch per (octave, layer): a 64x32 output tile is staged through shared memory with its
@@ -111,8 +112,7 @@ struct BlurArgs {
     int rows, cols;
     float* dst;                // this layer, or null
     float* dog;                // DoG plane (this - previous), or null
-    float* mag;                // gradient magnitude of the previous layer, or null
-    float* ang;                // gradient angle of the previous layer (degrees), or null
+    float2* grad;              // gradient (magnitude, angle in degrees) of the previous layer, or null
     float* down;               // previous layer [::2, ::2], or null
     int down_cols;
 };
@@ -180,15 +180,15 @@ __global__ void __launch_bounds__(NT) k_blur(BlurArgs a) {
         if (a.dst) a.dst[at] = v;
         const float* c = &s_in[(yy + RAD) * SW + xx + RAD];   // previous layer at (gy, gx)
         if (a.dog) a.dog[at] = __fsub_rn(v, c[0]);
-        if (a.mag) {
+        if (a.grad) {
             float dx = 0.f, dy = 0.f;
             if (gy > 0 && gy < a.rows - 1 && gx > 0 && gx < a.cols - 1) {
                 dx = __fsub_rn(c[1], c[-1]);
                 dy = __fsub_rn(c[-SW], c[SW]);
             }
-            a.mag[at] = __fsqrt_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)));
-            float an = __fmul_rn(atan2f(dy, dx), kRad2Deg);
-            a.ang[at] = an < 0.f ? __fadd_rn(an, 360.f) : an;
+            const float mg = __fsqrt_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)));
+            const float an = __fmul_rn(atan2f(dy, dx), kRad2Deg);
+            a.grad[at] = make_float2(mg, an < 0.f ? __fadd_rn(an, 360.f) : an);
         }
         if (a.down && !(gy & 1) && !(gx & 1)) a.down[(size_t)(gy >> 1) * a.down_cols + (gx >> 1)] = c[0];
     }
@@ -216,15 +216,16 @@ struct LayerCall {
     int layer;
     const float* src;
     int R, C;
-    float *dst, *dog, *mag, *ang, *down;
+    float *dst, *dog;
+    float2* grad;
+    float* down;
     int dc;
     int* err;   // error word of the tile copies' bounded waits
     cudaStream_t s;
 };
 int32_t run_layer_call(void* p, int v) {
     const LayerCall* c = static_cast<const LayerCall*>(p);
-    return launch_layer_fast(c->layer, c->src, c->R, c->C, c->dst, c->dog, c->mag, c->ang, c->down, c->dc, v, c->err,
-                             c->s);
+    return launch_layer_fast(c->layer, c->src, c->R, c->C, c->dst, c->dog, c->grad, c->down, c->dc, v, c->err, c->s);
 }
 struct BaseCall {
     const uint8_t* img;
@@ -239,9 +240,9 @@ int32_t run_base_call(void* p, int v) {
 // one tuned per-layer launch: the tile height is chosen per (layer, octave size);
 // FSB_LAYER_VARIANT=k (read on every call) runs variant k everywhere instead, so each variant can
 // be checked against the others
-int32_t tuned_layer(int layer, const float* src, int R, int C, float* dst, float* dog, float* mag, float* ang,
+int32_t tuned_layer(int layer, const float* src, int R, int C, float* dst, float* dog, float2* grad,
                     float* down, int dc, int* err, cudaStream_t s) {
-    LayerCall c{layer, src, R, C, dst, dog, mag, ang, down, dc, err, s};
+    LayerCall c{layer, src, R, C, dst, dog, grad, down, dc, err, s};
     if (const char* fv = std::getenv("FSB_LAYER_VARIANT")) {
         const int v = std::atoi(fv);
         if (v >= 0 && v < layer_tile_variants()) return run_layer_call(&c, v);
@@ -274,7 +275,9 @@ namespace {
 struct OctaveCall {
     const float* src;
     int R, C;
-    float *x, *y, *dog, *mag, *ang, *down;
+    float *x, *y, *dog;
+    float2* grad;
+    float* down;
     int dc;
     cudaStream_t s;
     // with a side stream, the octave's tail (layer 5, or the L4-L5 group) runs there after `fork`,
@@ -296,23 +299,23 @@ int32_t run_octave_call(void* p, int v) {
     };
     if (v == 2) {
         // the whole octave in one launch: no tail to move to the side stream
-        FSB_TRY(launch_octave_strip(c->src, c->R, c->C, c->dog, c->mag, c->ang, c->down, c->dc, c->err, c->s));
+        FSB_TRY(launch_octave_strip(c->src, c->R, c->C, c->dog, c->grad, c->down, c->dc, c->err, c->s));
         if (c->side) FSB_CUDA(cudaEventRecord(c->join, c->s));
         return FSB_OK;
     }
     if (v == 1) {
-        FSB_TRY(launch_group_lower(c->src, c->R, c->C, c->dog, c->mag, c->ang, c->x, c->down, c->dc, c->s));
+        FSB_TRY(launch_group_lower(c->src, c->R, c->C, c->dog, c->grad, c->x, c->down, c->dc, c->s));
         FSB_TRY(fork());
         FSB_TRY(launch_group_upper(c->x, c->R, c->C, c->dog + 3 * RC, ts));
     } else {
-        FSB_TRY(tuned_layer(1, c->src, c->R, c->C, c->x, c->dog, nullptr, nullptr, nullptr, 0, c->err, c->s));
-        FSB_TRY(tuned_layer(2, c->x, c->R, c->C, c->y, c->dog + RC, c->mag, c->ang, nullptr, 0, c->err, c->s));
-        FSB_TRY(tuned_layer(3, c->y, c->R, c->C, c->x, c->dog + 2 * RC, c->mag + RC, c->ang + RC, nullptr, 0, c->err,
+        FSB_TRY(tuned_layer(1, c->src, c->R, c->C, c->x, c->dog, nullptr, nullptr, 0, c->err, c->s));
+        FSB_TRY(tuned_layer(2, c->x, c->R, c->C, c->y, c->dog + RC, c->grad, nullptr, 0, c->err, c->s));
+        FSB_TRY(tuned_layer(3, c->y, c->R, c->C, c->x, c->dog + 2 * RC, c->grad + RC, nullptr, 0, c->err,
                             c->s));
-        FSB_TRY(tuned_layer(4, c->x, c->R, c->C, c->y, c->dog + 3 * RC, c->mag + 2 * RC, c->ang + 2 * RC, c->down,
+        FSB_TRY(tuned_layer(4, c->x, c->R, c->C, c->y, c->dog + 3 * RC, c->grad + 2 * RC, c->down,
                             c->dc, c->err, c->s));
         FSB_TRY(fork());
-        FSB_TRY(tuned_layer(5, c->y, c->R, c->C, nullptr, c->dog + 4 * RC, nullptr, nullptr, nullptr, 0, c->err, ts));
+        FSB_TRY(tuned_layer(5, c->y, c->R, c->C, nullptr, c->dog + 4 * RC, nullptr, nullptr, 0, c->err, ts));
     }
     if (c->side) FSB_CUDA(cudaEventRecord(c->join, c->side));
     return FSB_OK;
@@ -326,8 +329,7 @@ int32_t run_pyramid(Workspace& ws, const uint8_t* d_img, int img_stride, bool ex
     int* err = ws.counters.as<int>() + PYR_ERR_WORD;
     FSB_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
     float* DF = ws.dog.as<float>();
-    float* MAG = ws.mag.as<float>();
-    float* ANG = ws.ang.as<float>();
+    float2* GRAD = ws.grad.as<float2>();
     BlurArgs a{};
     a.img = d_img;
     a.img_stride = img_stride;
@@ -372,8 +374,8 @@ int32_t run_pyramid(Workspace& ws, const uint8_t* d_img, int img_stride, bool ex
             float* pl[2];
             for (int k = 0, n = 0; k < 3 && n < 2; ++k)
                 if (P[k] != cur && P[k] != busy) pl[n++] = P[k];
-            OctaveCall c{cur, g.R[o], g.C[o], pl[0], pl[1], DF + g.dog_off[o], MAG + g.grad_off[o],
-                         ANG + g.grad_off[o], last ? nullptr : NB + (o & 1) * half, last ? 0 : g.C[o + 1], s,
+            OctaveCall c{cur, g.R[o], g.C[o], pl[0], pl[1], DF + g.dog_off[o], GRAD + g.grad_off[o],
+                         last ? nullptr : NB + (o & 1) * half, last ? 0 : g.C[o + 1], s,
                          nullptr, side ? ev[2 * o] : nullptr, side ? ev[2 * o + 1] : nullptr, err};
             int v = eng == Engine::Group ? 1 : eng == Engine::Strip ? 2 : 0;
             char key[64];
@@ -400,15 +402,14 @@ int32_t run_pyramid(Workspace& ws, const uint8_t* d_img, int img_stride, bool ex
     for (int o = 0; o < g.n_oct; ++o) {
         const long long RC = (long long)g.R[o] * g.C[o];
         float* dog = DF + g.dog_off[o];
-        float* mag = MAG + g.grad_off[o];
-        float* ang = ANG + g.grad_off[o];
+        float2* grad = GRAD + g.grad_off[o];
         float* other[2];
         for (int k = 0, n = 0; k < 3; ++k)
             if (P[k] != cur) other[n++] = P[k];
         if (!exact && g.C[o] >= kFusedMinCols) {
             // fused octave: reads cur, writes the next base into another plane
             float* down = o + 1 < g.n_oct ? other[0] : nullptr;
-            FSB_TRY(launch_octave_fused(cur, g.R[o], g.C[o], dog, mag, ang, down, o + 1 < g.n_oct ? g.C[o + 1] : 0, s));
+            FSB_TRY(launch_octave_fused(cur, g.R[o], g.C[o], dog, grad, down, o + 1 < g.n_oct ? g.C[o + 1] : 0, s));
             cur = other[0];
             continue;
         }
@@ -416,12 +417,12 @@ int32_t run_pyramid(Workspace& ws, const uint8_t* d_img, int img_stride, bool ex
             const int R = g.R[o], C = g.C[o];
             float* down = o + 1 < g.n_oct ? cur : nullptr;
             const int dc = o + 1 < g.n_oct ? g.C[o + 1] : 0;
-            FSB_TRY(tuned_layer(1, cur, R, C, other[0], dog, nullptr, nullptr, nullptr, 0, err, s));
-            FSB_TRY(tuned_layer(2, other[0], R, C, other[1], dog + RC, mag, ang, nullptr, 0, err, s));
-            FSB_TRY(tuned_layer(3, other[1], R, C, other[0], dog + 2 * RC, mag + RC, ang + RC, nullptr, 0, err, s));
-            FSB_TRY(tuned_layer(4, other[0], R, C, other[1], dog + 3 * RC, mag + 2 * RC, ang + 2 * RC, down, dc,
+            FSB_TRY(tuned_layer(1, cur, R, C, other[0], dog, nullptr, nullptr, 0, err, s));
+            FSB_TRY(tuned_layer(2, other[0], R, C, other[1], dog + RC, grad, nullptr, 0, err, s));
+            FSB_TRY(tuned_layer(3, other[1], R, C, other[0], dog + 2 * RC, grad + RC, nullptr, 0, err, s));
+            FSB_TRY(tuned_layer(4, other[0], R, C, other[1], dog + 3 * RC, grad + 2 * RC, down, dc,
                                 err, s));
-            FSB_TRY(tuned_layer(5, other[1], R, C, nullptr, dog + 4 * RC, nullptr, nullptr, nullptr, 0, err, s));
+            FSB_TRY(tuned_layer(5, other[1], R, C, nullptr, dog + 4 * RC, nullptr, nullptr, 0, err, s));
             continue;   // the next base is in `cur` (the dead L0 plane)
         }
         BlurArgs b{};
@@ -431,17 +432,17 @@ int32_t run_pyramid(Workspace& ws, const uint8_t* d_img, int img_stride, bool ex
         b.src = cur; b.dst = other[0]; b.dog = dog;
         launch<1, 5, false>(exact, b, s);
         // layer 2: L1 (X) -> Y, DoG 1, gradient of L1
-        b.src = other[0]; b.dst = other[1]; b.dog = dog + RC; b.mag = mag; b.ang = ang;
+        b.src = other[0]; b.dst = other[1]; b.dog = dog + RC; b.grad = grad;
         launch<2, 6, false>(exact, b, s);
         // layer 3: L2 (Y) -> X, DoG 2, gradient of L2
-        b.src = other[1]; b.dst = other[0]; b.dog = dog + 2 * RC; b.mag = mag + RC; b.ang = ang + RC;
+        b.src = other[1]; b.dst = other[0]; b.dog = dog + 2 * RC; b.grad = grad + RC;
         launch<3, 8, false>(exact, b, s);
         // layer 4: L3 (X) -> Y, DoG 3, gradient of L3, L3[::2, ::2] -> the (dead) base plane
-        b.src = other[0]; b.dst = other[1]; b.dog = dog + 3 * RC; b.mag = mag + 2 * RC; b.ang = ang + 2 * RC;
+        b.src = other[0]; b.dst = other[1]; b.dog = dog + 3 * RC; b.grad = grad + 2 * RC;
         if (o + 1 < g.n_oct) { b.down = cur; b.down_cols = g.C[o + 1]; }
         launch<4, 10, false>(exact, b, s);
         // layer 5: L4 (Y) -> DoG 4 only
-        b.src = other[1]; b.dst = nullptr; b.dog = dog + 4 * RC; b.mag = nullptr; b.ang = nullptr; b.down = nullptr;
+        b.src = other[1]; b.dst = nullptr; b.dog = dog + 4 * RC; b.grad = nullptr; b.down = nullptr;
         launch<5, 13, false>(exact, b, s);
     }
     FSB_CUDA(cudaGetLastError());
