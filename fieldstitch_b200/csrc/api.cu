@@ -68,12 +68,12 @@ void Workspace::release() {
 static int32_t prepare_workspace(Workspace& ws, int h, int w) {
     ws.g = make_geometry(h, w);
     const Geometry& g = ws.g;
-    const size_t sum = (size_t)g.grad_off[g.n_oct] / 3;   // sum of octave pixels
-    const size_t p0 = (size_t)g.R[0] * g.C[0];
+    const size_t sum = (size_t)g.grad_off[g.n_oct] / 3;   // sum of the octaves' pitched pixels
+    const size_t p0 = (size_t)g.R[0] * g.P[0];
     FSB_TRY(ws.dog.ensure(5 * sum * 4));
     FSB_TRY(ws.grad.ensure(3 * sum * 8));
     for (auto& b : ws.plane) FSB_TRY(b.ensure(p0 * 4));
-    if (g.n_oct > 1) FSB_TRY(ws.next_base.ensure(2 * (((size_t)g.R[1] * g.C[1] + 63) / 64 * 64) * 4));
+    if (g.n_oct > 1) FSB_TRY(ws.next_base.ensure(2 * (((size_t)g.R[1] * g.P[1] + 63) / 64 * 64) * 4));
     FSB_TRY(ws.img.ensure((size_t)h * w));
     if (ws.cap_cand < 65536) ws.cap_cand = 65536;
     if (ws.cap_cand < sum / 64) ws.cap_cand = sum / 64;
@@ -229,11 +229,15 @@ static int32_t detect_into(fsb_ctx* ctx, Workspace& ws, const uint8_t* img, int 
     return detect_dev(ctx, ws, ws.img.as<uint8_t>(), w, p, max_kp);
 }
 
-// one component of the gradient atlas: part 0 the magnitudes, 1 the angles
-__global__ void k_grad_part(const float2* __restrict__ g, long long n, int part, float* __restrict__ out) {
+// n rows of C values out of an atlas of row pitch P, packed: what 0 the DoG values, 1 the magnitudes,
+// 2 the angles of the gradient pairs
+__global__ void k_atlas_part(const float* __restrict__ src, long long n, int C, int P, int what,
+                             float* __restrict__ out) {
     const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-        out[i] = part ? g[i].y : g[i].x;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n * C; i += stride) {
+        const long long at = i / C * P + i % C;
+        out[i] = what ? src[2 * at + (what - 1)] : src[at];
+    }
 }
 
 // selected keypoints -> describe inputs (tx..tly) and optional interleaved xy / response outputs
@@ -699,7 +703,9 @@ int32_t fsb_state_atlas(fsb_state* st, int32_t which, float* out, int64_t n_floa
     FSB_ARG(st && st->magic == STATE_MAGIC, "invalid state");
     FSB_ARG(out && which >= 0 && which <= 2, "bad atlas request");
     const Geometry& g = st->ws->g;
-    const int64_t want = which == 0 ? g.dog_off[g.n_oct] : g.grad_off[g.n_oct];
+    const int layers = which == 0 ? 5 : 3;
+    int64_t want = 0;
+    for (int o = 0; o < g.n_oct; ++o) want += (int64_t)layers * g.R[o] * g.C[o];
     if (n_floats != want) {
         set_error("invalid argument: atlas %d holds %lld floats, %lld requested", which, (long long)want,
                   (long long)n_floats);
@@ -708,15 +714,18 @@ int32_t fsb_state_atlas(fsb_state* st, int32_t which, float* out, int64_t n_floa
     FSB_TRY(use_device(st->ctx));
     fsb_ctx* ctx = st->ctx;
     if (!want) return FSB_OK;
-    const float* src = st->ws->dog.as<float>();
-    if (which != 0) {   // the magnitudes or the angles of the (magnitude, angle) atlas
-        FSB_TRY(ctx->s_misc.ensure((size_t)want * 4));
-        const long long nb = (want + 255) / 256;
-        k_grad_part<<<(unsigned)std::min<long long>(nb, 148 * 64), 256, 0, ctx->stream>>>(
-            st->ws->grad.as<float2>(), want, which - 1, ctx->s_misc.as<float>());
+    FSB_TRY(ctx->s_misc.ensure((size_t)want * 4));
+    float* src = ctx->s_misc.as<float>();
+    int64_t at = 0;
+    for (int o = 0; o < g.n_oct; ++o) {
+        const long long rows = (long long)layers * g.R[o], n = rows * g.C[o];
+        const float* plane = which == 0 ? st->ws->dog.as<float>() + g.dog_off[o]
+                                        : st->ws->grad.as<float>() + 2 * g.grad_off[o];
+        k_atlas_part<<<(unsigned)std::min<long long>((n + 255) / 256, 148 * 64), 256, 0, ctx->stream>>>(
+            plane, rows, g.C[o], g.P[o], which, src + at);
         note_launch();
         FSB_CUDA(cudaGetLastError());
-        src = ctx->s_misc.as<float>();
+        at += n;
     }
     FSB_CUDA(cudaMemcpyAsync(out, src, (size_t)want * 4, cudaMemcpyDeviceToHost, ctx->stream));
     FSB_CUDA(cudaStreamSynchronize(ctx->stream));

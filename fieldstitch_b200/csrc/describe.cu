@@ -57,13 +57,13 @@ __global__ void __launch_bounds__(OW * 32) k_orient(const float2* __restrict__ G
     for (uint32_t t = k0 + blockIdx.x * OW + wid; t < k1; t += nw) {
         const uint32_t i = order[t];
         const Refined e = ref[i];
-        const int o = e.o, R = g.R[o], C = g.C[o];
+        const int o = e.o, R = g.R[o], C = g.C[o], P = g.P[o];
         const float scl = kp_scale(e.l, e.x2);
         const int rad = min((int)rintf(4.5f * scl), ORI_R_MAX);
         const float sw = 1.5f * scl;
         const float den = 2.f * (sw * sw);
         const int W = 2 * rad + 1;
-        const long long gb = g.grad_off[o] + (long long)(e.l - 1) * R * C;
+        const long long gb = g.grad_off[o] + (long long)(e.l - 1) * R * P;
         for (int b = 0; b < ORI_BINS; ++b) acc[b][lane] = (Acc)0;
         // lane takes samples s = lane, lane + 32, ... of the W x W window (row-major); the window
         // position advances by (32 / W, 32 % W) per step, one division per keypoint
@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(OW * 32) k_orient(const float2* __restrict__ G
             const int y1 = e.r + ii, x1 = e.c + jj, y2 = e.r + ii2, x2 = e.c + jj2;
             const bool in1 = y1 > 0 && y1 < R - 1 && x1 > 0 && x1 < C - 1;
             const bool in2 = s + 32 < W * W && y2 > 0 && y2 < R - 1 && x2 > 0 && x2 < C - 1;
-            const long long g1 = gb + (long long)y1 * C + x1, g2 = gb + (long long)y2 * C + x2;
+            const long long g1 = gb + (long long)y1 * P + x1, g2 = gb + (long long)y2 * P + x2;
             const float2 s1 = in1 ? __ldg(GRAD + g1) : make_float2(0.f, 0.f);
             const float2 s2 = in2 ? __ldg(GRAD + g2) : make_float2(0.f, 0.f);
             const float m1 = s1.x, a1 = s1.y, m2 = s2.x, a2 = s2.y;
@@ -193,7 +193,7 @@ struct SquareWalk {
     uint64_t row;                         // address of pixel (i, 0) less 8 times the bits of SQ_M
 
     __device__ __forceinline__ void init(float sn, float cs, float Rf, float Cf, float hw, int ilo, int ihi, int jlo,
-                                         int jhi, const float2* ctr, int cols, bool on) {
+                                         int jhi, const float2* ctr, int pitch, bool on) {
         // a slope below SQ_AMIN is a row condition: its interval is everything or empty either way
         const float a = copysignf(fmaxf(fabsf(sn), SQ_AMIN), sn), b = copysignf(fmaxf(fabsf(cs), SQ_AMIN), cs);
         const float ia = 1.f / a, ib = 1.f / b;
@@ -219,19 +219,19 @@ struct SquareWalk {
         const int is = max(ilo, (int)ceilf(imin - sl)) - 1;
         i = (float)is;
         i1 = on ? fminf((float)ihi, floorf(imax + sl)) : -1e30f;
-        row = reinterpret_cast<uint64_t>(ctr) + 8ll * ((long long)is * cols) - 8ull * __float_as_uint(SQ_M);
+        row = reinterpret_cast<uint64_t>(ctr) + 8ll * ((long long)is * pitch) - 8ull * __float_as_uint(SQ_M);
         jmin = (float)jlo;
         jmax = (float)jhi;
         j = SQ_M + 1.f;
         j1 = SQ_M;
     }
     // returns whether the walk stayed in its row
-    __device__ __forceinline__ bool step(int cols) {
+    __device__ __forceinline__ bool step(int pitch) {
         j += 1.f;
         const bool stay = j <= j1;
         if (!stay) {
             i += 1.f;
-            row += 8ll * cols;
+            row += 8ll * pitch;
             j = fmaxf(fmaxf(fmaf(i, kl1, kl0), fmaf(i, ml1, ml0)), jmin) + SQ_M;
             j1 = fminf(fminf(fmaf(i, kl1, kh0), fmaf(i, ml1, mh0)), jmax) + SQ_M;
         }
@@ -279,12 +279,12 @@ __global__ void __launch_bounds__(DW * 32) k_describe(const float2* __restrict__
         const double scl = (double)ks[k] * f * 0.5;
         double ori = 360.0 - (double)ka[k];
         if (fabs(ori - 360.0) < 1e-4) ori = 0.0;
-        const int rows = g.R[o], cols = g.C[o];
+        const int rows = g.R[o], cols = g.C[o], pitch = g.P[o];
         long long radl = llrint(3.0 * scl * 1.4142135623730951 * 5.0 * 0.5);
         const long long rmax = (long long)sqrt((double)rows * rows + (double)cols * cols);
         if (radl > rmax) radl = rmax;
         const int rad = (int)radl;
-        const long long gb = g.grad_off[o] + (long long)(li - 1) * rows * cols;
+        const long long gb = g.grad_off[o] + (long long)(li - 1) * rows * pitch;
         const int pr = (int)rint(py), pc = (int)rint(px);
         const double hw = 3.0 * scl;
         const double t = ori * 0.017453292519943295;
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(DW * 32) k_describe(const float2* __restrict__
         const float cos_f = (float)cos_d, sin_f = (float)sin_d, ori_f = (float)ori;
         SquareWalk wk;
         wk.init(sin_f, cos_f, (float)Rq, (float)Cq, (float)hw, max(-rad, 1 - pr), min(rad, rows - 2 - pr),
-                max(-rad, 1 - pc), min(rad, cols - 2 - pc), GRAD + gb + (long long)pr * cols + pc, cols, lane < NSQ);
+                max(-rad, 1 - pc), min(rad, cols - 2 - pc), GRAD + gb + (long long)pr * pitch + pc, pitch, lane < NSQ);
         // floor(rbin) = R' and rbin > -1: rbin in [rlo, R' + 1); the same for columns
         const float rlo = Rq < 0 ? -0x1.fffffep-1f : (float)Rq, clo = Cq < 0 ? -0x1.fffffep-1f : (float)Cq;
         const double rlo_d = Rq < 0 ? -0x1.fffffffffffffp-1 : (double)Rq;
@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(DW * 32) k_describe(const float2* __restrict__
         bool qv[DESC_AHEAD], qs[DESC_AHEAD], qo[DESC_AHEAD];   // valid; pair shared with the sample before; odd pixel
         bool pair_first = false;   // the walk's latest sample was the even pixel of a loaded pair
         auto fetch = [&](int u) {
-            const bool same_row = wk.step(cols);
+            const bool same_row = wk.step(pitch);
             const uint64_t px = wk.pixel();
             qv[u] = wk.valid();
             qi[u] = wk.i;

@@ -94,18 +94,18 @@ __global__ void __launch_bounds__(EX_T, 4) k_extrema(const float* __restrict__ D
     while (o + 1 < tl.n_oct && (int)blockIdx.x >= tl.first[o + 1]) ++o;
     const int b = blockIdx.x - tl.first[o];
     const int ry = b / tl.col_tiles[o], cx = b - ry * tl.col_tiles[o];
-    const int R = k.g.R[o], C = k.g.C[o];
-    const long long RC = (long long)R * C;
+    const int R = k.g.R[o], C = k.g.C[o], P = k.g.P[o];
+    const long long RC = (long long)R * P;
     const float* base = DF + k.g.dog_off[o];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int c = BORDER + (cx * (EX_T / 32) + wid) * EX_COLS + lane - 1;   // this lane's column
     const int cc = min(max(c, 0), C - 1);                                    // clamped for loading
     const bool col_ok = lane >= 1 && lane <= EX_COLS && c >= BORDER && c < C - BORDER;
     const int y0 = BORDER + ry * EX_ROWS, y1 = min(y0 + EX_ROWS, R - BORDER);   // output rows [y0, y1)
-    // one row of the 3-row window: horizontal max / min of the 5 layers and the centre values of
-    // layers 1..3
+    // one row of the 3-row window: for layers 1..3, the maximum / minimum over the three layers
+    // around and the three columns around, and the centre value
     struct Row {
-        float hx[5], hn[5], c[3];
+        float hx[N_LAYERS], hn[N_LAYERS], c[N_LAYERS];
     };
     // Row r's five layer values at this lane's column arrive by 4-byte cp.async into the lane's own
     // ring slot ((r - (y0 - 1)) % EX_DEPTH), EX_DEPTH rows ahead of the row being finished; only the
@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(EX_T, 4) k_extrema(const float* __restrict__ D
     int next_row = y0 - 1, next_slot = 0, take_slot = 0;
     auto issue_next = [&]() {
         if (next_row <= last_row) {
-            const float* src = colp + (long long)next_row * C;
+            const float* src = colp + (long long)next_row * P;
 #pragma unroll
             for (int l = 0; l < 5; ++l) ex_cp_async4(ring + (next_slot * 5 + l) * EX_T, src + l * RC);
         }
@@ -136,12 +136,11 @@ __global__ void __launch_bounds__(EX_T, 4) k_extrema(const float* __restrict__ D
     };
     auto finish_row = [&](Row& w, const float (&raw)[5]) {
 #pragma unroll
-        for (int l = 0; l < 5; ++l) {
-            const float v = raw[l];
-            const float vl = __shfl_up_sync(0xffffffffu, v, 1), vr = __shfl_down_sync(0xffffffffu, v, 1);
-            w.hx[l] = max3f(vl, v, vr);
-            w.hn[l] = min3f(vl, v, vr);
-            if (l >= 1 && l <= N_LAYERS) w.c[l - 1] = v;
+        for (int l = 0; l < N_LAYERS; ++l) {
+            const float mx = max3f(raw[l], raw[l + 1], raw[l + 2]), mn = min3f(raw[l], raw[l + 1], raw[l + 2]);
+            w.hx[l] = max3f(__shfl_up_sync(0xffffffffu, mx, 1), mx, __shfl_down_sync(0xffffffffu, mx, 1));
+            w.hn[l] = min3f(__shfl_up_sync(0xffffffffu, mn, 1), mn, __shfl_down_sync(0xffffffffu, mn, 1));
+            w.c[l] = raw[l + 1];
         }
     };
     auto load_row = [&](Row& w) {
@@ -149,25 +148,21 @@ __global__ void __launch_bounds__(EX_T, 4) k_extrema(const float* __restrict__ D
         take_row(raw);
         finish_row(w, raw);
     };
+    const float tmax = nextafterf(k.pthr, INFINITY), tmin = nextafterf(-k.pthr, -INFINITY);
     // test row y from the window (up, mid, dn), append its extrema, then finish row y + 2 into `up`
     // (no longer needed): the three windows rotate by name, not by register moves
     auto step = [&](Row& up, const Row& mid, const Row& dn, int y) {
-        float vmx[5], vmn[5];
-#pragma unroll
-        for (int l = 0; l < 5; ++l) {
-            vmx[l] = max3f(up.hx[l], mid.hx[l], dn.hx[l]);
-            vmn[l] = min3f(up.hn[l], mid.hn[l], dn.hn[l]);
-        }
         unsigned mask = 0;
-        if (col_ok) {
 #pragma unroll
-            for (int l = 1; l <= N_LAYERS; ++l) {
-                const float v = mid.c[l - 1];
-                const float mx = max3f(vmx[l - 1], vmx[l], vmx[l + 1]);
-                const float mn = min3f(vmn[l - 1], vmn[l], vmn[l + 1]);
-                if ((v >= mx && v > k.pthr) || (v <= mn && v < -k.pthr)) mask |= 1u << (l - 1);
-            }
+        for (int l = 0; l < N_LAYERS; ++l) {
+            // v is one of the 27 values, so v >= their maximum and v > pthr is v >= the larger of the
+            // maximum and the float after pthr; the same for the minimum
+            const float v = mid.c[l];
+            const float mx = fmaxf(max3f(up.hx[l], mid.hx[l], dn.hx[l]), tmax);
+            const float mn = fminf(min3f(up.hn[l], mid.hn[l], dn.hn[l]), tmin);
+            if (v >= mx || v <= mn) mask |= 1u << l;
         }
+        if (!col_ok) mask = 0;
         const unsigned any = __ballot_sync(0xffffffffu, mask != 0);
         if (any) {
             const int cntv = __popc(mask);
@@ -185,7 +180,7 @@ __global__ void __launch_bounds__(EX_T, 4) k_extrema(const float* __restrict__ D
             while (mask) {
                 const int bit = __ffs(mask) - 1;
                 mask &= mask - 1;
-                if (pos < cap) cand[pos] = (uint32_t)(k.g.dog_off[o] + (bit + 1) * RC + (long long)y * C + c);
+                if (pos < cap) cand[pos] = (uint32_t)(k.g.dog_off[o] + (bit + 1) * RC + (long long)y * P + c);
                 ++pos;
             }
         }
@@ -270,17 +265,17 @@ __global__ void __launch_bounds__(128) k_refine(const float* __restrict__ DF, De
         if (i < n) {
             const uint32_t f = cand[i];
             const int o = find_octave(k.g, f);
-            const int R = k.g.R[o], C = k.g.C[o];
-            const long long RC = (long long)R * C, ob = k.g.dog_off[o];
+            const int R = k.g.R[o], C = k.g.C[o], P = k.g.P[o];
+            const long long RC = (long long)R * P, ob = k.g.dog_off[o];
             const long long loc = (long long)f - ob;
             int l = (int)(loc / RC);
             const long long rem = loc - (long long)l * RC;
-            int r = (int)(rem / C);
-            int c = (int)(rem - (long long)r * C);
+            int r = (int)(rem / P);
+            int c = (int)(rem - (long long)r * P);
             float X0 = 0.f, X1 = 0.f, X2 = 0.f;
             bool done = false;
             for (int it = 0; it < MAX_INTERP; ++it) {
-                const Fit F = local_fit(DF, ob + l * RC + (long long)r * C + c, C, RC);
+                const Fit F = local_fit(DF, ob + l * RC + (long long)r * P + c, P, RC);
                 // adjugate solve of H x = g (gsift.py:182-198); x = -H^-1 g
                 const float a = F.dxx, b = F.dxy, cc = F.dxs, d = F.dxy, ee = F.dyy, ff = F.dys;
                 const float gg = F.dxs, hh = F.dys, ii = F.dss;
@@ -305,7 +300,7 @@ __global__ void __launch_bounds__(128) k_refine(const float* __restrict__ DF, De
                 if (l < 1 || l > N_LAYERS || c < BORDER || c >= C - BORDER || r < BORDER || r >= R - BORDER) break;
             }
             if (done) {
-                const Fit F = local_fit(DF, ob + l * RC + (long long)r * C + c, C, RC);
+                const Fit F = local_fit(DF, ob + l * RC + (long long)r * P + c, P, RC);
                 const float contr = F.v + 0.5f * ((F.dx * X0 + F.dy * X1) + F.ds * X2);
                 const float tr = F.dxx + F.dyy;
                 const float dt = F.dxx * F.dyy - F.dxy * F.dxy;

@@ -77,11 +77,13 @@ constexpr int D_WIDTH = 4;
 constexpr int D_BINS = 8;
 constexpr int MAXO = 16;
 
-// Octave geometry of one image: octave o is R[o] x C[o]; DoG layers 0..4 of octave o start at
-// dog_off[o] in the DoG atlas, gradient layers 1..3 (magnitude and angle) at grad_off[o].
+// Octave geometry of one image: octave o is R[o] x C[o], its planes have row pitch P[o] (C[o] rounded
+// up to a multiple of four, so rows start on 16-byte boundaries); DoG layers 0..4 of octave o start
+// at dog_off[o] in the DoG atlas, gradient layers 1..3 (magnitude and angle) at grad_off[o], both in
+// pitched pixels.
 struct Geometry {
     int h, w, n_oct;
-    int R[MAXO], C[MAXO];
+    int R[MAXO], C[MAXO], P[MAXO];
     long long dog_off[MAXO + 1];
     long long grad_off[MAXO + 1];
 };
@@ -225,19 +227,14 @@ int32_t run_pyramid(Workspace& ws, const uint8_t* d_img, int img_stride, bool ex
                     cudaStream_t side = nullptr, cudaEvent_t* ev = nullptr);
 // octave.cu
 int32_t upload_octave_taps(const float* taps, int stride, const int* counts);
-int32_t launch_octave_fused(const float* L0, int R, int C, float* dog, float2* grad, float* down,
-                            int down_cols, cudaStream_t s);
 int layer_tile_variants();
 int layer_tile_height(int variant);
-int32_t launch_layer_fast(int layer, const float* src, int R, int C, float* dst, float* dog, float2* grad,
-                          float* down, int down_cols, int variant, int* err, cudaStream_t s);
-int32_t launch_base_fast(const uint8_t* img, int stride, int ih, int iw, float* dst, int variant, cudaStream_t s);
-int32_t launch_group_lower(const float* src, int R, int C, float* dog, float2* grad, float* l3, float* down,
-                           int down_cols, cudaStream_t s);
-int32_t launch_group_upper(const float* src, int R, int C, float* dog3, cudaStream_t s);
-// strip engine: the whole float32 octave in one launch (err: device word set when a TMA wait gives up)
-int32_t launch_octave_strip(const float* L0, int R, int C, float* dog, float2* grad, float* down,
-                            int down_cols, int* err, cudaStream_t s);
+int32_t launch_layer_fast(int layer, const float* src, int R, int C, int P, float* dst, float* dog, float2* grad,
+                          float* down, int down_pitch, int variant, int* err, cudaStream_t s);
+int32_t launch_base_fast(const uint8_t* img, int stride, int ih, int iw, int P, float* dst, int variant, cudaStream_t s);
+int32_t launch_group_lower(const float* src, int R, int C, int P, float* dog, float2* grad, float* l3, float* down,
+                           int down_pitch, cudaStream_t s);
+int32_t launch_group_upper(const float* src, int R, int C, int P, float* dog3, cudaStream_t s);
 constexpr int PYR_ERR_WORD = 8;   // index of the pyramid's error word in Workspace::counters
 // autotune.cu: the fastest of n_variants launches of `run` for `key` (timed once per process and
 // device on `s`, then cached; FSB_AUTOTUNE=0 returns variant 0, FSB_AUTOTUNE_FILE persists choices)

@@ -4,8 +4,8 @@
 // 227-267 (DoG atlas, gradient magnitude / angle of gauss layers 1..3).
 //
 // Layout in HBM (per image):
-//   DoG atlas   float32 [octave][layer 0..4][R][C], octave o at Geometry::dog_off[o]
-//   GRAD        float2 (magnitude, angle) [octave][layer 1..3][R][C], octave o at Geometry::grad_off[o];
+//   DoG atlas   float32 [octave][layer 0..4][R][P], octave o at Geometry::dog_off[o], P the row pitch
+//   GRAD        float2 (magnitude, angle) [octave][layer 1..3][R][P], octave o at Geometry::grad_off[o];
 //               one 8-byte load gives a sample of the orientation and descriptor windows
 //   planes      three octave-0-sized float32 scratch planes for gauss layers in flight
 //
@@ -82,8 +82,9 @@ Geometry make_geometry(int h, int w) {
         g.C[o] = C;
         g.dog_off[o] = dog;
         g.grad_off[o] = grad;
-        dog += 5LL * R * C;
-        grad += 3LL * R * C;
+        g.P[o] = (C + 3) & ~3;
+        dog += 5LL * R * g.P[o];
+        grad += 3LL * R * g.P[o];
         g.n_oct = o + 1;
         R = (R + 1) / 2;   // layers[3][::2, ::2]
         C = (C + 1) / 2;
@@ -109,12 +110,12 @@ struct BlurArgs {
     const float* src;          // previous gauss layer (layer launches)
     const uint8_t* img;        // uint8 input (base launch)
     int img_stride, ih, iw;
-    int rows, cols;
+    int rows, cols, pitch;     // pitch: of every plane of the octave
     float* dst;                // this layer, or null
     float* dog;                // DoG plane (this - previous), or null
     float2* grad;              // gradient (magnitude, angle in degrees) of the previous layer, or null
     float* down;               // previous layer [::2, ::2], or null
-    int down_cols;
+    int down_pitch;
 };
 
 // Bilinear 2x upsample sample of the uint8 image at (Y, X) of the 2h x 2w grid, float32 with the
@@ -163,7 +164,7 @@ __global__ void __launch_bounds__(NT) k_blur(BlurArgs a) {
     for (int i = threadIdx.x; i < IH * IW; i += NT) {
         const int yy = i / IW, xx = i - yy * IW;
         const int gy = mirror(y0 + yy - RAD, a.rows), gx = mirror(x0 + xx - RAD, a.cols);
-        s_in[yy * SW + xx] = BASE ? up2_sample(a, gy, gx) : __ldg(a.src + (size_t)gy * a.cols + gx);
+        s_in[yy * SW + xx] = BASE ? up2_sample(a, gy, gx) : __ldg(a.src + (size_t)gy * a.pitch + gx);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < TY * IW; i += NT) {
@@ -176,7 +177,7 @@ __global__ void __launch_bounds__(NT) k_blur(BlurArgs a) {
         const int gy = y0 + yy, gx = x0 + xx;
         if (gy >= a.rows || gx >= a.cols) continue;
         const float v = conv<TS, RAD, EXACT>(&s_mid[yy * SW + xx], 1);
-        const size_t at = (size_t)gy * a.cols + gx;
+        const size_t at = (size_t)gy * a.pitch + gx;
         if (a.dst) a.dst[at] = v;
         const float* c = &s_in[(yy + RAD) * SW + xx + RAD];   // previous layer at (gy, gx)
         if (a.dog) a.dog[at] = __fsub_rn(v, c[0]);
@@ -190,7 +191,7 @@ __global__ void __launch_bounds__(NT) k_blur(BlurArgs a) {
             const float an = __fmul_rn(atan2f(dy, dx), kRad2Deg);
             a.grad[at] = make_float2(mg, an < 0.f ? __fadd_rn(an, 360.f) : an);
         }
-        if (a.down && !(gy & 1) && !(gx & 1)) a.down[(size_t)(gy >> 1) * a.down_cols + (gx >> 1)] = c[0];
+        if (a.down && !(gy & 1) && !(gx & 1)) a.down[(size_t)(gy >> 1) * a.down_pitch + (gx >> 1)] = c[0];
     }
 }
 
@@ -206,16 +207,11 @@ void launch(bool exact, const BlurArgs& a, cudaStream_t s) {
 
 }  // namespace
 
-// Float32 octave engines: the fused layer groups (k_group, octave.cu) by default; the tiled
-// per-layer kernels (k_layer) with FSB_PYRAMID=layer; the fused streaming kernel (k_octave) for
-// octaves at least kFusedMinCols wide with FSB_PYRAMID=fused.
-static const int kFusedMinCols = 2000;
-
 namespace {
 struct LayerCall {
     int layer;
     const float* src;
-    int R, C;
+    int R, C, P;
     float *dst, *dog;
     float2* grad;
     float* down;
@@ -225,24 +221,24 @@ struct LayerCall {
 };
 int32_t run_layer_call(void* p, int v) {
     const LayerCall* c = static_cast<const LayerCall*>(p);
-    return launch_layer_fast(c->layer, c->src, c->R, c->C, c->dst, c->dog, c->grad, c->down, c->dc, v, c->err, c->s);
+    return launch_layer_fast(c->layer, c->src, c->R, c->C, c->P, c->dst, c->dog, c->grad, c->down, c->dc, v, c->err, c->s);
 }
 struct BaseCall {
     const uint8_t* img;
-    int stride, h, w;
+    int stride, h, w, P;
     float* dst;
     cudaStream_t s;
 };
 int32_t run_base_call(void* p, int v) {
     const BaseCall* c = static_cast<const BaseCall*>(p);
-    return launch_base_fast(c->img, c->stride, c->h, c->w, c->dst, v == 1 ? 2 : 0, c->s);   // heights 32, 64
+    return launch_base_fast(c->img, c->stride, c->h, c->w, c->P, c->dst, v == 1 ? 2 : 0, c->s);   // heights 32, 64
 }
 // one tuned per-layer launch: the tile height is chosen per (layer, octave size);
 // FSB_LAYER_VARIANT=k (read on every call) runs variant k everywhere instead, so each variant can
 // be checked against the others
-int32_t tuned_layer(int layer, const float* src, int R, int C, float* dst, float* dog, float2* grad,
+int32_t tuned_layer(int layer, const float* src, int R, int C, int P, float* dst, float* dog, float2* grad,
                     float* down, int dc, int* err, cudaStream_t s) {
-    LayerCall c{layer, src, R, C, dst, dog, grad, down, dc, err, s};
+    LayerCall c{layer, src, R, C, P, dst, dog, grad, down, dc, err, s};
     if (const char* fv = std::getenv("FSB_LAYER_VARIANT")) {
         const int v = std::atoi(fv);
         if (v >= 0 && v < layer_tile_variants()) return run_layer_call(&c, v);
@@ -254,17 +250,15 @@ int32_t tuned_layer(int layer, const float* src, int R, int C, float* dst, float
 }
 }  // namespace
 
-// FSB_PYRAMID selects the float32 octave engine (all are bit-identical): unset, the autotuner picks
+// FSB_PYRAMID selects the float32 octave engine (both are bit-identical): unset, the autotuner picks
 // per octave size between the per-layer kernels (variant 0, also with FSB_AUTOTUNE=0) and the
-// fused layer groups (variant 1); "layer" / "group" force one; "fused" takes the streaming
-// kernel for octaves at least kFusedMinCols wide. Read on every call.
-enum class Engine { Auto, Group, Layer, Fused, Strip };
+// fused layer groups (variant 1); "layer" / "group" force one, other values choose as unset. Read on
+// every call.
+enum class Engine { Auto, Group, Layer };
 static Engine pyramid_engine() {
     const char* e = std::getenv("FSB_PYRAMID");
     if (e && std::strcmp(e, "layer") == 0) return Engine::Layer;
     if (e && std::strcmp(e, "group") == 0) return Engine::Group;
-    if (e && std::strcmp(e, "strip") == 0) return Engine::Strip;
-    if (e && std::strcmp(e, "fused") == 0) return Engine::Fused;
     return Engine::Auto;
 }
 
@@ -274,7 +268,7 @@ namespace {
 // either any number of times.
 struct OctaveCall {
     const float* src;
-    int R, C;
+    int R, C, P;
     float *x, *y, *dog;
     float2* grad;
     float* down;
@@ -284,11 +278,11 @@ struct OctaveCall {
     // since the next octave needs only L3's downsample; `join` marks its end
     cudaStream_t side;
     cudaEvent_t fork, join;
-    int* err;   // error word of the strip engine's bounded waits
+    int* err;   // error word of the tile copies' bounded waits
 };
 int32_t run_octave_call(void* p, int v) {
     const OctaveCall* c = static_cast<const OctaveCall*>(p);
-    const long long RC = (long long)c->R * c->C;
+    const long long RC = (long long)c->R * c->P;
     cudaStream_t ts = c->s;   // stream of the tail
     auto fork = [&]() -> int32_t {
         if (!c->side) return FSB_OK;
@@ -297,25 +291,19 @@ int32_t run_octave_call(void* p, int v) {
         ts = c->side;
         return FSB_OK;
     };
-    if (v == 2) {
-        // the whole octave in one launch: no tail to move to the side stream
-        FSB_TRY(launch_octave_strip(c->src, c->R, c->C, c->dog, c->grad, c->down, c->dc, c->err, c->s));
-        if (c->side) FSB_CUDA(cudaEventRecord(c->join, c->s));
-        return FSB_OK;
-    }
     if (v == 1) {
-        FSB_TRY(launch_group_lower(c->src, c->R, c->C, c->dog, c->grad, c->x, c->down, c->dc, c->s));
+        FSB_TRY(launch_group_lower(c->src, c->R, c->C, c->P, c->dog, c->grad, c->x, c->down, c->dc, c->s));
         FSB_TRY(fork());
-        FSB_TRY(launch_group_upper(c->x, c->R, c->C, c->dog + 3 * RC, ts));
+        FSB_TRY(launch_group_upper(c->x, c->R, c->C, c->P, c->dog + 3 * RC, ts));
     } else {
-        FSB_TRY(tuned_layer(1, c->src, c->R, c->C, c->x, c->dog, nullptr, nullptr, 0, c->err, c->s));
-        FSB_TRY(tuned_layer(2, c->x, c->R, c->C, c->y, c->dog + RC, c->grad, nullptr, 0, c->err, c->s));
-        FSB_TRY(tuned_layer(3, c->y, c->R, c->C, c->x, c->dog + 2 * RC, c->grad + RC, nullptr, 0, c->err,
+        FSB_TRY(tuned_layer(1, c->src, c->R, c->C, c->P, c->x, c->dog, nullptr, nullptr, 0, c->err, c->s));
+        FSB_TRY(tuned_layer(2, c->x, c->R, c->C, c->P, c->y, c->dog + RC, c->grad, nullptr, 0, c->err, c->s));
+        FSB_TRY(tuned_layer(3, c->y, c->R, c->C, c->P, c->x, c->dog + 2 * RC, c->grad + RC, nullptr, 0, c->err,
                             c->s));
-        FSB_TRY(tuned_layer(4, c->x, c->R, c->C, c->y, c->dog + 3 * RC, c->grad + 2 * RC, c->down,
+        FSB_TRY(tuned_layer(4, c->x, c->R, c->C, c->P, c->y, c->dog + 3 * RC, c->grad + 2 * RC, c->down,
                             c->dc, c->err, c->s));
         FSB_TRY(fork());
-        FSB_TRY(tuned_layer(5, c->y, c->R, c->C, nullptr, c->dog + 4 * RC, nullptr, nullptr, 0, c->err, ts));
+        FSB_TRY(tuned_layer(5, c->y, c->R, c->C, c->P, nullptr, c->dog + 4 * RC, nullptr, nullptr, 0, c->err, ts));
     }
     if (c->side) FSB_CUDA(cudaEventRecord(c->join, c->side));
     return FSB_OK;
@@ -337,18 +325,19 @@ int32_t run_pyramid(Workspace& ws, const uint8_t* d_img, int img_stride, bool ex
     a.iw = g.w;
     a.rows = g.R[0];
     a.cols = g.C[0];
+    a.pitch = g.P[0];
     a.dst = P[0];
     if (exact) {
         launch<0, 5, true>(exact, a, s);
     } else {
-        BaseCall bc{d_img, img_stride, g.h, g.w, P[0], s};
+        BaseCall bc{d_img, img_stride, g.h, g.w, g.P[0], P[0], s};
         char key[64];
         std::snprintf(key, sizeof(key), "k_base_%dx%d", g.h, g.w);
         int v = 0;
         FSB_TRY(autotune(key, 2, run_base_call, &bc, s, &v));
     }
     const Engine eng = exact ? Engine::Layer : pyramid_engine();
-    if (!exact && eng != Engine::Fused) {
+    if (!exact) {
         // octave o reads its base from P[0] (o = 0) or one half of next_base and writes the next
         // base into the other half; two of P[0..2] hold its layers in flight. With a side stream,
         // an octave's tail (reading one of those planes) overlaps the next octave, which then takes
@@ -356,7 +345,7 @@ int32_t run_pyramid(Workspace& ws, const uint8_t* d_img, int img_stride, bool ex
         // most one tail is in flight. While an octave size is being tuned its tail stays on s (the
         // tuner times s only).
         float* NB = ws.next_base.as<float>();
-        const long long half = g.n_oct > 1 ? ((long long)g.R[1] * g.C[1] + 63) / 64 * 64 : 0;
+        const long long half = g.n_oct > 1 ? ((long long)g.R[1] * g.P[1] + 63) / 64 * 64 : 0;
         const float* cur = P[0];
         const float* tail_plane = nullptr;    // plane the latest side-stream tail reads
         int prev_tail = -1, last_tail = -1;   // the two latest octaves whose tails ran on the side
@@ -374,16 +363,16 @@ int32_t run_pyramid(Workspace& ws, const uint8_t* d_img, int img_stride, bool ex
             float* pl[2];
             for (int k = 0, n = 0; k < 3 && n < 2; ++k)
                 if (P[k] != cur && P[k] != busy) pl[n++] = P[k];
-            OctaveCall c{cur, g.R[o], g.C[o], pl[0], pl[1], DF + g.dog_off[o], GRAD + g.grad_off[o],
-                         last ? nullptr : NB + (o & 1) * half, last ? 0 : g.C[o + 1], s,
+            OctaveCall c{cur, g.R[o], g.C[o], g.P[o], pl[0], pl[1], DF + g.dog_off[o], GRAD + g.grad_off[o],
+                         last ? nullptr : NB + (o & 1) * half, last ? 0 : g.P[o + 1], s,
                          nullptr, side ? ev[2 * o] : nullptr, side ? ev[2 * o + 1] : nullptr, err};
-            int v = eng == Engine::Group ? 1 : eng == Engine::Strip ? 2 : 0;
+            int v = eng == Engine::Group ? 1 : 0;
             char key[64];
             std::snprintf(key, sizeof(key), "k_octave3_%dx%d", g.R[o], g.C[o]);
-            const bool known = eng != Engine::Auto || autotune_cached(key, 3, &v);
-            if (known && side && v != 2) c.side = side;
+            const bool known = eng != Engine::Auto || autotune_cached(key, 2, &v);
+            if (known && side) c.side = side;
             if (eng == Engine::Auto && !known) {
-                FSB_TRY(autotune(key, 3, run_octave_call, &c, s, &v));
+                FSB_TRY(autotune(key, 2, run_octave_call, &c, s, &v));
             } else {
                 FSB_TRY(run_octave_call(&c, v));
             }
@@ -400,34 +389,16 @@ int32_t run_pyramid(Workspace& ws, const uint8_t* d_img, int img_stride, bool ex
     }
     float* cur = P[0];   // base of the current octave
     for (int o = 0; o < g.n_oct; ++o) {
-        const long long RC = (long long)g.R[o] * g.C[o];
+        const long long RC = (long long)g.R[o] * g.P[o];
         float* dog = DF + g.dog_off[o];
         float2* grad = GRAD + g.grad_off[o];
         float* other[2];
         for (int k = 0, n = 0; k < 3; ++k)
             if (P[k] != cur) other[n++] = P[k];
-        if (!exact && g.C[o] >= kFusedMinCols) {
-            // fused octave: reads cur, writes the next base into another plane
-            float* down = o + 1 < g.n_oct ? other[0] : nullptr;
-            FSB_TRY(launch_octave_fused(cur, g.R[o], g.C[o], dog, grad, down, o + 1 < g.n_oct ? g.C[o + 1] : 0, s));
-            cur = other[0];
-            continue;
-        }
-        if (!exact) {
-            const int R = g.R[o], C = g.C[o];
-            float* down = o + 1 < g.n_oct ? cur : nullptr;
-            const int dc = o + 1 < g.n_oct ? g.C[o + 1] : 0;
-            FSB_TRY(tuned_layer(1, cur, R, C, other[0], dog, nullptr, nullptr, 0, err, s));
-            FSB_TRY(tuned_layer(2, other[0], R, C, other[1], dog + RC, grad, nullptr, 0, err, s));
-            FSB_TRY(tuned_layer(3, other[1], R, C, other[0], dog + 2 * RC, grad + RC, nullptr, 0, err, s));
-            FSB_TRY(tuned_layer(4, other[0], R, C, other[1], dog + 3 * RC, grad + 2 * RC, down, dc,
-                                err, s));
-            FSB_TRY(tuned_layer(5, other[1], R, C, nullptr, dog + 4 * RC, nullptr, nullptr, 0, err, s));
-            continue;   // the next base is in `cur` (the dead L0 plane)
-        }
         BlurArgs b{};
         b.rows = g.R[o];
         b.cols = g.C[o];
+        b.pitch = g.P[o];
         // layer 1: L0 -> X, DoG 0
         b.src = cur; b.dst = other[0]; b.dog = dog;
         launch<1, 5, false>(exact, b, s);
@@ -439,7 +410,7 @@ int32_t run_pyramid(Workspace& ws, const uint8_t* d_img, int img_stride, bool ex
         launch<3, 8, false>(exact, b, s);
         // layer 4: L3 (X) -> Y, DoG 3, gradient of L3, L3[::2, ::2] -> the (dead) base plane
         b.src = other[0]; b.dst = other[1]; b.dog = dog + 3 * RC; b.grad = grad + 2 * RC;
-        if (o + 1 < g.n_oct) { b.down = cur; b.down_cols = g.C[o + 1]; }
+        if (o + 1 < g.n_oct) { b.down = cur; b.down_pitch = g.P[o + 1]; }
         launch<4, 10, false>(exact, b, s);
         // layer 5: L4 (Y) -> DoG 4 only
         b.src = other[1]; b.dst = nullptr; b.dog = dog + 4 * RC; b.grad = nullptr; b.down = nullptr;
