@@ -1271,40 +1271,32 @@ int32_t fsb_match_bf_batch_d(fsb_ctx* ctx, int32_t n_pairs, const uint8_t* const
         if (na[p] >= 2 && nb[p] >= 2) live.push_back(p);
     if (live.empty()) return FSB_OK;
     ctx->stage_begin(ST_MATCH);
-    std::vector<int> cnt(n_pairs, 0);
     FSB_TRY(ctx->s_count.ensure((size_t)n_pairs * 4 + 64));
     int* dn_all = ctx->s_count.as<int>();
     FSB_CUDA(cudaMemsetAsync(dn_all, 0, (size_t)n_pairs * 4, s));
-    if (precision == FSB_PREC_FP32) {
-        for (int p : live)
-            FSB_TRY(run_match_bf(ctx, d_a[p], na[p], d_b[p], nb[p], ratio, precision, d_q[p], d_t[p], dn_all + p, s));
-    } else {
-        std::vector<const uint8_t*> pa, pb;
-        std::vector<int64_t*> pq, pt;
-        std::vector<int> ra, rb;
-        for (int p : live) {
-            pa.push_back(d_a[p]);
-            pb.push_back(d_b[p]);
-            pq.push_back(d_q[p]);
-            pt.push_back(d_t[p]);
-            ra.push_back(na[p]);
-            rb.push_back(nb[p]);
-        }
-        int32_t* dn_live = dn_all;
-        FSB_TRY(run_match_bf_tc(ctx, (int)live.size(), pa.data(), ra.data(), pb.data(), rb.data(), ratio, precision,
-                                pq.data(), pt.data(), dn_live, &ctx->tc_stats, s));
-        std::vector<int> cl(live.size(), 0);
-        FSB_CUDA(cudaMemcpyAsync(cl.data(), dn_live, cl.size() * 4, cudaMemcpyDeviceToHost, s));
-        FSB_CUDA(cudaStreamSynchronize(s));
-        for (size_t i = 0; i < live.size(); ++i) cnt[live[i]] = cl[i];
-        ctx->stage_end(ST_MATCH);
-        for (int p = 0; p < n_pairs; ++p) n_out[p] = cnt[p];
-        return FSB_OK;
+    std::vector<const uint8_t*> pa, pb;
+    std::vector<int64_t*> pq, pt;
+    std::vector<int> ra, rb;
+    for (int p : live) {
+        pa.push_back(d_a[p]);
+        pb.push_back(d_b[p]);
+        pq.push_back(d_q[p]);
+        pt.push_back(d_t[p]);
+        ra.push_back(na[p]);
+        rb.push_back(nb[p]);
     }
-    FSB_CUDA(cudaMemcpyAsync(cnt.data(), dn_all, (size_t)n_pairs * 4, cudaMemcpyDeviceToHost, s));
+    const int nl = (int)live.size();
+    if (precision == FSB_PREC_FP32)
+        FSB_TRY(run_match_bf_batch(ctx, nl, pa.data(), ra.data(), pb.data(), rb.data(), ratio, pq.data(), pt.data(),
+                                   dn_all, s));
+    else
+        FSB_TRY(run_match_bf_tc(ctx, nl, pa.data(), ra.data(), pb.data(), rb.data(), ratio, precision, pq.data(),
+                                pt.data(), dn_all, &ctx->tc_stats, s));
+    std::vector<int> cl(nl, 0);
+    FSB_CUDA(cudaMemcpyAsync(cl.data(), dn_all, (size_t)nl * 4, cudaMemcpyDeviceToHost, s));
     FSB_CUDA(cudaStreamSynchronize(s));
+    for (int i = 0; i < nl; ++i) n_out[live[i]] = cl[i];
     ctx->stage_end(ST_MATCH);
-    for (int p = 0; p < n_pairs; ++p) n_out[p] = cnt[p];
     return FSB_OK;
 }
 

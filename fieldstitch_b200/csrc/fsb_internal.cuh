@@ -274,6 +274,10 @@ int32_t spread_dev(fsb_ctx* ctx, const float* d_x, const float* d_y, const float
 // ---------------------------------------------------------------- match.cu
 int32_t run_match_bf(fsb_ctx* ctx, const uint8_t* d_a, int na, const uint8_t* d_b, int nb, float ratio,
                      int precision, int64_t* d_q, int64_t* d_t, int* d_n, cudaStream_t s);
+// a batch of FP32 problems (na, nb >= 2); counts: device, one per pair
+int32_t run_match_bf_batch(fsb_ctx* ctx, int n, const uint8_t* const* d_a, const int* na, const uint8_t* const* d_b,
+                           const int* nb, float ratio, int64_t* const* d_q, int64_t* const* d_t, int32_t* counts,
+                           cudaStream_t s);
 // d_n null: candidates only (c_t, c_b12: best target or -1, b1, b2 per query; no ratio test, no _unique)
 int32_t run_match_guided(fsb_ctx* ctx, const double* d_pred, const uint8_t* d_a, int na, const double* d_bxy,
                          const uint8_t* d_b, int nb, double wb, double hb, double radius, int kc, float ratio,

@@ -1,8 +1,9 @@
 // Descriptor matching on uint8 RootSIFT descriptors.
 //
-//   k_bf_fp32     exhaustive nearest / second-nearest squared distance, CUDA-core FP32 tiles
-//                 (the plain path of matching._ratio_match_bf, app/planesite/matching.py:86-100)
-//   k_bf_merge    merge of the per-split top-2, float32 ratio test
+//   k_bf_exact    exhaustive nearest / second-nearest squared distance on the CUDA cores: exact
+//                 32-bit integer distances (the plain path of matching._ratio_match_bf,
+//                 app/planesite/matching.py:86-100)
+//   k_bf_merge    merge of the per-split top-2, float32 ratio test, one-to-one keys
 //   k_guided      prior-guided candidates within a radius on a uniform grid, exact integer
 //                 distances (matching._guided, app/planesite/matching.py:113-152)
 //   k_unique      one match per target: atomicMin on (distance << 32 | query) keys
@@ -15,6 +16,7 @@
 // on the values and the tie rules, which follow the reference.
 #include <cub/cub.cuh>
 
+#include <atomic>
 #include <mutex>
 
 #include "fsb_internal.cuh"
@@ -35,8 +37,10 @@ __global__ void k_norms(const uint8_t* __restrict__ d, int n, int32_t* __restric
     if (lane == 0) out[row] = s;
 }
 
-// ------------------------------------------------------------------------- FP32 dense tiles
-constexpr int BM = 128, BN = 128, BK = 32, TM = 8, TN = 8, BF_THREADS = 256;
+// ------------------------------------------------------------------------- dense tiles
+constexpr int BN = 128;            // target rows per tile
+constexpr int BF_PITCH = 144;      // bytes per staged row: rows 16 bytes apart mod 128, so the eight
+                                   // rows of a quarter-warp's loads fall in different banks
 
 struct Top2 {
     float b1, b2;
@@ -63,113 +67,303 @@ __device__ __forceinline__ Top2 top2_merge(Top2 a, Top2 b) {
     return r;
 }
 
-// grid: (row blocks, splits of B). Each CTA sweeps B rows [n0, n1) for 128 A rows and writes the
-// per-row top-2 of its split.
-__global__ void __launch_bounds__(BF_THREADS) k_bf_fp32(const uint8_t* __restrict__ A, int na,
-                                                        const uint8_t* __restrict__ B, int nb,
-                                                        const int32_t* __restrict__ nA, const int32_t* __restrict__ nB,
-                                                        int split_len, Top2* __restrict__ part) {
-    // operand tiles during the sweep; the same bytes hold the row merge afterwards
-    constexpr size_t kTileBytes = 2 * sizeof(float) * BK * (BM + 4);
-    constexpr size_t kRedBytes = sizeof(Top2) * 16 * BM;
-    __shared__ __align__(16) unsigned char smem[kTileBytes > kRedBytes ? kTileBytes : kRedBytes];
-    float (*As)[BM + 4] = reinterpret_cast<float (*)[BM + 4]>(smem);
-    float (*Bs)[BN + 4] = reinterpret_cast<float (*)[BN + 4]>(smem + sizeof(float) * BK * (BM + 4));
-    const int tid = threadIdx.x;
-    const int tx = tid & 15, ty = tid >> 4;
-    const int m0 = blockIdx.x * BM;
-    const int n_begin = blockIdx.y * split_len;
-    const int n_end = min(nb, n_begin + split_len);
-    Top2 best[TM];
+__device__ __forceinline__ void bf_cp_async(void* dst, const void* src, bool wide) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    if (wide) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
+    } else {
 #pragma unroll
-    for (int i = 0; i < TM; ++i) best[i] = Top2{INFINITY, INFINITY, -1};
-    float rn[TM];
-#pragma unroll
-    for (int i = 0; i < TM; ++i) {
-        const int r = m0 + ty + 16 * i;
-        rn[i] = r < na ? (float)nA[r] : 0.f;
-    }
-    for (int n0 = n_begin; n0 < n_end; n0 += BN) {
-        float acc[TM][TN];
-#pragma unroll
-        for (int i = 0; i < TM; ++i)
-#pragma unroll
-            for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
-        for (int k0 = 0; k0 < 128; k0 += BK) {
-            // stage 128 x 32 bytes of A and B as float, transposed (k-major)
-            for (int e = tid; e < BM * (BK / 4); e += BF_THREADS) {
-                const int r = e / (BK / 4), q = e - r * (BK / 4);
-                uint32_t wa = 0, wb = 0;
-                if (m0 + r < na) wa = reinterpret_cast<const uint32_t*>(A + (size_t)(m0 + r) * 128 + k0)[q];
-                if (n0 + r < n_end) wb = reinterpret_cast<const uint32_t*>(B + (size_t)(n0 + r) * 128 + k0)[q];
-#pragma unroll
-                for (int b = 0; b < 4; ++b) {
-                    As[q * 4 + b][r] = (float)((wa >> (8 * b)) & 255u);
-                    Bs[q * 4 + b][r] = (float)((wb >> (8 * b)) & 255u);
-                }
-            }
-            __syncthreads();
-#pragma unroll 4
-            for (int kk = 0; kk < BK; ++kk) {
-                float a[TM], b[TN];
-#pragma unroll
-                for (int i = 0; i < TM; ++i) a[i] = As[kk][ty + 16 * i];
-#pragma unroll
-                for (int j = 0; j < TN; ++j) b[j] = Bs[kk][tx + 16 * j];
-#pragma unroll
-                for (int i = 0; i < TM; ++i)
-#pragma unroll
-                    for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-            }
-            __syncthreads();
-        }
-#pragma unroll
-        for (int j = 0; j < TN; ++j) {
-            const int c = n0 + tx + 16 * j;
-            if (c >= n_end) continue;
-            const float cn = (float)nB[c];
-#pragma unroll
-            for (int i = 0; i < TM; ++i) top2_push(best[i], (rn[i] + cn) - 2.f * acc[i][j], c);
-        }
-    }
-    // merge the 16 column groups of each row through shared memory
-    Top2 (*red)[BM] = reinterpret_cast<Top2 (*)[BM]>(smem);
-#pragma unroll
-    for (int i = 0; i < TM; ++i) red[tx][ty + 16 * i] = best[i];
-    __syncthreads();
-    if (tid < BM) {
-        Top2 t = red[0][tid];
-        for (int g = 1; g < 16; ++g) t = top2_merge(t, red[g][tid]);
-        const int r = m0 + tid;
-        if (r < na) part[(size_t)blockIdx.y * na + r] = t;
+        for (int k = 0; k < 16; k += 4)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d + k), "l"((const char*)src + k) : "memory");
     }
 }
 
-// merge the splits, ratio test (float32, app/planesite/matching.py:96-99)
-__global__ void k_bf_merge(const Top2* __restrict__ part, int na, int splits, float ratio,
-                           int32_t* __restrict__ t_row, uint32_t* __restrict__ d_row) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+// rows r0 .. r0 + ROWS - 1 of D (zero rows from `end` on) into a staged tile; wide: D is 16-byte aligned
+template <int ROWS, int NTH>
+__device__ __forceinline__ void bf_stage(unsigned char* tile, const uint8_t* __restrict__ D, int r0, int end, bool wide) {
+#pragma unroll
+    for (int e = threadIdx.x; e < ROWS * 8; e += NTH) {
+        const int r = e >> 3, q = e & 7;
+        unsigned char* dst = tile + r * BF_PITCH + q * 16;
+        if (r0 + r < end)
+            bf_cp_async(dst, D + (size_t)(r0 + r) * 128 + q * 16, wide);
+        else
+            *reinterpret_cast<uint4*>(dst) = make_uint4(0u, 0u, 0u, 0u);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+
+// squared norms of the staged rows (threads 2r, 2r + 1 take a half each); rows from `live` on get a
+// value above every distance
+template <int ROWS, int NTH>
+__device__ __forceinline__ void bf_norms(const unsigned char* tile, int live, int* out) {
+    for (int e = threadIdx.x; e < ROWS * 2; e += NTH) {
+        const uint4* p = reinterpret_cast<const uint4*>(tile + (e >> 1) * BF_PITCH + (e & 1) * 64);
+        unsigned s = 0;
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+            const uint4 w = p[v];
+            s = __dp4a(w.x, w.x, s);
+            s = __dp4a(w.y, w.y, s);
+            s = __dp4a(w.z, w.z, s);
+            s = __dp4a(w.w, w.w, s);
+        }
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        if ((e & 1) == 0) out[e >> 1] = (e >> 1) < live ? (int)s : 0x3fffffff;
+    }
+}
+
+// One dense problem of a batch (an array in device memory, or one by value).
+struct BfPair {
+    const uint8_t *a, *b;
+    Top2* part;                // splits x na
+    unsigned long long* key;   // nb one-to-one keys
+    int64_t *q, *t;
+    int32_t* n;
+    int na, nb, split_len, splits;
+    int item0;                 // first CTA of the pair in the batch's grid
+};
+
+// the pair a CTA works on: the last one whose first item is not after `item`
+__device__ __forceinline__ int bf_find(const BfPair* __restrict__ tab, int n, int item) {
+    int lo = 0, hi = n - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (tab[mid].item0 <= item) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
+
+// A CTA per (row block of 32 WR queries, split of B) of every pair: it sweeps B rows [n0, n1) for its
+// queries and writes the per-row top-2 of its split. Squared distances of uint8 rows are integers below
+// 2^24: four products and their sum per dp4a in 32-bit integers give exactly the values that float32
+// multiply-adds give, a row's 128 bytes stay bytes in shared memory, and a thread's 8 x 8 block
+// reads 16 bytes of 16 rows per 256 dp4a. The query norm is added once at the end (it is the same for
+// every target of a row), and eight columns enter the running top-2 only when their smallest distance
+// beats the second best, which happens a few times per row.
+// Bound by the dp4a rate (half that of a multiply-add, four products each). Four pairs of about
+// 7000 x 7000: 2318 -> 667 us for the whole call against float32 multiply-adds on tiles converted to
+// float in shared memory, one pair after another; 1500 x 1500 from host arrays: 183 -> 102 us.
+template <int WR>
+__global__ void __launch_bounds__(64 * WR, WR == 4 ? 2 : 4)
+    k_bf_exact(const __grid_constant__ BfPair one, const BfPair* __restrict__ tab, int n_pairs) {
+    constexpr int BM = 32 * WR, NTH = 64 * WR;
+    extern __shared__ __align__(16) unsigned char bf_sm[];
+    unsigned char* sA = bf_sm;                                  // BM rows
+    unsigned char* sB = bf_sm + BM * BF_PITCH;                  // two tiles of BN rows
+    int* s_nb = reinterpret_cast<int*>(sB + 2 * BN * BF_PITCH);   // two tiles' norms
+    int* s_na = s_nb + 2 * BN;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int row0 = (warp >> 1) * 32 + (lane >> 3), col0 = (warp & 1) * 64 + (lane & 7);
+    const BfPair& P = tab ? tab[bf_find(tab, n_pairs, blockIdx.x)] : one;
+    const uint8_t* __restrict__ A = P.a;
+    const uint8_t* __restrict__ B = P.b;
+    const int na = P.na, item = blockIdx.x - P.item0, split = item % P.splits;
+    const int m0 = (item / P.splits) * BM;
+    const int n_begin = split * P.split_len;
+    const int n_end = min(P.nb, n_begin + P.split_len);
+    const bool wa = (reinterpret_cast<uintptr_t>(A) & 15) == 0, wb = (reinterpret_cast<uintptr_t>(B) & 15) == 0;
+    bf_stage<BM, NTH>(sA, A, m0, na, wa);
+    bf_stage<BN, NTH>(sB, B, n_begin, n_end, wb);
+    int b1[8], b2[8], i1[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        b1[i] = b2[i] = 0x3fffffff;
+        i1[i] = -1;
+    }
+    const unsigned char* pa = sA + row0 * BF_PITCH;
+    int buf = 0;
+    for (int n0 = n_begin; n0 < n_end; n0 += BN, buf ^= 1) {
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        __syncthreads();   // this tile is in; every thread is done with the other one
+        const unsigned char* tile = sB + buf * BN * BF_PITCH;
+        if (n0 + BN < n_end) bf_stage<BN, NTH>(sB + (buf ^ 1) * BN * BF_PITCH, B, n0 + BN, n_end, wb);
+        bf_norms<BN, NTH>(tile, n_end - n0, s_nb + buf * BN);
+        const unsigned char* pb = tile + col0 * BF_PITCH;
+        unsigned acc[8][8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[i][j] = 0u;
+#pragma unroll 2
+        for (int k = 0; k < 128; k += 8) {
+            uint2 a[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const uint2*>(pa + 4 * i * BF_PITCH + k);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const uint2 b = *reinterpret_cast<const uint2*>(pb + 8 * j * BF_PITCH + k);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) acc[i][j] = __dp4a(a[i].x, b.x, acc[i][j]);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) acc[i][j] = __dp4a(a[i].y, b.y, acc[i][j]);
+            }
+        }
+        __syncthreads();   // the tile's norms
+        int cn[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) cn[j] = s_nb[buf * BN + col0 + 8 * j];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            int d[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) d[j] = cn[j] - 2 * (int)acc[i][j];
+            const int m = min(min(min(d[0], d[1]), min(d[2], d[3])), min(min(d[4], d[5]), min(d[6], d[7])));
+            if (m < b2[i]) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const bool less = d[j] < b1[i];
+                    b2[i] = min(b2[i], max(b1[i], d[j]));
+                    b1[i] = less ? d[j] : b1[i];
+                    i1[i] = less ? n0 + col0 + 8 * j : i1[i];
+                }
+            }
+        }
+    }
+    // merge the 16 column groups of each row through shared memory (the staged targets are dead)
+    bf_norms<BM, NTH>(sA, BM, s_na);
+    __syncthreads();
+    int3 (*red)[BM] = reinterpret_cast<int3 (*)[BM]>(sB);
+    static_assert(sizeof(int3) * 16 * BM <= 2 * BN * BF_PITCH, "merge area");
+    const int grp = (warp & 1) * 8 + (lane & 7);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) red[grp][row0 + 4 * i] = make_int3(b1[i], b2[i], i1[i]);
+    __syncthreads();
+    if (tid < BM && m0 + tid < na) {
+        const float norm = (float)s_na[tid];
+        Top2 t{INFINITY, INFINITY, -1};
+        for (int g = 0; g < 16; ++g) {
+            const int3 v = red[g][tid];
+            Top2 o{INFINITY, INFINITY, v.z};
+            if (v.x < 0x20000000) o.b1 = norm + (float)v.x;   // exact: integers below 2^24
+            if (v.y < 0x20000000) o.b2 = norm + (float)v.y;
+            t = top2_merge(t, o);
+        }
+        P.part[(size_t)split * na + m0 + tid] = t;
+    }
+}
+
+template <int WR>
+constexpr int bf_smem() {
+    return 32 * WR * BF_PITCH + 2 * BN * BF_PITCH + (2 * BN + 32 * WR) * 4;
+}
+
+// How a batch of dense problems is cut into CTAs: WR = 4 (128 queries per CTA) once the 128 x 128 tiles
+// outnumber two per SM, else WR = 2 (twice the CTAs); every pair's targets in splits of `tps` tiles,
+// the number that gives the shortest schedule (waves of resident CTAs x (tiles + 1 for a CTA's
+// own staging and merge)), bounded by the top-2 table's capacity.
+struct BfPlan {
+    int wr, tps, items;
+    size_t parts;   // top-2 records
+};
+BfPlan bf_plan(const int* na, const int* nb, int n, size_t max_parts) {
+    auto tiles = [&](int p) { return (nb[p] + BN - 1) / BN; };
+    long long units = 0;
+    int most = 1;
+    for (int p = 0; p < n; ++p) {
+        units += (long long)((na[p] + 127) / 128) * tiles(p);
+        most = std::max(most, tiles(p));
+    }
+    BfPlan best{};
+    best.wr = units >= 2 * 148 ? 4 : 2;
+    const int bm = 32 * best.wr, slots = best.wr == 4 ? 2 * 148 : 4 * 148;
+    double cost = 0.0;
+    // with many tiles, finer steps than 1/64 of the longest sweep change little
+    for (int tps = most; tps >= 1; tps -= std::max(1, tps / 64)) {
+        long long items = 0;
+        size_t parts = 0;
+        for (int p = 0; p < n; ++p) {
+            const long long sp = (tiles(p) + tps - 1) / tps;
+            items += sp * ((na[p] + bm - 1) / bm);
+            parts += (size_t)sp * na[p];
+        }
+        if (parts > max_parts || items > 0x7fffffffLL) break;   // more splits from here on
+        const double c = (double)((items + slots - 1) / slots) * (tps + 1.0);
+        if (best.tps == 0 || c < cost) {
+            best.tps = tps;
+            best.items = (int)items;
+            best.parts = parts;
+            cost = c;
+        }
+    }
+    return best;
+}
+// fills p's split and first item; returns the next pair's first item
+int bf_place(const BfPlan& pl, BfPair& p, int item0) {
+    const int tiles = (p.nb + BN - 1) / BN, bm = 32 * pl.wr;
+    p.split_len = pl.tps * BN;
+    p.splits = (tiles + pl.tps - 1) / pl.tps;
+    p.item0 = item0;
+    return item0 + p.splits * ((p.na + bm - 1) / bm);
+}
+int32_t launch_bf(const BfPlan& pl, const BfPair& one, const BfPair* tab, int n, cudaStream_t s) {
+    static std::atomic<int> a2[64], a4[64];
+    if (pl.wr == 4) {
+        FSB_TRY(smem_attr((const void*)k_bf_exact<4>, bf_smem<4>(), a4));
+        k_bf_exact<4><<<pl.items, 256, bf_smem<4>(), s>>>(one, tab, n);
+    } else {
+        FSB_TRY(smem_attr((const void*)k_bf_exact<2>, bf_smem<2>(), a2));
+        k_bf_exact<2><<<pl.items, 128, bf_smem<2>(), s>>>(one, tab, n);
+    }
+    note_launch();
+    FSB_CUDA(cudaGetLastError());
+    return FSB_OK;
+}
+
+// merge the splits, ratio test (float32, app/planesite/matching.py:96-99), one-to-one key of the target
+__global__ void k_bf_merge(const __grid_constant__ BfPair one, const BfPair* __restrict__ tab, float ratio) {
+    const BfPair& P = tab ? tab[blockIdx.y] : one;
+    const int r = blockIdx.x * blockDim.x + threadIdx.x, na = P.na;
     if (r >= na) return;
-    Top2 t = part[r];
-    for (int s = 1; s < splits; ++s) t = top2_merge(t, part[(size_t)s * na + r]);
+    Top2 t = P.part[r];
+    for (int s = 1; s < P.splits; ++s) t = top2_merge(t, P.part[(size_t)s * na + r]);
     const float b1 = fmaxf(t.b1, 0.f), b2 = fmaxf(t.b2, 0.f);
     const bool ok = __fsqrt_rn(b1) < __fmul_rn(ratio, __fsqrt_rn(b2));
-    t_row[r] = ok ? t.i1 : -1;
-    d_row[r] = (uint32_t)b1;
+    if (ok && t.i1 >= 0) atomicMin(P.key + t.i1, ((unsigned long long)(uint32_t)b1 << 32) | (unsigned)r);
 }
 
 // ------------------------------------------------------------------------------ one-to-one
-__global__ void k_fill_u64(unsigned long long* p, int n, unsigned long long v) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = v;
-}
-
 __global__ void k_unique_keys(const int32_t* __restrict__ t_row, const uint32_t* __restrict__ d_row, int na,
                               unsigned long long* __restrict__ key) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= na) return;
     const int t = t_row[r];
     if (t >= 0) atomicMin(key + t, ((unsigned long long)d_row[r] << 32) | (unsigned)r);
+}
+
+// target-ordered compaction of the one-to-one keys by one block: one launch where flags, a device
+// select (two kernels) and a gather take four; up to kCompactMax targets (5 us at 9000)
+constexpr int kCompactMax = 32768;
+constexpr int COMPACT_T = 1024;
+__device__ __forceinline__ void unique_compact(const unsigned long long* __restrict__ key, int nb, int64_t* __restrict__ q,
+                                               int64_t* __restrict__ t, int32_t* __restrict__ n_out) {
+    typedef cub::BlockScan<int, COMPACT_T> Scan;
+    __shared__ typename Scan::TempStorage tmp;
+    const int per = (nb + COMPACT_T - 1) / COMPACT_T;
+    const int t0 = threadIdx.x * per, t1 = min(nb, t0 + per);
+    int cnt = 0;
+    for (int i = t0; i < t1; ++i) cnt += key[i] != ~0ull;
+    int off = 0, total = 0;
+    Scan(tmp).ExclusiveSum(cnt, off, total);
+    for (int i = t0; i < t1; ++i) {
+        const unsigned long long k = key[i];
+        if (k != ~0ull) {
+            q[off] = (int64_t)(k & 0xffffffffull);
+            t[off] = i;
+            ++off;
+        }
+    }
+    if (threadIdx.x == 0) *n_out = total;
+}
+__global__ void __launch_bounds__(COMPACT_T) k_unique_compact(const unsigned long long* __restrict__ key, int nb,
+                                                              int64_t* __restrict__ q, int64_t* __restrict__ t,
+                                                              int32_t* __restrict__ n_out) {
+    unique_compact(key, nb, q, t, n_out);
+}
+// a block per pair of a batch
+__global__ void __launch_bounds__(COMPACT_T) k_bf_compact(const BfPair* __restrict__ tab) {
+    const BfPair& P = tab[blockIdx.x];
+    unique_compact(P.key, P.nb, P.q, P.t, P.n);
 }
 
 __global__ void k_unique_flags(const unsigned long long* __restrict__ key, int nb, uint8_t* __restrict__ flag,
@@ -393,26 +587,40 @@ __global__ void k_perspective(const double* __restrict__ xy, int n, const double
     out[2 * i + 1] = v;
 }
 
-// one-to-one filter + compaction ordered by target: q[i], t[i], *d_n
-int32_t run_unique(fsb_ctx* ctx, const int32_t* t_row, const uint32_t* d_row, int na, int nb, int64_t* d_q,
-                   int64_t* d_t, int* d_n, cudaStream_t s) {
-    FSB_TRY(ctx->s_u64.ensure((size_t)nb * 8 + 64));
+// the one-to-one keys of nb targets -> matches ordered by target: q[i], t[i], *d_n
+int32_t emit_unique(fsb_ctx* ctx, const unsigned long long* key, int nb, int64_t* d_q, int64_t* d_t, int* d_n,
+                    cudaStream_t s) {
+    if (nb <= kCompactMax) {
+        k_unique_compact<<<1, COMPACT_T, 0, s>>>(key, nb, d_q, d_t, d_n);
+        note_launch();
+        FSB_CUDA(cudaGetLastError());
+        return FSB_OK;
+    }
     FSB_TRY(ctx->s_misc2.ensure((size_t)nb * 9 + 1024));
-    unsigned long long* key = ctx->s_u64.as<unsigned long long>();
     uint8_t* flag = ctx->s_misc2.as<uint8_t>();
     int32_t* iota = reinterpret_cast<int32_t*>(flag + ((nb + 255) / 256) * 256);
     int32_t* tsel = iota + nb;
-    k_fill_u64<<<blocks(nb, 256), 256, 0, s>>>(key, nb, ~0ull);
-    k_unique_keys<<<blocks(na, 256), 256, 0, s>>>(t_row, d_row, na, key);
     k_unique_flags<<<blocks(nb, 256), 256, 0, s>>>(key, nb, flag, iota);
     size_t tb = 0;
     cub::DeviceSelect::Flagged(nullptr, tb, iota, flag, tsel, d_n, nb, s);
     FSB_TRY(ctx->s_cub.ensure(tb + 16));
     FSB_CUDA(cub::DeviceSelect::Flagged(ctx->s_cub.p, tb, iota, flag, tsel, d_n, nb, s));
     k_unique_emit<<<blocks(nb, 256), 256, 0, s>>>(key, tsel, d_n, d_q, d_t);
-    note_launch(4);
+    note_launch(2);
     FSB_CUDA(cudaGetLastError());
     return FSB_OK;
+}
+
+// one-to-one filter + compaction ordered by target
+int32_t run_unique(fsb_ctx* ctx, const int32_t* t_row, const uint32_t* d_row, int na, int nb, int64_t* d_q,
+                   int64_t* d_t, int* d_n, cudaStream_t s) {
+    FSB_TRY(ctx->s_u64.ensure((size_t)nb * 8 + 64));
+    unsigned long long* key = ctx->s_u64.as<unsigned long long>();
+    FSB_CUDA(cudaMemsetAsync(key, 0xff, (size_t)nb * 8, s));
+    k_unique_keys<<<blocks(na, 256), 256, 0, s>>>(t_row, d_row, na, key);
+    note_launch();
+    FSB_CUDA(cudaGetLastError());
+    return emit_unique(ctx, key, nb, d_q, d_t, d_n, s);
 }
 
 __device__ __forceinline__ uint32_t orderable(float f) {
@@ -640,26 +848,60 @@ int32_t run_match_bf(fsb_ctx* ctx, const uint8_t* d_a, int na, const uint8_t* d_
     }
     if (precision != FSB_PREC_FP32)
         return run_match_bf_tc(ctx, 1, &d_a, &na, &d_b, &nb, ratio, precision, &d_q, &d_t, d_n, &ctx->tc_stats, s);
-    const int row_blocks = (na + BM - 1) / BM;
-    int splits = 1;
-    while (row_blocks * splits < 2 * 148 && (nb + splits * 2 - 1) / (splits * 2) >= BN) splits *= 2;
-    int split_len = (nb + splits - 1) / splits;
-    split_len = ((split_len + BN - 1) / BN) * BN;
-    splits = (nb + split_len - 1) / split_len;
-    FSB_TRY(ctx->s_i32.ensure((size_t)(na + nb) * 4 + (size_t)na * 8 + 64));
-    int32_t* nA = ctx->s_i32.as<int32_t>();
-    int32_t* nB = nA + na;
-    int32_t* t_row = nB + nb;
-    uint32_t* d_row = reinterpret_cast<uint32_t*>(t_row + na);
-    FSB_TRY(ctx->s_misc.ensure((size_t)splits * na * sizeof(Top2) + 64));
-    Top2* part = ctx->s_misc.as<Top2>();
-    k_norms<<<blocks(na, 8), 256, 0, s>>>(d_a, na, nA);
-    k_norms<<<blocks(nb, 8), 256, 0, s>>>(d_b, nb, nB);
-    k_bf_fp32<<<dim3(row_blocks, splits), BF_THREADS, 0, s>>>(d_a, na, d_b, nb, nA, nB, split_len, part);
-    k_bf_merge<<<blocks(na, 256), 256, 0, s>>>(part, na, splits, ratio, t_row, d_row);
-    note_launch(4);
+    const BfPlan pl = bf_plan(&na, &nb, 1, (size_t)1 << 40);
+    FSB_TRY(ctx->s_misc.ensure(pl.parts * sizeof(Top2) + 64));
+    FSB_TRY(ctx->s_u64.ensure((size_t)nb * 8 + 64));
+    BfPair one{d_a, d_b, ctx->s_misc.as<Top2>(), ctx->s_u64.as<unsigned long long>(), d_q, d_t, d_n, na, nb};
+    bf_place(pl, one, 0);
+    FSB_CUDA(cudaMemsetAsync(one.key, 0xff, (size_t)nb * 8, s));
+    FSB_TRY(launch_bf(pl, one, nullptr, 1, s));
+    k_bf_merge<<<blocks(na, 256), 256, 0, s>>>(one, nullptr, ratio);
+    note_launch();
     FSB_CUDA(cudaGetLastError());
-    return run_unique(ctx, t_row, d_row, na, nb, d_q, d_t, d_n, s);
+    return emit_unique(ctx, one.key, nb, d_q, d_t, d_n, s);
+}
+
+// A batch of FP32 dense problems (each na, nb >= 2) in one set of launches: counts (device, one per
+// pair). Pairs with more targets than one block compacts run one after another instead.
+int32_t run_match_bf_batch(fsb_ctx* ctx, int n, const uint8_t* const* d_a, const int* na, const uint8_t* const* d_b,
+                           const int* nb, float ratio, int64_t* const* d_q, int64_t* const* d_t, int32_t* counts,
+                           cudaStream_t s) {
+    bool one_by_one = n == 1 || n > 65535;   // a grid's second dimension
+    for (int p = 0; p < n; ++p) one_by_one = one_by_one || nb[p] > kCompactMax;
+    if (one_by_one) {
+        for (int p = 0; p < n; ++p)
+            FSB_TRY(run_match_bf(ctx, d_a[p], na[p], d_b[p], nb[p], ratio, FSB_PREC_FP32, d_q[p], d_t[p], counts + p, s));
+        return FSB_OK;
+    }
+    const BfPlan pl = bf_plan(na, nb, n, (size_t)1 << 40);
+    size_t keys = 0;
+    int max_na = 0;
+    for (int p = 0; p < n; ++p) {
+        keys += (size_t)nb[p];
+        max_na = std::max(max_na, na[p]);
+    }
+    FSB_TRY(ctx->s_misc.ensure(pl.parts * sizeof(Top2) + 64));
+    FSB_TRY(ctx->s_u64.ensure(keys * 8 + 64));
+    FSB_TRY(ctx->s_i32.ensure((size_t)n * sizeof(BfPair)));
+    std::vector<BfPair> tab(n);
+    Top2* part = ctx->s_misc.as<Top2>();
+    unsigned long long* key = ctx->s_u64.as<unsigned long long>();
+    int item = 0;
+    for (int p = 0; p < n; ++p) {
+        tab[p] = BfPair{d_a[p], d_b[p], part, key, d_q[p], d_t[p], counts + p, na[p], nb[p]};
+        item = bf_place(pl, tab[p], item);
+        part += (size_t)tab[p].splits * na[p];
+        key += nb[p];
+    }
+    BfPair* d_tab = ctx->s_i32.as<BfPair>();
+    FSB_CUDA(cudaMemcpyAsync(d_tab, tab.data(), (size_t)n * sizeof(BfPair), cudaMemcpyHostToDevice, s));
+    FSB_CUDA(cudaMemsetAsync(ctx->s_u64.p, 0xff, keys * 8, s));
+    FSB_TRY(launch_bf(pl, tab[0], d_tab, n, s));
+    k_bf_merge<<<dim3(blocks(max_na, 256), (unsigned)n), 256, 0, s>>>(tab[0], d_tab, ratio);
+    k_bf_compact<<<n, COMPACT_T, 0, s>>>(d_tab);
+    note_launch(2);
+    FSB_CUDA(cudaGetLastError());
+    return FSB_OK;
 }
 
 int32_t run_unique_rows(fsb_ctx* ctx, const int32_t* t_row, const uint32_t* d_row, int na, int nb, int64_t* d_q,
@@ -881,7 +1123,7 @@ int32_t run_match_guided_batch(fsb_ctx* ctx, int n_pairs, const double* const* d
 // serving), host frameworks that own the CUDA allocator and forbid allocations behind their back,
 // and real-time loops where an allocation may block or fail in the middle of a frame. For them
 // this entry point runs the FP32 dense matcher with all of its scratch in one file-scope device
-// array of fixed size (kNoAllocScratchBytes, about 1.9 MiB), so a call allocates nothing: the
+// array of fixed size (kNoAllocScratchBytes, about 1.6 MiB), so a call allocates nothing: the
 // caller passes device inputs and outputs and a stream.
 //
 // The array lives in every GPU that loads this library until the process exits. Host code may
@@ -899,7 +1141,6 @@ namespace {
 constexpr int kNoAllocMaxRows = 16384;
 constexpr int kNoAllocSplitRows = 8 * kNoAllocMaxRows;   // capacity of the per-split top-2 table
 constexpr size_t kNoAllocScratchBytes =
-    4 * sizeof(int32_t) * kNoAllocMaxRows +                // norms of A and B, best target, distance
     sizeof(unsigned long long) * kNoAllocMaxRows +         // one-to-one keys per target
     sizeof(Top2) * (size_t)kNoAllocSplitRows;              // per-split top-2 of every A row
 
@@ -953,30 +1194,6 @@ int32_t noalloc_scratch(void** out) {
     return FSB_OK;
 }
 
-// single-CTA, target-ordered compaction of the one-to-one keys (nb <= kNoAllocMaxRows)
-constexpr int kCompactThreads = 1024;
-__global__ void __launch_bounds__(kCompactThreads) k_noalloc_compact(const unsigned long long* __restrict__ key, int nb,
-                                                                      int64_t* __restrict__ q, int64_t* __restrict__ t,
-                                                                      int32_t* __restrict__ n_out) {
-    typedef cub::BlockScan<int, kCompactThreads> Scan;
-    __shared__ typename Scan::TempStorage tmp;
-    const int per = (nb + kCompactThreads - 1) / kCompactThreads;
-    const int t0 = threadIdx.x * per, t1 = min(nb, t0 + per);
-    int cnt = 0;
-    for (int i = t0; i < t1; ++i) cnt += key[i] != ~0ull;
-    int off = 0, total = 0;
-    Scan(tmp).ExclusiveSum(cnt, off, total);
-    for (int i = t0; i < t1; ++i) {
-        const unsigned long long k = key[i];
-        if (k != ~0ull) {
-            q[off] = (int64_t)(k & 0xffffffffull);
-            t[off] = i;
-            ++off;
-        }
-    }
-    if (threadIdx.x == 0) *n_out = total;
-}
-
 }  // namespace
 }  // namespace fsb
 
@@ -998,29 +1215,17 @@ extern "C" int32_t fsb_match_bf_noalloc(const uint8_t* d_a, int32_t na, const ui
     }
     void* base = nullptr;
     FSB_TRY(noalloc_scratch(&base));
-    int32_t* nA = static_cast<int32_t*>(base);
-    int32_t* nB = nA + kNoAllocMaxRows;
-    int32_t* t_row = nB + kNoAllocMaxRows;
-    uint32_t* d_row = reinterpret_cast<uint32_t*>(t_row + kNoAllocMaxRows);
-    unsigned long long* key = reinterpret_cast<unsigned long long*>(d_row + kNoAllocMaxRows);
+    unsigned long long* key = static_cast<unsigned long long*>(base);
     Top2* part = reinterpret_cast<Top2*>(key + kNoAllocMaxRows);
-    // same split rule as the allocating matcher, bounded by the top-2 table's capacity
-    const int row_blocks = (na + BM - 1) / BM;
-    const int max_splits = kNoAllocSplitRows / na;
-    int splits = 1;
-    while (row_blocks * splits < 2 * 148 && (nb + splits * 2 - 1) / (splits * 2) >= BN && splits * 2 <= max_splits)
-        splits *= 2;
-    int split_len = (nb + splits - 1) / splits;
-    split_len = ((split_len + BN - 1) / BN) * BN;
-    splits = (nb + split_len - 1) / split_len;
-    k_norms<<<blocks(na, 8), 256, 0, s>>>(d_a, na, nA);
-    k_norms<<<blocks(nb, 8), 256, 0, s>>>(d_b, nb, nB);
-    k_bf_fp32<<<dim3(row_blocks, splits), BF_THREADS, 0, s>>>(d_a, na, d_b, nb, nA, nB, split_len, part);
-    k_bf_merge<<<blocks(na, 256), 256, 0, s>>>(part, na, splits, ratio, t_row, d_row);
-    k_fill_u64<<<blocks(nb, 256), 256, 0, s>>>(key, nb, ~0ull);
-    k_unique_keys<<<blocks(na, 256), 256, 0, s>>>(t_row, d_row, na, key);
-    k_noalloc_compact<<<1, kCompactThreads, 0, s>>>(key, nb, d_q, d_t, d_n);
-    note_launch(7);
+    // the allocating matcher's plan, bounded by the top-2 table's capacity
+    const BfPlan pl = bf_plan(&na, &nb, 1, kNoAllocSplitRows);
+    BfPair one{d_a, d_b, part, key, d_q, d_t, d_n, na, nb};
+    bf_place(pl, one, 0);
+    FSB_CUDA(cudaMemsetAsync(key, 0xff, (size_t)nb * 8, s));
+    FSB_TRY(launch_bf(pl, one, nullptr, 1, s));
+    k_bf_merge<<<blocks(na, 256), 256, 0, s>>>(one, nullptr, ratio);
+    k_unique_compact<<<1, COMPACT_T, 0, s>>>(key, nb, d_q, d_t, d_n);
+    note_launch(2);
     FSB_CUDA(cudaGetLastError());
     return FSB_OK;
 }

@@ -30,7 +30,7 @@ extern "C" {
 #define FSB_ERR_OVERFLOW 7    /* an internal capacity was exceeded and could not be grown */
 
 /* dense matcher precision (fsb_match_bf) */
-#define FSB_PREC_FP32 0 /* CUDA-core FP32 distances: the plain path */
+#define FSB_PREC_FP32 0 /* CUDA-core distances (exact 32-bit values): the plain path */
 #define FSB_PREC_BF16 1 /* tcgen05 BF16 x BF16 -> FP32 (exact for uint8 rows), exact integer re-rank */
 #define FSB_PREC_FP8 2  /* tcgen05 E4M3 (per-row power-of-two scale) -> FP32, exact integer re-rank of
                            the best 4 x 32 columns, certified ratio test, exact fallback rows */
@@ -292,7 +292,7 @@ int32_t fsb_mlp_filter_d(fsb_ctx* ctx, int32_t na, const int32_t* d_t1, const fl
    cudaMalloc: processes that reserve their whole device-memory budget up front, host frameworks
    that own the CUDA allocator, real-time loops that must not block or fail in an allocation.
    No counterpart in the reference (PlaneSite allocates through CuPy/NumPy). All scratch lives in
-   one fixed device array inside the library (about 1.9 MiB, held on every GPU that loads the
+   one fixed device array inside the library (about 1.6 MiB, held on every GPU that loads the
    library until exit); na and nb must be <= 16384, larger sizes are rejected with FSB_ERR_ARG.
    Inputs d_a (na x 128), d_b (nb x 128) and outputs d_q, d_t (capacity na, int64) and d_n (one
    int32, the number of pairs, ordered by target) are device pointers; the work is queued on
