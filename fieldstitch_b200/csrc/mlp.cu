@@ -12,9 +12,9 @@
 //                     2 log2(size_b / size_a), 3 signed angle difference / 180 (wrapped),
 //                     4 prior residual |pred_a - xy_b| / radius, 5 response_a, 6 response_b,
 //                     7 octave_a
-//   k_mlp_fwd_bwd     one mini-batch slice per block (128 samples): forward (ReLU, sigmoid),
-//                     mean binary cross-entropy gradient; activations and deltas staged in shared
-//                     memory, per-block partial gradients (fixed summation order)
+//   k_mlp_fwd_bwd     one mini-batch slice (128 samples) per cluster of 1, 2 or 4 blocks: forward (ReLU,
+//                     sigmoid), mean binary cross-entropy gradient; activations and deltas staged in
+//                     shared memory, partial gradients per slice (fixed summation order)
 //   k_mlp_adam        sums the partials in block order and applies one Adam step
 //   k_mlp_infer       inference, FP32 or BF16 (BF16 weights, inputs and hidden activations,
 //                     FP32 accumulation)
@@ -22,8 +22,8 @@
 //                     -> (target, distance) rows for the one-to-one filter
 //
 // Parameter vector (float32): W1[64][8], b1[64], W2[64][64], b2[64], w3[64], b3, then the input
-// normalisation mu[8], sigma[8] (not trained). An epoch (device-side shuffle + every step) is
-// captured once as a CUDA graph and replayed.
+// normalisation mu[8], sigma[8] (not trained).
+#include <cooperative_groups.h>
 #include <cub/cub.cuh>
 #include <cuda_bf16.h>
 
@@ -39,8 +39,9 @@ constexpr int NF = 8, H = 64;
 constexpr int OFF_W1 = 0, OFF_B1 = OFF_W1 + H * NF, OFF_W2 = OFF_B1 + H, OFF_B2 = OFF_W2 + H * H,
               OFF_W3 = OFF_B2 + H, OFF_B3 = OFF_W3 + H, N_TRAIN = OFF_B3 + 1, OFF_MU = N_TRAIN,
               OFF_SIG = OFF_MU + NF, N_PARAM = OFF_SIG + NF;
-constexpr int MB = 128;          // samples per block in k_mlp_fwd_bwd
-constexpr int HP = H + 1;        // padded row of the shared activation tiles
+constexpr int MB = 128;          // samples per slice (one partial gradient) of k_mlp_fwd_bwd
+constexpr int HP = H + 4;        // row of the shared activation tiles: 16-byte rows, banks shifted by 4
+constexpr int MT = 256;          // threads per block
 
 inline unsigned nblk(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
@@ -76,117 +77,374 @@ __global__ void k_mlp_features(int n, const int32_t* __restrict__ t1, const floa
 // ------------------------------------------------------------------------ training
 __device__ __forceinline__ float sigmoidf_(float z) { return 1.f / (1.f + __expf(-z)); }
 
-// Per-block partial gradient of mean BCE over `count` samples (sample = idx[base + s]); part has
-// N_TRAIN floats per block. loss_sum (nullable) accumulates the summed loss.
-__global__ void __launch_bounds__(MB) k_mlp_fwd_bwd(const float* __restrict__ prm, const float* __restrict__ feat,
+// acc[q][i] += sum over c = 0..63, in order, of W[c][i0 + i] * act[s_q][c] for NS samples s_q = s0 + 16 q
+// and four outputs (W rows of pitch WP, act rows of pitch HP; the chain of fused multiply-adds of
+// each output is one after another, so the blocking changes no rounding). Per four c: four 16-byte
+// loads of W, NS of the activations, 8 NS packed multiply-adds.
+template <int NS, int WP>
+__device__ __forceinline__ void mlp_tile(const float* __restrict__ W, const float* __restrict__ act, int s0, int i0,
+                                         float2 (&acc)[NS][2]) {
+#pragma unroll 2
+    for (int c = 0; c < H; c += 4) {
+        float4 w[4], h[NS];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) w[k] = *reinterpret_cast<const float4*>(W + (c + k) * WP + i0);
+#pragma unroll
+        for (int q = 0; q < NS; ++q) h[q] = *reinterpret_cast<const float4*>(act + (s0 + 16 * q) * HP + c);
+#pragma unroll
+        for (int q = 0; q < NS; ++q) {
+            const float hv[4] = {h[q].x, h[q].y, h[q].z, h[q].w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float2 hh = make_float2(hv[k], hv[k]);
+                acc[q][0] = __ffma2_rn(make_float2(w[k].x, w[k].y), hh, acc[q][0]);
+                acc[q][1] = __ffma2_rn(make_float2(w[k].z, w[k].w), hh, acc[q][1]);
+            }
+        }
+    }
+}
+
+// h1 rows of `n` samples from the normalised features: a = b1[i] + sum_k W1[i][k] x[k] in order, ReLU,
+// rounded to BF16 with BF16
+template <bool BF16>
+__device__ __forceinline__ float mlp_act(float a) {
+    a = fmaxf(a, 0.f);
+    return BF16 ? __bfloat162float(__float2bfloat16_rn(a)) : a;
+}
+// (W1T: [feature][output]); put(sample, first output, four values) stores
+template <bool BF16, class Put>
+__device__ __forceinline__ void mlp_h1(const float* __restrict__ W1T, const float* __restrict__ B1,
+                                       const float* __restrict__ X, int n, Put put) {
+    const int i0 = 4 * (threadIdx.x & 15);
+    const float4 b = *reinterpret_cast<const float4*>(B1 + i0);
+    float4 w[NF];
+#pragma unroll
+    for (int k = 0; k < NF; ++k) w[k] = *reinterpret_cast<const float4*>(W1T + k * H + i0);
+    for (int s = threadIdx.x >> 4; s < n; s += MT / 16) {
+        const float4 xa = *reinterpret_cast<const float4*>(X + s * NF), xb = *reinterpret_cast<const float4*>(X + s * NF + 4);
+        const float x[NF] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
+        float4 a = b;
+#pragma unroll
+        for (int k = 0; k < NF; ++k) {
+            a.x = fmaf(w[k].x, x[k], a.x);
+            a.y = fmaf(w[k].y, x[k], a.y);
+            a.z = fmaf(w[k].z, x[k], a.z);
+            a.w = fmaf(w[k].w, x[k], a.w);
+        }
+        put(s, i0, make_float4(mlp_act<BF16>(a.x), mlp_act<BF16>(a.y), mlp_act<BF16>(a.z), mlp_act<BF16>(a.w)));
+    }
+}
+// the weights in shared memory, W1 and W2 transposed (W2T rows of pitch HP); W2 too when wanted
+template <bool BF16, bool KEEP_W2>
+__device__ __forceinline__ void mlp_weights(const float* __restrict__ prm, float* __restrict__ W1T, float* __restrict__ B1,
+                                            float* __restrict__ W2, float* __restrict__ W2T, float* __restrict__ B2,
+                                            float* __restrict__ W3) {
+    auto wgt = [](float w) { return BF16 ? __bfloat162float(__float2bfloat16_rn(w)) : w; };
+    const int tid = threadIdx.x;
+    float t1[H * NF / MT], t2[H * H / MT], b[3] = {0.f, 0.f, 0.f};   // every load in flight at once
+#pragma unroll
+    for (int k = 0; k < H * NF / MT; ++k) t1[k] = prm[OFF_W1 + tid + k * MT];
+#pragma unroll
+    for (int k = 0; k < H * H / MT; ++k) t2[k] = prm[OFF_W2 + tid + k * MT];
+    if (tid < H) {
+        b[0] = prm[OFF_B1 + tid];
+        b[1] = prm[OFF_B2 + tid];
+        b[2] = prm[OFF_W3 + tid];
+    }
+#pragma unroll
+    for (int k = 0; k < H * NF / MT; ++k) {
+        const int i = tid + k * MT;
+        W1T[(i & (NF - 1)) * H + i / NF] = wgt(t1[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < H * H / MT; ++k) {
+        const int i = tid + k * MT;
+        if (KEEP_W2) W2[i] = t2[k];
+        W2T[(i & (H - 1)) * HP + (i >> 6)] = wgt(t2[k]);
+    }
+    if (tid < H) {
+        B1[tid] = b[0];
+        B2[tid] = b[1];
+        W3[tid] = wgt(b[2]);
+    }
+}
+// h2 = act(b2 + W2 h1) of 16 NS samples (W2T: [input][output], pitch HP)
+template <int NS, bool BF16, class Put>
+__device__ __forceinline__ void mlp_h2(const float* __restrict__ W2T, const float* __restrict__ B2,
+                                       const float* __restrict__ H1, Put put) {
+    const int s0 = threadIdx.x >> 4, i0 = 4 * (threadIdx.x & 15);
+    float2 acc[NS][2];
+    const float4 b = *reinterpret_cast<const float4*>(B2 + i0);
+#pragma unroll
+    for (int q = 0; q < NS; ++q) {
+        acc[q][0] = make_float2(b.x, b.y);
+        acc[q][1] = make_float2(b.z, b.w);
+    }
+    mlp_tile<NS, HP>(W2T, H1, s0, i0, acc);
+#pragma unroll
+    for (int q = 0; q < NS; ++q)
+        put(s0 + 16 * q, i0, make_float4(mlp_act<BF16>(acc[q][0].x), mlp_act<BF16>(acc[q][0].y),
+                                         mlp_act<BF16>(acc[q][1].x), mlp_act<BF16>(acc[q][1].y)));
+}
+// z = b3 + sum_i w3[i] h2[i], in order
+__device__ __forceinline__ float mlp_z(const float* __restrict__ W3, float b3, const float* __restrict__ h2) {
+    float z = b3;
+#pragma unroll
+    for (int i = 0; i < H; i += 4) {
+        const float4 w = *reinterpret_cast<const float4*>(W3 + i), h = *reinterpret_cast<const float4*>(h2 + i);
+        z = fmaf(w.x, h.x, z);
+        z = fmaf(w.y, h.y, z);
+        z = fmaf(w.z, h.z, z);
+        z = fmaf(w.w, h.w, z);
+    }
+    return z;
+}
+
+// Shared memory of a training block (floats): the weights, then every activation and delta of the
+// slice's 128 samples. A block of a cluster computes its own 128 / CS samples and stores what another
+// block's gradients need into that block's shared memory too.
+struct MlpSmem {
+    static constexpr int W1 = 0, B1 = W1 + H * NF, W2 = B1 + H, W2T = W2 + H * H, B2 = W2T + H * HP, W3 = B2 + H,
+                         X = W3 + H, H1 = X + MB * NF, H2 = H1 + MB * HP, D2 = H2 + MB * HP, D1 = D2 + MB * HP,
+                         DZ = D1 + MB * HP, LOSS = DZ + MB, ONE = LOSS + MB, END = ONE + 4;
+};
+
+// Partial gradient of mean BCE over one slice of 128 of `count` samples (sample = idx[base + s], the
+// identity when idx is null) per cluster of CS blocks; part has N_TRAIN floats per slice. loss_sum
+// (nullable) accumulates the summed loss. Block r of a cluster runs samples 128 r / CS .. of the
+// forward and backward passes, and once the blocks have exchanged activations and deltas, sums the
+// gradients of rows 64 r / CS .. of W1 and W2 (and their biases and w3) over the slice's samples in
+// order: every gradient is one chain over samples 0 .. 127 whatever CS is.
+// Bound by latency: a step of 8192 samples is 64 slices, 3.6 MFLOP each, on 148 SMs. One thread per
+// sample with two shared loads per multiply-add on 64 SMs took 82 us a step with its Adam update;
+// blocked tiles on clusters of two take 16 us (the launch, the weights and the Adam update 6 of them).
+template <int CS>
+__global__ void __launch_bounds__(MT) k_mlp_fwd_bwd(const float* __restrict__ prm, const float* __restrict__ feat,
                                                     const float* __restrict__ label,
                                                     const int32_t* __restrict__ idx, int base, int count,
                                                     float inv_batch, float* __restrict__ part,
                                                     double* __restrict__ loss_sum) {
-    extern __shared__ float sm[];
-    float* sW1 = sm;                       // H*NF
-    float* sB1 = sW1 + H * NF;             // H
-    float* sW2 = sB1 + H;                  // H*H
-    float* sB2 = sW2 + H * H;              // H
-    float* sW3 = sB2 + H;                  // H
-    float* sX = sW3 + H;                   // MB*NF
-    float* sH1 = sX + MB * NF;             // MB*HP
-    float* sH2 = sH1 + MB * HP;            // MB*HP
-    float* sD2 = sH2 + MB * HP;            // MB*HP
-    float* sD1 = sD2 + MB * HP;            // MB*HP
-    float* sDz = sD1 + MB * HP;            // MB
-    __shared__ float s_loss[MB / 32];
+    using S = MlpSmem;
+    constexpr int SPC = MB / CS, NS = SPC / 16;   // samples of this block; per thread of a 16 x 16 tile grid
+    constexpr int NI = H / CS;                    // gradient rows of this block
+    extern __shared__ __align__(16) float sm[];
     const int tid = threadIdx.x;
-    for (int i = tid; i < OFF_B3; i += MB) sm[i] = prm[i];
-    const float b3 = prm[OFF_B3];
+    const int rank = CS > 1 ? (int)(blockIdx.x % CS) : 0, slice = blockIdx.x / CS;
+    const int l0 = rank * SPC;                    // first sample of this block within the slice
+    // the samples do not depend on the step before: they load while it finishes
+    constexpr int XN = (SPC * NF + MT - 1) / MT;
+    float xr[XN], yr = 0.f;
+    cudaTriggerProgrammaticLaunchCompletion();
+#pragma unroll
+    for (int k = 0; k < XN; ++k) {
+        const int e = tid + k * MT, gi = slice * MB + l0 + e / NF;
+        xr[k] = 0.f;
+        if (e < SPC * NF && gi < count) xr[k] = feat[(size_t)(idx ? idx[base + gi] : base + gi) * NF + (e & (NF - 1))];
+    }
+    if (tid < SPC) {
+        const int gi = slice * MB + l0 + tid;
+        if (gi < count) yr = label[idx ? idx[base + gi] : base + gi];
+    }
+    cudaGridDependencySynchronize();   // the parameters of the step before (no-op without that launch attribute)
+    mlp_weights<false, true>(prm, sm + S::W1, sm + S::B1, sm + S::W2, sm + S::W2T, sm + S::B2, sm + S::W3);
+    const float mu = prm[OFF_MU + (tid & (NF - 1))], sig = prm[OFF_SIG + (tid & (NF - 1))], b3 = prm[OFF_B3];
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    float* peer[CS];   // the shared memory of the cluster's blocks, this one's included
+#pragma unroll
+    for (int r = 0; r < CS; ++r) peer[r] = CS > 1 ? cl.map_shared_rank(sm, r) : sm;
+    if constexpr (CS > 1) cl.sync();   // every block of the cluster runs: its shared memory may be written
+    if (tid == 0) sm[S::ONE] = 1.f;
+#pragma unroll
+    for (int k = 0; k < XN; ++k) {   // feature e % 8 = tid % 8
+        const int e = tid + k * MT, gi = slice * MB + l0 + e / NF;
+        if (e < SPC * NF) {
+            const float x = gi < count ? (xr[k] - mu) / sig : 0.f;
+#pragma unroll
+            for (int r = 0; r < CS; ++r) peer[r][S::X + l0 * NF + e] = x;
+        }
+    }
     __syncthreads();
-    const int s = tid;
-    const int gi = blockIdx.x * MB + s;
-    const bool live = gi < count;
-    float loss = 0.f;
-    {
-        float x[NF];
-        const int id = live ? idx[base + gi] : 0;
+    // h1 of every sample goes to every block; of h2, d2 and d1 each column to the block that sums its
+    // gradients
+    auto all = [&](int at, float4 v) {
 #pragma unroll
-        for (int k = 0; k < NF; ++k) {
-            x[k] = live ? (feat[(size_t)id * NF + k] - prm[OFF_MU + k]) / prm[OFF_SIG + k] : 0.f;
-            sX[s * NF + k] = x[k];
-        }
-        for (int i = 0; i < H; ++i) {
-            float a = sB1[i];
-#pragma unroll
-            for (int k = 0; k < NF; ++k) a = fmaf(sW1[i * NF + k], x[k], a);
-            sH1[s * HP + i] = fmaxf(a, 0.f);
-        }
-        float z = b3;
-        for (int i = 0; i < H; ++i) {
-            float a = sB2[i];
-            for (int j = 0; j < H; ++j) a = fmaf(sW2[i * H + j], sH1[s * HP + j], a);
-            a = fmaxf(a, 0.f);
-            sH2[s * HP + i] = a;
-            z = fmaf(sW3[i], a, z);
-        }
-        const float y = live ? label[id] : 0.f;
+        for (int r = 0; r < CS; ++r) *reinterpret_cast<float4*>(peer[r] + at) = v;
+    };
+    auto own = [&](int at, int col, float4 v) {
+        *reinterpret_cast<float4*>(sm + at) = v;
+        if (CS > 1 && col / NI != rank) *reinterpret_cast<float4*>(cl.map_shared_rank(sm, col / NI) + at) = v;
+    };
+    mlp_h1<false>(sm + S::W1, sm + S::B1, sm + S::X + l0 * NF, SPC,
+                  [&](int s, int i, float4 v) { all(S::H1 + (l0 + s) * HP + i, v); });
+    __syncthreads();
+    mlp_h2<NS, false>(sm + S::W2T, sm + S::B2, sm + S::H1 + l0 * HP,
+                      [&](int s, int i, float4 v) { own(S::H2 + (l0 + s) * HP + i, i, v); });
+    __syncthreads();
+    if (tid < SPC) {
+        const int s = l0 + tid, gi = slice * MB + s;
+        const bool live = gi < count;
+        const float z = mlp_z(sm + S::W3, b3, sm + S::H2 + s * HP);
+        const float y = yr;
         const float p = sigmoidf_(z);
         // BCE with logits: max(z, 0) - z y + log(1 + exp(-|z|))
-        loss = live ? fmaxf(z, 0.f) - z * y + log1pf(__expf(-fabsf(z))) : 0.f;
+        peer[0][S::LOSS + s] = live ? fmaxf(z, 0.f) - z * y + log1pf(__expf(-fabsf(z))) : 0.f;
         const float dz = live ? (p - y) * inv_batch : 0.f;
-        sDz[s] = dz;
-        for (int i = 0; i < H; ++i) sD2[s * HP + i] = sH2[s * HP + i] > 0.f ? dz * sW3[i] : 0.f;
-        for (int j = 0; j < H; ++j) {
-            float a = 0.f;
-            if (sH1[s * HP + j] > 0.f)
-                for (int i = 0; i < H; ++i) a = fmaf(sW2[i * H + j], sD2[s * HP + i], a);
-            sD1[s * HP + j] = a;
-        }
+#pragma unroll
+        for (int r = 0; r < CS; ++r) peer[r][S::DZ + s] = dz;
     }
-    for (int o = 16; o; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
-    if ((tid & 31) == 0) s_loss[tid >> 5] = loss;
     __syncthreads();
-    if (tid == 0 && loss_sum) {
-        float l = 0.f;
-        for (int w = 0; w < MB / 32; ++w) l += s_loss[w];
-        atomicAdd(loss_sum, (double)l);
+    for (int e = tid; e < SPC * (H / 4); e += MT) {
+        const int s = l0 + (e >> 4), i0 = 4 * (e & 15);
+        const float dz = sm[S::DZ + s];
+        const float4 h = *reinterpret_cast<const float4*>(sm + S::H2 + s * HP + i0);
+        const float4 w = *reinterpret_cast<const float4*>(sm + S::W3 + i0);
+        own(S::D2 + s * HP + i0, i0,
+            make_float4(h.x > 0.f ? dz * w.x : 0.f, h.y > 0.f ? dz * w.y : 0.f, h.z > 0.f ? dz * w.z : 0.f,
+                        h.w > 0.f ? dz * w.w : 0.f));
     }
-    // partial gradients, one output per thread and loop step, summed over the block's samples in order
-    float* out = part + (size_t)blockIdx.x * N_TRAIN;
-    for (int e = tid; e < N_TRAIN; e += MB) {
-        float g = 0.f;
-        if (e < OFF_B1) {                       // W1[i][k] = sum d1[s][i] x[s][k]
-            const int i = e / NF, k = e - i * NF;
-            for (int q = 0; q < MB; ++q) g = fmaf(sD1[q * HP + i], sX[q * NF + k], g);
-        } else if (e < OFF_W2) {                // b1[i]
-            const int i = e - OFF_B1;
-            for (int q = 0; q < MB; ++q) g += sD1[q * HP + i];
-        } else if (e < OFF_B2) {                // W2[i][j] = sum d2[s][i] h1[s][j]
-            const int r = e - OFF_W2, i = r / H, j = r - i * H;
-            for (int q = 0; q < MB; ++q) g = fmaf(sD2[q * HP + i], sH1[q * HP + j], g);
-        } else if (e < OFF_W3) {                // b2[i]
-            const int i = e - OFF_B2;
-            for (int q = 0; q < MB; ++q) g += sD2[q * HP + i];
-        } else if (e < OFF_B3) {                // w3[i] = sum dz[s] h2[s][i]
-            const int i = e - OFF_W3;
-            for (int q = 0; q < MB; ++q) g = fmaf(sDz[q], sH2[q * HP + i], g);
-        } else {                                // b3
-            for (int q = 0; q < MB; ++q) g += sDz[q];
+    __syncthreads();
+    {   // d1[s][j] = sum_i W2[i][j] d2[s][i] where h1[s][j] > 0
+        const int s0 = l0 + (tid >> 4), j0 = 4 * (tid & 15);
+        float2 acc[NS][2];
+#pragma unroll
+        for (int q = 0; q < NS; ++q) acc[q][0] = acc[q][1] = make_float2(0.f, 0.f);
+        mlp_tile<NS, H>(sm + S::W2, sm + S::D2, s0, j0, acc);
+#pragma unroll
+        for (int q = 0; q < NS; ++q) {
+            const float4 h = *reinterpret_cast<const float4*>(sm + S::H1 + (s0 + 16 * q) * HP + j0);
+            own(S::D1 + (s0 + 16 * q) * HP + j0, j0,
+                make_float4(h.x > 0.f ? acc[q][0].x : 0.f, h.y > 0.f ? acc[q][0].y : 0.f, h.z > 0.f ? acc[q][1].x : 0.f,
+                            h.w > 0.f ? acc[q][1].y : 0.f));
         }
-        out[e] = g;
+    }
+    if constexpr (CS > 1) cl.sync();   // every block's stores have landed; no remote access after this
+    else __syncthreads();
+    float* out = part + (size_t)slice * N_TRAIN;
+    const int ib = rank * NI;
+    if (tid < 128) {
+        // W2[i][j] = sum_s d2[s][i] h1[s][j], s in order: TI rows x four columns per thread
+        constexpr int TI = NI / 8;
+        const int i0 = ib + (tid >> 4) * TI, j0 = 4 * (tid & 15);
+        float2 g[TI][2];
+#pragma unroll
+        for (int i = 0; i < TI; ++i) g[i][0] = g[i][1] = make_float2(0.f, 0.f);
+#pragma unroll 4
+        for (int q = 0; q < MB; ++q) {
+            const float4 h = *reinterpret_cast<const float4*>(sm + S::H1 + q * HP + j0);
+            float d[TI];
+            const float* dp = sm + S::D2 + q * HP + i0;
+            if constexpr (TI % 4 == 0) {
+#pragma unroll
+                for (int i = 0; i < TI; i += 4) {
+                    const float4 v = *reinterpret_cast<const float4*>(dp + i);
+                    d[i] = v.x;
+                    d[i + 1] = v.y;
+                    d[i + 2] = v.z;
+                    d[i + 3] = v.w;
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < TI; ++i) d[i] = dp[i];
+            }
+#pragma unroll
+            for (int i = 0; i < TI; ++i) {
+                g[i][0] = __ffma2_rn(make_float2(d[i], d[i]), make_float2(h.x, h.y), g[i][0]);
+                g[i][1] = __ffma2_rn(make_float2(d[i], d[i]), make_float2(h.z, h.w), g[i][1]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < TI; ++i) {
+            float* o = out + OFF_W2 + (i0 + i) * H + j0;   // N_TRAIN is odd: no wide stores
+            o[0] = g[i][0].x;
+            o[1] = g[i][0].y;
+            o[2] = g[i][1].x;
+            o[3] = g[i][1].y;
+        }
+    } else {
+        // The others, all chains of a thread in one branch-free sweep (so that the loads of several
+        // samples are in flight): W1[i][k] = sum d1 x for KN features; and EX of b1 = sum 1 d1,
+        // b2 = sum 1 d2, w3 = sum dz h2, b3 = sum dz 1 (a multiply-add by one rounds like an addition).
+        constexpr int G = 128 / NI;                     // groups of NI threads
+        constexpr int KN = G >= NF ? 1 : NF / G, EX = G >= 4 ? 1 : 4 / G;
+        const int u = tid - 128, i = ib + u % NI, grp = u / NI, k0 = grp * KN;
+        const float *pa[EX], *pb[EX];
+        int sa[EX], sb[EX], what[EX];
+#pragma unroll
+        for (int x = 0; x < EX; ++x) {
+            what[x] = grp * EX + x;
+            pa[x] = pb[x] = sm + S::ONE;
+            sa[x] = sb[x] = 0;
+            if (what[x] == 0) pb[x] = sm + S::D1 + i;
+            if (what[x] == 1) pb[x] = sm + S::D2 + i;
+            if (what[x] == 2) pb[x] = sm + S::H2 + i;
+            if (what[x] <= 2) sb[x] = HP;
+            if (what[x] == 2 || what[x] == 3) {
+                pa[x] = sm + S::DZ;
+                sa[x] = 1;
+            }
+        }
+        const float* px = sm + S::X + min(k0, NF - KN);
+        const float* pd = sm + S::D1 + i;
+        float g[KN], ge[EX];
+#pragma unroll
+        for (int k = 0; k < KN; ++k) g[k] = 0.f;
+#pragma unroll
+        for (int x = 0; x < EX; ++x) ge[x] = 0.f;
+#pragma unroll 8
+        for (int q = 0; q < MB; ++q) {
+            const float d1 = pd[q * HP];
+#pragma unroll
+            for (int k = 0; k < KN; ++k) g[k] = fmaf(d1, px[q * NF + k], g[k]);
+#pragma unroll
+            for (int x = 0; x < EX; ++x) ge[x] = fmaf(pa[x][q * sa[x]], pb[x][q * sb[x]], ge[x]);
+        }
+        if (k0 < NF) {
+#pragma unroll
+            for (int k = 0; k < KN; ++k) out[OFF_W1 + i * NF + k0 + k] = g[k];
+        }
+#pragma unroll
+        for (int x = 0; x < EX; ++x) {
+            if (what[x] == 0) out[OFF_B1 + i] = ge[x];
+            if (what[x] == 1) out[OFF_B2 + i] = ge[x];
+            if (what[x] == 2) out[OFF_W3 + i] = ge[x];
+            if (what[x] == 3 && i == 0) out[OFF_B3] = ge[x];
+        }
+    }
+    if (loss_sum && rank == 0 && tid < 32) {
+        // sums of 32 samples by lane pairs, the four sums in order
+        float l = 0.f;
+        for (int w = 0; w < MB / 32; ++w) {
+            float v = sm[S::LOSS + 32 * w + tid];
+            for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            l += v;
+        }
+        if (tid == 0) atomicAdd(loss_sum, (double)l);
     }
 }
 
-// Sum of the partial gradients (block order) and one Adam step. step_ctr holds the number of
-// steps taken so far; k_mlp_step_done increments it after the update.
-__global__ void k_mlp_adam(float* __restrict__ prm, float* __restrict__ m, float* __restrict__ v,
-                           const float* __restrict__ part, int nparts, const int* __restrict__ step_ctr, float lr,
-                           float* __restrict__ grad_out) {
+// Sum of the partial gradients (slice order) and Adam step number t (from 1).
+constexpr int AT = 64;   // threads per block: 75 blocks for the 4 737 parameters
+__global__ void __launch_bounds__(AT) k_mlp_adam(float* __restrict__ prm, float* __restrict__ m, float* __restrict__ v,
+                                                 const float* __restrict__ part, int nparts,
+                                                 int t, float lr, float* __restrict__ grad_out) {
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= N_TRAIN) return;
     float g = 0.f;
-    for (int b = 0; b < nparts; ++b) g += part[(size_t)b * N_TRAIN + e];
+    int b = 0;
+    for (; b + 32 <= nparts; b += 32) {   // 32 loads in flight, added in order
+        float p[32];
+#pragma unroll
+        for (int k = 0; k < 32; ++k) p[k] = part[(size_t)(b + k) * N_TRAIN + e];
+#pragma unroll
+        for (int k = 0; k < 32; ++k) g += p[k];
+    }
+    for (; b < nparts; ++b) g += part[(size_t)b * N_TRAIN + e];
     if (grad_out) grad_out[e] = g;
     if (!m) return;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    const int t = *step_ctr + 1;
     const float mm = b1 * m[e] + (1.f - b1) * g;
     const float vv = b2 * v[e] + (1.f - b2) * g * g;
     m[e] = mm;
@@ -195,14 +453,12 @@ __global__ void k_mlp_adam(float* __restrict__ prm, float* __restrict__ m, float
     prm[e] -= lr * mh / (sqrtf(vh) + eps);
 }
 
-__global__ void k_mlp_step_done(int* step_ctr) { ++*step_ctr; }
-
-__global__ void k_mlp_perm_keys(int n, const int* __restrict__ epoch_ctr, uint32_t seed, uint32_t* __restrict__ key,
+__global__ void k_mlp_perm_keys(int n, int epoch, uint32_t seed, uint32_t* __restrict__ key,
                                 int32_t* __restrict__ val) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     // splitmix-style 32-bit hash of (seed, epoch, i)
-    uint32_t h = seed ^ (0x9E3779B9u * (uint32_t)(*epoch_ctr + 1)) ^ (0x85EBCA6Bu * (uint32_t)i);
+    uint32_t h = seed ^ (0x9E3779B9u * (uint32_t)(epoch + 1)) ^ (0x85EBCA6Bu * (uint32_t)i);
     h ^= h >> 16;
     h *= 0x7FEB352Du;
     h ^= h >> 15;
@@ -212,47 +468,47 @@ __global__ void k_mlp_perm_keys(int n, const int* __restrict__ epoch_ctr, uint32
     val[i] = i;
 }
 
-__global__ void k_mlp_epoch_done(int* epoch_ctr) { ++*epoch_ctr; }
-
 // ------------------------------------------------------------------------ inference
 __device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
+// Inference of 128 samples per block and step (blocks walk the samples): the training pass's tiles, so
+// every pre-activation is the same chain of multiply-adds. Bound by the multiply-adds (4 672 a sample);
+// one thread per sample with a shared load per multiply-add took 223 us for 390 000 samples, the
+// tiles take 100 us.
+struct InferSmem {
+    static constexpr int W1 = 0, B1 = W1 + H * NF, W2T = B1 + H, B2 = W2T + H * HP, W3 = B2 + H, X = W3 + H,
+                         H1 = X + MB * NF, H2 = H1 + MB * HP, END = H2 + MB * HP;
+};
 template <bool BF16>
-__global__ void __launch_bounds__(256) k_mlp_infer(const float* __restrict__ prm, int n, const float* __restrict__ feat,
-                                                   float* __restrict__ prob) {
-    __shared__ float sW[OFF_B3 + 1];
-    for (int i = threadIdx.x; i <= OFF_B3; i += blockDim.x) {
-        const bool weight = i < OFF_B1 || (i >= OFF_W2 && i < OFF_B2) || (i >= OFF_W3 && i < OFF_B3);
-        sW[i] = BF16 && weight ? bf16r(prm[i]) : prm[i];
-    }
-    __syncthreads();
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n) return;
-    float x[NF];
+__global__ void __launch_bounds__(MT, 2) k_mlp_infer(const float* __restrict__ prm, int n, const float* __restrict__ feat,
+                                                     float* __restrict__ prob) {
+    using S = InferSmem;
+    extern __shared__ __align__(16) float sm[];
+    const int tid = threadIdx.x;
+    mlp_weights<BF16, false>(prm, sm + S::W1, sm + S::B1, nullptr, sm + S::W2T, sm + S::B2, sm + S::W3);
+    const float b3 = prm[OFF_B3];
+    const float mu = prm[OFF_MU + (tid & 7)], sig = prm[OFF_SIG + (tid & 7)];
+    const int tiles = (n + MB - 1) / MB;
+    for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const int base = t * MB;
+        __syncthreads();   // the previous tile's rows are done (first pass: the weights)
 #pragma unroll
-    for (int k = 0; k < NF; ++k) {
-        x[k] = (feat[(size_t)s * NF + k] - prm[OFF_MU + k]) / prm[OFF_SIG + k];
-        if (BF16) x[k] = bf16r(x[k]);
+        for (int e = tid; e < MB * NF; e += MT) {   // k = e % 8 = tid % 8
+            float x = 0.f;
+            if (base + (e >> 3) < n) x = (feat[(size_t)base * NF + e] - mu) / sig;
+            sm[S::X + e] = BF16 ? bf16r(x) : x;
+        }
+        __syncthreads();
+        mlp_h1<BF16>(sm + S::W1, sm + S::B1, sm + S::X, MB, [&](int s, int i, float4 v) {
+            *reinterpret_cast<float4*>(sm + S::H1 + s * HP + i) = v;
+        });
+        __syncthreads();
+        mlp_h2<MB / 16, BF16>(sm + S::W2T, sm + S::B2, sm + S::H1, [&](int s, int i, float4 v) {
+            *reinterpret_cast<float4*>(sm + S::H2 + s * HP + i) = v;
+        });
+        __syncthreads();
+        if (tid < MB && base + tid < n) prob[base + tid] = sigmoidf_(mlp_z(sm + S::W3, b3, sm + S::H2 + tid * HP));
     }
-    float h1[H];
-#pragma unroll
-    for (int i = 0; i < H; ++i) {
-        float a = sW[OFF_B1 + i];
-#pragma unroll
-        for (int k = 0; k < NF; ++k) a = fmaf(sW[OFF_W1 + i * NF + k], x[k], a);
-        a = fmaxf(a, 0.f);
-        h1[i] = BF16 ? bf16r(a) : a;
-    }
-    float z = sW[OFF_B3];
-    for (int i = 0; i < H; ++i) {
-        float a = sW[OFF_B2 + i];
-#pragma unroll
-        for (int j = 0; j < H; ++j) a = fmaf(sW[OFF_W2 + i * H + j], h1[j], a);
-        a = fmaxf(a, 0.f);
-        if (BF16) a = bf16r(a);
-        z = fmaf(sW[OFF_W3 + i], a, z);
-    }
-    prob[s] = sigmoidf_(z);
 }
 
 __global__ void k_mlp_accept(int n, const int32_t* __restrict__ t1, const float* __restrict__ b12,
@@ -273,11 +529,68 @@ __global__ void k_mlp_accept(int n, const int32_t* __restrict__ t1, const float*
     d_row[i] = ok ? (uint32_t)b12[2 * i] : 0u;
 }
 
-size_t fwd_bwd_smem() { return sizeof(float) * (size_t)(OFF_B3 + MB * NF + 4 * MB * HP + MB); }
-
-int32_t configure_fwd_bwd() {
+template <int CS>
+int32_t launch_fwd_bwd_t(int slices, const float* prm, const float* feat, const float* label, const int32_t* idx, int base,
+                         int count, float inv_batch, float* part, double* loss, bool overlap, cudaStream_t s) {
     static std::atomic<int> done[64];
-    return smem_attr((const void*)k_mlp_fwd_bwd, (int)fwd_bwd_smem(), done);
+    constexpr int bytes = MlpSmem::END * 4;
+    FSB_TRY(smem_attr((const void*)k_mlp_fwd_bwd<CS>, bytes, done));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)slices * CS);
+    cfg.blockDim = dim3(MT);
+    cfg.dynamicSmemBytes = bytes;
+    cfg.stream = s;
+    cudaLaunchAttribute at[2];
+    int na = 0;
+    if (CS > 1) {
+        at[na].id = cudaLaunchAttributeClusterDimension;
+        at[na].val.clusterDim.x = CS;
+        at[na].val.clusterDim.y = 1;
+        at[na++].val.clusterDim.z = 1;
+    }
+    if (overlap) {
+        at[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[na++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = na;
+    FSB_CUDA(cudaLaunchKernelEx(&cfg, k_mlp_fwd_bwd<CS>, prm, feat, label, idx, base, count, inv_batch, part, loss));
+    note_launch();
+    return FSB_OK;
+}
+// blocks per slice: as many as keep every slice resident at once (one block per SM), at most four
+// (clusters of eight such blocks find few places: 55 us a step of 2048 against 13 with four).
+// overlap: the launch may start while the kernel before it (an Adam step, which nothing but the
+// parameters and the partials of this kernel depend on) is running
+int32_t launch_fwd_bwd(int slices, const float* prm, const float* feat, const float* label, const int32_t* idx, int base,
+                       int count, float inv_batch, float* part, double* loss, bool overlap, cudaStream_t s) {
+    auto* f = slices * 4 <= 128 ? launch_fwd_bwd_t<4> : slices * 2 <= 140 ? launch_fwd_bwd_t<2> : launch_fwd_bwd_t<1>;
+    return f(slices, prm, feat, label, idx, base, count, inv_batch, part, loss, overlap, s);
+}
+int32_t launch_adam(float* prm, float* m, float* v, const float* part, int nparts, int t, float lr, float* grad,
+                    cudaStream_t s) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(nblk(N_TRAIN, AT));
+    cfg.blockDim = dim3(AT);
+    cfg.stream = s;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    FSB_CUDA(cudaLaunchKernelEx(&cfg, k_mlp_adam, prm, m, v, part, nparts, t, lr, grad));
+    note_launch();
+    return FSB_OK;
+}
+template <bool BF16>
+int32_t launch_infer(const float* prm, int n, const float* feat, float* prob, cudaStream_t s) {
+    static std::atomic<int> done[64];
+    constexpr int bytes = InferSmem::END * 4;
+    FSB_TRY(smem_attr((const void*)k_mlp_infer<BF16>, bytes, done));
+    k_mlp_infer<BF16><<<std::min(nblk(n, MB), 2u * 148u), MT, bytes, s>>>(prm, n, feat, prob);
+    note_launch();
+    FSB_CUDA(cudaGetLastError());
+    return FSB_OK;
 }
 
 }  // namespace
@@ -299,11 +612,7 @@ int32_t run_mlp_features(int n, const int32_t* t1, const float* b12, const doubl
 
 int32_t run_mlp_infer(const float* prm, int n, const float* feat, bool bf16, float* prob, cudaStream_t s) {
     if (n <= 0) return FSB_OK;
-    if (bf16) k_mlp_infer<true><<<nblk(n, 256), 256, 0, s>>>(prm, n, feat, prob);
-    else k_mlp_infer<false><<<nblk(n, 256), 256, 0, s>>>(prm, n, feat, prob);
-    note_launch();
-    FSB_CUDA(cudaGetLastError());
-    return FSB_OK;
+    return bf16 ? launch_infer<true>(prm, n, feat, prob, s) : launch_infer<false>(prm, n, feat, prob, s);
 }
 
 int32_t run_mlp_accept(int n, const int32_t* t1, const float* b12, const float* prob, float thr, float ratio,
@@ -318,21 +627,15 @@ int32_t run_mlp_accept(int n, const int32_t* t1, const float* b12, const float* 
 // Mean-BCE gradient over samples idx[0..n) (identity when idx is null) into grad (N_TRAIN floats).
 int32_t run_mlp_grad(fsb_ctx* ctx, const float* prm, int n, const float* feat, const float* label, float* grad,
                      double* loss, cudaStream_t s) {
-    FSB_TRY(configure_fwd_bwd());
     const int nb = (int)nblk(n, MB);
     auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
-    FSB_TRY(ctx->s_misc.ensure(al((size_t)nb * N_TRAIN * 4) + al((size_t)n * 4) + al(64)));
+    FSB_TRY(ctx->s_misc.ensure(al((size_t)nb * N_TRAIN * 4) + al(64)));
     uint8_t* base = ctx->s_misc.as<uint8_t>();
     float* part = reinterpret_cast<float*>(base);
-    int32_t* idx = reinterpret_cast<int32_t*>(base + al((size_t)nb * N_TRAIN * 4));
-    double* dl = reinterpret_cast<double*>(base + al((size_t)nb * N_TRAIN * 4) + al((size_t)n * 4));
-    std::vector<int32_t> iota(n);
-    for (int i = 0; i < n; ++i) iota[i] = i;
-    FSB_CUDA(cudaMemcpyAsync(idx, iota.data(), (size_t)n * 4, cudaMemcpyHostToDevice, s));
+    double* dl = reinterpret_cast<double*>(base + al((size_t)nb * N_TRAIN * 4));
     FSB_CUDA(cudaMemsetAsync(dl, 0, 8, s));
-    k_mlp_fwd_bwd<<<nb, MB, fwd_bwd_smem(), s>>>(prm, feat, label, idx, 0, n, 1.f / (float)n, part, dl);
-    k_mlp_adam<<<nblk(N_TRAIN, 256), 256, 0, s>>>(nullptr, nullptr, nullptr, part, nb, nullptr, 0.f, grad);
-    note_launch(2);
+    FSB_TRY(launch_fwd_bwd(nb, prm, feat, label, nullptr, 0, n, 1.f / (float)n, part, dl, false, s));
+    FSB_TRY(launch_adam(nullptr, nullptr, nullptr, part, nb, 0, 0.f, grad, s));
     FSB_CUDA(cudaGetLastError());
     double h = 0.0;
     FSB_CUDA(cudaMemcpyAsync(&h, dl, 8, cudaMemcpyDeviceToHost, s));
@@ -343,11 +646,11 @@ int32_t run_mlp_grad(fsb_ctx* ctx, const float* prm, int n, const float* feat, c
 
 // Mini-batch Adam over n samples for `epochs` epochs. prm (N_PARAM), m, v (N_TRAIN) in device memory.
 // Each epoch: shuffle (hash keys + radix sort), then floor(n / batch) steps (one step of n when
-// n < batch). The epoch is captured once as a CUDA graph and replayed. losses (host, nullable,
-// `epochs` entries) receives the mean training loss of every epoch.
+// n < batch). Two launches a step, queued without a host wait until the end; each may start while the
+// one before it drains (the samples of a step load during the Adam step before it). losses (host,
+// nullable, `epochs` entries) receives the mean training loss of every epoch.
 int32_t run_mlp_train(fsb_ctx* ctx, float* prm, float* m, float* v, int n, const float* feat, const float* label,
                       int epochs, int batch, float lr, uint32_t seed, double* losses, cudaStream_t s) {
-    FSB_TRY(configure_fwd_bwd());
     batch = std::max(MB, (batch / MB) * MB);
     const int bsz = n < batch ? n : batch;
     const int steps = n < batch ? 1 : n / batch;
@@ -356,7 +659,8 @@ int32_t run_mlp_train(fsb_ctx* ctx, float* prm, float* m, float* v, int n, const
     cub::DeviceRadixSort::SortPairs(nullptr, tb, (uint32_t*)nullptr, (uint32_t*)nullptr, (int32_t*)nullptr,
                                     (int32_t*)nullptr, n, 0, 32, s);
     auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
-    const size_t need = al((size_t)nb * N_TRAIN * 4) + 4 * al((size_t)n * 4) + al(tb) + 2 * al(64);
+    if (epochs < 0) epochs = 0;
+    const size_t need = al((size_t)nb * N_TRAIN * 4) + 4 * al((size_t)n * 4) + al(tb) + al((size_t)epochs * 8 + 8);
     FSB_TRY(ctx->s_misc.ensure(need));
     uint8_t* cur = ctx->s_misc.as<uint8_t>();
     auto take = [&](size_t bytes) {
@@ -370,62 +674,27 @@ int32_t run_mlp_train(fsb_ctx* ctx, float* prm, float* m, float* v, int n, const
     int32_t* vals = reinterpret_cast<int32_t*>(take((size_t)n * 4));
     int32_t* perm = reinterpret_cast<int32_t*>(take((size_t)n * 4));
     void* tmp = take(tb);
-    int* ctr = reinterpret_cast<int*>(take(64));      // [0] steps, [1] epochs
-    double* dl = reinterpret_cast<double*>(take(64));
-    FSB_CUDA(cudaMemsetAsync(ctr, 0, 64, s));
-    FSB_CUDA(cudaMemsetAsync(dl, 0, 64, s));
+    double* dl = reinterpret_cast<double*>(take((size_t)epochs * 8 + 8));   // loss sums of the epochs
+    FSB_CUDA(cudaMemsetAsync(dl, 0, (size_t)epochs * 8 + 8, s));
     FSB_CUDA(cudaMemsetAsync(m, 0, (size_t)N_TRAIN * 4, s));
     FSB_CUDA(cudaMemsetAsync(v, 0, (size_t)N_TRAIN * 4, s));
+    for (int e = 0; e < epochs; ++e) {
+        k_mlp_perm_keys<<<nblk(n, 256), 256, 0, s>>>(n, e, seed, keys, vals);
+        size_t tbe = tb;
+        FSB_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tbe, keys, keys2, vals, perm, n, 0, 32, s));
+        note_launch(2);
+        for (int st = 0; st < steps; ++st) {
+            FSB_TRY(launch_fwd_bwd(nb, prm, feat, label, perm, st * bsz, bsz, 1.f / (float)bsz, part, dl + e, st > 0, s));
+            FSB_TRY(launch_adam(prm, m, v, part, nb, e * steps + st + 1, lr, nullptr, s));
+        }
+    }
+    FSB_CUDA(cudaGetLastError());
+    std::vector<double> h(epochs > 0 ? epochs : 1, 0.0);
+    if (losses && epochs > 0)
+        FSB_CUDA(cudaMemcpyAsync(h.data(), dl, (size_t)epochs * 8, cudaMemcpyDeviceToHost, s));
     FSB_CUDA(cudaStreamSynchronize(s));
-    // capture one epoch
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    FSB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    k_mlp_perm_keys<<<nblk(n, 256), 256, 0, s>>>(n, ctr + 1, seed, keys, vals);
-    cub::DeviceRadixSort::SortPairs(tmp, tb, keys, keys2, vals, perm, n, 0, 32, s);
-    for (int st = 0; st < steps; ++st) {
-        k_mlp_fwd_bwd<<<nb, MB, fwd_bwd_smem(), s>>>(prm, feat, label, perm, st * bsz, bsz, 1.f / (float)bsz, part, dl);
-        k_mlp_adam<<<nblk(N_TRAIN, 256), 256, 0, s>>>(prm, m, v, part, nb, ctr, lr, nullptr);
-        k_mlp_step_done<<<1, 1, 0, s>>>(ctr);
-    }
-    k_mlp_epoch_done<<<1, 1, 0, s>>>(ctr + 1);
-    cudaError_t ce = cudaStreamEndCapture(s, &graph);
-    if (ce != cudaSuccess) {
-        set_error("graph capture of the training epoch failed: %s", cudaGetErrorString(ce));
-        return FSB_ERR_CUDA;
-    }
-    ce = cudaGraphInstantiate(&exec, graph, 0);
-    if (ce != cudaSuccess) {
-        cudaGraphDestroy(graph);
-        set_error("graph instantiation failed: %s", cudaGetErrorString(ce));
-        return FSB_ERR_CUDA;
-    }
-    int32_t rc = FSB_OK;
-    for (int e = 0; e < epochs && rc == FSB_OK; ++e) {
-        if (cudaMemsetAsync(dl, 0, 8, s) != cudaSuccess || cudaGraphLaunch(exec, s) != cudaSuccess) {
-            set_error("training epoch launch failed: %s", cudaGetErrorString(cudaGetLastError()));
-            rc = FSB_ERR_CUDA;
-            break;
-        }
-        note_launch(3 * steps + 3);
-        if (losses) {
-            double h = 0.0;
-            cudaMemcpyAsync(&h, dl, 8, cudaMemcpyDeviceToHost, s);
-            if (cudaStreamSynchronize(s) != cudaSuccess) {
-                set_error("training epoch failed: %s", cudaGetErrorString(cudaGetLastError()));
-                rc = FSB_ERR_CUDA;
-                break;
-            }
-            losses[e] = h / ((double)steps * bsz);
-        }
-    }
-    if (rc == FSB_OK && cudaStreamSynchronize(s) != cudaSuccess) {
-        set_error("training failed: %s", cudaGetErrorString(cudaGetLastError()));
-        rc = FSB_ERR_CUDA;
-    }
-    cudaGraphExecDestroy(exec);
-    cudaGraphDestroy(graph);
-    return rc;
+    for (int e = 0; losses && e < epochs; ++e) losses[e] = h[e] / ((double)steps * bsz);
+    return FSB_OK;
 }
 
 }  // namespace fsb

@@ -4,8 +4,8 @@ PlaneSite accepts a query's best guided candidate by the ratio test (matching._g
 app/planesite/matching.py:142-146) and then verifies the accepted set with a RANSAC homography
 (matching.py:205-233). Here an 8-64-64-1 MLP scores every query's best candidate from 8 features
 (ratio, best distance, log2 scale ratio, angle difference, prior residual, both responses,
-octave); it is trained on the GPU (libfsb200's own forward/backward/Adam kernels, one CUDA graph
-per epoch) on labels that the plain pipeline produces by its own verification: a candidate is an
+octave); it is trained on the GPU (libfsb200's own forward/backward/Adam kernels, every step queued
+without a host wait) on labels that the plain pipeline produces by its own verification: a candidate is an
 inlier when the RANSAC homography fitted to the plain pipeline's matches maps it within 2 px.
 The plain ratio test stays the fallback (``MatchFilter.matches`` without a trained network) and
 the yardstick of the filter's precision and recall (``score``).

@@ -272,7 +272,7 @@ int32_t fsb_mlp_features_d(fsb_ctx* ctx, int32_t n, const int32_t* d_t1, const f
 int32_t fsb_mlp_grad_d(fsb_ctx* ctx, const float* d_params, int32_t n, const float* d_feat,
                        const float* d_label, float* d_grad, double* loss);
 /* Mini-batch Adam (beta 0.9 / 0.999) on the GPU: each epoch shuffles the samples on the device
-   (seeded) and takes floor(n / batch) steps; the epoch runs as one captured CUDA graph. d_m, d_v:
+   (seeded) and takes floor(n / batch) steps, queued without a host wait until the end. d_m, d_v:
    Adam moments (trainable count each, reset here). losses (host, nullable) receives the mean
    loss of each of the `epochs` epochs. */
 int32_t fsb_mlp_train_d(fsb_ctx* ctx, float* d_params, float* d_m, float* d_v, int32_t n,
