@@ -516,8 +516,6 @@ int32_t fsb_destroy(fsb_ctx* ctx) {
                      &ctx->s_u64, &ctx->s_misc, &ctx->s_misc2, &ctx->s_host_stage, &ctx->s_cub,
                      &ctx->s_tc_pack, &ctx->s_tc_part, &ctx->s_tc_aux, &ctx->s_count, &ctx->s_gb};
     for (DevBuf* b : all) b->release();
-    if (ctx->gb_graph.exec) cudaGraphExecDestroy(ctx->gb_graph.exec);
-    if (ctx->gb_graph.graph) cudaGraphDestroy(ctx->gb_graph.graph);
     {
         auto& x = ctx->xb;
         for (cudaStream_t cs : x.streams) cudaStreamSynchronize(cs);
@@ -1221,10 +1219,9 @@ int32_t fsb_match_guided_d(fsb_ctx* ctx, const double* d_pred, const uint8_t* d_
     FSB_TRY(ctx->s_count.ensure(64));
     int* dn = ctx->s_count.as<int>();
     ctx->stage_begin(ST_MATCH);
-    FSB_TRY(run_match_guided(ctx, d_pred, d_a, na, d_bxy, d_b, nb, w_b, h_b, radius, kc, ratio, d_q, d_t, dn, s));
     int n = 0;
-    FSB_CUDA(cudaMemcpyAsync(&n, dn, sizeof(int), cudaMemcpyDeviceToHost, s));
-    FSB_CUDA(cudaStreamSynchronize(s));
+    FSB_TRY(run_match_guided_batch(ctx, 1, &d_pred, &d_a, &na, &d_bxy, &d_b, &nb, &w_b, &h_b, radius, kc, ratio, &d_q,
+                                   &d_t, dn, &n, s));
     ctx->stage_end(ST_MATCH);
     *n_out = n;
     return FSB_OK;
@@ -1321,9 +1318,13 @@ int32_t fsb_match_guided_cand_d(fsb_ctx* ctx, const double* d_pred, const uint8_
     FSB_TRY(use_device(ctx));
     cudaStream_t s = ctx->stream;
     ctx->stage_begin(ST_MATCH);
-    FSB_TRY(run_match_guided(ctx, d_pred, d_a, na, d_bxy, d_b, nb, w_b, h_b, radius, kc, 1.f, nullptr, nullptr,
-                             nullptr, s, d_t1, d_b12));
-    FSB_CUDA(cudaStreamSynchronize(s));
+    if (nb < 1 || !(radius > 0.0)) {   // no candidates
+        FSB_CUDA(cudaMemsetAsync(d_t1, 0xff, (size_t)na * 4, s));
+        FSB_CUDA(cudaStreamSynchronize(s));
+    } else {
+        FSB_TRY(run_match_guided_batch(ctx, 1, &d_pred, &d_a, &na, &d_bxy, &d_b, &nb, &w_b, &h_b, radius, kc, 1.f,
+                                       nullptr, nullptr, nullptr, nullptr, s, d_t1, d_b12));
+    }
     ctx->stage_end(ST_MATCH);
     return FSB_OK;
 }
@@ -1369,11 +1370,9 @@ int32_t fsb_match_guided_batch_d(fsb_ctx* ctx, int32_t n_pairs, const double* co
     FSB_TRY(ctx->s_count.ensure(L * 4 + 64));
     int32_t* dn = ctx->s_count.as<int32_t>();
     ctx->stage_begin(ST_MATCH);
+    std::vector<int32_t> cnt(L, 0);
     FSB_TRY(run_match_guided_batch(ctx, (int)L, pr.data(), pa.data(), ra.data(), bx.data(), pb.data(), rb.data(),
-                                   wv.data(), hv.data(), radius, kc, ratio, pq.data(), pt.data(), dn, s));
-    std::vector<int> cnt(L, 0);
-    FSB_CUDA(cudaMemcpyAsync(cnt.data(), dn, L * 4, cudaMemcpyDeviceToHost, s));
-    FSB_CUDA(cudaStreamSynchronize(s));
+                                   wv.data(), hv.data(), radius, kc, ratio, pq.data(), pt.data(), dn, cnt.data(), s));
     ctx->stage_end(ST_MATCH);
     for (size_t i = 0; i < L; ++i) n_out[live[i]] = cnt[i];
     return FSB_OK;
@@ -1534,11 +1533,11 @@ int32_t fsb_match_guided(fsb_ctx* ctx, const double* pred_xy, const uint8_t* a, 
     int64_t* dt = dq + na;
     FSB_TRY(ctx->s_count.ensure(64));
     int* dn = ctx->s_count.as<int>();
-    FSB_TRY(run_match_guided(ctx, dp, ctx->s_u8a.as<uint8_t>(), na, dbx, ctx->s_u8b.as<uint8_t>(), nb, w_b, h_b, radius,
-                             kc, ratio, dq, dt, dn, s));
+    const uint8_t *da = ctx->s_u8a.as<uint8_t>(), *db = ctx->s_u8b.as<uint8_t>();
+    const double *dpc = dp, *dbc = dbx;
     int n = 0;
-    FSB_CUDA(cudaMemcpyAsync(&n, dn, sizeof(int), cudaMemcpyDeviceToHost, s));
-    FSB_CUDA(cudaStreamSynchronize(s));
+    FSB_TRY(run_match_guided_batch(ctx, 1, &dpc, &da, &na, &dbc, &db, &nb, &w_b, &h_b, radius, kc, ratio, &dq, &dt, dn,
+                                   &n, s));
     const HostCopy out[2] = {{q, dq, (size_t)n * 8}, {t, dt, (size_t)n * 8}};
     FSB_TRY(copy_out(ctx, out, n ? 2 : 0));
     *n_out = n;

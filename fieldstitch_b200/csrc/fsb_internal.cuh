@@ -129,8 +129,8 @@ struct TcStats {
     float mean_abs_err = 0.f;      // and its mean
 };
 
-// A captured guided-batch graph and the exact inputs it was captured for.
-struct GuidedGraph {
+// A captured batch graph and the exact inputs it was captured for.
+struct BatchGraph {
     std::vector<char> key;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -172,8 +172,7 @@ struct fsb_ctx {
     fsb::DevBuf s_cub;   // CUB temporary storage (one primitive at a time)
     fsb::DevBuf s_tc_pack, s_tc_part, s_tc_aux;   // tensor-core matcher: packed operands, candidates, tables
     fsb::DevBuf s_count;   // result counts of the API calls; never grown by the internal stages
-    fsb::DevBuf s_gb;      // guided batch scratch (addresses captured in gb_graph)
-    fsb::GuidedGraph gb_graph;
+    fsb::DevBuf s_gb;      // guided matching scratch
     fsb::TcStats tc_stats{};                      // of the last tensor-core dense match
     // sync-free batched extraction (fsb_sift_features_batch_d): chains of images, each with its own
     // stream and workspace, captured as one CUDA graph and replayed while the call is unchanged
@@ -185,8 +184,8 @@ struct fsb_ctx {
         cudaStream_t upload = nullptr;            // host-image batches: the uploads, in image order
         std::vector<cudaEvent_t> uploaded;        // image i on the device (captured edges)
         std::vector<cudaGraphNode_t> copy_nodes;  // the upload of image i in the captured graph
-        fsb::GuidedGraph graph;
-        fsb::GuidedGraph pyr_graph;   // fsb_pyramid_batch_d
+        fsb::BatchGraph graph;
+        fsb::BatchGraph pyr_graph;   // fsb_pyramid_batch_d
         int pyr_h = 0, pyr_w = 0;     // geometry whose pyramid ran once outside a capture (autotuned)
         fsb::DevBuf status;
         fsb::AsyncCaps caps{};
@@ -278,15 +277,13 @@ int32_t run_match_bf(fsb_ctx* ctx, const uint8_t* d_a, int na, const uint8_t* d_
 int32_t run_match_bf_batch(fsb_ctx* ctx, int n, const uint8_t* const* d_a, const int* na, const uint8_t* const* d_b,
                            const int* nb, float ratio, int64_t* const* d_q, int64_t* const* d_t, int32_t* counts,
                            cudaStream_t s);
-// d_n null: candidates only (c_t, c_b12: best target or -1, b1, b2 per query; no ratio test, no _unique)
-int32_t run_match_guided(fsb_ctx* ctx, const double* d_pred, const uint8_t* d_a, int na, const double* d_bxy,
-                         const uint8_t* d_b, int nb, double wb, double hb, double radius, int kc, float ratio,
-                         int64_t* d_q, int64_t* d_t, int* d_n, cudaStream_t s, int32_t* c_t = nullptr,
-                         float* c_b12 = nullptr);
+// guided matching of a batch (na, nb >= 1, radius > 0), waits; c_t, c_b12 (one pair): the best target or -1
+// and b1, b2 per query instead of matches
 int32_t run_match_guided_batch(fsb_ctx* ctx, int n_pairs, const double* const* d_pred, const uint8_t* const* d_a,
                                const int* na, const double* const* d_bxy, const uint8_t* const* d_b, const int* nb,
                                const double* wb, const double* hb, double radius, int kc, float ratio,
-                               int64_t* const* d_q, int64_t* const* d_t, int32_t* counts, cudaStream_t s);
+                               int64_t* const* d_q, int64_t* const* d_t, int32_t* d_n, int32_t* h_counts, cudaStream_t s,
+                               int32_t* c_t = nullptr, float* c_b12 = nullptr);
 int32_t run_unique_rows(fsb_ctx* ctx, const int32_t* t_row, const uint32_t* d_row, int na, int nb, int64_t* d_q,
                         int64_t* d_t, int* d_n, cudaStream_t s);
 // mlp.cu

@@ -4,8 +4,8 @@
 //                 32-bit integer distances (the plain path of matching._ratio_match_bf,
 //                 app/planesite/matching.py:86-100)
 //   k_bf_merge    merge of the per-split top-2, float32 ratio test, one-to-one keys
-//   k_guided      prior-guided candidates within a radius on a uniform grid, exact integer
-//                 distances (matching._guided, app/planesite/matching.py:113-152)
+//   k_gb_*        prior-guided candidates within a radius on a uniform grid, exact integer
+//                 distances (matching._guided, app/planesite/matching.py:113-152), one pair or a batch
 //   k_unique      one match per target: atomicMin on (distance << 32 | query) keys
 //                 (matching._unique, app/planesite/matching.py:103-110), then target-ordered
 //                 compaction
@@ -25,17 +25,6 @@ namespace fsb {
 namespace {
 
 inline unsigned blocks(long long n, int t) { return (unsigned)((n + t - 1) / t); }
-
-// squared L2 norm of each uint8 row (exact integer)
-__global__ void k_norms(const uint8_t* __restrict__ d, int n, int32_t* __restrict__ out) {
-    const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (row >= n) return;
-    const uint32_t w = reinterpret_cast<const uint32_t*>(d + (size_t)row * 128)[lane];
-    int s = (int)__dp4a(w, w, 0u);
-    for (int sh = 16; sh; sh >>= 1) s += __shfl_xor_sync(0xffffffffu, s, sh);
-    if (lane == 0) out[row] = s;
-}
 
 // ------------------------------------------------------------------------- dense tiles
 constexpr int BN = 128;            // target rows per tile
@@ -394,181 +383,240 @@ __device__ __forceinline__ int cell_of(double v, double o, double cs, int n) {
     return f < 0.0 ? 0 : (f >= (double)(n - 1) ? n - 1 : (int)f);
 }
 
-__global__ void k_grid_count(const double* __restrict__ bxy, int nb, GridSpec gs, int32_t* __restrict__ cell,
-                             int32_t* __restrict__ count) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nb) return;
-    const int cx = cell_of(bxy[2 * i], gs.x0, gs.cs, gs.gw), cy = cell_of(bxy[2 * i + 1], gs.y0, gs.cs, gs.gh);
-    const int c = cy * gs.gw + cx;
-    cell[i] = c;
+constexpr int G_WARPS = 4, G_CAND = 512;
+constexpr int G_QUERIES = 16;   // queries of a block (four per warp)
+
+// One pair of a guided batch (an array in device memory, or one by value).
+struct GPair {
+    const double* pred;
+    const uint8_t* a;
+    const double* bxy;
+    const uint8_t* b;
+    int na, nb;
+    double wb, hb;
+    GridSpec gs;
+    int cell0;   // first cell of this pair's grid
+    int item0;   // first target (B row) in the concatenated target arrays
+    int64_t* q_out;
+    int64_t* t_out;
+    int32_t* n_out;
+};
+
+__global__ void k_gb_count(const __grid_constant__ GPair one, const GPair* __restrict__ tab, int32_t* __restrict__ cell,
+                           int32_t* __restrict__ count) {
+    const GPair& P = tab ? tab[blockIdx.y] : one;
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= P.nb) return;
+    const int cx = cell_of(P.bxy[2 * j], P.gs.x0, P.gs.cs, P.gs.gw), cy = cell_of(P.bxy[2 * j + 1], P.gs.y0, P.gs.cs, P.gs.gh);
+    const int c = P.cell0 + cy * P.gs.gw + cx;
+    cell[P.item0 + j] = c;
     atomicAdd(count + c, 1);
 }
 
-__global__ void k_grid_fill(const int32_t* __restrict__ cell, int nb, const int32_t* __restrict__ start,
-                            int32_t* __restrict__ cursor, int32_t* __restrict__ items) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nb) return;
-    const int c = cell[i];
-    items[start[c] + atomicAdd(cursor + c, 1)] = i;
+// targets in cell order: index and position
+__global__ void k_gb_fill(const __grid_constant__ GPair one, const GPair* __restrict__ tab, const int32_t* __restrict__ cell,
+                          const int32_t* __restrict__ start, int32_t* __restrict__ cursor, int32_t* __restrict__ items,
+                          double2* __restrict__ pos) {
+    const GPair& P = tab ? tab[blockIdx.y] : one;
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= P.nb) return;
+    const int c = cell[P.item0 + j];
+    const int at = start[c] + atomicAdd(cursor + c, 1);
+    items[at] = j;   // local target index
+    pos[at] = make_double2(P.bxy[2 * j], P.bxy[2 * j + 1]);
 }
 
-constexpr int G_WARPS = 4, G_CAND = 512;
-
-__device__ __forceinline__ int exact_d2(const uint32_t* __restrict__ qa, const uint8_t* __restrict__ B, int j,
-                                        int qn, const int32_t* __restrict__ nB) {
-    const uint4* pb = reinterpret_cast<const uint4*>(B + (size_t)j * 128);
-    unsigned dot = 0;
-#pragma unroll
-    for (int v = 0; v < 8; ++v) {
-        const uint4 w = __ldg(pb + v);
-        dot = __dp4a(qa[4 * v + 0], w.x, dot);
-        dot = __dp4a(qa[4 * v + 1], w.y, dot);
-        dot = __dp4a(qa[4 * v + 2], w.z, dot);
-        dot = __dp4a(qa[4 * v + 3], w.w, dot);
+__device__ __forceinline__ void top2_push_tie(Top2& t, float d, int j) {   // equal distances: smaller index
+    if (d < t.b1 || (d == t.b1 && j < t.i1)) {
+        t.b2 = t.b1;
+        t.b1 = d;
+        t.i1 = j;
+    } else if (d < t.b2) {
+        t.b2 = d;
     }
-    return (qn + nB[j]) - 2 * (int)dot;
 }
 
-// One query of the guided matcher (one warp): candidates of the prior window, exact distances,
-// top-2, ratio test; writes t_row/d_row (nullable) and the pre-ratio candidate (c_t, nullable).
-__device__ __forceinline__ void guided_query(int q, const double* __restrict__ pred, const uint8_t* __restrict__ A,
-                                             int na, const double* __restrict__ bxy,
-                                             const uint8_t* __restrict__ B, int nb,
-                                             const int32_t* __restrict__ nA, const int32_t* __restrict__ nB,
-                                             GridSpec gs, const int32_t* __restrict__ start,
-                                             const int32_t* __restrict__ items, double wb, double hb,
-                                             double radius, int kc, float ratio,
-                                             int32_t* __restrict__ t_row, uint32_t* __restrict__ d_row,
-                                             int32_t* __restrict__ c_t, float* __restrict__ c_b12,
-                                             int* __restrict__ overflow, uint32_t (*s_q)[32],
-                                             double (*s_cd)[G_CAND], int32_t (*s_ci)[G_CAND]) {
-    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (q >= na) return;
-    const double px = pred[2 * q], py = pred[2 * q + 1];
-    int32_t res_t = -1;
-    uint32_t res_d = 0;
-    int32_t cand_t = -1;
-    float cand_b1 = INFINITY, cand_b2 = INFINITY;
-    const bool inside = px > -radius && px < wb + radius && py > -radius && py < hb + radius;
-    if (inside) {
-        s_q[wid][lane] = reinterpret_cast<const uint32_t*>(A + (size_t)q * 128)[lane];
-        __syncwarp();
-        uint32_t qa[32];
+// exact squared distances of the query row (16-byte segment a4 of this lane, squared norm qn) to the m
+// targets of `list`, into this lane's top-2: eight lanes per target, one 16-byte load each, and
+// |b|^2 - 2 a.b summed over the eight; eight targets in flight
+__device__ __forceinline__ void guided_distances(const uint4& a4, int qn, const uint8_t* __restrict__ B,
+                                                 const int32_t* list, int m, Top2& best) {
+    const int lane = threadIdx.x & 31, seg = lane & 7, g = lane >> 3;
+    for (int c0 = 0; c0 < m; c0 += 8) {
+        int j[2], v[2];
+        uint4 b[2];
 #pragma unroll
-        for (int v = 0; v < 32; ++v) qa[v] = s_q[wid][v];
-        const int qn = nA[q];
-        const double r2 = radius * radius;
-        const int cx = cell_of(px, gs.x0, gs.cs, gs.gw), cy = cell_of(py, gs.y0, gs.cs, gs.gh);
-        Top2 best{INFINITY, INFINITY, -1};
-        if (kc <= 0) {
-            // every B keypoint strictly within the radius is a candidate
-            for (int yy = max(cy - 1, 0); yy <= min(cy + 1, gs.gh - 1); ++yy)
-                for (int xx = max(cx - 1, 0); xx <= min(cx + 1, gs.gw - 1); ++xx) {
-                    const int c = yy * gs.gw + xx;
-                    const int s0 = start[c], s1 = start[c + 1];
-                    for (int p = s0 + lane; p < s1; p += 32) {
-                        const int j = items[p];
-                        const double dx = __dsub_rn(bxy[2 * j], px), dy = __dsub_rn(bxy[2 * j + 1], py);
-                        const double d2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
-                        if (d2 < r2) top2_push(best, (float)exact_d2(qa, B, j, qn, nB), j);
-                    }
-                }
-        } else {
-            // collect candidates (spatial distance, index) in shared memory
-            int cnt = 0;
-            for (int yy = max(cy - 1, 0); yy <= min(cy + 1, gs.gh - 1); ++yy)
-                for (int xx = max(cx - 1, 0); xx <= min(cx + 1, gs.gw - 1); ++xx) {
-                    const int c = yy * gs.gw + xx;
-                    const int s0 = start[c], s1 = start[c + 1];
-                    for (int p0 = s0; p0 < s1; p0 += 32) {
-                        const int p = p0 + lane;
-                        bool hit = false;
-                        double d2 = 0.0;
-                        int j = 0;
-                        if (p < s1) {
-                            j = items[p];
-                            const double dx = __dsub_rn(bxy[2 * j], px), dy = __dsub_rn(bxy[2 * j + 1], py);
-                            d2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
-                            hit = d2 < r2;
-                        }
-                        const unsigned m = __ballot_sync(0xffffffffu, hit);
-                        if (hit) {
-                            const int pos = cnt + __popc(m & ((1u << lane) - 1u));
-                            if (pos < G_CAND) {
-                                s_cd[wid][pos] = d2;
-                                s_ci[wid][pos] = j;
-                            }
-                        }
-                        cnt += __popc(m);
-                    }
-                }
-            __syncwarp();
-            if (cnt > G_CAND) {
-                if (lane == 0) atomicExch(overflow, 1);
-                cnt = G_CAND;
-            }
-            // keep the kc nearest (ties: smaller B index)
-            for (int e = lane; e < cnt; e += 32) {
-                const double de = s_cd[wid][e];
-                const int ie = s_ci[wid][e];
-                int rank = 0;
-                if (cnt > kc)
-                    for (int f = 0; f < cnt; ++f) {
-                        const double df = s_cd[wid][f];
-                        rank += (df < de || (df == de && s_ci[wid][f] < ie)) ? 1 : 0;
-                    }
-                if (rank < kc) top2_push(best, (float)exact_d2(qa, B, ie, qn, nB), ie);
-            }
+        for (int u = 0; u < 2; ++u) {
+            j[u] = list[min(c0 + 4 * u + g, m - 1)];
+            b[u] = __ldg(reinterpret_cast<const uint4*>(B + (size_t)j[u] * 128) + seg);
         }
-        // warp merge of the per-lane top-2
 #pragma unroll
-        for (int sh = 16; sh; sh >>= 1) {
-            Top2 o;
-            o.b1 = __shfl_xor_sync(0xffffffffu, best.b1, sh);
-            o.b2 = __shfl_xor_sync(0xffffffffu, best.b2, sh);
-            o.i1 = __shfl_xor_sync(0xffffffffu, best.i1, sh);
-            best = top2_merge(best, o);
-        }
-        cand_t = best.i1;
-        cand_b1 = best.b1;
-        cand_b2 = best.b2;
-        if (best.i1 >= 0) {
-            // single candidate: b2 = inf passes (app/planesite/matching.py:142-146)
-            const bool ok = __fsqrt_rn(best.b1) < __fmul_rn(ratio, __fsqrt_rn(best.b2));
-            if (ok) {
-                res_t = best.i1;
-                res_d = (uint32_t)best.b1;
-            }
-        }
-    }
-    if (lane == 0) {
-        if (t_row) {
-            t_row[q] = res_t;
-            d_row[q] = res_d;
-        }
-        if (c_t) {   // the best candidate before the ratio test (learned filter input)
-            c_t[q] = cand_t;
-            c_b12[2 * q] = cand_b1;
-            c_b12[2 * q + 1] = cand_b2;
+        for (int u = 0; u < 2; ++u) {
+            unsigned ab = __dp4a(a4.x, b[u].x, 0u), bb = __dp4a(b[u].x, b[u].x, 0u);
+            ab = __dp4a(a4.y, b[u].y, ab);
+            bb = __dp4a(b[u].y, b[u].y, bb);
+            ab = __dp4a(a4.z, b[u].z, ab);
+            bb = __dp4a(b[u].z, b[u].z, bb);
+            ab = __dp4a(a4.w, b[u].w, ab);
+            bb = __dp4a(b[u].w, b[u].w, bb);
+            v[u] = (int)bb - 2 * (int)ab;
+#pragma unroll
+            for (int sh = 1; sh < 8; sh <<= 1) v[u] += __shfl_xor_sync(0xffffffffu, v[u], sh);
+            if (c0 + 4 * u + g < m) top2_push_tie(best, (float)(qn + v[u]), j[u]);
         }
     }
 }
 
-__global__ void __launch_bounds__(G_WARPS * 32) k_guided(const double* __restrict__ pred, const uint8_t* __restrict__ A,
-                                                         int na, const double* __restrict__ bxy,
-                                                         const uint8_t* __restrict__ B, int nb,
-                                                         const int32_t* __restrict__ nA, const int32_t* __restrict__ nB,
-                                                         GridSpec gs, const int32_t* __restrict__ start,
-                                                         const int32_t* __restrict__ items, double wb, double hb,
-                                                         double radius, int kc, float ratio,
-                                                         int32_t* __restrict__ t_row, uint32_t* __restrict__ d_row,
-                                                         int32_t* __restrict__ c_t, float* __restrict__ c_b12,
-                                                         int* __restrict__ overflow) {
-    __shared__ uint32_t s_q[G_WARPS][32];
+// Guided matcher, one warp per query: the candidates of the prior window, exact distances, top-2, ratio
+// test and the one-to-one key of the target; or (c_t set) the best candidate before the ratio test.
+// The three grid rows of the window are three contiguous runs of the cell-ordered targets, so the
+// window is one list read 32 positions at a time (about 25 at 9000 targets of a 2640 x 1978 frame and
+// a radius of 40) instead of nine cells one after another, and a candidate's row is one coalesced
+// 128-byte read instead of eight strided ones.
+// Bound by the latency of the dependent reads (cell starts, positions, rows). 64 pairs of 2000-16000
+// features: 1219 us with nine cells and a lane per candidate (plus 188 us for norms), GB_TIMES now.
+__global__ void __launch_bounds__(G_WARPS * 32) k_gb_guided(const __grid_constant__ GPair one, const GPair* __restrict__ tab,
+                                                            const int32_t* __restrict__ start,
+                                                            const int32_t* __restrict__ items,
+                                                            const double2* __restrict__ pos, double radius, int kc,
+                                                            float ratio, unsigned long long* __restrict__ key,
+                                                            int32_t* __restrict__ c_t, float* __restrict__ c_b12,
+                                                            int* __restrict__ overflow) {
     __shared__ double s_cd[G_WARPS][G_CAND];
     __shared__ int32_t s_ci[G_WARPS][G_CAND];
-    guided_query(blockIdx.x * G_WARPS + (threadIdx.x >> 5), pred, A, na, bxy, B, nb, nA, nB, gs, start, items, wb, hb,
-                 radius, kc, ratio, t_row, d_row, c_t, c_b12, overflow, s_q, s_cd, s_ci);
+    const GPair& P = tab ? tab[blockIdx.y] : one;
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, seg = lane & 7;
+    double* cd = s_cd[wid];
+    int32_t* ci = s_ci[wid];
+    const unsigned lt = (1u << lane) - 1u;
+    const bool wide = (reinterpret_cast<uintptr_t>(P.a) & 15) == 0;
+    const int q1 = min(P.na, (int)(blockIdx.x + 1) * G_QUERIES);
+    for (int q = blockIdx.x * G_QUERIES + wid; q < q1; q += G_WARPS) {
+        const double px = P.pred[2 * (size_t)q], py = P.pred[2 * (size_t)q + 1];
+        Top2 best{INFINITY, INFINITY, -1};
+        if (px > -radius && px < P.wb + radius && py > -radius && py < P.hb + radius) {
+            uint4 a4;
+            const uint8_t* ar = P.a + (size_t)q * 128 + seg * 16;
+            if (wide) {
+                a4 = __ldg(reinterpret_cast<const uint4*>(ar));
+            } else {
+                const uint32_t* aw = reinterpret_cast<const uint32_t*>(ar);
+                a4 = make_uint4(__ldg(aw), __ldg(aw + 1), __ldg(aw + 2), __ldg(aw + 3));
+            }
+            const int cx = cell_of(px, P.gs.x0, P.gs.cs, P.gs.gw), cy = cell_of(py, P.gs.y0, P.gs.cs, P.gs.gh);
+            // lane r < 3: the run of grid row cy - 1 + r
+            int s0 = 0, len = 0;
+            const int yy = cy - 1 + lane;
+            if (lane < 3 && yy >= 0 && yy < P.gs.gh) {
+                const int32_t* row = start + P.cell0 + yy * P.gs.gw;
+                s0 = row[max(cx - 1, 0)];
+                len = row[min(cx + 1, P.gs.gw - 1) + 1] - s0;
+            }
+            const int l0 = __shfl_sync(0xffffffffu, len, 0), l1 = __shfl_sync(0xffffffffu, len, 1);
+            const int l2 = __shfl_sync(0xffffffffu, len, 2);
+            // slot of the window's e-th target: e + the offset of its run
+            const int o0 = __shfl_sync(0xffffffffu, s0, 0), o1 = __shfl_sync(0xffffffffu, s0, 1) - l0;
+            const int o2 = __shfl_sync(0xffffffffu, s0, 2) - l0 - l1;
+            const int n = l0 + l1 + l2;
+            unsigned qn = __dp4a(a4.x, a4.x, 0u);
+            qn = __dp4a(a4.y, a4.y, qn);
+            qn = __dp4a(a4.z, a4.z, qn);
+            qn = __dp4a(a4.w, a4.w, qn);
+#pragma unroll
+            for (int sh = 1; sh < 8; sh <<= 1) qn += __shfl_xor_sync(0xffffffffu, qn, sh);
+            const double r2 = radius * radius;
+            int cnt = 0;
+            for (int e0 = 0; e0 < n; e0 += 32) {
+                const int e = e0 + lane;
+                bool hit = false;
+                double d2 = 0.0;
+                int j = 0;
+                if (e < n) {
+                    const int at = e + (e < l0 ? o0 : e < l0 + l1 ? o1 : o2);
+                    j = __ldg(items + at);
+                    const double2 p = __ldg(pos + at);
+                    const double dx = __dsub_rn(p.x, px), dy = __dsub_rn(p.y, py);
+                    d2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
+                    hit = d2 < r2;
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, hit);
+                if (hit) {
+                    const int at = cnt + __popc(m & lt);
+                    if (at < G_CAND) {
+                        cd[at] = d2;
+                        ci[at] = j;
+                    }
+                }
+                cnt += __popc(m);
+                if (kc <= 0) {   // every target strictly within the radius: no list to keep
+                    __syncwarp();
+                    guided_distances(a4, (int)qn, P.b, ci, cnt, best);
+                    __syncwarp();
+                    cnt = 0;
+                }
+            }
+            __syncwarp();
+            if (kc > 0) {
+                if (cnt > G_CAND) {
+                    if (lane == 0) atomicExch(overflow, 1);
+                    cnt = G_CAND;
+                }
+                if (cnt > kc) {
+                    // keep the kc nearest (ties: smaller B index): bit c of `keep` is entry 32 c + lane
+                    unsigned keep = 0;
+                    for (int e = lane, c = 0; e < cnt; e += 32, ++c) {
+                        const double de = cd[e];
+                        const int ie = ci[e];
+                        int rank = 0;
+                        for (int f = 0; f < cnt; ++f) {
+                            const double df = cd[f];
+                            rank += (df < de || (df == de && ci[f] < ie)) ? 1 : 0;
+                        }
+                        if (rank < kc) keep |= 1u << c;
+                    }
+                    __syncwarp();
+                    int kept = 0;
+                    for (int e0 = 0, c = 0; e0 < cnt; e0 += 32, ++c) {
+                        const bool k = keep >> c & 1u;
+                        const int j = k ? ci[e0 + lane] : 0;
+                        const unsigned m = __ballot_sync(0xffffffffu, k);
+                        if (k) ci[kept + __popc(m & lt)] = j;   // at or before its own entry
+                        kept += __popc(m);
+                        __syncwarp();
+                    }
+                    cnt = kept;
+                }
+                if (cnt > 0) guided_distances(a4, (int)qn, P.b, ci, cnt, best);
+                __syncwarp();
+            }
+            // merge the four groups' top-2
+#pragma unroll
+            for (int sh = 8; sh < 32; sh <<= 1) {
+                Top2 o;
+                o.b1 = __shfl_xor_sync(0xffffffffu, best.b1, sh);
+                o.b2 = __shfl_xor_sync(0xffffffffu, best.b2, sh);
+                o.i1 = __shfl_xor_sync(0xffffffffu, best.i1, sh);
+                best = top2_merge(best, o);
+            }
+        }
+        if (lane == 0) {
+            if (c_t) {   // the best candidate before the ratio test (learned filter input)
+                c_t[q] = best.i1;
+                c_b12[2 * (size_t)q] = best.b1;
+                c_b12[2 * (size_t)q + 1] = best.b2;
+            } else if (best.i1 >= 0 && __fsqrt_rn(best.b1) < __fmul_rn(ratio, __fsqrt_rn(best.b2))) {
+                // single candidate: b2 = inf passes (app/planesite/matching.py:142-146)
+                atomicMin(key + P.item0 + best.i1, ((unsigned long long)(uint32_t)best.b1 << 32) | (unsigned)q);
+            }
+        }
+    }
+}
+
+// matches of each pair ordered by target: a block per pair
+__global__ void __launch_bounds__(COMPACT_T) k_gb_compact(const __grid_constant__ GPair one, const GPair* __restrict__ tab,
+                                                          const unsigned long long* __restrict__ key) {
+    const GPair& P = tab ? tab[blockIdx.x] : one;
+    unique_compact(key + P.item0, P.nb, P.q_out, P.t_out, P.n_out);
 }
 
 __global__ void k_perspective(const double* __restrict__ xy, int n, const double* __restrict__ hm,
@@ -656,105 +704,6 @@ __global__ void k_uq_emit(const uint32_t* __restrict__ pos, const int* __restric
     to[i] = t[pos[i]];
 }
 
-
-// ------------------------------------------------------------------------------ guided batch
-// Many guided problems in one set of launches (blockIdx.y = pair): concatenated norms, one grid
-// per pair in one concatenated cell array (one prefix sum for all), one guided kernel over every
-// query of every pair, and _unique per pair over concatenated target keys.
-struct GPair {
-    const double* pred;
-    const uint8_t* a;
-    const double* bxy;
-    const uint8_t* b;
-    int na, nb;
-    double wb, hb;
-    GridSpec gs;
-    int cell0;   // first cell of this pair's grid
-    int item0;   // first target (B row) in the concatenated target arrays
-    int row0;    // first query (A row) in the concatenated query arrays
-    int64_t* q_out;
-    int64_t* t_out;
-};
-
-__global__ void k_gb_norms(const GPair* __restrict__ pairs, int which, int32_t* __restrict__ out) {
-    const GPair& P = pairs[blockIdx.y];
-    const int n = which ? P.nb : P.na;
-    const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (row >= n) return;
-    const uint8_t* d = which ? P.b : P.a;
-    const uint32_t w = reinterpret_cast<const uint32_t*>(d + (size_t)row * 128)[lane];
-    int s = (int)__dp4a(w, w, 0u);
-    for (int sh = 16; sh; sh >>= 1) s += __shfl_xor_sync(0xffffffffu, s, sh);
-    if (lane == 0) out[(which ? P.item0 : P.row0) + row] = s;
-}
-
-__global__ void k_gb_count(const GPair* __restrict__ pairs, int32_t* __restrict__ cell, int32_t* __restrict__ count) {
-    const GPair& P = pairs[blockIdx.y];
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= P.nb) return;
-    const int cx = cell_of(P.bxy[2 * j], P.gs.x0, P.gs.cs, P.gs.gw), cy = cell_of(P.bxy[2 * j + 1], P.gs.y0, P.gs.cs, P.gs.gh);
-    const int c = P.cell0 + cy * P.gs.gw + cx;
-    cell[P.item0 + j] = c;
-    atomicAdd(count + c, 1);
-}
-
-__global__ void k_gb_fill(const GPair* __restrict__ pairs, const int32_t* __restrict__ cell,
-                          const int32_t* __restrict__ start, int32_t* __restrict__ cursor, int32_t* __restrict__ items) {
-    const GPair& P = pairs[blockIdx.y];
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= P.nb) return;
-    const int c = cell[P.item0 + j];
-    items[start[c] + atomicAdd(cursor + c, 1)] = j;   // local target index
-}
-
-__global__ void __launch_bounds__(G_WARPS * 32) k_gb_guided(const GPair* __restrict__ pairs, const int32_t* __restrict__ nA,
-                                                            const int32_t* __restrict__ nB,
-                                                            const int32_t* __restrict__ start,
-                                                            const int32_t* __restrict__ items, double radius, int kc,
-                                                            float ratio, int32_t* __restrict__ t_row,
-                                                            uint32_t* __restrict__ d_row, int* __restrict__ overflow) {
-    __shared__ uint32_t s_q[G_WARPS][32];
-    __shared__ double s_cd[G_WARPS][G_CAND];
-    __shared__ int32_t s_ci[G_WARPS][G_CAND];
-    const GPair& P = pairs[blockIdx.y];
-    guided_query(blockIdx.x * G_WARPS + (threadIdx.x >> 5), P.pred, P.a, P.na, P.bxy, P.b, P.nb, nA + P.row0,
-                 nB + P.item0, P.gs, start + P.cell0, items, P.wb, P.hb, radius, kc, ratio, t_row + P.row0,
-                 d_row + P.row0, nullptr, nullptr, overflow, s_q, s_cd, s_ci);
-}
-
-__global__ void k_gb_fill_keys(unsigned long long* __restrict__ key, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) key[i] = ~0ull;
-}
-
-__global__ void k_gb_keys(const GPair* __restrict__ pairs, const int32_t* __restrict__ t_row,
-                          const uint32_t* __restrict__ d_row, unsigned long long* __restrict__ key) {
-    const GPair& P = pairs[blockIdx.y];
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= P.na) return;
-    const int t = t_row[P.row0 + q];
-    if (t >= 0) atomicMin(key + P.item0 + t, ((unsigned long long)d_row[P.row0 + q] << 32) | (unsigned)q);
-}
-
-__global__ void k_gb_flags(const unsigned long long* __restrict__ key, int n, int32_t* __restrict__ flag) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i <= n) flag[i] = i < n && key[i] != ~0ull;
-}
-
-__global__ void k_gb_emit(const GPair* __restrict__ pairs, const unsigned long long* __restrict__ key,
-                          const int32_t* __restrict__ pos, int32_t* __restrict__ counts) {
-    const GPair& P = pairs[blockIdx.y];
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= P.nb) return;
-    const int i = P.item0 + j;
-    if (j == P.nb - 1) counts[blockIdx.y] = pos[P.item0 + P.nb] - pos[P.item0];
-    const unsigned long long k = key[i];
-    if (k == ~0ull) return;
-    const int o = pos[i] - pos[P.item0];
-    P.q_out[o] = (int64_t)(k & 0xffffffffull);
-    P.t_out[o] = j;
-}
 
 }  // namespace
 
@@ -909,73 +858,14 @@ int32_t run_unique_rows(fsb_ctx* ctx, const int32_t* t_row, const uint32_t* d_ro
     return run_unique(ctx, t_row, d_row, na, nb, d_q, d_t, d_n, s);
 }
 
-int32_t run_match_guided(fsb_ctx* ctx, const double* d_pred, const uint8_t* d_a, int na, const double* d_bxy,
-                         const uint8_t* d_b, int nb, double wb, double hb, double radius, int kc, float ratio,
-                         int64_t* d_q, int64_t* d_t, int* d_n, cudaStream_t s, int32_t* c_t, float* c_b12) {
-    if (na < 1 || nb < 1 || !(radius > 0.0)) {
-        if (d_n) FSB_CUDA(cudaMemsetAsync(d_n, 0, sizeof(int), s));
-        if (c_t && na > 0) FSB_CUDA(cudaMemsetAsync(c_t, 0xff, (size_t)na * 4, s));
-        return FSB_OK;
-    }
-    GridSpec gs;
-    gs.x0 = 0.0;
-    gs.y0 = 0.0;
-    gs.cs = radius;
-    double gwd = (wb > 0 ? wb : 1.0) / radius + 1.0, ghd = (hb > 0 ? hb : 1.0) / radius + 1.0;
-    while (gwd * ghd > 4.0e6) {
-        gs.cs *= 2.0;
-        gwd = (wb > 0 ? wb : 1.0) / gs.cs + 1.0;
-        ghd = (hb > 0 ? hb : 1.0) / gs.cs + 1.0;
-    }
-    gs.gw = (int)gwd;
-    gs.gh = (int)ghd;
-    const int ncell = gs.gw * gs.gh;
-    FSB_TRY(ctx->s_i32.ensure((size_t)(na + nb) * 4 + (size_t)na * 8 + (size_t)nb * 8 + (size_t)ncell * 12 + 256));
-    int32_t* nA = ctx->s_i32.as<int32_t>();
-    int32_t* nB = nA + na;
-    int32_t* t_row = nB + nb;
-    uint32_t* d_row = reinterpret_cast<uint32_t*>(t_row + na);
-    int32_t* cell = reinterpret_cast<int32_t*>(d_row + na);
-    int32_t* items = cell + nb;
-    int32_t* count = items + nb;      // ncell + 1
-    int32_t* start = count + ncell + 1;
-    int32_t* cursor = start + ncell + 1;
-    int* overflow = cursor + ncell;
-    FSB_CUDA(cudaMemsetAsync(count, 0, (size_t)(ncell + 1) * 4, s));
-    FSB_CUDA(cudaMemsetAsync(cursor, 0, (size_t)ncell * 4 + 4, s));
-    k_norms<<<blocks(na, 8), 256, 0, s>>>(d_a, na, nA);
-    k_norms<<<blocks(nb, 8), 256, 0, s>>>(d_b, nb, nB);
-    k_grid_count<<<blocks(nb, 256), 256, 0, s>>>(d_bxy, nb, gs, cell, count);
-    size_t tb = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, tb, count, start, ncell + 1, s);
-    FSB_TRY(ctx->s_cub.ensure(tb + 16));
-    FSB_CUDA(cub::DeviceScan::ExclusiveSum(ctx->s_cub.p, tb, count, start, ncell + 1, s));
-    k_grid_fill<<<blocks(nb, 256), 256, 0, s>>>(cell, nb, start, cursor, items);
-    note_launch(5);
-    k_guided<<<blocks(na, G_WARPS), G_WARPS * 32, 0, s>>>(d_pred, d_a, na, d_bxy, d_b, nb, nA, nB, gs, start, items,
-                                                          wb, hb, radius, kc, ratio, d_n ? t_row : nullptr,
-                                                          d_row, c_t, c_b12, overflow);
-    FSB_CUDA(cudaGetLastError());
-    int h_over = 0;
-    FSB_CUDA(cudaMemcpyAsync(&h_over, overflow, sizeof(int), cudaMemcpyDeviceToHost, s));
-    FSB_CUDA(cudaStreamSynchronize(s));
-    if (h_over) {
-        set_error("more than %d B keypoints within the radius of one prediction (kc mode)", G_CAND);
-        return FSB_ERR_OVERFLOW;
-    }
-    if (!d_n) return FSB_OK;   // candidates only
-    return run_unique(ctx, t_row, d_row, na, nb, d_q, d_t, d_n, s);
-}
-
-
-// Guided matching of a batch of pairs (each na, nb >= 1, radius > 0) with _unique, as one CUDA
-// graph on the context's stream: captured on the first call with a given pair table and replayed
-// while the table (pointers, sizes, frames) and the scratch addresses stay the same. counts:
-// device, one per pair.
+// Guided matching of a batch of pairs (each na, nb >= 1, radius > 0) with _unique in one set of
+// launches: h_counts (host) receives the match count of each pair; the call waits. With c_t / c_b12
+// (one pair only) the candidates before the ratio test are written instead. d_n: device, one per pair.
 int32_t run_match_guided_batch(fsb_ctx* ctx, int n_pairs, const double* const* d_pred, const uint8_t* const* d_a,
                                const int* na, const double* const* d_bxy, const uint8_t* const* d_b, const int* nb,
                                const double* wb, const double* hb, double radius, int kc, float ratio,
-                               int64_t* const* d_q, int64_t* const* d_t, int32_t* counts, cudaStream_t s) {
+                               int64_t* const* d_q, int64_t* const* d_t, int32_t* d_n, int32_t* h_counts, cudaStream_t s,
+                               int32_t* c_t, float* c_b12) {
     if (n_pairs <= 0) return FSB_OK;
     std::vector<GPair> hp(n_pairs);
     long long cells = 0, rows = 0, items = 0;
@@ -1005,9 +895,9 @@ int32_t run_match_guided_batch(fsb_ctx* ctx, int n_pairs, const double* const* d
         P.gs = gs;
         P.cell0 = (int)cells;
         P.item0 = (int)items;
-        P.row0 = (int)rows;
-        P.q_out = d_q[p];
-        P.t_out = d_t[p];
+        P.q_out = d_q ? d_q[p] : nullptr;
+        P.t_out = d_t ? d_t[p] : nullptr;
+        P.n_out = d_n ? d_n + p : nullptr;
         cells += (long long)gs.gw * gs.gh;
         rows += na[p];
         items += nb[p];
@@ -1018,91 +908,51 @@ int32_t run_match_guided_batch(fsb_ctx* ctx, int n_pairs, const double* const* d
         set_error("guided batch too large (%lld cells, %lld targets, %lld queries)", cells, items, rows);
         return FSB_ERR_ARG;
     }
-    size_t tb1 = 0, tb2 = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, tb1, (int32_t*)nullptr, (int32_t*)nullptr, (int)(cells + 1), s);
-    cub::DeviceScan::ExclusiveSum(nullptr, tb2, (int32_t*)nullptr, (int32_t*)nullptr, (int)(items + 1), s);
+    size_t tb = 0;
+    cub::DeviceScan::ExclusiveSum(nullptr, tb, (int32_t*)nullptr, (int32_t*)nullptr, (int)(cells + 1), s);
     auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
-    const size_t b_pairs = al((size_t)n_pairs * sizeof(GPair)), b_rows = al((size_t)rows * 4), b_items = al((size_t)items * 4);
-    const size_t b_cells = al((size_t)(cells + 1) * 4), b_keys = al((size_t)items * 8), b_flag = al((size_t)(items + 1) * 4);
-    const size_t need = b_pairs + 3 * b_rows + 3 * b_items + 3 * b_cells + b_keys + 2 * b_flag + al(std::max(tb1, tb2)) + 512;
-    void* before = ctx->s_gb.p;
-    FSB_TRY(ctx->s_gb.ensure(need));
+    const size_t b_pairs = n_pairs > 1 ? al((size_t)n_pairs * sizeof(GPair)) : 0, b_items = al((size_t)items * 4);
+    const size_t b_cells = al((size_t)(cells + 1) * 4);
+    FSB_TRY(ctx->s_gb.ensure(b_pairs + 2 * b_items + al((size_t)items * 16) + 3 * b_cells + 256 + al((size_t)items * 8) +
+                             al(tb)));
     uint8_t* cur = ctx->s_gb.as<uint8_t>();
     auto take = [&](size_t bytes) {
         uint8_t* p = cur;
         cur += bytes;
         return p;
     };
-    GPair* d_pairs = reinterpret_cast<GPair*>(take(b_pairs));
-    int32_t* nA = reinterpret_cast<int32_t*>(take(b_rows));
-    int32_t* t_row = reinterpret_cast<int32_t*>(take(b_rows));
-    uint32_t* d_row = reinterpret_cast<uint32_t*>(take(b_rows));
-    int32_t* nB = reinterpret_cast<int32_t*>(take(b_items));
+    GPair* tab = n_pairs > 1 ? reinterpret_cast<GPair*>(take(b_pairs)) : nullptr;
     int32_t* cell = reinterpret_cast<int32_t*>(take(b_items));
     int32_t* gitems = reinterpret_cast<int32_t*>(take(b_items));
-    int32_t* count = reinterpret_cast<int32_t*>(take(b_cells));
+    double2* pos = reinterpret_cast<double2*>(take(al((size_t)items * 16)));
     int32_t* start = reinterpret_cast<int32_t*>(take(b_cells));
-    int32_t* cursor = reinterpret_cast<int32_t*>(take(b_cells));
-    unsigned long long* keys = reinterpret_cast<unsigned long long*>(take(b_keys));
-    int32_t* flag = reinterpret_cast<int32_t*>(take(b_flag));
-    int32_t* pos = reinterpret_cast<int32_t*>(take(b_flag));
-    void* tmp = take(al(std::max(tb1, tb2)));
+    int32_t* count = reinterpret_cast<int32_t*>(take(b_cells));    // count, cursor and the overflow
+    int32_t* cursor = reinterpret_cast<int32_t*>(take(b_cells));   // flag are cleared together
     int* overflow = reinterpret_cast<int*>(take(256));
-    // the graph is valid for exactly this table, these scratch addresses and parameters
-    GuidedGraph& G = ctx->gb_graph;
-    std::vector<char> key(sizeof(GPair) * n_pairs + 64);
-    memcpy(key.data(), hp.data(), sizeof(GPair) * n_pairs);
-    {
-        char* k = key.data() + sizeof(GPair) * n_pairs;
-        memcpy(k, &radius, 8);
-        memcpy(k + 8, &kc, 4);
-        memcpy(k + 12, &ratio, 4);
-        memcpy(k + 16, &counts, 8);
-        void* base = ctx->s_gb.p;
-        memcpy(k + 24, &base, 8);
-        const size_t nb_ = ctx->s_gb.bytes;
-        memcpy(k + 32, &nb_, 8);
-    }
-    const bool reuse = G.exec && before == ctx->s_gb.p && G.key == key;
-    if (!reuse) {
-        if (G.exec) cudaGraphExecDestroy(G.exec);
-        if (G.graph) cudaGraphDestroy(G.graph);
-        G.exec = nullptr;
-        G.graph = nullptr;
-        G.key.clear();
-        FSB_CUDA(cudaMemcpyAsync(d_pairs, hp.data(), (size_t)n_pairs * sizeof(GPair), cudaMemcpyHostToDevice, s));
-        FSB_CUDA(cudaStreamSynchronize(s));
-        FSB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        const unsigned py = (unsigned)n_pairs;
-        cudaMemsetAsync(count, 0, (size_t)(cells + 1) * 4, s);
-        cudaMemsetAsync(cursor, 0, (size_t)(cells + 1) * 4, s);
-        cudaMemsetAsync(overflow, 0, 4, s);
-        k_gb_norms<<<dim3(blocks(max_na, 8), py), 256, 0, s>>>(d_pairs, 0, nA);
-        k_gb_norms<<<dim3(blocks(max_nb, 8), py), 256, 0, s>>>(d_pairs, 1, nB);
-        k_gb_count<<<dim3(blocks(max_nb, 256), py), 256, 0, s>>>(d_pairs, cell, count);
-        cub::DeviceScan::ExclusiveSum(tmp, tb1, count, start, (int)(cells + 1), s);
-        k_gb_fill<<<dim3(blocks(max_nb, 256), py), 256, 0, s>>>(d_pairs, cell, start, cursor, gitems);
-        k_gb_guided<<<dim3(blocks(max_na, G_WARPS), py), G_WARPS * 32, 0, s>>>(d_pairs, nA, nB, start, gitems, radius,
-                                                                             kc, ratio, t_row, d_row, overflow);
-        k_gb_fill_keys<<<blocks(items, 256), 256, 0, s>>>(keys, (int)items);
-        k_gb_keys<<<dim3(blocks(max_na, 256), py), 256, 0, s>>>(d_pairs, t_row, d_row, keys);
-        k_gb_flags<<<blocks(items + 1, 256), 256, 0, s>>>(keys, (int)items, flag);
-        cub::DeviceScan::ExclusiveSum(tmp, tb2, flag, pos, (int)(items + 1), s);
-        k_gb_emit<<<dim3(blocks(max_nb, 256), py), 256, 0, s>>>(d_pairs, keys, pos, counts);
-        cudaError_t ce = cudaStreamEndCapture(s, &G.graph);
-        if (ce == cudaSuccess) ce = cudaGraphInstantiate(&G.exec, G.graph, 0);
-        if (ce != cudaSuccess) {
-            if (G.graph) cudaGraphDestroy(G.graph);
-            G.graph = nullptr;
-            G.exec = nullptr;
-            cudaGetLastError();
-            set_error("guided batch graph: %s", cudaGetErrorString(ce));
-            return FSB_ERR_CUDA;
+    unsigned long long* keys = reinterpret_cast<unsigned long long*>(take(al((size_t)items * 8)));
+    void* tmp = take(al(tb));
+    if (tab) FSB_CUDA(cudaMemcpyAsync(tab, hp.data(), (size_t)n_pairs * sizeof(GPair), cudaMemcpyHostToDevice, s));
+    FSB_CUDA(cudaMemsetAsync(count, 0, 2 * b_cells + 256, s));
+    const unsigned py = (unsigned)n_pairs;
+    k_gb_count<<<dim3(blocks(max_nb, 256), py), 256, 0, s>>>(hp[0], tab, cell, count);
+    FSB_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb, count, start, (int)(cells + 1), s));
+    k_gb_fill<<<dim3(blocks(max_nb, 256), py), 256, 0, s>>>(hp[0], tab, cell, start, cursor, gitems, pos);
+    if (!c_t) FSB_CUDA(cudaMemsetAsync(keys, 0xff, (size_t)items * 8, s));
+    k_gb_guided<<<dim3(blocks(max_na, G_QUERIES), py), G_WARPS * 32, 0, s>>>(hp[0], tab, start, gitems, pos, radius, kc,
+                                                                           ratio, keys, c_t, c_b12, overflow);
+    note_launch(4);
+    FSB_CUDA(cudaGetLastError());
+    if (!c_t) {
+        if (max_nb <= kCompactMax) {
+            k_gb_compact<<<py, COMPACT_T, 0, s>>>(hp[0], tab, keys);
+            note_launch();
+            FSB_CUDA(cudaGetLastError());
+        } else {
+            for (const GPair& P : hp)
+                FSB_TRY(emit_unique(ctx, keys + P.item0, P.nb, P.q_out, P.t_out, P.n_out, s));
         }
-        G.key = key;
+        if (h_counts) FSB_CUDA(cudaMemcpyAsync(h_counts, d_n, (size_t)n_pairs * 4, cudaMemcpyDeviceToHost, s));
     }
-    FSB_CUDA(cudaGraphLaunch(G.exec, s));
-    note_launch(13);
     int h_over = 0;
     FSB_CUDA(cudaMemcpyAsync(&h_over, overflow, sizeof(int), cudaMemcpyDeviceToHost, s));
     FSB_CUDA(cudaStreamSynchronize(s));
