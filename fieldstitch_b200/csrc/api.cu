@@ -1283,15 +1283,16 @@ int32_t fsb_match_bf_batch_d(fsb_ctx* ctx, int32_t n_pairs, const uint8_t* const
         rb.push_back(nb[p]);
     }
     const int nl = (int)live.size();
-    if (precision == FSB_PREC_FP32)
+    std::vector<int> cl(nl, 0);
+    if (precision == FSB_PREC_FP32) {
         FSB_TRY(run_match_bf_batch(ctx, nl, pa.data(), ra.data(), pb.data(), rb.data(), ratio, pq.data(), pt.data(),
                                    dn_all, s));
-    else
+        FSB_CUDA(cudaMemcpyAsync(cl.data(), dn_all, (size_t)nl * 4, cudaMemcpyDeviceToHost, s));
+        FSB_CUDA(cudaStreamSynchronize(s));
+    } else {
         FSB_TRY(run_match_bf_tc(ctx, nl, pa.data(), ra.data(), pb.data(), rb.data(), ratio, precision, pq.data(),
-                                pt.data(), dn_all, &ctx->tc_stats, s));
-    std::vector<int> cl(nl, 0);
-    FSB_CUDA(cudaMemcpyAsync(cl.data(), dn_all, (size_t)nl * 4, cudaMemcpyDeviceToHost, s));
-    FSB_CUDA(cudaStreamSynchronize(s));
+                                pt.data(), dn_all, cl.data(), &ctx->tc_stats, s));
+    }
     for (int i = 0; i < nl; ++i) n_out[live[i]] = cl[i];
     ctx->stage_end(ST_MATCH);
     return FSB_OK;

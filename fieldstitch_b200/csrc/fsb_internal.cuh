@@ -301,10 +301,10 @@ int32_t run_mlp_grad(fsb_ctx* ctx, const float* prm, int n, const float* feat, c
 int32_t run_mlp_train(fsb_ctx* ctx, float* prm, float* m, float* v, int n, const float* feat, const float* label,
                       int epochs, int batch, float lr, uint32_t seed, double* losses, cudaStream_t s);
 // tc_match.cu: tensor-core dense matching of a batch of pairs (na, nb >= 1), _unique included;
-// counts (device, one per pair), q_out/t_out device arrays of capacity na[p]
+// counts (device, one per pair; h_counts host, nullable), q_out/t_out device arrays of capacity na[p]; waits
 int32_t run_match_bf_tc(fsb_ctx* ctx, int n_pairs, const uint8_t* const* d_a, const int* na,
                         const uint8_t* const* d_b, const int* nb, float ratio, int precision, int64_t* const* q_out,
-                        int64_t* const* t_out, int32_t* counts, TcStats* stats, cudaStream_t s);
+                        int64_t* const* t_out, int32_t* counts, int32_t* h_counts, TcStats* stats, cudaStream_t s);
 // ransac.cu
 int32_t run_ransac_h(const long long* d_off, int n_pairs, const double2* d_src, const double2* d_dst, double thr,
                      int iters, unsigned long long seed, double* d_H, uint8_t* d_mask, int* d_ninl, cudaStream_t s);

@@ -20,6 +20,7 @@
 #include <mutex>
 
 #include "fsb_internal.cuh"
+#include "unique.cuh"
 
 namespace fsb {
 namespace {
@@ -320,30 +321,6 @@ __global__ void k_unique_keys(const int32_t* __restrict__ t_row, const uint32_t*
     if (t >= 0) atomicMin(key + t, ((unsigned long long)d_row[r] << 32) | (unsigned)r);
 }
 
-// target-ordered compaction of the one-to-one keys by one block: one launch where flags, a device
-// select (two kernels) and a gather take four; up to kCompactMax targets (5 us at 9000)
-constexpr int kCompactMax = 32768;
-constexpr int COMPACT_T = 1024;
-__device__ __forceinline__ void unique_compact(const unsigned long long* __restrict__ key, int nb, int64_t* __restrict__ q,
-                                               int64_t* __restrict__ t, int32_t* __restrict__ n_out) {
-    typedef cub::BlockScan<int, COMPACT_T> Scan;
-    __shared__ typename Scan::TempStorage tmp;
-    const int per = (nb + COMPACT_T - 1) / COMPACT_T;
-    const int t0 = threadIdx.x * per, t1 = min(nb, t0 + per);
-    int cnt = 0;
-    for (int i = t0; i < t1; ++i) cnt += key[i] != ~0ull;
-    int off = 0, total = 0;
-    Scan(tmp).ExclusiveSum(cnt, off, total);
-    for (int i = t0; i < t1; ++i) {
-        const unsigned long long k = key[i];
-        if (k != ~0ull) {
-            q[off] = (int64_t)(k & 0xffffffffull);
-            t[off] = i;
-            ++off;
-        }
-    }
-    if (threadIdx.x == 0) *n_out = total;
-}
 __global__ void __launch_bounds__(COMPACT_T) k_unique_compact(const unsigned long long* __restrict__ key, int nb,
                                                               int64_t* __restrict__ q, int64_t* __restrict__ t,
                                                               int32_t* __restrict__ n_out) {
@@ -474,7 +451,7 @@ __device__ __forceinline__ void guided_distances(const uint4& a4, int qn, const 
 // a radius of 40) instead of nine cells one after another, and a candidate's row is one coalesced
 // 128-byte read instead of eight strided ones.
 // Bound by the latency of the dependent reads (cell starts, positions, rows). 64 pairs of 2000-16000
-// features: 1219 us with nine cells and a lane per candidate (plus 188 us for norms), GB_TIMES now.
+// features: 1219 us with nine cells and a lane per candidate (plus 188 us for norms), 404 us now.
 __global__ void __launch_bounds__(G_WARPS * 32) k_gb_guided(const __grid_constant__ GPair one, const GPair* __restrict__ tab,
                                                             const int32_t* __restrict__ start,
                                                             const int32_t* __restrict__ items,
@@ -796,7 +773,8 @@ int32_t run_match_bf(fsb_ctx* ctx, const uint8_t* d_a, int na, const uint8_t* d_
         return FSB_OK;
     }
     if (precision != FSB_PREC_FP32)
-        return run_match_bf_tc(ctx, 1, &d_a, &na, &d_b, &nb, ratio, precision, &d_q, &d_t, d_n, &ctx->tc_stats, s);
+        return run_match_bf_tc(ctx, 1, &d_a, &na, &d_b, &nb, ratio, precision, &d_q, &d_t, d_n, nullptr,
+                               &ctx->tc_stats, s);
     const BfPlan pl = bf_plan(&na, &nb, 1, (size_t)1 << 40);
     FSB_TRY(ctx->s_misc.ensure(pl.parts * sizeof(Top2) + 64));
     FSB_TRY(ctx->s_u64.ensure((size_t)nb * 8 + 64));

@@ -17,12 +17,14 @@
 //                      targets are not scaled (uint8 never exceeds the E4M3 range). A power-of-two
 //                      scale moves only the exponent, so for uint8 values it changes no rounded
 //                      value; it is kept for inputs whose range needs it.
-//   k_tc_dense   persistent warp-specialised kernel. Warp 0 streams 128-row target tiles into a
+//   k_tc_dense   persistent warp-specialised kernel. Warp 0 streams 256-row target tiles into a
 //                shared-memory ring with bulk asynchronous copies (no tensor map, no multicast);
-//                warp 1 issues the MMAs (M=128, N=128) for the two 128-row halves of a 256-row
-//                query block into double-buffered FP32 accumulators (4 x 128 of the 512 TMEM
-//                columns); warps 2-9 read the accumulators with tcgen05.ld (a 128-column row per wait)
-//                and keep, per query row, the two largest 32-column maxima and their chunks.
+//                warp 1 issues the MMAs (M=128, N=256) for the two 128-row halves of a 256-row
+//                query block into FP32 accumulators (2 x 256 of the 512 TMEM columns); warps 2-9
+//                read the accumulators with tcgen05.ld (four 32-column loads per wait), a half being
+//                drained while the other is computed, and keep, per query row, the two largest
+//                16-column maxima and their chunks. At N = 128 an MMA's operands take the whole
+//                shared-memory read bandwidth (8 KB per 64 cycles); at N = 256 three quarters of it.
 //   k_tc_finish  per query row: the two best chunks over all column splits and the exact integer
 //                distances (dp4a) of their columns (BF16: the best chunk only; the second chunk's
 //                maximum is already exact), top-2, the float32 ratio test of the reference, and a
@@ -36,8 +38,8 @@
 // The best target, the exact best distance and the accept decision are therefore the same as
 // those of the CUDA-core FP32 path and of the reference, for every precision.
 #include <cub/cub.cuh>
-#include <cuda_fp8.h>
 
+#include <algorithm>
 #include <cfloat>
 #include <climits>
 #include <cmath>
@@ -45,6 +47,7 @@
 #include <vector>
 
 #include "fsb_internal.cuh"
+#include "unique.cuh"
 
 namespace fsb {
 namespace {
@@ -53,8 +56,8 @@ inline unsigned nblk(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
 constexpr int TC_THREADS = 320;      // producer warp, MMA warp, 8 epilogue warps
 constexpr int TC_ROWS = 256;         // query rows per work item (two M=128 halves)
-constexpr int TC_N = 128;            // target rows per tile (MMA N)
-constexpr int TC_CHUNK = 32;         // columns per tcgen05.ld
+constexpr int TC_N = 256;            // target rows per tile (MMA N)
+constexpr int TC_CHUNK = 16;         // columns per candidate chunk
 constexpr int TC_MAX_SPLITS = 8;
 constexpr long long TC_TIMEOUT_CYCLES = 4000000000ll;   // about two seconds at full clock
 
@@ -68,20 +71,22 @@ template <int PREC> struct TcTraits;
 template <> struct TcTraits<FSB_PREC_BF16> {
     static constexpr int ROW_BYTES = 288;   // 128 + 16 BF16 values
     static constexpr int MAIN_STEPS = 8;    // K = 16 BF16 per MMA (32 bytes)
-    static constexpr int STAGES = 4;
+    static constexpr int STAGES = 2;
     static constexpr int TOPK = 2;
 };
 template <> struct TcTraits<FSB_PREC_FP8> {
     static constexpr int ROW_BYTES = 160;   // 128 E4M3 + 16 BF16 values
     static constexpr int MAIN_STEPS = 4;    // K = 32 E4M3 per MMA (32 bytes)
-    static constexpr int STAGES = 8;
+    static constexpr int STAGES = 4;
     static constexpr int TOPK = 2;
 };
 
-template <int PREC> constexpr int tile_bytes() { return 128 * TcTraits<PREC>::ROW_BYTES; }
+template <int PREC> constexpr int half_bytes() { return 128 * TcTraits<PREC>::ROW_BYTES; }    // a query half
+template <int PREC> constexpr int tile_bytes() { return TC_N * TcTraits<PREC>::ROW_BYTES; }   // a target tile
 template <int PREC> constexpr int smem_bytes() {
-    return 2 * tile_bytes<PREC>() + TcTraits<PREC>::STAGES * tile_bytes<PREC>() + 2048;
+    return 2 * half_bytes<PREC>() + TcTraits<PREC>::STAGES * tile_bytes<PREC>() + 2048;
 }
+static_assert(smem_bytes<FSB_PREC_BF16>() <= 227 * 1024 && smem_bytes<FSB_PREC_FP8>() <= 227 * 1024, "shared memory");
 
 // Byte offset of (row, k-byte) inside a 128-row block: core matrix (row / 8, kb / 16) at
 // (row / 8) * SBO + (kb / 16) * 128 with SBO = ROW_BYTES * 8; the descriptor's LBO is 128.
@@ -94,7 +99,7 @@ struct TcPair {
     const uint8_t* a;      // uint8 query rows (na x 128)
     const uint8_t* b;      // uint8 target rows (nb x 128)
     const uint8_t* pa;     // packed query blocks (nrb x 256 rows)
-    const uint8_t* pb;     // packed target tiles (ntiles x 128 rows)
+    const uint8_t* pb;     // packed target tiles (ntiles x TC_N rows)
     const float* rowsc;    // E4M3: per query (s, 1 / s, |a|, |alpha|)
     const float* bmax;     // E4M3: (max |b|, max |beta|) over the targets
     const int32_t* nA;     // |a|^2
@@ -106,11 +111,13 @@ struct TcPair {
     int row0;              // first row in the concatenated row arrays
     long long part0;       // first candidate record
     long long key0;        // first target in the concatenated key array
+    unsigned long long* key;   // one-to-one keys of the targets
+    int32_t* count;        // number of matches
 };
 
 struct Cand {
-    float v;   // largest s * (a.b - |b|^2 / 2) of a 32-column chunk, as computed by the tensor cores
-    int j;     // the chunk (column / 32), -1 when empty
+    float v;   // largest s * (a.b - |b|^2 / 2) of a chunk of columns, as computed by the tensor cores
+    int j;     // the chunk (column / TC_CHUNK), -1 when empty
 };
 
 // Packing job: `n` rows of `src` (padded with zero rows to n_pad) into `dst`.
@@ -134,81 +141,121 @@ __device__ __forceinline__ int upper_index(const T* __restrict__ arr, int n, lon
 }
 
 // ------------------------------------------------------------------------ packing
-__device__ __forceinline__ uint16_t bf16_bits(float x) {
-    return (uint16_t)(__float_as_uint(x) >> 16);   // exact for the integers 0..255 and powers of two
+// byte k of w as float (exact): its bits under the exponent of 2^23, less 2^23
+__device__ __forceinline__ float byte_float(uint32_t w, int k) {
+    return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u | (unsigned)k)) - 8388608.f;
+}
+// a BF16 pair from two exactly representable floats
+__device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) {
+    return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632u);
 }
 
-// One warp per packed row; blockIdx.y is the job.
+// Four packed rows per warp, eight lanes per row (16 bytes each); blockIdx.y is the job. Bound by HBM
+// (128 bytes in, ROW_BYTES out per row). One row per warp with a conversion instruction per value
+// took 92 us (BF16, 524 000 rows) and 268 us (E4M3, 433 000 rows, one more pass back to float and two
+// atomics per target); byte permutes and integer rounding take 45 and 79 us.
+constexpr int PACK_T = 256, PACK_ROWS = PACK_T / 8;
 template <int PREC>
-__global__ void k_tc_pack(const PackSeg* __restrict__ segs) {
+__global__ void __launch_bounds__(PACK_T) k_tc_pack(const PackSeg* __restrict__ segs) {
     constexpr int RB = TcTraits<PREC>::ROW_BYTES;
     constexpr int XB = RB - 32;   // byte offset of the norm slots
     const PackSeg& S = segs[blockIdx.y];
-    const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (row >= S.n_pad) return;
+    const int lane = threadIdx.x & 31, seg = lane & 7;
+    const int row = blockIdx.x * PACK_ROWS + (threadIdx.x >> 3);
+    if (blockIdx.x * PACK_ROWS >= S.n_pad) return;   // n_pad is a multiple of PACK_ROWS: uniform per block
     uint8_t* blk = S.dst + (size_t)(row >> 7) * (128 * RB);
     const int r = row & 127;
     const bool live = row < S.n;
-    const uint32_t w = live ? reinterpret_cast<const uint32_t*>(S.src + (size_t)row * 128)[lane] : 0u;
-    int nrm = (int)__dp4a(w, w, 0u);
-    for (int sh = 16; sh; sh >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, sh);
-    if (lane == 0 && live) S.norms[row] = nrm;
+    uint4 w = make_uint4(0u, 0u, 0u, 0u);
+    if (live) w = __ldg(reinterpret_cast<const uint4*>(S.src + (size_t)row * 128) + seg);
+    const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+    unsigned un = 0;
+#pragma unroll
+    for (int v = 0; v < 4; ++v) un = __dp4a(ww[v], ww[v], un);
+#pragma unroll
+    for (int sh = 1; sh < 8; sh <<= 1) un += __shfl_xor_sync(0xffffffffu, un, sh);
+    const int nrm = (int)un;
+    if (seg == 0 && live) S.norms[row] = nrm;
     float s = 1.f;
     if constexpr (PREC == FSB_PREC_BF16) {
-        uint2 v;
-        v.x = (uint32_t)bf16_bits((float)(w & 255u)) | ((uint32_t)bf16_bits((float)((w >> 8) & 255u)) << 16);
-        v.y = (uint32_t)bf16_bits((float)((w >> 16) & 255u)) | ((uint32_t)bf16_bits((float)(w >> 24)) << 16);
-        *reinterpret_cast<uint2*>(blk + core_off(r, lane * 8, RB)) = v;
+        uint32_t o[8];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+            o[2 * v] = bf16_pair(byte_float(ww[v], 0), byte_float(ww[v], 1));
+            o[2 * v + 1] = bf16_pair(byte_float(ww[v], 2), byte_float(ww[v], 3));
+        }
+        *reinterpret_cast<uint4*>(blk + core_off(r, seg * 32, RB)) = make_uint4(o[0], o[1], o[2], o[3]);
+        *reinterpret_cast<uint4*>(blk + core_off(r, seg * 32 + 16, RB)) = make_uint4(o[4], o[5], o[6], o[7]);
     } else {
-        if (S.role == 0) {   // per-query power-of-two scale: the largest e <= 8 with max * 2^e <= 448
-            uint32_t mx = max(max(w & 255u, (w >> 8) & 255u), max((w >> 16) & 255u, w >> 24));
-            for (int sh = 16; sh; sh >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, sh));
-            int e = 8;
-            while (e > 0 && (mx << e) > 448u) --e;
+        int e = 0;
+        if (S.role == 0) {
+            // per-query power-of-two scale: the largest e <= 8 with max * 2^e <= 448 = 1.75 * 2^8
+            uint32_t mx = __vmaxu4(__vmaxu4(ww[0], ww[1]), __vmaxu4(ww[2], ww[3]));
+            mx = __vmaxu4(mx, mx >> 16);
+            mx = max(mx & 255u, (mx >> 8) & 255u);
+#pragma unroll
+            for (int sh = 1; sh < 8; sh <<= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, sh));
+            e = 8;
+            if (mx) {
+                const int k = 31 - __clz(mx);
+                e = max(0, (mx << (8 - k)) <= 448u ? 8 - k : 7 - k);
+            }
             s = (float)(1 << e);
         }
-        uint32_t packed = 0;
+        // E4M3 of x 2^e for an integer x in 1..255: three mantissa bits, round to nearest even (the carry
+        // moves the exponent), exponent re-biased by 7 - 127; the scale is an exponent shift, so the
+        // rounding error of x itself does not depend on it
+        uint32_t o[4];
         float err2 = 0.f;
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const float x = (float)((w >> (8 * b)) & 255u);
-            const __nv_fp8_storage_t q = __nv_cvt_float_to_fp8(x * s, __NV_SATFINITE, __NV_E4M3);
-            const float back = __half2float(__half(__nv_cvt_fp8_to_halfraw(q, __NV_E4M3))) / s;
-            err2 = fmaf(back - x, back - x, err2);
-            packed |= (uint32_t)q << (8 * b);
-        }
-        for (int sh = 16; sh; sh >>= 1) err2 += __shfl_xor_sync(0xffffffffu, err2, sh);
-        *reinterpret_cast<uint32_t*>(blk + core_off(r, lane * 4, RB)) = packed;
-        const float len = live ? sqrtf((float)nrm) * (1.f + 1e-6f) : 0.f;
-        const float elen = live ? sqrtf(err2) * (1.f + 1e-6f) : 0.f;
-        if (lane == 0 && live && S.role == 0)
-            reinterpret_cast<float4*>(S.rowsc)[row] = make_float4(s, 1.f / s, len, elen);
-        if (lane == 0 && live && S.role == 1) {
-            // the largest |b| and |beta| of the job (non-negative floats order like their bit
-            // patterns); the atomic is skipped once the running maximum is already larger
-            int* bm = reinterpret_cast<int*>(S.bmax);
-            if (__float_as_int(len) > *reinterpret_cast<volatile int*>(bm)) atomicMax(bm, __float_as_int(len));
-            if (__float_as_int(elen) > *reinterpret_cast<volatile int*>(bm + 1)) atomicMax(bm + 1, __float_as_int(elen));
-        }
-    }
-    if (lane < 4) {   // the 16 norm slots (32 bytes), 8 bytes per lane
-        uint16_t e[4] = {0, 0, 0, 0};
-        if (lane == 0 && live) {
-            if (S.role == 0) {
-                e[0] = bf16_bits(-32768.f * s);
-                e[1] = bf16_bits(-128.f * s);
-                e[2] = bf16_bits(-0.5f * s);
-            } else {
-                e[0] = bf16_bits((float)((nrm >> 16) & 255));
-                e[1] = bf16_bits((float)((nrm >> 8) & 255));
-                e[2] = bf16_bits((float)(nrm & 255));
+        for (int v = 0; v < 4; ++v) {
+            o[v] = 0;
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const float x = byte_float(ww[v], b);
+                const uint32_t u = __float_as_uint(x);
+                const uint32_t q = (u + 0x7FFFFu + ((u >> 20) & 1u)) >> 20;
+                const float back = __uint_as_float(q << 20);
+                err2 = fmaf(back - x, back - x, err2);
+                const uint32_t code = x > 0.f ? q + (uint32_t)(8 * e - 960) : 0u;
+                o[v] |= code << (8 * b);
             }
         }
-        uint2 x;
-        x.x = (uint32_t)e[0] | ((uint32_t)e[1] << 16);
-        x.y = (uint32_t)e[2] | ((uint32_t)e[3] << 16);
-        *reinterpret_cast<uint2*>(blk + core_off(r, XB + lane * 8, RB)) = x;
+#pragma unroll
+        for (int sh = 1; sh < 8; sh <<= 1) err2 += __shfl_xor_sync(0xffffffffu, err2, sh);
+        *reinterpret_cast<uint4*>(blk + core_off(r, seg * 16, RB)) = make_uint4(o[0], o[1], o[2], o[3]);
+        const float len = live ? sqrtf((float)nrm) * (1.f + 1e-6f) : 0.f;
+        const float elen = live ? sqrtf(err2) * (1.f + 1e-6f) : 0.f;
+        if (S.role == 0) {
+            if (seg == 0 && live) reinterpret_cast<float4*>(S.rowsc)[row] = make_float4(s, 1.f / s, len, elen);
+        } else {
+            // the largest |b| and |beta| of the job (non-negative floats order like their bit
+            // patterns): one pair of atomics per warp, skipped once the running maximum is larger
+            int ml = __float_as_int(len), me = __float_as_int(elen);
+#pragma unroll
+            for (int sh = 8; sh < 32; sh <<= 1) {
+                ml = max(ml, __shfl_xor_sync(0xffffffffu, ml, sh));
+                me = max(me, __shfl_xor_sync(0xffffffffu, me, sh));
+            }
+            if (lane == 0) {
+                int* bm = reinterpret_cast<int*>(S.bmax);
+                if (ml > *reinterpret_cast<volatile int*>(bm)) atomicMax(bm, ml);
+                if (me > *reinterpret_cast<volatile int*>(bm + 1)) atomicMax(bm + 1, me);
+            }
+        }
+    }
+    if (seg < 2) {   // the 16 norm slots (32 bytes), 16 bytes per lane
+        uint4 x = make_uint4(0u, 0u, 0u, 0u);
+        if (seg == 0 && live) {
+            if (S.role == 0) {
+                x.x = bf16_pair(-32768.f * s, -128.f * s);
+                x.y = bf16_pair(-0.5f * s, 0.f);
+            } else {
+                x.x = bf16_pair(byte_float((uint32_t)nrm, 2), byte_float((uint32_t)nrm, 1));
+                x.y = bf16_pair(byte_float((uint32_t)nrm, 0), 0.f);
+            }
+        }
+        *reinterpret_cast<uint4*>(blk + core_off(r, XB + seg * 16, RB)) = x;
     }
 }
 
@@ -320,28 +367,35 @@ __device__ __forceinline__ void top_insert(float (&t)[K], int (&j)[K], float v, 
     }
 }
 
+// The item of CTA `cta` in round w: items are in descending length (the pairs are sorted by their
+// number of target tiles), and every other round runs backwards, so that the CTAs' sums even out.
+// Rounds end at w * grid >= n_items; an item past the end is skipped.
+__device__ __forceinline__ int tc_item(int w, int cta, int grid) {
+    return w * grid + ((w & 1) ? grid - 1 - cta : cta);
+}
+
 // ------------------------------------------------------------------------ the dense kernel
 template <int PREC>
 __global__ void __launch_bounds__(TC_THREADS, 1)
     k_tc_dense(const TcPair* __restrict__ pairs, int n_pairs, int n_items, Cand* __restrict__ part,
                int* __restrict__ err) {
     using T = TcTraits<PREC>;
-    constexpr int TB = tile_bytes<PREC>();
+    constexpr int TB = tile_bytes<PREC>(), HB = half_bytes<PREC>();
     constexpr int NST = T::STAGES;
     constexpr int K = T::TOPK;
     constexpr uint32_t SBO = T::ROW_BYTES * 8;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem =
         reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    unsigned char* sA = smem;            // 2 x TB
-    unsigned char* sB = smem + 2 * TB;   // NST x TB
+    unsigned char* sA = smem;            // 2 x HB
+    unsigned char* sB = smem + 2 * HB;   // NST x TB
     uint64_t* bars = reinterpret_cast<uint64_t*>(sB + NST * TB);
     uint64_t* b_full = bars;             // NST
     uint64_t* b_empty = bars + NST;      // NST
     uint64_t* a_full = bars + 2 * NST;
     uint64_t* a_empty = a_full + 1;
-    uint64_t* acc_full = a_full + 2;     // 2
-    uint64_t* acc_empty = a_full + 4;    // 2
+    uint64_t* acc_full = a_full + 2;     // per query half
+    uint64_t* acc_empty = a_full + 4;    // per query half
     uint64_t* done_bar = a_full + 6;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(a_full + 8);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -357,7 +411,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         mbar_init(a_empty, 1);
         for (int i = 0; i < 2; ++i) {
             mbar_init(acc_full + i, 1);
-            mbar_init(acc_empty + i, 8);
+            mbar_init(acc_empty + i, 4);
         }
         mbar_init(done_bar, 1);
         *abort_flag = 0;
@@ -383,7 +437,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             int pend[NST];
             for (int i = 0; i < NST; ++i) pend[i] = -1;
             int a_pend = -1;
-            for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++wi) {
+            for (int w = 0; w * (int)gridDim.x < n_items && ok; ++w) {
+                const int item = tc_item(w, blockIdx.x, gridDim.x);
+                if (item >= n_items) continue;
                 const TcPair& P = pairs[upper_index(pairs, n_pairs, item, item0_of)];
                 const int local = item - P.item0;
                 const int rb = local / P.splits, sp = local - rb * P.splits;
@@ -401,9 +457,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                 if (!ok) break;
                 ok = mbar_wait(a_empty, (wi & 1) ^ 1, abort_flag);
                 if (!ok) break;
-                mbar_expect_tx(a_full, 2 * TB);
-                bulk_load(sA, P.pa + (size_t)rb * 2 * TB, TB, a_full);
-                bulk_load(sA + TB, P.pa + (size_t)rb * 2 * TB + TB, TB, a_full);
+                mbar_expect_tx(a_full, 2 * HB);
+                bulk_load(sA, P.pa + (size_t)rb * 2 * HB, HB, a_full);
+                bulk_load(sA + HB, P.pa + (size_t)rb * 2 * HB + HB, HB, a_full);
                 a_pend = wi & 1;
                 for (int t = t0 + pre; t < t1 && ok; ++t, ++bit) {
                     const int st = bit % NST;
@@ -413,6 +469,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                     bulk_load(sB + st * TB, P.pb + (size_t)t * TB, TB, b_full + st);
                     pend[st] = (int)((bit / NST) & 1);
                 }
+                ++wi;
             }
             if (!ok) {
                 // let every copy already issued land before the CTA leaves (bounded)
@@ -434,7 +491,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             int wi = 0;
             bool ok = true, issued = false;
             const uint32_t a0 = saddr(sA), b0 = saddr(sB);
-            for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++wi) {
+            for (int w = 0; w * (int)gridDim.x < n_items && ok; ++w) {
+                const int item = tc_item(w, blockIdx.x, gridDim.x);
+                if (item >= n_items) continue;
                 const TcPair& P = pairs[upper_index(pairs, n_pairs, item, item0_of)];
                 const int local = item - P.item0;
                 const int sp = local % P.splits;
@@ -444,16 +503,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                 tc_fence_after();
                 for (int t = t0; t < t1; ++t, ++bit, ++tit) {
                     const int st = bit % NST;
-                    const int ac = tit & 1;
                     ok = mbar_wait(b_full + st, (bit / NST) & 1, abort_flag);
                     if (!ok) break;
-                    ok = mbar_wait(acc_empty + ac, ((tit >> 1) & 1) ^ 1, abort_flag);
-                    if (!ok) break;
-                    tc_fence_after();
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
-                        const uint32_t d = tmem + (uint32_t)(ac * 256 + h * 128);
-                        const uint32_t ra = a0 + h * TB, rb = b0 + st * TB;
+                        // half h of the accumulators is drained while the other half is computed
+                        ok = ok && mbar_wait(acc_empty + h, (tit & 1) ^ 1, abort_flag);
+                        if (!ok) break;
+                        tc_fence_after();
+                        const uint32_t d = tmem + (uint32_t)(h * TC_N);
+                        const uint32_t ra = a0 + h * HB, rb = b0 + st * TB;
 #pragma unroll
                         for (int k = 0; k < T::MAIN_STEPS; ++k) {
                             if constexpr (PREC == FSB_PREC_BF16)
@@ -463,13 +522,15 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                         }
                         mma_bf16(d, smem_desc(ra + T::MAIN_STEPS * 256, SBO), smem_desc(rb + T::MAIN_STEPS * 256, SBO),
                                  1u);
+                        issued = true;
+                        mma_commit(acc_full + h);
                     }
-                    issued = true;
+                    if (!ok) break;
                     mma_commit(b_empty + st);
-                    mma_commit(acc_full + ac);
                 }
                 if (!ok) break;
                 mma_commit(a_empty);
+                ++wi;
             }
             // every MMA issued by this thread has completed before TMEM is released
             if (issued) {
@@ -488,7 +549,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         const int rloc = h * 128 + lq * 32 + lane;
         uint32_t tit = 0;
         bool ok = true;
-        for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+        for (int w = 0; w * (int)gridDim.x < n_items && ok; ++w) {
+            const int item = tc_item(w, blockIdx.x, gridDim.x);
+            if (item >= n_items) continue;
             const TcPair& P = pairs[upper_index(pairs, n_pairs, item, item0_of)];
             const int local = item - P.item0;
             const int rb = local / P.splits, sp = local - rb * P.splits;
@@ -502,41 +565,41 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                 tj[i] = -1;
             }
             for (int t = t0; t < t1; ++t, ++tit) {
-                const int ac = tit & 1;
-                ok = mbar_wait(acc_full + ac, (tit >> 1) & 1, abort_flag);
+                ok = mbar_wait(acc_full + h, tit & 1, abort_flag);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t base = tmem + ((uint32_t)(lq * 32) << 16) + (uint32_t)(ac * 256 + h * 128);
-                // the whole 128-column row at once (four loads, one wait), then the accumulator is free
-                uint32_t r[TC_N / TC_CHUNK][32];
+                const uint32_t base = tmem + ((uint32_t)(lq * 32) << 16) + (uint32_t)(h * TC_N);
+#pragma unroll 1
+                for (int c0 = 0; c0 < TC_N; c0 += 128) {
+                    // 128 columns of the row at once (four loads, one wait); after the last ones the
+                    // accumulator is free
+                    uint32_t r[4][32];
 #pragma unroll
-                for (int ch = 0; ch < TC_N / TC_CHUNK; ++ch) tmem_ld32(base + ch * TC_CHUNK, r[ch]);
-                tmem_wait_ld();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(acc_empty + ac);
-#pragma unroll
-                for (int ch = 0; ch < TC_N / TC_CHUNK; ++ch) {
-                    const int j0 = t * TC_N + ch * TC_CHUNK;
-                    float v[32];
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[ch][i]);
-                    if (j0 + TC_CHUNK > P.nb) {
-#pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            if (j0 + i >= P.nb) v[i] = -INFINITY;
+                    for (int ch = 0; ch < 4; ++ch) tmem_ld32(base + c0 + ch * 32, r[ch]);
+                    tmem_wait_ld();
+                    if (c0 + 128 == TC_N) {
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(acc_empty + h);
                     }
-                    float a0 = max3(v[0], v[1], v[2]), a1 = max3(v[3], v[4], v[5]), a2 = max3(v[6], v[7], v[8]);
-                    float a3 = max3(v[9], v[10], v[11]), a4 = max3(v[12], v[13], v[14]);
-                    float a5 = max3(v[15], v[16], v[17]), a6 = max3(v[18], v[19], v[20]);
-                    float a7 = max3(v[21], v[22], v[23]), a8 = max3(v[24], v[25], v[26]);
-                    float a9 = max3(v[27], v[28], v[29]), a10 = fmaxf(v[30], v[31]);
-                    a0 = max3(a0, a1, a2);
-                    a3 = max3(a3, a4, a5);
-                    a6 = max3(a6, a7, a8);
-                    a9 = fmaxf(a9, a10);
-                    const float mx = fmaxf(max3(a0, a3, a6), a9);
-                    if (mx > tv[K - 1]) top_insert<K>(tv, tj, mx, j0 / TC_CHUNK);
+#pragma unroll
+                    for (int ch = 0; ch < 128 / TC_CHUNK; ++ch) {
+                        const int j0 = t * TC_N + c0 + ch * TC_CHUNK;
+                        float v[TC_CHUNK];
+#pragma unroll
+                        for (int i = 0; i < TC_CHUNK; ++i)
+                            v[i] = __uint_as_float(r[ch / (32 / TC_CHUNK)][ch % (32 / TC_CHUNK) * TC_CHUNK + i]);
+                        if (j0 + TC_CHUNK > P.nb) {
+#pragma unroll
+                            for (int i = 0; i < TC_CHUNK; ++i)
+                                if (j0 + i >= P.nb) v[i] = -INFINITY;
+                        }
+                        static_assert(TC_CHUNK == 16, "maximum tree");
+                        const float a0 = max3(v[0], v[1], v[2]), a1 = max3(v[3], v[4], v[5]), a2 = max3(v[6], v[7], v[8]);
+                        const float a3 = max3(v[9], v[10], v[11]), a4 = max3(v[12], v[13], v[14]);
+                        const float mx = fmaxf(max3(a0, a1, a2), max3(a3, a4, v[15]));
+                        if (mx > tv[K - 1]) top_insert<K>(tv, tj, mx, j0 / TC_CHUNK);
+                    }
                 }
             }
             if (!ok) break;
@@ -614,17 +677,16 @@ __device__ __forceinline__ void group_top2(long long& k1, long long& d2) {
 // segment of the 128-byte rows that the lane multiplies. Per row:
 //   1. the K best chunks over the column splits (value descending, chunk ascending; one split's
 //      records are already in that order);
-//   2. the exact distances of the re-ranked chunks' 32 columns each: 32 independent 16-byte loads
-//      and dp4a per lane, then a transposed butterfly over seg (16 + 8 + 4 shuffles) leaves lane
-//      seg the whole dots of columns 4 seg .. 4 seg + 3; top-2 over the row's lanes;
+//   2. the exact distances of the re-ranked chunks' 16 columns each: 16 independent 16-byte loads
+//      and dp4a per lane, then a transposed butterfly over seg (8 + 4 + 2 shuffles) leaves lane seg
+//      the whole dots of columns 2 seg, 2 seg + 1; top-2 over the row's lanes;
 //   3. (lane seg 0) the certificate and the float32 ratio test of the reference: BF16, the best
 //      chunk's tensor-core maximum must equal the exact best (the values are exact) and the next
 //      chunk's maximum is the exact best outside it; E4M3, the rounding bound must settle the
 //      decision. Unsettled rows go to k_tc_exact_rows.
 template <int K>
 __global__ void __launch_bounds__(256) k_tc_finish(const TcPair* __restrict__ pairs, const Cand* __restrict__ part,
-                                                   float ratio, int prec, int32_t* __restrict__ t_row,
-                                                   uint32_t* __restrict__ d_row, int32_t* __restrict__ flagged,
+                                                   float ratio, int prec, int32_t* __restrict__ flagged,
                                                    int* __restrict__ n_flagged, float* __restrict__ err_stat) {
     __shared__ float s_mx, s_sum;
     __shared__ int s_n;
@@ -707,9 +769,9 @@ __global__ void __launch_bounds__(256) k_tc_finish(const TcPair* __restrict__ pa
         for (int k = 0; k < K; ++k) {
             if (k >= nre) break;   // warp-uniform
             const int jc = sc[k] < 0 ? P.nb : sc[k] * TC_CHUNK;   // an empty chunk: no valid column
-            uint32_t p[32];
+            uint32_t p[TC_CHUNK];
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
+            for (int i = 0; i < TC_CHUNK; ++i) {
                 const int j = jc + i;
                 uint32_t dot = 0;
                 if (j < P.nb) {
@@ -721,18 +783,19 @@ __global__ void __launch_bounds__(256) k_tc_finish(const TcPair* __restrict__ pa
                 }
                 p[i] = dot;
             }
+            constexpr int C2 = TC_CHUNK / 2, C4 = TC_CHUNK / 4, C8 = TC_CHUNK / 8;
 #pragma unroll
-            for (int t = 0; t < 16; ++t)
-                p[t] = (h4 ? p[t + 16] : p[t]) + __shfl_xor_sync(0xffffffffu, h4 ? p[t] : p[t + 16], 4);
+            for (int t = 0; t < C2; ++t)
+                p[t] = (h4 ? p[t + C2] : p[t]) + __shfl_xor_sync(0xffffffffu, h4 ? p[t] : p[t + C2], 4);
 #pragma unroll
-            for (int t = 0; t < 8; ++t)
-                p[t] = (h2 ? p[t + 8] : p[t]) + __shfl_xor_sync(0xffffffffu, h2 ? p[t] : p[t + 8], 2);
+            for (int t = 0; t < C4; ++t)
+                p[t] = (h2 ? p[t + C4] : p[t]) + __shfl_xor_sync(0xffffffffu, h2 ? p[t] : p[t + C4], 2);
 #pragma unroll
-            for (int t = 0; t < 4; ++t)
-                p[t] = (h1 ? p[t + 4] : p[t]) + __shfl_xor_sync(0xffffffffu, h1 ? p[t] : p[t + 4], 1);
+            for (int t = 0; t < C8; ++t)
+                p[t] = (h1 ? p[t + C8] : p[t]) + __shfl_xor_sync(0xffffffffu, h1 ? p[t] : p[t + C8], 1);
 #pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                const int j = jc + 4 * seg + t;
+            for (int t = 0; t < C8; ++t) {
+                const int j = jc + C8 * seg + t;
                 if (j < P.nb) {
                     const long long d = na + __ldg(P.nB + j) - 2ll * (long long)p[t];
                     const long long key = (d << 32) | (unsigned)j;
@@ -781,17 +844,10 @@ __global__ void __launch_bounds__(256) k_tc_finish(const TcPair* __restrict__ pa
             acc.sum += err;
             ++acc.n;
         }
-        if (!mismatch && accept) {
-            t_row[g] = j1;
-            d_row[g] = (uint32_t)e1;
-        } else if (!mismatch && reject) {
-            t_row[g] = -1;
-            d_row[g] = has1 ? (uint32_t)e1 : 0u;
-        } else {
-            t_row[g] = -1;
-            d_row[g] = 0u;
+        if (!mismatch && accept)
+            atomicMin(P.key + j1, ((unsigned long long)(uint32_t)e1 << 32) | (unsigned)q);
+        else if (mismatch || !reject)
             flagged[atomicAdd(n_flagged, 1)] = g;
-        }
     }
     if (acc.n) {   // err >= 0: its bits order like the values
         atomicMax(reinterpret_cast<int*>(&s_mx), __float_as_int(acc.mx));
@@ -809,8 +865,7 @@ __global__ void __launch_bounds__(256) k_tc_finish(const TcPair* __restrict__ pa
 // Exact fallback for rows the certificate could not settle: one CTA per row, every target.
 __global__ void __launch_bounds__(256) k_tc_exact_rows(const TcPair* __restrict__ pairs, int n_pairs,
                                                        const int32_t* __restrict__ rows, const int* __restrict__ n_rows,
-                                                       float ratio, int32_t* __restrict__ t_row,
-                                                       uint32_t* __restrict__ d_row) {
+                                                       float ratio) {
     __shared__ long long s_k1[8], s_d2[8];
     const int nr = *n_rows;
     for (int ri = blockIdx.x; ri < nr; ri += gridDim.x) {
@@ -850,42 +905,32 @@ __global__ void __launch_bounds__(256) k_tc_exact_rows(const TcPair* __restrict_
             const long long e1 = b1 >> 32;
             const float f1 = (float)e1, f2 = b2 > (1ll << 24) ? 16777216.f : (float)b2;
             const bool ok = b1 != LLONG_MAX && ratio_ok(f1, f2, ratio);
-            t_row[g] = ok ? (int32_t)(b1 & 0xffffffffll) : -1;
-            d_row[g] = b1 != LLONG_MAX ? (uint32_t)e1 : 0u;
+            if (ok) atomicMin(P.key + (b1 & 0xffffffffll), ((unsigned long long)(uint32_t)e1 << 32) | (unsigned)q);
         }
         __syncthreads();
     }
 }
 
 // ------------------------------------------------------------------------ batched _unique
-__global__ void k_tcu_fill(unsigned long long* __restrict__ key, long long n) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) key[i] = ~0ull;
+// matches of each pair by target: a block per pair
+__global__ void __launch_bounds__(COMPACT_T) k_tcu_compact(const TcPair* __restrict__ pairs) {
+    const TcPair& P = pairs[blockIdx.x];
+    unique_compact(P.key, P.nb, P.q_out, P.t_out, P.count);
 }
 
-__global__ void k_tcu_keys(const TcPair* __restrict__ pairs, const int32_t* __restrict__ t_row,
-                           const uint32_t* __restrict__ d_row, unsigned long long* __restrict__ key) {
-    const TcPair& P = pairs[blockIdx.y];
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= P.na) return;
-    const int g = P.row0 + q;
-    const int t = t_row[g];
-    if (t >= 0) atomicMin(key + P.key0 + t, ((unsigned long long)d_row[g] << 32) | (unsigned)q);
-}
-
+// the same for pairs with more targets than a block compacts: flags, a scan over the batch, the gather
 __global__ void k_tcu_flags(const unsigned long long* __restrict__ key, long long n, int32_t* __restrict__ flag) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i <= n) flag[i] = i < n && key[i] != ~0ull;
 }
 
 __global__ void k_tcu_emit(const TcPair* __restrict__ pairs, const unsigned long long* __restrict__ key,
-                           const int32_t* __restrict__ pos, int32_t* __restrict__ counts) {
-    const int p = blockIdx.y;
-    const TcPair& P = pairs[p];
+                           const int32_t* __restrict__ pos) {
+    const TcPair& P = pairs[blockIdx.y];
     const int local = blockIdx.x * blockDim.x + threadIdx.x;
     if (local >= P.nb) return;
     const long long i = P.key0 + local;
-    if (local == P.nb - 1) counts[p] = pos[P.key0 + P.nb] - pos[P.key0];
+    if (local == P.nb - 1) *P.count = pos[P.key0 + P.nb] - pos[P.key0];
     const unsigned long long k = key[i];
     if (k == ~0ull) return;
     const int o = pos[i] - pos[P.key0];
@@ -906,11 +951,12 @@ int32_t tc_launch_dense(const TcPair* d_pairs, int n_pairs, int n_items, Cand* p
 }  // namespace
 
 // Tensor-core dense matching of a batch of pairs, _unique included: pair p writes counts[p]
-// (device) matches into q_out[p], t_out[p] (device, capacity na[p]). Pairs need na, nb >= 1.
+// (device; h_counts, host, nullable) matches into q_out[p], t_out[p] (device, capacity na[p]). Pairs need
+// na, nb >= 1. Waits.
 // Scratch comes from ctx; stats (nullable) receives the certificate and error statistics.
 int32_t run_match_bf_tc(fsb_ctx* ctx, int n_pairs, const uint8_t* const* d_a, const int* na,
                         const uint8_t* const* d_b, const int* nb, float ratio, int precision, int64_t* const* q_out,
-                        int64_t* const* t_out, int32_t* counts, TcStats* stats, cudaStream_t s) {
+                        int64_t* const* t_out, int32_t* counts, int32_t* h_counts, TcStats* stats, cudaStream_t s) {
     if (precision != FSB_PREC_BF16 && precision != FSB_PREC_FP8) {
         set_error("precision %d has no tensor-core path", precision);
         return FSB_ERR_UNSUPPORTED;
@@ -926,19 +972,25 @@ int32_t run_match_bf_tc(fsb_ctx* ctx, int n_pairs, const uint8_t* const* d_a, co
         FSB_CUDA(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev));
     }
     auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
+    // longest sweeps first (see tc_item)
+    std::vector<int> order(n_pairs);
+    for (int p = 0; p < n_pairs; ++p) order[p] = p;
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return nb[x] > nb[y]; });
     std::vector<TcPair> hp(n_pairs);
     size_t off_pa = 0, off_pb = 0, n_norm = 0, n_parts = 0;
     long long n_keys = 0, rb_total = 0;
     int items = 0, rows = 0;
     for (int p = 0; p < n_pairs; ++p) rb_total += (na[p] + TC_ROWS - 1) / TC_ROWS;
-    for (int p = 0; p < n_pairs; ++p) {
-        TcPair& P = hp[p];
+    for (int k = 0; k < n_pairs; ++k) {
+        TcPair& P = hp[k];
+        const int p = order[k];
         P.a = d_a[p];
         P.b = d_b[p];
         P.na = na[p];
         P.nb = nb[p];
         P.q_out = q_out[p];
         P.t_out = t_out[p];
+        P.count = counts + p;
         P.nrb = (na[p] + TC_ROWS - 1) / TC_ROWS;
         P.ntiles = (nb[p] + TC_N - 1) / TC_N;
         int splits = 1;
@@ -965,10 +1017,14 @@ int32_t run_match_bf_tc(fsb_ctx* ctx, int n_pairs, const uint8_t* const* d_a, co
     // scratch layout
     const size_t b_pairs = al((size_t)n_pairs * sizeof(TcPair)), b_segs = al((size_t)2 * n_pairs * sizeof(PackSeg));
     const size_t b_norm = al(n_norm * 4), b_rowsc = fp8 ? al((size_t)rows * 16) : 0, b_bmax = al((size_t)n_pairs * 8);
-    const size_t b_rowi = al((size_t)rows * 4), b_keys = al((size_t)n_keys * 8), b_flag = al((size_t)(n_keys + 1) * 4);
+    const size_t b_rowi = al((size_t)rows * 4), b_keys = al((size_t)n_keys * 8);
+    bool small_targets = true;
+    for (int p = 0; p < n_pairs; ++p) small_targets = small_targets && nb[p] <= kCompactMax;
+    const size_t b_flag = small_targets ? 0 : al((size_t)(n_keys + 1) * 4);
+    if (small_targets) tb_scan = 0;
     FSB_TRY(ctx->s_tc_pack.ensure(al(off_pa) + al(off_pb)));
     FSB_TRY(ctx->s_tc_part.ensure(al(n_parts * sizeof(Cand)) + 256));
-    FSB_TRY(ctx->s_tc_aux.ensure(b_pairs + b_segs + b_norm + b_rowsc + b_bmax + 4 * b_rowi + b_keys + 2 * b_flag +
+    FSB_TRY(ctx->s_tc_aux.ensure(b_pairs + b_segs + b_norm + b_rowsc + b_bmax + b_rowi + b_keys + 2 * b_flag +
                                  al(tb_scan) + 512));
     uint8_t* pack = ctx->s_tc_pack.as<uint8_t>();
     uint8_t* cur = ctx->s_tc_aux.as<uint8_t>();
@@ -982,10 +1038,7 @@ int32_t run_match_bf_tc(fsb_ctx* ctx, int n_pairs, const uint8_t* const* d_a, co
     int32_t* norms = reinterpret_cast<int32_t*>(take(b_norm));
     float* rowsc = reinterpret_cast<float*>(take(b_rowsc));
     float* bmax = reinterpret_cast<float*>(take(b_bmax));
-    int32_t* t_row = reinterpret_cast<int32_t*>(take(b_rowi));
-    uint32_t* d_row = reinterpret_cast<uint32_t*>(take(b_rowi));
     int32_t* flagged = reinterpret_cast<int32_t*>(take(b_rowi));
-    take(b_rowi);
     unsigned long long* keys = reinterpret_cast<unsigned long long*>(take(b_keys));
     int32_t* flag = reinterpret_cast<int32_t*>(take(b_flag));
     int32_t* pos = reinterpret_cast<int32_t*>(take(b_flag));
@@ -1005,6 +1058,7 @@ int32_t run_match_bf_tc(fsb_ctx* ctx, int n_pairs, const uint8_t* const* d_a, co
         P.nB = norms + nn + P.na;
         P.rowsc = fp8 ? rowsc + 4 * rr : nullptr;
         P.bmax = bmax + 2 * p;
+        P.key = keys + P.key0;
         const int pad_a = P.nrb * TC_ROWS, pad_b = P.ntiles * TC_N;
         max_pad = std::max(max_pad, std::max(pad_a, pad_b));
         max_na = std::max(max_na, P.na);
@@ -1020,11 +1074,12 @@ int32_t run_match_bf_tc(fsb_ctx* ctx, int n_pairs, const uint8_t* const* d_a, co
     }
     FSB_CUDA(cudaMemcpyAsync(d_pairs, hp.data(), (size_t)n_pairs * sizeof(TcPair), cudaMemcpyHostToDevice, s));
     FSB_CUDA(cudaMemcpyAsync(d_segs, segs.data(), segs.size() * sizeof(PackSeg), cudaMemcpyHostToDevice, s));
-    const dim3 pack_grid(nblk(max_pad, 8), (unsigned)segs.size());
+    FSB_CUDA(cudaMemsetAsync(keys, 0xff, (size_t)n_keys * 8, s));
+    const dim3 pack_grid(nblk(max_pad, PACK_ROWS), (unsigned)segs.size());
     if (fp8)
-        k_tc_pack<FSB_PREC_FP8><<<pack_grid, 256, 0, s>>>(d_segs);
+        k_tc_pack<FSB_PREC_FP8><<<pack_grid, PACK_T, 0, s>>>(d_segs);
     else
-        k_tc_pack<FSB_PREC_BF16><<<pack_grid, 256, 0, s>>>(d_segs);
+        k_tc_pack<FSB_PREC_BF16><<<pack_grid, PACK_T, 0, s>>>(d_segs);
     note_launch(1);
     FSB_CUDA(cudaGetLastError());
     Cand* part = ctx->s_tc_part.as<Cand>();
@@ -1036,34 +1091,34 @@ int32_t run_match_bf_tc(fsb_ctx* ctx, int n_pairs, const uint8_t* const* d_a, co
     float* err_stat = stats ? reinterpret_cast<float*>(small + 2) : nullptr;
     const dim3 fin_grid(nblk(max_na, 8 * 4 * FIN_PASSES), (unsigned)n_pairs);
     if (fp8)
-        k_tc_finish<TcTraits<FSB_PREC_FP8>::TOPK><<<fin_grid, 256, 0, s>>>(d_pairs, part, ratio, precision, t_row,
-                                                                           d_row, flagged, small + 1, err_stat);
+        k_tc_finish<TcTraits<FSB_PREC_FP8>::TOPK><<<fin_grid, 256, 0, s>>>(d_pairs, part, ratio, precision, flagged,
+                                                                           small + 1, err_stat);
     else
-        k_tc_finish<TcTraits<FSB_PREC_BF16>::TOPK><<<fin_grid, 256, 0, s>>>(d_pairs, part, ratio, precision, t_row,
-                                                                            d_row, flagged, small + 1, err_stat);
-    note_launch(1);
+        k_tc_finish<TcTraits<FSB_PREC_BF16>::TOPK><<<fin_grid, 256, 0, s>>>(d_pairs, part, ratio, precision, flagged,
+                                                                            small + 1, err_stat);
+    // the rows the certificate did not settle (their number is on the device; usually none, and the blocks leave)
+    k_tc_exact_rows<<<std::min(rows, 2 * num_sms), 256, 0, s>>>(d_pairs, n_pairs, flagged, small + 1, ratio);
+    note_launch(2);
+    FSB_CUDA(cudaGetLastError());
+    // _unique of every pair
+    if (small_targets) {
+        k_tcu_compact<<<n_pairs, COMPACT_T, 0, s>>>(d_pairs);
+        note_launch(1);
+    } else {
+        k_tcu_flags<<<nblk(n_keys + 1, 256), 256, 0, s>>>(keys, n_keys, flag);
+        FSB_CUDA(cub::DeviceScan::ExclusiveSum(scan_tmp, tb_scan, flag, pos, (int)(n_keys + 1), s));
+        k_tcu_emit<<<dim3(nblk(max_nb, 256), (unsigned)n_pairs), 256, 0, s>>>(d_pairs, keys, pos);
+        note_launch(2);
+    }
     FSB_CUDA(cudaGetLastError());
     int host_small[5] = {0, 0, 0, 0, 0};
     FSB_CUDA(cudaMemcpyAsync(host_small, small, sizeof(host_small), cudaMemcpyDeviceToHost, s));
+    if (h_counts) FSB_CUDA(cudaMemcpyAsync(h_counts, counts, (size_t)n_pairs * 4, cudaMemcpyDeviceToHost, s));
     FSB_CUDA(cudaStreamSynchronize(s));
     if (host_small[0]) {
         set_error("tensor-core matcher: a pipeline wait timed out");
         return FSB_ERR_CUDA;
     }
-    if (host_small[1] > 0) {
-        k_tc_exact_rows<<<std::min(host_small[1], 8 * num_sms), 256, 0, s>>>(d_pairs, n_pairs, flagged, small + 1,
-                                                                            ratio, t_row, d_row);
-        note_launch(1);
-        FSB_CUDA(cudaGetLastError());
-    }
-    // _unique of every pair
-    k_tcu_fill<<<nblk(n_keys, 256), 256, 0, s>>>(keys, n_keys);
-    k_tcu_keys<<<dim3(nblk(max_na, 256), (unsigned)n_pairs), 256, 0, s>>>(d_pairs, t_row, d_row, keys);
-    k_tcu_flags<<<nblk(n_keys + 1, 256), 256, 0, s>>>(keys, n_keys, flag);
-    FSB_CUDA(cub::DeviceScan::ExclusiveSum(scan_tmp, tb_scan, flag, pos, (int)(n_keys + 1), s));
-    k_tcu_emit<<<dim3(nblk(max_nb, 256), (unsigned)n_pairs), 256, 0, s>>>(d_pairs, keys, pos, counts);
-    note_launch(5);
-    FSB_CUDA(cudaGetLastError());
     if (stats) {
         float mx, sum;
         memcpy(&mx, &host_small[2], 4);
