@@ -48,19 +48,19 @@ __device__ __forceinline__ void warp_append(bool flag, const T& v, T* out, uint3
     }
 }
 
-// k_extrema: a block is 8 warps side by side over 240 interior columns of an EX_ROWS-row chunk of
+// k_extrema: a block is EX_W warps side by side over 62 EX_W interior columns of a chunk of `rows` rows of
 // one octave; each warp walks its chunk row by row (see the kernel).
-constexpr int EX_T = 256;            // 8 warps per block
-constexpr int EX_COLS = 30;          // output columns per warp (lanes 1..30; lanes 0 and 31 are halo)
-constexpr int EX_ROWS = 64;          // rows per block (a chunk of the octave's interior rows)
+constexpr int EX_W = 4, EX_T = 32 * EX_W;   // warps, threads per block
+constexpr int EX_COLS = 62;                 // output columns per warp: two per lane, the outermost two are halo
+constexpr int EX_BLOCKS = 7;                // resident blocks per SM
 
 struct ExTiles {
-    int n_oct;
+    int n_oct, rows;
     int col_tiles[MAXO], row_tiles[MAXO];
     int first[MAXO + 1];     // first block of each octave
 };
 
-constexpr int EX_DEPTH = 9;          // rows in flight per lane (the shared-memory ring's slots)
+constexpr int EX_DEPTH = 5;          // rows in flight per lane (the shared-memory ring's slots)
 
 // three-input maximum / minimum (one instruction on sm_100); exact, so the same values as two
 // two-input ones
@@ -75,21 +75,25 @@ __device__ __forceinline__ float min3f(float a, float b, float c) {
     return d;
 }
 
-__device__ __forceinline__ void ex_cp_async4(float* dst, const float* src) {
+__device__ __forceinline__ void ex_cp_async8(float2* dst, const float* src) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
 }
 
-// Streaming 3x3x3 extremum test: each warp walks down a chunk of rows of 30 interior columns;
-// every DoG value is read once (coalesced, EX_DEPTH rows ahead through a shared-memory ring),
-// horizontal neighbours come from the adjacent lanes,
-// the 3-row vertical window of the horizontal maxima / minima stays in registers. A voxel is an
-// extremum when it equals the maximum (minimum) of its 27-neighbourhood - ties count - and is
-// beyond the threshold, as scipy's maximum_filter / minimum_filter test in the reference
-// (gsift.py:293-319). Candidates of a row are appended with one warp-aggregated atomic.
-__global__ void __launch_bounds__(EX_T, 4) k_extrema(const float* __restrict__ DF, DetectConsts k, ExTiles tl,
+// Streaming 3x3x3 extremum test: each warp walks down a chunk of rows of 62 interior columns, two columns
+// per lane; every DoG value is read once (coalesced, EX_DEPTH rows ahead through a shared-memory ring).
+// Per row and column the maxima / minima over the three layers around layers 1..3 come first, then
+// over the three columns (a lane's other column and one shuffled neighbour), and over the 3-row
+// window kept in registers. A voxel is an extremum when it equals the maximum (minimum) of its
+// 27-neighbourhood - ties count - and is beyond the threshold, as scipy's maximum_filter / minimum_filter
+// test in the reference (gsift.py:293-319). Candidates of a row are appended with one atomic.
+//
+// Bound by instruction issue (max / min on the ALU pipe at half rate; HBM, 557 MB, would allow 85 us). Two
+// columns per lane share a row's addresses, copies, loop and half of its shuffles, and a smaller window
+// (the layers are reduced first) leaves the registers for it. 2640 x 1978: 181 -> 138 us.
+__global__ void __launch_bounds__(EX_T, EX_BLOCKS) k_extrema(const float* __restrict__ DF, DetectConsts k, ExTiles tl,
                                                   uint32_t* __restrict__ cand, uint32_t* counter, uint32_t cap) {
-    __shared__ float ex_ring[EX_DEPTH * 5 * EX_T];
+    __shared__ float2 ex_ring[EX_DEPTH * 5 * EX_T];
     int o = 0;
     while (o + 1 < tl.n_oct && (int)blockIdx.x >= tl.first[o + 1]) ++o;
     const int b = blockIdx.x - tl.first[o];
@@ -98,95 +102,99 @@ __global__ void __launch_bounds__(EX_T, 4) k_extrema(const float* __restrict__ D
     const long long RC = (long long)R * P;
     const float* base = DF + k.g.dog_off[o];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int c = BORDER + (cx * (EX_T / 32) + wid) * EX_COLS + lane - 1;   // this lane's column
-    const int cc = min(max(c, 0), C - 1);                                    // clamped for loading
-    const bool col_ok = lane >= 1 && lane <= EX_COLS && c >= BORDER && c < C - BORDER;
-    const int y0 = BORDER + ry * EX_ROWS, y1 = min(y0 + EX_ROWS, R - BORDER);   // output rows [y0, y1)
-    // one row of the 3-row window: for layers 1..3, the maximum / minimum over the three layers
-    // around and the three columns around, and the centre value
+    // this lane's columns c, c + 1: even, so a pair is one aligned 8-byte copy (clamped into the pitch)
+    const int c = BORDER - 1 + (cx * EX_W + wid) * EX_COLS + 2 * lane;
+    static_assert((BORDER - 1) % 2 == 0 && EX_COLS % 2 == 0, "8-byte column pairs");
+    const bool ok0 = lane > 0 && c < C - BORDER, ok1 = lane < 31 && c + 1 < C - BORDER;
+    const int y0 = BORDER + ry * tl.rows, y1 = min(y0 + tl.rows, R - BORDER);   // output rows [y0, y1)
+    // one row of the 3-row window, per column: the maximum / minimum over the three layers around layers
+    // 1..3 and the three columns around
     struct Row {
-        float hx[N_LAYERS], hn[N_LAYERS], c[N_LAYERS];
+        float hx[2][N_LAYERS], hn[2][N_LAYERS], c[2][N_LAYERS];
     };
-    // Row r's five layer values at this lane's column arrive by 4-byte cp.async into the lane's own
-    // ring slot ((r - (y0 - 1)) % EX_DEPTH), EX_DEPTH rows ahead of the row being finished; only the
-    // lane that copied a value reads it, so a lane waits on its own copy groups and no barrier is
-    // needed. One commit group per row (empty past the last needed row) keeps the count uniform.
-    float* ring = ex_ring + threadIdx.x;   // element (slot, l) at ring[(slot * 5 + l) * EX_T]
-    const float* colp = base + cc;
+    // Row r's five layer pairs arrive by 8-byte cp.async into the lane's own ring slot, EX_DEPTH rows ahead
+    // of the row being finished; only the lane that copied a value reads it, so a lane waits on its own
+    // copy groups and no barrier is needed. One commit group per row (empty past the last needed row)
+    // keeps the count uniform; the slot just read takes the next row.
+    float2* ring = ex_ring + threadIdx.x;   // element (slot, l) at ring[(slot * 5 + l) * EX_T]
     const int last_row = min(y1 + 1, R - 1);
-    int next_row = y0 - 1, next_slot = 0, take_slot = 0;
-    auto issue_next = [&]() {
-        if (next_row <= last_row) {
-            const float* src = colp + (long long)next_row * P;
+    const float* next = base + (long long)(y0 - 1) * P + min(c, P - 2);
+    int rows_left = last_row - (y0 - 1) + 1, slot = 0;
+    auto issue_next = [&](int at) {
+        if (rows_left > 0) {
 #pragma unroll
-            for (int l = 0; l < 5; ++l) ex_cp_async4(ring + (next_slot * 5 + l) * EX_T, src + l * RC);
+            for (int l = 0; l < 5; ++l) ex_cp_async8(ring + at + l * EX_T, next + l * RC);
+            next += P;
+            --rows_left;
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
-        ++next_row;
-        next_slot = next_slot + 1 == EX_DEPTH ? 0 : next_slot + 1;
-    };
-    // the oldest row in flight, once landed (EX_DEPTH groups outstanding -> wait for all but the
-    // newest EX_DEPTH - 1), then its slot gets the next row
-    auto take_row = [&](float (&raw)[5]) {
-        asm volatile("cp.async.wait_group %0;\n" ::"n"(EX_DEPTH - 1) : "memory");
-#pragma unroll
-        for (int l = 0; l < 5; ++l) raw[l] = ring[(take_slot * 5 + l) * EX_T];
-        take_slot = take_slot + 1 == EX_DEPTH ? 0 : take_slot + 1;
-        issue_next();
-    };
-    auto finish_row = [&](Row& w, const float (&raw)[5]) {
-#pragma unroll
-        for (int l = 0; l < N_LAYERS; ++l) {
-            const float mx = max3f(raw[l], raw[l + 1], raw[l + 2]), mn = min3f(raw[l], raw[l + 1], raw[l + 2]);
-            w.hx[l] = max3f(__shfl_up_sync(0xffffffffu, mx, 1), mx, __shfl_down_sync(0xffffffffu, mx, 1));
-            w.hn[l] = min3f(__shfl_up_sync(0xffffffffu, mn, 1), mn, __shfl_down_sync(0xffffffffu, mn, 1));
-            w.c[l] = raw[l + 1];
-        }
     };
     auto load_row = [&](Row& w) {
-        float raw[5];
-        take_row(raw);
-        finish_row(w, raw);
+        // the oldest row in flight, once landed (EX_DEPTH groups outstanding -> wait for all but the
+        // newest EX_DEPTH - 1)
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(EX_DEPTH - 1) : "memory");
+        float2 raw[5];
+#pragma unroll
+        for (int l = 0; l < 5; ++l) raw[l] = ring[slot + l * EX_T];
+        issue_next(slot);
+        slot = slot == (EX_DEPTH - 1) * 5 * EX_T ? 0 : slot + 5 * EX_T;
+#pragma unroll
+        for (int l = 0; l < N_LAYERS; ++l) {
+            const float mx0 = max3f(raw[l].x, raw[l + 1].x, raw[l + 2].x), mx1 = max3f(raw[l].y, raw[l + 1].y, raw[l + 2].y);
+            const float mn0 = min3f(raw[l].x, raw[l + 1].x, raw[l + 2].x), mn1 = min3f(raw[l].y, raw[l + 1].y, raw[l + 2].y);
+            w.hx[0][l] = max3f(__shfl_up_sync(0xffffffffu, mx1, 1), mx0, mx1);
+            w.hx[1][l] = max3f(mx0, mx1, __shfl_down_sync(0xffffffffu, mx0, 1));
+            w.hn[0][l] = min3f(__shfl_up_sync(0xffffffffu, mn1, 1), mn0, mn1);
+            w.hn[1][l] = min3f(mn0, mn1, __shfl_down_sync(0xffffffffu, mn0, 1));
+            w.c[0][l] = raw[l + 1].x;
+            w.c[1][l] = raw[l + 1].y;
+        }
     };
     const float tmax = nextafterf(k.pthr, INFINITY), tmin = nextafterf(-k.pthr, -INFINITY);
+    const uint32_t flat0 = (uint32_t)(k.g.dog_off[o] + RC + c);   // layer 1, row 0 of this lane's first column
     // test row y from the window (up, mid, dn), append its extrema, then finish row y + 2 into `up`
     // (no longer needed): the three windows rotate by name, not by register moves
     auto step = [&](Row& up, const Row& mid, const Row& dn, int y) {
-        unsigned mask = 0;
+        bool hit[2][N_LAYERS];
+        bool any = false;
 #pragma unroll
-        for (int l = 0; l < N_LAYERS; ++l) {
-            // v is one of the 27 values, so v >= their maximum and v > pthr is v >= the larger of the
-            // maximum and the float after pthr; the same for the minimum
-            const float v = mid.c[l];
-            const float mx = fmaxf(max3f(up.hx[l], mid.hx[l], dn.hx[l]), tmax);
-            const float mn = fminf(min3f(up.hn[l], mid.hn[l], dn.hn[l]), tmin);
-            if (v >= mx || v <= mn) mask |= 1u << l;
-        }
-        if (!col_ok) mask = 0;
-        const unsigned any = __ballot_sync(0xffffffffu, mask != 0);
-        if (any) {
-            const int cntv = __popc(mask);
-            int incl = cntv;
+        for (int q = 0; q < 2; ++q)
 #pragma unroll
-            for (int sh = 1; sh < 32; sh <<= 1) {
-                const int t = __shfl_up_sync(0xffffffffu, incl, sh);
-                if (lane >= sh) incl += t;
+            for (int l = 0; l < N_LAYERS; ++l) {
+                // v is one of the 27 values, so v >= their maximum and v > pthr is v >= the larger of
+                // the maximum and the float after pthr; the same for the minimum
+                const float v = mid.c[q][l];
+                const float mx = fmaxf(max3f(up.hx[q][l], mid.hx[q][l], dn.hx[q][l]), tmax);
+                const float mn = fminf(min3f(up.hn[q][l], mid.hn[q][l], dn.hn[q][l]), tmin);
+                hit[q][l] = (q ? ok1 : ok0) && (v >= mx || v <= mn);
+                any = any || hit[q][l];
             }
-            const int total = __shfl_sync(0xffffffffu, incl, 31);
-            uint32_t basepos = 0;
-            if (lane == 31) basepos = atomicAdd(counter, (uint32_t)total);
-            basepos = __shfl_sync(0xffffffffu, basepos, 31);
-            uint32_t pos = basepos + (uint32_t)(incl - cntv);
-            while (mask) {
-                const int bit = __ffs(mask) - 1;
-                mask &= mask - 1;
-                if (pos < cap) cand[pos] = (uint32_t)(k.g.dog_off[o] + (bit + 1) * RC + (long long)y * P + c);
-                ++pos;
-            }
+        if (__any_sync(0xffffffffu, any)) {
+            unsigned m[2][N_LAYERS];
+            int total = 0;
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+#pragma unroll
+                for (int l = 0; l < N_LAYERS; ++l) {
+                    m[q][l] = __ballot_sync(0xffffffffu, hit[q][l]);
+                    total += __popc(m[q][l]);
+                }
+            uint32_t pos = 0;
+            if (lane == 0) pos = atomicAdd(counter, (uint32_t)total);
+            pos = __shfl_sync(0xffffffffu, pos, 0);
+            const unsigned lt = (1u << lane) - 1u;
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+#pragma unroll
+                for (int l = 0; l < N_LAYERS; ++l) {
+                    const uint32_t at = pos + __popc(m[q][l] & lt);
+                    if (hit[q][l] && at < cap) cand[at] = flat0 + (uint32_t)((long long)l * RC + (long long)y * P + q);
+                    pos += __popc(m[q][l]);
+                }
         }
         load_row(up);   // row y + 2
     };
-    for (int i = 0; i < EX_DEPTH; ++i) issue_next();   // rows y0 - 1 .. y0 + EX_DEPTH - 2
+    for (int i = 0; i < EX_DEPTH; ++i) issue_next(i * 5 * EX_T);   // rows y0 - 1 .. y0 + EX_DEPTH - 2
     Row w0, w1, w2;
     load_row(w0);   // y0 - 1
     load_row(w1);   // y0
@@ -201,20 +209,40 @@ __global__ void __launch_bounds__(EX_T, 4) k_extrema(const float* __restrict__ D
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");   // no copy outlives the block
 }
 
-ExTiles make_tiles(const Geometry& g, int* total) {
+ExTiles make_tiles_rows(const Geometry& g, int rows, int* total) {
     ExTiles t{};
     t.n_oct = g.n_oct;
+    t.rows = rows;
     int acc = 0;
     for (int o = 0; o < g.n_oct; ++o) {
         t.first[o] = acc;
         const int inner_c = g.C[o] - 2 * BORDER, inner_r = g.R[o] - 2 * BORDER;
-        t.col_tiles[o] = inner_c > 0 ? (inner_c + (EX_T / 32) * EX_COLS - 1) / ((EX_T / 32) * EX_COLS) : 0;
-        t.row_tiles[o] = inner_r > 0 ? (inner_r + EX_ROWS - 1) / EX_ROWS : 0;
+        t.col_tiles[o] = inner_c > 0 ? (inner_c + EX_W * EX_COLS - 1) / (EX_W * EX_COLS) : 0;
+        t.row_tiles[o] = inner_r > 0 ? (inner_r + rows - 1) / rows : 0;
         acc += t.col_tiles[o] * t.row_tiles[o];
     }
     t.first[g.n_oct] = acc;
     *total = acc;
     return t;
+}
+// Rows per chunk: the shortest schedule of waves of resident blocks, a chunk costing its rows plus
+// about ten (the two halo rows and filling the ring). A small image takes short chunks - its blocks all
+// run at once, and a chunk's rows are one after another (320 x 240: 50 us with 64-row chunks, 16 us) -
+// a large one the chunk that fills its last wave.
+ExTiles make_tiles(const Geometry& g, int* total) {
+    ExTiles best{};
+    long long cost = 0;
+    for (int rows = 96; rows >= 8; rows -= 4) {
+        int n = 0;
+        const ExTiles t = make_tiles_rows(g, rows, &n);
+        const long long c = (long long)((n + EX_BLOCKS * 148 - 1) / (EX_BLOCKS * 148)) * (rows + 10);
+        if (rows == 96 || c < cost) {
+            best = t;
+            cost = c;
+            *total = n;
+        }
+    }
+    return best;
 }
 
 // The extremum candidates of every octave in one launch, appended to `cand` through `cnt[0]`.
