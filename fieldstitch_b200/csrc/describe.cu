@@ -32,7 +32,9 @@ __device__ __forceinline__ float kp_scale(int l, float x2) {
 }
 
 // --------------------------------------------------------------------------------- orientation
-constexpr int OW = 4;   // warps per block
+constexpr int OW = 4;          // warps per block
+constexpr int ORI_AHEAD = 4;   // gradient gathers in flight per lane (two, issued together: 86 us; these: 77 us for
+                               // 18 000 extrema of a 2640 x 1978 photo; bound by the gathers' latency)
 
 // Acc = double reproduces the reference's float64 bincount in every case that matters (exact
 // mode); Acc = float (per-lane sums of at most 35 samples, then a float64 lane reduction) halves
@@ -69,47 +71,55 @@ __global__ void __launch_bounds__(OW * 32) k_orient(const float2* __restrict__ G
         // position advances by (32 / W, 32 % W) per step, one division per keypoint
         const int dq = 32 / W, dr = 32 - dq * W;
         int ii = lane / W - rad, jj = lane - (lane / W) * W - rad;
-        // two samples per step: both gathers are issued before either is accumulated (the
-        // accumulation order of the lane is unchanged)
-        for (int s = lane; s < W * W; s += 64) {
-            int ii2 = ii + dq, jj2 = jj + dr;
-            if (jj2 > rad) {
-                jj2 -= W;
-                ++ii2;
-            }
-            const int y1 = e.r + ii, x1 = e.c + jj, y2 = e.r + ii2, x2 = e.c + jj2;
-            const bool in1 = y1 > 0 && y1 < R - 1 && x1 > 0 && x1 < C - 1;
-            const bool in2 = s + 32 < W * W && y2 > 0 && y2 < R - 1 && x2 > 0 && x2 < C - 1;
-            const long long g1 = gb + (long long)y1 * P + x1, g2 = gb + (long long)y2 * P + x2;
-            const float2 s1 = in1 ? __ldg(GRAD + g1) : make_float2(0.f, 0.f);
-            const float2 s2 = in2 ? __ldg(GRAD + g2) : make_float2(0.f, 0.f);
-            const float m1 = s1.x, a1 = s1.y, m2 = s2.x, a2 = s2.y;
-            if (in1) {
-                const float w = expf(-(float)(ii * ii + jj * jj) / den);
-                int b = (int)rintf(a1 * 0.1f);   // angles lie in [0, 360]: b in [0, 36]
-                if (b >= ORI_BINS) b -= ORI_BINS;
-                if (b < 0) b += ORI_BINS;
-                acc[b][lane] += (Acc)(m1 * w);
-            }
-            if (in2) {
-                const float w = expf(-(float)(ii2 * ii2 + jj2 * jj2) / den);
-                int b = (int)rintf(a2 * 0.1f);
-                if (b >= ORI_BINS) b -= ORI_BINS;
-                if (b < 0) b += ORI_BINS;
-                acc[b][lane] += (Acc)(m2 * w);
-            }
-            ii = ii2 + dq;
-            jj = jj2 + dr;
+        // ORI_AHEAD samples in flight: a slot's next gather is issued before the slot's sample is
+        // accumulated (the accumulation order of the lane is row-major)
+        int qd[ORI_AHEAD];      // squared distance, -1 outside the window's interior
+        float2 qg[ORI_AHEAD];
+        int s_next = lane;
+        auto fetch = [&](int u) {
+            const int y = e.r + ii, x = e.c + jj;
+            const bool in = s_next < W * W && y > 0 && y < R - 1 && x > 0 && x < C - 1;
+            qd[u] = in ? ii * ii + jj * jj : -1;
+            if (in) qg[u] = __ldg(GRAD + gb + (long long)y * P + x);
+            s_next += 32;
+            ii += dq;
+            jj += dr;
             if (jj > rad) {
                 jj -= W;
                 ++ii;
             }
+        };
+#pragma unroll
+        for (int u = 0; u < ORI_AHEAD; ++u) {
+            qg[u] = make_float2(0.f, 0.f);
+            fetch(u);
+        }
+        for (int s = 0; s < W * W; s += 32 * ORI_AHEAD) {
+#pragma unroll
+            for (int u = 0; u < ORI_AHEAD; ++u) {
+                const int d2 = qd[u];
+                const float2 gv = qg[u];
+                fetch(u);
+                if (d2 >= 0) {
+                    const float w = expf(-(float)d2 / den);
+                    int b = (int)rintf(gv.y * 0.1f);   // angles lie in [0, 360]: b in [0, 36]
+                    if (b >= ORI_BINS) b -= ORI_BINS;
+                    if (b < 0) b += ORI_BINS;
+                    acc[b][lane] += (Acc)(gv.x * w);
+                }
+            }
         }
         __syncwarp();
-        for (int b = lane; b < ORI_BINS; b += 32) {
-            double t = 0.0;
-            for (int l = 0; l < 32; ++l) t += (double)acc[b][l];
-            s_raw[wid][b] = (float)t;
+        {   // lane order in float64: a bin per lane, then the last four bins by lanes 0..3 on the same sweep
+            double t = 0.0, u = 0.0;
+            const int b2 = 32 + (lane & 3);
+#pragma unroll 8
+            for (int l = 0; l < 32; ++l) {
+                t += (double)acc[lane][l];
+                u += (double)acc[b2][l];
+            }
+            s_raw[wid][lane] = (float)t;
+            if (lane < ORI_BINS - 32) s_raw[wid][32 + lane] = (float)u;
         }
         __syncwarp();
         float hmax = 0.f;
