@@ -232,8 +232,8 @@ int32_t launch_layer_fast(int layer, const float* src, int R, int C, int P, floa
                           float* down, int down_pitch, int variant, int* err, cudaStream_t s);
 int32_t launch_base_fast(const uint8_t* img, int stride, int ih, int iw, int P, float* dst, int variant, cudaStream_t s);
 int32_t launch_group_lower(const float* src, int R, int C, int P, float* dog, float2* grad, float* l3, float* down,
-                           int down_pitch, cudaStream_t s);
-int32_t launch_group_upper(const float* src, int R, int C, int P, float* dog3, cudaStream_t s);
+                           int down_pitch, bool small, cudaStream_t s);
+int32_t launch_group_upper(const float* src, int R, int C, int P, float* dog3, bool small, cudaStream_t s);
 constexpr int PYR_ERR_WORD = 8;   // index of the pyramid's error word in Workspace::counters
 // autotune.cu: the fastest of n_variants launches of `run` for `key` (timed once per process and
 // device on `s`, then cached; FSB_AUTOTUNE=0 returns variant 0, FSB_AUTOTUNE_FILE persists choices)

@@ -639,7 +639,8 @@ int32_t launch_layer_t(const LayerArgs& a, int variant, cudaStream_t s) {
 
 // ------------------------------------------------------------------------------------------------
 // Fused layer groups (float32 path): one persistent kernel computes consecutive layers of an
-// octave for 128 x 32 output tiles,
+// octave for output tiles of 128 x 32 (or smaller ones for octaves that would leave SMs idle, see
+// launch_group_small),
 //   group 0: L1, L2, L3 from L0 -> DoG 0..2, gradients of L1..L3, L3 and L3[::2, ::2]
 //   group 1: L4, L5 from L3     -> DoG 3, 4
 // Every level is held in shared memory on the tile plus the halo the levels above it need (row
@@ -652,7 +653,14 @@ int32_t launch_layer_t(const LayerArgs& a, int variant, cudaStream_t s) {
 // kernel's (8-row register window of column pairs; row-pair-interleaved horizontal pass), with
 // the DoG / gradient epilogue of a level run by the horizontal pass of the level above it. One
 // CTA per SM walks the tiles; the next tile's input arrives by cp.async while this one computes.
-constexpr int GX = 128, GY = 32, GNT = 512;
+// tile and threads: the large tile has the least halo, the small ones the shortest chain of passes
+template <int X, int Y, int T>
+struct GTile {
+    static constexpr int GX = X, GY = Y, GNT = T;
+};
+using GLarge = GTile<128, 32, 512>;
+using GMid = GTile<64, 16, 384>;
+using GSmall = GTile<32, 16, 256>;
 
 __host__ __device__ constexpr int cmax(int a, int b) { return a > b ? a : b; }
 
@@ -660,8 +668,10 @@ __host__ __device__ constexpr int cmax(int a, int b) { return a > b ? a : b; }
 // the level below (Hi, Xi). The vertical pass covers input columns VS .. VS + VW - 1 (VS even);
 // column j of its output sits at float2 index j + E of a row pair, so the horizontal pass's
 // 16-byte loads start on an even index.
-template <int Hi, int Xi, int Ho, int Xo, int r>
-struct GLevel {
+template <class Tile, int Hi, int Xi, int Ho, int Xo, int r>
+struct GLevel : Tile {
+    using Tile::GX;
+    using Tile::GY;
     static constexpr int HIN = Hi, XIN = Xi, HOUT = Ho, XOUT = Xo, RAD = r;
     static constexpr int NIN = GY + 2 * Hi, MIN = GX + 2 * Xi;     // input rows, columns (= pitch)
     static constexpr int NOUT = GY + 2 * Ho, MOUT = GX + 2 * Xo;   // output rows, columns (= pitch)
@@ -677,31 +687,32 @@ struct GLevel {
     static_assert(VS + VW <= MIN, "vertical pass inside the input level");
 };
 
-template <int G>
+template <int G, class Tile>
 struct GSpec;
-template <>
-struct GSpec<0> {
-    using A = GLevel<20, 28, 15, 20, 5>;   // L0 -> L1
-    using B = GLevel<15, 20, 9, 12, 6>;    // L1 -> L2
-    using C = GLevel<9, 12, 1, 4, 8>;      // L2 -> L3 (halo 1: gradient of L3)
+template <class Tile>
+struct GSpec<0, Tile> {
+    using A = GLevel<Tile, 20, 28, 15, 20, 5>;   // L0 -> L1
+    using B = GLevel<Tile, 15, 20, 9, 12, 6>;    // L1 -> L2
+    using C = GLevel<Tile, 9, 12, 1, 4, 8>;      // L2 -> L3 (halo 1: gradient of L3)
     static constexpr int BUF0 = (cmax(A::IN_FLOATS, cmax(B::V_FLOATS, C::V_FLOATS)) + 3) & ~3;   // L0 / V2 / V3
     static constexpr int BUF1 = (cmax(A::V_FLOATS, B::OUT_FLOATS) + 3) & ~3;                     // V1 / L2
     static constexpr int BUF2 = (cmax(A::OUT_FLOATS, C::OUT_FLOATS) + 3) & ~3;                   // L1 / L3
 };
-template <>
-struct GSpec<1> {
-    using A = GLevel<23, 28, 13, 16, 10>;   // L3 -> L4
-    using B = GLevel<13, 16, 0, 0, 13>;     // L4 -> L5 (tile only)
+template <class Tile>
+struct GSpec<1, Tile> {
+    using A = GLevel<Tile, 23, 28, 13, 16, 10>;   // L3 -> L4
+    using B = GLevel<Tile, 13, 16, 0, 0, 13>;     // L4 -> L5 (tile only)
     static constexpr int BUF0 = (cmax(A::IN_FLOATS, B::V_FLOATS) + 3) & ~3;   // L3 / V5
     static constexpr int BUF1 = (A::V_FLOATS + 3) & ~3;                       // V4
     static constexpr int BUF2 = (A::OUT_FLOATS + 3) & ~3;                     // L4
 };
 // two input buffers (this tile's, the next tile's) and the two others
-template <int G>
+template <int G, class Tile>
 constexpr int group_smem() {
-    return (2 * GSpec<G>::BUF0 + GSpec<G>::BUF1 + GSpec<G>::BUF2) * 4;
+    return (2 * GSpec<G, Tile>::BUF0 + GSpec<G, Tile>::BUF1 + GSpec<G, Tile>::BUF2) * 4;
 }
-static_assert(group_smem<0>() <= 227 * 1024 && group_smem<1>() <= 227 * 1024, "group shared memory");
+static_assert(group_smem<0, GLarge>() <= 227 * 1024 && group_smem<1, GLarge>() <= 227 * 1024, "group shared memory");
+static_assert(group_smem<0, GMid>() <= 113 * 1024 && group_smem<0, GSmall>() <= 75 * 1024, "two and three per SM");
 
 struct GroupArgs {
     const float* src;   // the group's input level, R x C
@@ -717,7 +728,8 @@ struct GroupArgs {
 // input level of tile t (rows y0 - HIN .., columns x0 - XIN .., reflect-101 outside) by cp.async
 template <class L>
 __device__ __forceinline__ void g_load(const GroupArgs& a, int t, float* dst) {
-    const int y0 = (t / a.tiles_x) * GY, cx = (t % a.tiles_x) * GX - L::XIN;
+    constexpr int GNT = L::GNT;
+    const int y0 = (t / a.tiles_x) * L::GY, cx = (t % a.tiles_x) * L::GX - L::XIN;
     if (cx >= 0 && cx + L::MIN <= a.C) {
         // eight lanes per row (the mirrored row address once per row)
         for (int row = threadIdx.x >> 3; row < L::NIN; row += GNT / 8) {
@@ -743,7 +755,7 @@ __device__ __forceinline__ void g_load(const GroupArgs& a, int t, float* dst) {
 // are computed (a tile that reaches past the image needs its level only to the halo beyond it).
 template <int TS, class L>
 __device__ __forceinline__ void g_vpass(const float* __restrict__ pin, float2* __restrict__ v, int kmax, int jmax) {
-    constexpr int r = L::RAD, NQ = L::VW / 2, NG = (L::NOUT + 7) / 8;
+    constexpr int r = L::RAD, NQ = L::VW / 2, NG = (L::NOUT + 7) / 8, GNT = L::GNT;
     static_assert(L::NOUT >= 8 && L::NIN == L::NOUT + 2 * r + 2 * L::ROFF, "vertical pass rows");
     float2 w[r + 1];
     load_taps<TS, r>(w);
@@ -773,7 +785,7 @@ __device__ __forceinline__ void g_vpass(const float* __restrict__ pin, float2* _
 template <int TS, class L, class Epi>
 __device__ __forceinline__ void g_hpass(const float2* __restrict__ v, float* __restrict__ pout, Epi epi, int kmax,
                                         int jmax) {
-    constexpr int r = L::RAD, NC = L::MOUT / 4, NP = L::NOUT / 2;
+    constexpr int r = L::RAD, NC = L::MOUT / 4, NP = L::NOUT / 2, GNT = L::GNT;
     float2 w[r + 1];
     load_taps<TS, r>(w);
     for (int it = threadIdx.x; it < NP * NC; it += GNT) {
@@ -817,7 +829,7 @@ __device__ __forceinline__ void g_dog_grad(const GroupArgs& a, int yy, int xx, c
 
 // epilogue of a level: for the tile pixels of an item, DoG (this level - prev) and the gradient of
 // prev, prev being the shared level (halo PH, PX, pitch P) below
-template <int PH, int PX, int P>
+template <class Tile, int PH, int PX, int P>
 struct GEpi {
     const GroupArgs& a;
     int y0, x0;
@@ -825,19 +837,20 @@ struct GEpi {
     float* dog;
     float2* grad;
     __device__ __forceinline__ void operator()(int ty, int tx, float4 top, float4 bot) const {
-        if (tx < 0 || tx >= GX || x0 + tx >= a.C) return;
+        if (tx < 0 || tx >= Tile::GX || x0 + tx >= a.C) return;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int t = ty + h;
-            if (t < 0 || t >= GY || y0 + t >= a.R) continue;
+            if (t < 0 || t >= Tile::GY || y0 + t >= a.R) continue;
             g_dog_grad<P>(a, y0 + t, x0 + tx, prev + (PH + t) * P + PX + tx, h ? bot : top, dog, grad);
         }
     }
 };
 
-template <int G>
-__global__ void __launch_bounds__(GNT, 1) k_group(GroupArgs a) {
-    using Sp = GSpec<G>;
+template <int G, class Tile>
+__global__ void __launch_bounds__(Tile::GNT, Tile::GX == 128 ? 1 : Tile::GX == 64 ? 2 : 3) k_group(GroupArgs a) {
+    constexpr int GX = Tile::GX, GY = Tile::GY, GNT = Tile::GNT;
+    using Sp = GSpec<G, Tile>;
     using LA = typename Sp::A;
     extern __shared__ __align__(16) float sm[];
     float* b1 = sm + 2 * Sp::BUF0;
@@ -861,19 +874,19 @@ __global__ void __launch_bounds__(GNT, 1) k_group(GroupArgs a) {
             g_vpass<1, LA>(b0, reinterpret_cast<float2*>(b1), vy + 2 * LA::HOUT, vx + 2 * LA::XOUT);  // L0 -> V1
             __syncthreads();
             g_hpass<1, LA>(reinterpret_cast<const float2*>(b1), b2,                               // V1 -> L1
-                           GEpi<LA::HIN, LA::XIN, LA::MIN>{a, y0, x0, b0, a.dog[0], nullptr},
+                           GEpi<Tile, LA::HIN, LA::XIN, LA::MIN>{a, y0, x0, b0, a.dog[0], nullptr},
                            vy + 2 * LA::HOUT, vx + 2 * LA::XOUT);
             __syncthreads();
             g_vpass<2, LB>(b2, reinterpret_cast<float2*>(b0), vy + 2 * LB::HOUT, vx + 2 * LB::XOUT);  // L1 -> V2
             __syncthreads();
             g_hpass<2, LB>(reinterpret_cast<const float2*>(b0), b1,                               // V2 -> L2
-                           GEpi<LB::HIN, LB::XIN, LB::MIN>{a, y0, x0, b2, a.dog[1], a.grad[0]},
+                           GEpi<Tile, LB::HIN, LB::XIN, LB::MIN>{a, y0, x0, b2, a.dog[1], a.grad[0]},
                            vy + 2 * LB::HOUT, vx + 2 * LB::XOUT);
             __syncthreads();
             g_vpass<3, LC>(b1, reinterpret_cast<float2*>(b0), vy + 2 * LC::HOUT, vx + 2 * LC::XOUT);  // L2 -> V3
             __syncthreads();
             g_hpass<3, LC>(reinterpret_cast<const float2*>(b0), b2,                               // V3 -> L3
-                           GEpi<LC::HIN, LC::XIN, LC::MIN>{a, y0, x0, b1, a.dog[2], a.grad[1]},
+                           GEpi<Tile, LC::HIN, LC::XIN, LC::MIN>{a, y0, x0, b1, a.dog[2], a.grad[1]},
                            vy + 2 * LC::HOUT, vx + 2 * LC::XOUT);
             __syncthreads();
             // gradient of L3, L3 and L3[::2, ::2] on the tile
@@ -899,13 +912,13 @@ __global__ void __launch_bounds__(GNT, 1) k_group(GroupArgs a) {
             g_vpass<4, LA>(b0, reinterpret_cast<float2*>(b1), vy + 2 * LA::HOUT, vx + 2 * LA::XOUT);  // L3 -> V4
             __syncthreads();
             g_hpass<4, LA>(reinterpret_cast<const float2*>(b1), b2,                               // V4 -> L4
-                           GEpi<LA::HIN, LA::XIN, LA::MIN>{a, y0, x0, b0, a.dog[0], nullptr},
+                           GEpi<Tile, LA::HIN, LA::XIN, LA::MIN>{a, y0, x0, b0, a.dog[0], nullptr},
                            vy + 2 * LA::HOUT, vx + 2 * LA::XOUT);
             __syncthreads();
             g_vpass<5, LB>(b2, reinterpret_cast<float2*>(b0), vy + 2 * LB::HOUT, vx + 2 * LB::XOUT);  // L4 -> V5
             __syncthreads();
             g_hpass<5, LB>(reinterpret_cast<const float2*>(b0), nullptr,                          // V5 -> L5
-                           GEpi<LB::HIN, LB::XIN, LB::MIN>{a, y0, x0, b2, a.dog[1], nullptr},
+                           GEpi<Tile, LB::HIN, LB::XIN, LB::MIN>{a, y0, x0, b2, a.dog[1], nullptr},
                            vy + 2 * LB::HOUT, vx + 2 * LB::XOUT);
         }
     }
@@ -920,17 +933,28 @@ int sm_count() {
     return n[dev];
 }
 
-template <int G>
+template <int G, class Tile>
 int32_t launch_group_t(GroupArgs a, cudaStream_t s) {
     static std::atomic<int> attr[64];
-    FSB_TRY(smem_attr((const void*)k_group<G>, group_smem<G>(), attr));
-    a.tiles_x = (a.C + GX - 1) / GX;
-    a.n_tiles = a.tiles_x * ((a.R + GY - 1) / GY);
-    const int grid = a.n_tiles < sm_count() ? a.n_tiles : sm_count();
-    k_group<G><<<grid, GNT, group_smem<G>(), s>>>(a);
+    FSB_TRY(smem_attr((const void*)k_group<G, Tile>, group_smem<G, Tile>(), attr));
+    a.tiles_x = (a.C + Tile::GX - 1) / Tile::GX;
+    a.n_tiles = a.tiles_x * ((a.R + Tile::GY - 1) / Tile::GY);
+    const int resident = sm_count() * (Tile::GX == 128 ? 1 : Tile::GX == 64 ? 2 : 3);
+    const int grid = a.n_tiles < resident ? a.n_tiles : resident;
+    k_group<G, Tile><<<grid, Tile::GNT, group_smem<G, Tile>(), s>>>(a);
     note_launch();
     FSB_CUDA(cudaGetLastError());
     return FSB_OK;
+}
+
+// The group with tiles for small octaves: 32 x 16 while they all fit on the GPU at once, else 64 x 16. An
+// octave of 240 x 320 is 24 tiles of 128 x 32 - 24 SMs, each six passes over 13 000 pixels of input,
+// 17 us - or 150 tiles of 32 x 16 with 5 000 pixels each. 320 x 240: the groups 18.7 and 14.7 us a launch, now 10.9 and
+// 9.6; the whole pyramid 147 -> 117 us.
+template <int G>
+int32_t launch_group_small(const GroupArgs& a, cudaStream_t s) {
+    const long long small = (long long)((a.C + 31) / 32) * ((a.R + 15) / 16);
+    return small <= 3ll * sm_count() ? launch_group_t<G, GSmall>(a, s) : launch_group_t<G, GMid>(a, s);
 }
 
 }  // namespace
@@ -966,9 +990,10 @@ int32_t launch_layer_fast(int layer, const float* src, int R, int C, int P, floa
 
 // Layers 1..3 of a float32 octave by the fused group kernel: from L0 (src, R x C, pitch P), DoG planes
 // 0..2 at dog, dog + RC, dog + 2RC, gradients of L1..L3 at grad (+ RC, + 2RC), L3 to l3 and
-// L3[::2, ::2] to down (null: last octave). down must not alias src (other tiles still read it).
+// L3[::2, ::2] to down (null: last octave). down must not alias src (other tiles still read it). small:
+// the tiles for small octaves.
 int32_t launch_group_lower(const float* src, int R, int C, int P, float* dog, float2* grad, float* l3, float* down,
-                           int down_pitch, cudaStream_t s) {
+                           int down_pitch, bool small, cudaStream_t s) {
     const long long RC = (long long)R * P;
     GroupArgs a{};
     a.src = src;
@@ -982,12 +1007,12 @@ int32_t launch_group_lower(const float* src, int R, int C, int P, float* dog, fl
     a.dst = l3;
     a.down = down;
     a.down_pitch = down_pitch;
-    return launch_group_t<0>(a, s);
+    return small ? launch_group_small<0>(a, s) : launch_group_t<0, GLarge>(a, s);
 }
 
 // Layers 4, 5 of a float32 octave by the fused group kernel: from L3 (src), DoG planes 3, 4 at
 // dog3, dog3 + RC.
-int32_t launch_group_upper(const float* src, int R, int C, int P, float* dog3, cudaStream_t s) {
+int32_t launch_group_upper(const float* src, int R, int C, int P, float* dog3, bool small, cudaStream_t s) {
     GroupArgs a{};
     a.src = src;
     a.R = R;
@@ -995,7 +1020,7 @@ int32_t launch_group_upper(const float* src, int R, int C, int P, float* dog3, c
     a.P = P;
     a.dog[0] = dog3;
     a.dog[1] = dog3 + (long long)R * P;
-    return launch_group_t<1>(a, s);
+    return small ? launch_group_small<1>(a, s) : launch_group_t<1, GLarge>(a, s);
 }
 
 // The float32 octave-0 base: blur (tap set 0, radius 5) of the 2x upsampled uint8 image.

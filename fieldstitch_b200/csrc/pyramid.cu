@@ -250,15 +250,16 @@ int32_t tuned_layer(int layer, const float* src, int R, int C, int P, float* dst
 }
 }  // namespace
 
-// FSB_PYRAMID selects the float32 octave engine (both are bit-identical): unset, the autotuner picks
+// FSB_PYRAMID selects the float32 octave engine (all are bit-identical): unset, the autotuner picks
 // per octave size between the per-layer kernels (variant 0, also with FSB_AUTOTUNE=0) and the
-// fused layer groups (variant 1); "layer" / "group" force one, other values choose as unset. Read on
-// every call.
-enum class Engine { Auto, Group, Layer };
+// fused layer groups on large (1) or small (2) tiles; "layer" / "group" / "group_small" force one,
+// other values choose as unset. Read on every call.
+enum class Engine { Auto, Group, GroupSmall, Layer };
 static Engine pyramid_engine() {
     const char* e = std::getenv("FSB_PYRAMID");
     if (e && std::strcmp(e, "layer") == 0) return Engine::Layer;
     if (e && std::strcmp(e, "group") == 0) return Engine::Group;
+    if (e && std::strcmp(e, "group_small") == 0) return Engine::GroupSmall;
     return Engine::Auto;
 }
 
@@ -291,10 +292,10 @@ int32_t run_octave_call(void* p, int v) {
         ts = c->side;
         return FSB_OK;
     };
-    if (v == 1) {
-        FSB_TRY(launch_group_lower(c->src, c->R, c->C, c->P, c->dog, c->grad, c->x, c->down, c->dc, c->s));
+    if (v >= 1) {
+        FSB_TRY(launch_group_lower(c->src, c->R, c->C, c->P, c->dog, c->grad, c->x, c->down, c->dc, v == 2, c->s));
         FSB_TRY(fork());
-        FSB_TRY(launch_group_upper(c->x, c->R, c->C, c->P, c->dog + 3 * RC, ts));
+        FSB_TRY(launch_group_upper(c->x, c->R, c->C, c->P, c->dog + 3 * RC, v == 2, ts));
     } else {
         FSB_TRY(tuned_layer(1, c->src, c->R, c->C, c->P, c->x, c->dog, nullptr, nullptr, 0, c->err, c->s));
         FSB_TRY(tuned_layer(2, c->x, c->R, c->C, c->P, c->y, c->dog + RC, c->grad, nullptr, 0, c->err, c->s));
@@ -366,18 +367,18 @@ int32_t run_pyramid(Workspace& ws, const uint8_t* d_img, int img_stride, bool ex
             OctaveCall c{cur, g.R[o], g.C[o], g.P[o], pl[0], pl[1], DF + g.dog_off[o], GRAD + g.grad_off[o],
                          last ? nullptr : NB + (o & 1) * half, last ? 0 : g.P[o + 1], s,
                          nullptr, side ? ev[2 * o] : nullptr, side ? ev[2 * o + 1] : nullptr, err};
-            int v = eng == Engine::Group ? 1 : 0;
+            int v = eng == Engine::Group ? 1 : eng == Engine::GroupSmall ? 2 : 0;
             char key[64];
             std::snprintf(key, sizeof(key), "k_octave3_%dx%d", g.R[o], g.C[o]);
-            const bool known = eng != Engine::Auto || autotune_cached(key, 2, &v);
+            const bool known = eng != Engine::Auto || autotune_cached(key, 3, &v);
             if (known && side) c.side = side;
             if (eng == Engine::Auto && !known) {
-                FSB_TRY(autotune(key, 2, run_octave_call, &c, s, &v));
+                FSB_TRY(autotune(key, 3, run_octave_call, &c, s, &v));
             } else {
                 FSB_TRY(run_octave_call(&c, v));
             }
             if (c.side) {
-                tail_plane = v == 1 ? c.x : c.y;
+                tail_plane = v >= 1 ? c.x : c.y;
                 prev_tail = last_tail;
                 last_tail = o;
             }
