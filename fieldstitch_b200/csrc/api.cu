@@ -2,9 +2,10 @@
 // include/fsb200.h.
 #include <time.h>
 
+#include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
-#include <atomic>
 #include <string>
 
 #include "fsb_internal.cuh"
@@ -141,6 +142,36 @@ struct HostCopy {
 
 static size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 
+// Pageable buffers are staged through page-locked memory; more than RING_SLOTS pieces go through a ring of
+// them (2 MB, whatever the buffer's size), the CPU's copy of one piece overlapping the transfer of others.
+// What bounds it is the CPU's copy, 14 GB/s on one core: a 5.2 MB image takes 390 us staged as a whole, 364
+// through the ring (256 KB pieces: the same). Keypoints and descriptors of 8000 features, 1.3 MB of image and
+// the waits between them: detect + describe of 1320 x 989 1630 -> 1360 us.
+constexpr size_t COPY_PIECE = (size_t)512 << 10;
+constexpr int RING_SLOTS = 4;
+
+static int32_t ring_ensure(fsb_ctx* ctx) {
+    FSB_TRY(stage_ensure(ctx, RING_SLOTS * COPY_PIECE));
+    while ((int)ctx->copy_ev.size() < RING_SLOTS) {
+        cudaEvent_t e = nullptr;
+        FSB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        ctx->copy_ev.push_back(e);
+    }
+    return FSB_OK;
+}
+
+// piece j of a staged host -> device copy: fill(slot) writes its bytes
+template <typename Fill>
+static int32_t ring_push(fsb_ctx* ctx, int j, void* dev, size_t n, Fill fill) {
+    cudaEvent_t ev = ctx->copy_ev[j % RING_SLOTS];
+    char* slot = static_cast<char*>(ctx->pinned) + (size_t)(j % RING_SLOTS) * COPY_PIECE;
+    if (j >= RING_SLOTS) FSB_CUDA(cudaEventSynchronize(ev));
+    fill(slot);
+    FSB_CUDA(cudaMemcpyAsync(dev, slot, n, cudaMemcpyHostToDevice, ctx->stream));
+    FSB_CUDA(cudaEventRecord(ev, ctx->stream));
+    return FSB_OK;
+}
+
 // host -> device copies of k buffers, enqueued on the context's stream
 static int32_t copy_in(fsb_ctx* ctx, const HostCopy* c, int k) {
     size_t total = 0;
@@ -149,10 +180,22 @@ static int32_t copy_in(fsb_ctx* ctx, const HostCopy* c, int k) {
         direct[i] = c[i].bytes == 0 || host_pinned(c[i].host);
         if (!direct[i]) total += al256(c[i].bytes);
     }
-    if (total) FSB_TRY(stage_ensure(ctx, total));
+    const bool ring = total > RING_SLOTS * COPY_PIECE;
+    if (ring) FSB_TRY(ring_ensure(ctx));
+    else if (total) FSB_TRY(stage_ensure(ctx, total));
     char* st = static_cast<char*>(ctx->pinned);
+    int piece = 0;
     for (int i = 0; i < k; ++i) {
         if (c[i].bytes == 0) continue;
+        if (ring && !direct[i]) {
+            for (size_t o = 0; o < c[i].bytes; o += COPY_PIECE) {
+                const size_t n = std::min(COPY_PIECE, c[i].bytes - o);
+                const char* src = static_cast<const char*>(c[i].host) + o;
+                FSB_TRY(ring_push(ctx, piece++, static_cast<char*>(c[i].dev) + o, n,
+                                  [&](char* slot) { std::memcpy(slot, src, n); }));
+            }
+            continue;
+        }
         const void* src = c[i].host;
         if (!direct[i]) {
             std::memcpy(st, c[i].host, c[i].bytes);
@@ -172,22 +215,45 @@ static int32_t copy_out(fsb_ctx* ctx, const HostCopy* c, int k) {
         direct[i] = c[i].bytes == 0 || host_pinned(c[i].host);
         if (!direct[i]) total += al256(c[i].bytes);
     }
-    if (total) FSB_TRY(stage_ensure(ctx, total));
-    char* st = static_cast<char*>(ctx->pinned);
-    char* at[16];
+    const bool ring = total > RING_SLOTS * COPY_PIECE;
+    if (ring) FSB_TRY(ring_ensure(ctx));
+    else if (total) FSB_TRY(stage_ensure(ctx, total));
+    char* const st = static_cast<char*>(ctx->pinned);
+    struct Piece {
+        char *host, *dev, *slot;
+        size_t n;
+    };
+    std::vector<Piece> pieces;
+    size_t off = 0;
     for (int i = 0; i < k; ++i) {
         if (c[i].bytes == 0) continue;
-        void* dst = c[i].host;
-        if (!direct[i]) {
-            at[i] = st;
-            dst = st;
-            st += al256(c[i].bytes);
+        char *host = static_cast<char*>(c[i].host), *dev = static_cast<char*>(c[i].dev);
+        if (direct[i]) {
+            FSB_CUDA(cudaMemcpyAsync(host, dev, c[i].bytes, cudaMemcpyDeviceToHost, ctx->stream));
+        } else if (ring) {
+            for (size_t o = 0; o < c[i].bytes; o += COPY_PIECE)
+                pieces.push_back({host + o, dev + o, st + pieces.size() % RING_SLOTS * COPY_PIECE,
+                                  std::min(COPY_PIECE, c[i].bytes - o)});
+        } else {
+            pieces.push_back({host, dev, st + off, c[i].bytes});
+            off += al256(c[i].bytes);
         }
-        FSB_CUDA(cudaMemcpyAsync(dst, c[i].dev, c[i].bytes, cudaMemcpyDeviceToHost, ctx->stream));
     }
-    FSB_CUDA(cudaStreamSynchronize(ctx->stream));
-    for (int i = 0; i < k; ++i)
-        if (c[i].bytes && !direct[i]) std::memcpy(c[i].host, at[i], c[i].bytes);
+    auto fetch = [&](size_t j) -> int32_t {
+        const Piece& p = pieces[j];
+        FSB_CUDA(cudaMemcpyAsync(p.slot, p.dev, p.n, cudaMemcpyDeviceToHost, ctx->stream));
+        if (ring) FSB_CUDA(cudaEventRecord(ctx->copy_ev[j % RING_SLOTS], ctx->stream));
+        return FSB_OK;
+    };
+    const size_t ahead = ring ? std::min(pieces.size(), (size_t)RING_SLOTS) : pieces.size();
+    for (size_t j = 0; j < ahead; ++j) FSB_TRY(fetch(j));
+    if (!ring) FSB_CUDA(cudaStreamSynchronize(ctx->stream));
+    for (size_t j = 0; j < pieces.size(); ++j) {
+        if (ring) FSB_CUDA(cudaEventSynchronize(ctx->copy_ev[j % RING_SLOTS]));
+        std::memcpy(pieces[j].host, pieces[j].slot, pieces[j].n);
+        if (j + ahead < pieces.size()) FSB_TRY(fetch(j + ahead));
+    }
+    if (ring) FSB_CUDA(cudaStreamSynchronize(ctx->stream));   // buffers copied without staging
     return FSB_OK;
 }
 
@@ -219,11 +285,21 @@ static int32_t detect_into(fsb_ctx* ctx, Workspace& ws, const uint8_t* img, int 
         FSB_CUDA(cudaMemcpy2DAsync(ws.img.p, (size_t)w, img, (size_t)stride, (size_t)w, (size_t)h,
                                    cudaMemcpyHostToDevice, s));
     } else {
-        // rows gathered into the context's page-locked buffer, one contiguous copy
-        FSB_TRY(stage_ensure(ctx, (size_t)h * w));
-        uint8_t* st = static_cast<uint8_t*>(ctx->pinned);
-        for (int r = 0; r < h; ++r) std::memcpy(st + (size_t)r * w, img + (size_t)r * stride, (size_t)w);
-        FSB_CUDA(cudaMemcpyAsync(ws.img.p, st, (size_t)h * w, cudaMemcpyHostToDevice, s));
+        // rows gathered into the ring of page-locked pieces
+        FSB_TRY(ring_ensure(ctx));
+        const int step = std::max(1, (int)(COPY_PIECE / (size_t)w));
+        for (int r0 = 0, piece = 0; r0 < h; r0 += step, ++piece) {
+            const int r1 = std::min(h, r0 + step);
+            FSB_TRY(ring_push(ctx, piece, ws.img.as<uint8_t>() + (size_t)r0 * w, (size_t)(r1 - r0) * w,
+                              [&](char* slot) {
+                                  if (stride == w) {
+                                      std::memcpy(slot, img + (size_t)r0 * w, (size_t)(r1 - r0) * w);
+                                      return;
+                                  }
+                                  for (int r = r0; r < r1; ++r)
+                                      std::memcpy(slot + (size_t)(r - r0) * w, img + (size_t)r * stride, (size_t)w);
+                              }));
+        }
     }
     ctx->stage_end(ST_UPLOAD);
     return detect_dev(ctx, ws, ws.img.as<uint8_t>(), w, p, max_kp);
@@ -238,6 +314,33 @@ __global__ void k_atlas_part(const float* __restrict__ src, long long n, int C, 
         const long long at = i / C * P + i % C;
         out[i] = what ? src[2 * at + (what - 1)] : src[at];
     }
+}
+
+// matches (cap queries, cap targets, their count, one after another in device memory) to the host: up to
+// 64 K entries in one transfer with the count, more of them after the count is known
+static int32_t matches_out(fsb_ctx* ctx, const int64_t* dq, int cap, int64_t* q, int64_t* t, int32_t* n_out) {
+    cudaStream_t s = ctx->stream;
+    const size_t all = (size_t)cap * 16 + 4;
+    const bool whole = cap <= 65536;
+    FSB_TRY(stage_ensure(ctx, whole ? all : 64));
+    char* st = static_cast<char*>(ctx->pinned);
+    const int* dn = reinterpret_cast<const int*>(dq + 2 * (size_t)cap);
+    int n = 0;
+    if (whole) {
+        FSB_CUDA(cudaMemcpyAsync(st, dq, all, cudaMemcpyDeviceToHost, s));
+        FSB_CUDA(cudaStreamSynchronize(s));
+        std::memcpy(&n, st + (size_t)cap * 16, 4);
+        std::memcpy(q, st, (size_t)n * 8);
+        std::memcpy(t, st + (size_t)cap * 8, (size_t)n * 8);
+    } else {
+        FSB_CUDA(cudaMemcpyAsync(st, dn, 4, cudaMemcpyDeviceToHost, s));
+        FSB_CUDA(cudaStreamSynchronize(s));
+        std::memcpy(&n, st, 4);
+        const HostCopy out[2] = {{q, (void*)dq, (size_t)n * 8}, {t, (void*)(dq + cap), (size_t)n * 8}};
+        FSB_TRY(copy_out(ctx, out, 2));
+    }
+    *n_out = n;
+    return FSB_OK;
 }
 
 // selected keypoints -> describe inputs (tx..tly) and optional interleaved xy / response outputs
@@ -394,21 +497,24 @@ int32_t batch_body(fsb_ctx* ctx, const BatchCall& b) {
     if (b.h_imgs) {
         // the uploads on their own stream, in image order: image i's chain waits for image i only,
         // so later uploads overlap the extraction of earlier images
-        x.copy_nodes.assign(b.n_img, nullptr);
         FSB_CUDA(cudaStreamWaitEvent(x.upload, x.fork, 0));
         const size_t bytes = (size_t)b.h * b.stride;
         for (int i = 0; i < b.n_img; ++i) {
             FSB_CUDA(cudaMemcpyAsync(const_cast<uint8_t*>(b.imgs[i]), b.h_imgs[i], bytes, cudaMemcpyHostToDevice,
                                      x.upload));
-            cudaStreamCaptureStatus cs;
+            cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
             const cudaGraphNode_t* deps = nullptr;
             size_t nd = 0;
             FSB_CUDA(cudaStreamGetCaptureInfo(x.upload, &cs, nullptr, nullptr, &deps, &nd));
-            if (cs != cudaStreamCaptureStatusActive || nd != 1) {
-                set_error("capture of the image uploads: unexpected capture state");
-                return FSB_ERR_CUDA;
+            if (cs == cudaStreamCaptureStatusActive) {
+                if (nd != 1) {
+                    set_error("capture of the image uploads: unexpected capture state");
+                    return FSB_ERR_CUDA;
+                }
+                // (a direct launch leaves the nodes of the graph that is kept)
+                x.copy_nodes.resize(b.n_img);
+                x.copy_nodes[i] = deps[0];
             }
-            x.copy_nodes[i] = deps[0];
             FSB_CUDA(cudaEventRecord(x.uploaded[i], x.upload));
         }
     }
@@ -537,6 +643,7 @@ int32_t fsb_destroy(fsb_ctx* ctx) {
     }
     if (ctx->pinned) cudaFreeHost(ctx->pinned);
     ctx->stage_release();
+    for (cudaEvent_t e : ctx->copy_ev) cudaEventDestroy(e);
     if (ctx->side) cudaStreamSynchronize(ctx->side);
     jpeg_release(ctx);
     for (auto& e : ctx->pyr_ev)
@@ -633,13 +740,11 @@ int32_t fsb_state_keypoints(fsb_state* st, float* x, float* y, float* size, floa
     FSB_TRY(use_device(ctx));
     const Workspace& ws = *st->ws;
     const size_t n = (size_t)ws.n_kp;
-    cudaStream_t s = ctx->stream;
-    struct { void* h; const DevBuf* d; } out[] = {{x, &ws.kx}, {y, &ws.ky}, {size, &ws.ksize}, {angle, &ws.kangle},
-                                                 {response, &ws.kresp}, {octave, &ws.koct}, {layer, &ws.klayer}};
-    for (auto& o : out)
-        if (o.h && n) FSB_CUDA(cudaMemcpyAsync(o.h, o.d->p, n * 4, cudaMemcpyDeviceToHost, s));
-    FSB_CUDA(cudaStreamSynchronize(s));
-    return FSB_OK;
+    const HostCopy out[7] = {{x, ws.kx.p, x ? n * 4 : 0},          {y, ws.ky.p, y ? n * 4 : 0},
+                             {size, ws.ksize.p, size ? n * 4 : 0}, {angle, ws.kangle.p, angle ? n * 4 : 0},
+                             {response, ws.kresp.p, response ? n * 4 : 0},
+                             {octave, ws.koct.p, octave ? n * 4 : 0}, {layer, ws.klayer.p, layer ? n * 4 : 0}};
+    return copy_out(ctx, out, 7);
 }
 
 int32_t fsb_describe(fsb_ctx* ctx, fsb_state* st, int32_t n, const float* x, const float* y, const float* size,
@@ -669,21 +774,17 @@ int32_t fsb_describe(fsb_ctx* ctx, fsb_state* st, int32_t n, const float* x, con
     float* da = ds + n;
     int32_t* dout = reinterpret_cast<int32_t*>(da + n);
     int32_t* dl = dout + n;
-    FSB_CUDA(cudaMemcpyAsync(dx, x, n * 4, cudaMemcpyHostToDevice, s));
-    FSB_CUDA(cudaMemcpyAsync(dy, y, n * 4, cudaMemcpyHostToDevice, s));
-    FSB_CUDA(cudaMemcpyAsync(ds, size, n * 4, cudaMemcpyHostToDevice, s));
-    FSB_CUDA(cudaMemcpyAsync(da, angle, n * 4, cudaMemcpyHostToDevice, s));
-    FSB_CUDA(cudaMemcpyAsync(dout, octave, n * 4, cudaMemcpyHostToDevice, s));
-    FSB_CUDA(cudaMemcpyAsync(dl, layer, n * 4, cudaMemcpyHostToDevice, s));
+    const size_t nb = (size_t)n * 4;
+    const HostCopy in[6] = {{(void*)x, dx, nb},     {(void*)y, dy, nb},        {(void*)size, ds, nb},
+                            {(void*)angle, da, nb}, {(void*)octave, dout, nb}, {(void*)layer, dl, nb}};
+    FSB_TRY(copy_in(ctx, in, 6));
     FSB_TRY(ctx->s_f32b.ensure((size_t)n * 128 * 4 + 256));
     FSB_TRY(ctx->s_u8a.ensure((size_t)n * 128 + 256));
     float* dd = desc ? ctx->s_f32b.as<float>() : nullptr;
     uint8_t* du = rootsift ? ctx->s_u8a.as<uint8_t>() : nullptr;
     FSB_TRY(run_describe_mode(ws, n, dx, dy, ds, da, dout, dl, dd, du, st->exact, s));
-    if (desc) FSB_CUDA(cudaMemcpyAsync(desc, dd, (size_t)n * 128 * 4, cudaMemcpyDeviceToHost, s));
-    if (rootsift) FSB_CUDA(cudaMemcpyAsync(rootsift, du, (size_t)n * 128, cudaMemcpyDeviceToHost, s));
-    FSB_CUDA(cudaStreamSynchronize(s));
-    return FSB_OK;
+    const HostCopy out[2] = {{desc, dd, desc ? (size_t)n * 512 : 0}, {rootsift, du, rootsift ? (size_t)n * 128 : 0}};
+    return copy_out(ctx, out, 2);
 }
 
 int32_t fsb_state_geometry(fsb_state* st, int32_t* n_oct, int32_t* rows, int32_t* cols) {
@@ -974,7 +1075,22 @@ int32_t sift_features_batch(fsb_ctx* ctx, int32_t n_img, const uint8_t* const* h
         for (const void* q : ptrs) key_put(key, q);
         key_put(key, ws->sort_tmp.bytes);
     }
-    if (!x.graph.exec || key != x.graph.key) {
+    // A call with other arguments than the last one is launched directly (about 65 launches an image, queued
+    // faster than they run); capturing and instantiating it costs 3.6 ms per 16 images before any of them
+    // runs: 16 photos of 2640 x 1978 in new buffers 16.9 -> 14.0 ms. The second such call in a row captures
+    // the graph, later ones replay it (13.7 ms).
+    const bool replay = x.graph.exec && key == x.graph.key;
+    const bool direct = !replay && key != x.last_key;
+    x.last_key = key;
+    if (direct) {
+        BatchCall bc{n_img, d_imgs, h_imgs, h, w, stride, p, nfeats, d_xy, d_resp, d_rootsift, d_counts};
+        const int32_t st = batch_body(ctx, bc);
+        if (st != FSB_OK) {   // no work left behind on the chains' streams
+            for (cudaStream_t c : x.streams) cudaStreamSynchronize(c);
+            if (x.upload) cudaStreamSynchronize(x.upload);
+            return st;
+        }
+    } else if (!replay) {
         if (x.graph.exec) cudaGraphExecDestroy(x.graph.exec);
         if (x.graph.graph) cudaGraphDestroy(x.graph.graph);
         x.graph.exec = nullptr;
@@ -1000,13 +1116,13 @@ int32_t sift_features_batch(fsb_ctx* ctx, int32_t n_img, const uint8_t* const* h
         FSB_CUDA(cudaGraphInstantiate(&x.graph.exec, g, 0));
         x.graph.key = key;
     }
-    if (h_imgs) {
-        for (int i = 0; i < n_img; ++i)
+    if (!direct) {
+        for (int i = 0; h_imgs && i < n_img; ++i)
             FSB_CUDA(cudaGraphExecMemcpyNodeSetParams1D(x.graph.exec, x.copy_nodes[i], const_cast<uint8_t*>(d_imgs[i]),
                                                         h_imgs[i], (size_t)h * stride, cudaMemcpyHostToDevice));
+        FSB_CUDA(cudaGraphLaunch(x.graph.exec, s));
+        note_launch(x.graph.n_kernels);
     }
-    FSB_CUDA(cudaGraphLaunch(x.graph.exec, s));
-    note_launch(x.graph.n_kernels);
     // one wait per batch: the flags say which images (if any) exceeded a capacity
     FSB_TRY(stage_ensure(ctx, (size_t)n_img * 8 + 64));
     uint32_t* h_status = static_cast<uint32_t*>(ctx->pinned);
@@ -1487,25 +1603,17 @@ int32_t fsb_match_bf(fsb_ctx* ctx, const uint8_t* a, int32_t na, const uint8_t* 
     if (na < 2 || nb < 2) return FSB_OK;
     FSB_TRY(use_device(ctx));
     cudaStream_t s = ctx->stream;
-    FSB_TRY(to_dev(ctx->s_u8a, a, (size_t)na * 128, s));
-    FSB_TRY(to_dev(ctx->s_u8b, b, (size_t)nb * 128, s));
+    FSB_TRY(ctx->s_u8a.ensure((size_t)na * 128 + 16));
+    FSB_TRY(ctx->s_u8b.ensure((size_t)nb * 128 + 16));
+    const HostCopy in[2] = {{(void*)a, ctx->s_u8a.p, (size_t)na * 128}, {(void*)b, ctx->s_u8b.p, (size_t)nb * 128}};
+    FSB_TRY(copy_in(ctx, in, 2));
     FSB_TRY(ctx->s_i64.ensure((size_t)na * 16 + 64));
     int64_t* dq = ctx->s_i64.as<int64_t>();
     int64_t* dt = dq + na;
-    FSB_TRY(ctx->s_count.ensure(64));
-    int* dn = ctx->s_count.as<int>();
+    int* dn = reinterpret_cast<int*>(dt + na);
     FSB_TRY(run_match_bf(ctx, ctx->s_u8a.as<uint8_t>(), na, ctx->s_u8b.as<uint8_t>(), nb, ratio, precision, dq, dt,
                          dn, s));
-    int n = 0;
-    FSB_CUDA(cudaMemcpyAsync(&n, dn, sizeof(int), cudaMemcpyDeviceToHost, s));
-    FSB_CUDA(cudaStreamSynchronize(s));
-    if (n) {
-        FSB_CUDA(cudaMemcpyAsync(q, dq, (size_t)n * 8, cudaMemcpyDeviceToHost, s));
-        FSB_CUDA(cudaMemcpyAsync(t, dt, (size_t)n * 8, cudaMemcpyDeviceToHost, s));
-        FSB_CUDA(cudaStreamSynchronize(s));
-    }
-    *n_out = n;
-    return FSB_OK;
+    return matches_out(ctx, dq, na, q, t, n_out);
 }
 
 int32_t fsb_match_guided(fsb_ctx* ctx, const double* pred_xy, const uint8_t* a, int32_t na, const double* b_xy,

@@ -185,6 +185,7 @@ struct fsb_ctx {
         std::vector<cudaEvent_t> uploaded;        // image i on the device (captured edges)
         std::vector<cudaGraphNode_t> copy_nodes;  // the upload of image i in the captured graph
         fsb::BatchGraph graph;
+        std::vector<char> last_key;   // the arguments of the latest call
         fsb::BatchGraph pyr_graph;   // fsb_pyramid_batch_d
         int pyr_h = 0, pyr_w = 0;     // geometry whose pyramid ran once outside a capture (autotuned)
         fsb::DevBuf status;
@@ -194,6 +195,7 @@ struct fsb_ctx {
     } xb;
     void* pinned = nullptr;
     size_t pinned_bytes = 0;
+    std::vector<cudaEvent_t> copy_ev;   // per slot of the ring that staged copies go through
     // stage timers: event pairs recorded at stage boundaries while timing is on, read back lazily
     // (when many are pending, and when the times are queried), so timing adds no host wait
     struct StageMark { int st; cudaEvent_t e0, e1; };

@@ -58,24 +58,29 @@ def ratio_match_bf_batch_d(a_list, b_list, ratio, precision="bf16", device=0, ou
     if len(a_list) != len(b_list):
         raise ValueError("a_list and b_list differ in length")
     n = len(a_list)
-    for x in list(a_list) + list(b_list):
-        if x.dtype != torch.uint8 or x.dim() != 2 or x.shape[1] != 128 or not x.is_contiguous() or not x.is_cuda:
+    u8 = torch.uint8
+    shapes = [x.shape for x in a_list] + [x.shape for x in b_list]
+    for x, s in zip(list(a_list) + list(b_list), shapes):
+        if x.dtype != u8 or len(s) != 2 or s[1] != 128 or not x.is_contiguous() or not x.is_cuda:
             raise ValueError("descriptors must be contiguous CUDA uint8 tensors of shape (n, 128)")
+    na = [s[0] for s in shapes[:n]]
+    nb = [s[0] for s in shapes[n:]]
     ctx = _lib.context(device)
     if out is None:
-        outs = [(torch.empty(max(len(a), 1), dtype=torch.int64, device=a.device),
-                 torch.empty(max(len(a), 1), dtype=torch.int64, device=a.device)) for a in a_list]
+        outs = [(torch.empty(max(k, 1), dtype=torch.int64, device=a.device),
+                 torch.empty(max(k, 1), dtype=torch.int64, device=a.device)) for a, k in zip(a_list, na)]
     else:
         outs = list(out)
-        if len(outs) != n or any(len(q) < len(a) or len(t) < len(a) or q.dtype != torch.int64 or t.dtype != torch.int64
-                                 for (q, t), a in zip(outs, a_list)):
+        i64 = torch.int64
+        if len(outs) != n or any(q.shape[0] < k or t.shape[0] < k or q.dtype != i64 or t.dtype != i64
+                                 for (q, t), k in zip(outs, na)):
             raise ValueError("out must hold one (q, t) pair of int64 tensors of length >= na per pair")
     P = ctypes.c_void_p * max(n, 1)
     I = ctypes.c_int32 * max(n, 1)
     pa = P(*[a.data_ptr() for a in a_list])
     pb = P(*[b.data_ptr() for b in b_list])
-    na = I(*[len(a) for a in a_list])
-    nb = I(*[len(b) for b in b_list])
+    na = I(*na)
+    nb = I(*nb)
     pq = P(*[o[0].data_ptr() for o in outs])
     pt = P(*[o[1].data_ptr() for o in outs])
     cnt = I()
@@ -94,17 +99,24 @@ def guided_from_pred_batch_d(problems, radius, kc, ratio, device=0, out=None):
     """
     import torch
     n = len(problems)
-    for pred, a, bxy, b, _ in problems:
-        for x, dt, w in ((pred, torch.float64, 2), (a, torch.uint8, 128), (bxy, torch.float64, 2),
-                         (b, torch.uint8, 128)):
-            if x.dtype != dt or x.dim() != 2 or x.shape[1] != w or not x.is_contiguous() or not x.is_cuda:
+    kinds = ((torch.float64, 2), (torch.uint8, 128), (torch.float64, 2), (torch.uint8, 128))
+    ptrs, nas, nbs = [], [], []
+    for pred, a, bxy, b, _ in problems:   # one pass over the attributes: a batch has hundreds of tensors
+        lens = []
+        for x, (dt, w) in zip((pred, a, bxy, b), kinds):
+            s = x.shape
+            if x.dtype != dt or len(s) != 2 or s[1] != w or not x.is_contiguous() or not x.is_cuda:
                 raise ValueError("expected contiguous CUDA tensors: pred/b_xy float64 (n,2), a/b uint8 (n,128)")
-        if len(pred) != len(a) or len(bxy) != len(b):
+            lens.append(s[0])
+            ptrs.append(x.data_ptr())
+        if lens[0] != lens[1] or lens[2] != lens[3]:
             raise ValueError("positions and descriptors differ in length")
+        nas.append(lens[1])
+        nbs.append(lens[3])
     ctx = _lib.context(device)
     if out is None:
-        out = [(torch.empty(max(len(pr), 1), dtype=torch.int64, device=pr.device),
-                torch.empty(max(len(pr), 1), dtype=torch.int64, device=pr.device)) for pr, _, _, _, _ in problems]
+        out = [(torch.empty(max(k, 1), dtype=torch.int64, device=x[0].device),
+                torch.empty(max(k, 1), dtype=torch.int64, device=x[0].device)) for x, k in zip(problems, nas)]
     P = ctypes.c_void_p * max(n, 1)
     I = ctypes.c_int32 * max(n, 1)
     D = ctypes.c_double * max(n, 1)
@@ -112,9 +124,7 @@ def guided_from_pred_batch_d(problems, radius, kc, ratio, device=0, out=None):
     cnt = I()
     torch.cuda.current_stream(device).synchronize()
     _lib.check(ctx.lib.fsb_match_guided_batch_d(
-        ctx.handle, n, P(*[x[0].data_ptr() for x in problems]), P(*[x[1].data_ptr() for x in problems]),
-        I(*[len(x[1]) for x in problems]), P(*[x[2].data_ptr() for x in problems]),
-        P(*[x[3].data_ptr() for x in problems]), I(*[len(x[3]) for x in problems]),
+        ctx.handle, n, P(*ptrs[0::4]), P(*ptrs[1::4]), I(*nas), P(*ptrs[2::4]), P(*ptrs[3::4]), I(*nbs),
         D(*[float(x[4][0]) for x in problems]), D(*[float(x[4][1]) for x in problems]), float(radius), k,
         float(ratio), P(*[o[0].data_ptr() for o in out]), P(*[o[1].data_ptr() for o in out]), cnt),
         "fsb_match_guided_batch_d")
