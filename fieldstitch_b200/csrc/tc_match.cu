@@ -37,6 +37,7 @@
 //
 // The best target, the exact best distance and the accept decision are therefore the same as
 // those of the CUDA-core FP32 path and of the reference, for every precision.
+#include <cuda_fp16.h>
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -127,6 +128,7 @@ struct PackSeg {
     int32_t* norms;
     float* rowsc;   // E4M3 queries
     float* bmax;    // E4M3 targets
+    unsigned long long* key;   // targets: the one-to-one keys, set to ~0
     int n, n_pad, role;   // role 0: query, 1: target
 };
 
@@ -150,112 +152,137 @@ __device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) {
     return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632u);
 }
 
-// Four packed rows per warp, eight lanes per row (16 bytes each); blockIdx.y is the job. Bound by HBM
-// (128 bytes in, ROW_BYTES out per row). One row per warp with a conversion instruction per value
-// took 92 us (BF16, 524 000 rows) and 268 us (E4M3, 433 000 rows, one more pass back to float and two
-// atomics per target); byte permutes and integer rounding take 45 and 79 us.
-constexpr int PACK_T = 256, PACK_ROWS = PACK_T / 8;
+__device__ __forceinline__ __half2 as_half2(uint32_t u) { return *reinterpret_cast<const __half2*>(&u); }
+__device__ __forceinline__ uint32_t as_bits(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
+
+// Eight lanes per row (16 bytes each), four rows per warp at a time, PACK_IT times with all loads up front;
+// blockIdx.y is the job. Bound by HBM (128 bytes in, ROW_BYTES out per row), E4M3 also by the conversions.
+// One row per warp with a conversion instruction per value took 92 us (BF16, 524 000 rows) and 268 us (E4M3,
+// 433 000 rows, one more pass back to float and two atomics per target). Byte permutes and integer rounding
+// with four rows per warp took 54 and 80 us; four loads in flight 52 and 57 with one pair of atomics per block
+// (per warp, they queue on one line of L2); two bytes per instruction as FP16 pairs (E4M3) 42.
+constexpr int PACK_T = 256, PACK_IT = 4, PACK_ROWS = PACK_T / 8 * PACK_IT;
 template <int PREC>
 __global__ void __launch_bounds__(PACK_T) k_tc_pack(const PackSeg* __restrict__ segs) {
     constexpr int RB = TcTraits<PREC>::ROW_BYTES;
     constexpr int XB = RB - 32;   // byte offset of the norm slots
+    __shared__ int s_max[2];
     const PackSeg& S = segs[blockIdx.y];
     const int lane = threadIdx.x & 31, seg = lane & 7;
-    const int row = blockIdx.x * PACK_ROWS + (threadIdx.x >> 3);
     if (blockIdx.x * PACK_ROWS >= S.n_pad) return;   // n_pad is a multiple of PACK_ROWS: uniform per block
-    uint8_t* blk = S.dst + (size_t)(row >> 7) * (128 * RB);
-    const int r = row & 127;
-    const bool live = row < S.n;
-    uint4 w = make_uint4(0u, 0u, 0u, 0u);
-    if (live) w = __ldg(reinterpret_cast<const uint4*>(S.src + (size_t)row * 128) + seg);
-    const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
-    unsigned un = 0;
+    const int role = S.role, n = S.n;
+    uint8_t* const blk = S.dst + (size_t)blockIdx.x * (PACK_ROWS * RB);   // PACK_ROWS is the block of core_off
+    uint4 wv[PACK_IT];
 #pragma unroll
-    for (int v = 0; v < 4; ++v) un = __dp4a(ww[v], ww[v], un);
+    for (int it = 0; it < PACK_IT; ++it) {
+        const int row = blockIdx.x * PACK_ROWS + it * (PACK_T / 8) + (threadIdx.x >> 3);
+        wv[it] = make_uint4(0u, 0u, 0u, 0u);
+        if (row < n) wv[it] = __ldg(reinterpret_cast<const uint4*>(S.src + (size_t)row * 128) + seg);
+    }
+    if (PREC == FSB_PREC_FP8 && role == 1) {
+        if (threadIdx.x < 2) s_max[threadIdx.x] = 0;
+        __syncthreads();
+    }
+    int ml = 0, me = 0;   // E4M3 targets: the largest |b| and |beta| (non-negative floats order like their bits)
 #pragma unroll
-    for (int sh = 1; sh < 8; sh <<= 1) un += __shfl_xor_sync(0xffffffffu, un, sh);
-    const int nrm = (int)un;
-    if (seg == 0 && live) S.norms[row] = nrm;
-    float s = 1.f;
-    if constexpr (PREC == FSB_PREC_BF16) {
-        uint32_t o[8];
+    for (int it = 0; it < PACK_IT; ++it) {
+        const int r = it * (PACK_T / 8) + (threadIdx.x >> 3);
+        const int row = blockIdx.x * PACK_ROWS + r;
+        const bool live = row < n;
+        const uint4 w = wv[it];
+        const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+        unsigned un = 0;
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            o[2 * v] = bf16_pair(byte_float(ww[v], 0), byte_float(ww[v], 1));
-            o[2 * v + 1] = bf16_pair(byte_float(ww[v], 2), byte_float(ww[v], 3));
-        }
-        *reinterpret_cast<uint4*>(blk + core_off(r, seg * 32, RB)) = make_uint4(o[0], o[1], o[2], o[3]);
-        *reinterpret_cast<uint4*>(blk + core_off(r, seg * 32 + 16, RB)) = make_uint4(o[4], o[5], o[6], o[7]);
-    } else {
-        int e = 0;
-        if (S.role == 0) {
-            // per-query power-of-two scale: the largest e <= 8 with max * 2^e <= 448 = 1.75 * 2^8
-            uint32_t mx = __vmaxu4(__vmaxu4(ww[0], ww[1]), __vmaxu4(ww[2], ww[3]));
-            mx = __vmaxu4(mx, mx >> 16);
-            mx = max(mx & 255u, (mx >> 8) & 255u);
+        for (int v = 0; v < 4; ++v) un = __dp4a(ww[v], ww[v], un);
 #pragma unroll
-            for (int sh = 1; sh < 8; sh <<= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, sh));
-            e = 8;
-            if (mx) {
-                const int k = 31 - __clz(mx);
-                e = max(0, (mx << (8 - k)) <= 448u ? 8 - k : 7 - k);
+        for (int sh = 1; sh < 8; sh <<= 1) un += __shfl_xor_sync(0xffffffffu, un, sh);
+        const int nrm = (int)un;
+        if (seg == 0 && live) S.norms[row] = nrm;
+        if (role == 1 && seg == 1 && live) S.key[row] = ~0ull;
+        float s = 1.f;
+        if constexpr (PREC == FSB_PREC_BF16) {
+            uint32_t o[8];
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+                o[2 * v] = bf16_pair(byte_float(ww[v], 0), byte_float(ww[v], 1));
+                o[2 * v + 1] = bf16_pair(byte_float(ww[v], 2), byte_float(ww[v], 3));
             }
-            s = (float)(1 << e);
-        }
-        // E4M3 of x 2^e for an integer x in 1..255: three mantissa bits, round to nearest even (the carry
-        // moves the exponent), exponent re-biased by 7 - 127; the scale is an exponent shift, so the
-        // rounding error of x itself does not depend on it
-        uint32_t o[4];
-        float err2 = 0.f;
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            o[v] = 0;
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                const float x = byte_float(ww[v], b);
-                const uint32_t u = __float_as_uint(x);
-                const uint32_t q = (u + 0x7FFFFu + ((u >> 20) & 1u)) >> 20;
-                const float back = __uint_as_float(q << 20);
-                err2 = fmaf(back - x, back - x, err2);
-                const uint32_t code = x > 0.f ? q + (uint32_t)(8 * e - 960) : 0u;
-                o[v] |= code << (8 * b);
-            }
-        }
-#pragma unroll
-        for (int sh = 1; sh < 8; sh <<= 1) err2 += __shfl_xor_sync(0xffffffffu, err2, sh);
-        *reinterpret_cast<uint4*>(blk + core_off(r, seg * 16, RB)) = make_uint4(o[0], o[1], o[2], o[3]);
-        const float len = live ? sqrtf((float)nrm) * (1.f + 1e-6f) : 0.f;
-        const float elen = live ? sqrtf(err2) * (1.f + 1e-6f) : 0.f;
-        if (S.role == 0) {
-            if (seg == 0 && live) reinterpret_cast<float4*>(S.rowsc)[row] = make_float4(s, 1.f / s, len, elen);
+            *reinterpret_cast<uint4*>(blk + core_off(r, seg * 32, RB)) = make_uint4(o[0], o[1], o[2], o[3]);
+            *reinterpret_cast<uint4*>(blk + core_off(r, seg * 32 + 16, RB)) = make_uint4(o[4], o[5], o[6], o[7]);
         } else {
-            // the largest |b| and |beta| of the job (non-negative floats order like their bit
-            // patterns): one pair of atomics per warp, skipped once the running maximum is larger
-            int ml = __float_as_int(len), me = __float_as_int(elen);
+            int e = 0;
+            if (role == 0) {
+                // per-query power-of-two scale: the largest e <= 8 with max * 2^e <= 448 = 1.75 * 2^8
+                uint32_t mx = __vmaxu4(__vmaxu4(ww[0], ww[1]), __vmaxu4(ww[2], ww[3]));
+                mx = __vmaxu4(mx, mx >> 16);
+                mx = max(mx & 255u, (mx >> 8) & 255u);
 #pragma unroll
-            for (int sh = 8; sh < 32; sh <<= 1) {
-                ml = max(ml, __shfl_xor_sync(0xffffffffu, ml, sh));
-                me = max(me, __shfl_xor_sync(0xffffffffu, me, sh));
+                for (int sh = 1; sh < 8; sh <<= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, sh));
+                e = 8;
+                if (mx) {
+                    const int k = 31 - __clz(mx);
+                    e = max(0, (mx << (8 - k)) <= 448u ? 8 - k : 7 - k);
+                }
+                s = (float)(1 << e);
             }
-            if (lane == 0) {
-                int* bm = reinterpret_cast<int*>(S.bmax);
-                if (ml > *reinterpret_cast<volatile int*>(bm)) atomicMax(bm, ml);
-                if (me > *reinterpret_cast<volatile int*>(bm + 1)) atomicMax(bm + 1, me);
+            // E4M3 of x 2^e for an integer x in 1..255: three mantissa bits, round to nearest even (the carry
+            // moves the exponent), exponent re-biased by 7 - 15; the scale is an exponent shift, so the
+            // rounding error of x itself does not depend on it. Two bytes at a time as FP16 (exact: integers
+            // below 2048, and the squared errors of a lane's bytes add up to at most 8 * 64 per half)
+            uint32_t o[4];
+            __half2 e2 = __float2half2_rn(0.f);
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+                uint32_t c[2];
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    const uint32_t biased = __byte_perm(ww[v], 0x64u, 0x4140u + 0x0202u * b);   // 1024 + x
+                    const __half2 x = __hsub2(as_half2(biased), as_half2(0x64006400u));
+                    const uint32_t u = as_bits(x);
+                    const uint32_t back = (u + 0x003F003Fu + ((u >> 7) & 0x00010001u)) & 0xFF80FF80u;
+                    const __half2 d = __hsub2(as_half2(back), x);
+                    e2 = __hfma2(d, d, e2);
+                    const uint32_t q = back >> 7;
+                    c[b] = q - __vminu2(q, 0x00010001u) * (uint32_t)(64 - 8 * e);   // 0 stays 0
+                }
+                o[v] = __byte_perm(c[0], c[1], 0x6420u);
             }
+            float err2 = __low2float(e2) + __high2float(e2);
+#pragma unroll
+            for (int sh = 1; sh < 8; sh <<= 1) err2 += __shfl_xor_sync(0xffffffffu, err2, sh);
+            *reinterpret_cast<uint4*>(blk + core_off(r, seg * 16, RB)) = make_uint4(o[0], o[1], o[2], o[3]);
+            const float len = live ? sqrtf((float)nrm) * (1.f + 1e-6f) : 0.f;
+            const float elen = live ? sqrtf(err2) * (1.f + 1e-6f) : 0.f;
+            if (role == 0) {
+                if (seg == 0 && live) reinterpret_cast<float4*>(S.rowsc)[row] = make_float4(s, 1.f / s, len, elen);
+            } else {
+                ml = max(ml, __float_as_int(len));
+                me = max(me, __float_as_int(elen));
+            }
+        }
+        if (seg < 2) {   // the 16 norm slots (32 bytes), 16 bytes per lane
+            uint4 x = make_uint4(0u, 0u, 0u, 0u);
+            if (seg == 0 && live) {
+                if (role == 0) {
+                    x.x = bf16_pair(-32768.f * s, -128.f * s);
+                    x.y = bf16_pair(-0.5f * s, 0.f);
+                } else {
+                    x.x = bf16_pair(byte_float((uint32_t)nrm, 2), byte_float((uint32_t)nrm, 1));
+                    x.y = bf16_pair(byte_float((uint32_t)nrm, 0), 0.f);
+                }
+            }
+            *reinterpret_cast<uint4*>(blk + core_off(r, XB + seg * 16, RB)) = x;
         }
     }
-    if (seg < 2) {   // the 16 norm slots (32 bytes), 16 bytes per lane
-        uint4 x = make_uint4(0u, 0u, 0u, 0u);
-        if (seg == 0 && live) {
-            if (S.role == 0) {
-                x.x = bf16_pair(-32768.f * s, -128.f * s);
-                x.y = bf16_pair(-0.5f * s, 0.f);
-            } else {
-                x.x = bf16_pair(byte_float((uint32_t)nrm, 2), byte_float((uint32_t)nrm, 1));
-                x.y = bf16_pair(byte_float((uint32_t)nrm, 0), 0.f);
-            }
+    if (PREC == FSB_PREC_FP8 && role == 1) {   // one pair of atomics per block (see above)
+        ml = __reduce_max_sync(0xffffffffu, ml);
+        me = __reduce_max_sync(0xffffffffu, me);
+        if (lane == 0) {
+            atomicMax(s_max, ml);
+            atomicMax(s_max + 1, me);
         }
-        *reinterpret_cast<uint4*>(blk + core_off(r, XB + seg * 16, RB)) = x;
+        __syncthreads();
+        if (threadIdx.x < 2) atomicMax(reinterpret_cast<int*>(S.bmax) + threadIdx.x, s_max[threadIdx.x]);
     }
 }
 
@@ -651,8 +678,6 @@ __device__ __forceinline__ void warp_top2(long long& k1, long long& d2) {
 
 constexpr long long NO_D = LLONG_MAX >> 32;   // "no distance" (above every uint8 distance)
 
-constexpr int FIN_PASSES = 2;   // a warp finishes 4 rows per pass
-
 // Per-lane error statistics of the certificate (kept by the lane that finishes a row, summed per
 // block, then one global update per block: a global atomic per row on one address serialises the
 // whole kernel).
@@ -661,33 +686,42 @@ struct ErrAcc {
     int n = 0;
 };
 
-// Top-2 merge of (key1 = d << 32 | j, d2) over the 8 lanes of a row group (xor 1, 2, 4).
-__device__ __forceinline__ void group_top2(long long& k1, long long& d2) {
+// The exact dots of a row's 16 bytes with the 16 columns of a chunk; FULL: every column exists, else the
+// columns from lim on repeat the last one (or the first row of the job).
+template <bool FULL>
+__device__ __forceinline__ void chunk_dots(const uint4& a4, const uint8_t* __restrict__ base, int lim,
+                                           uint32_t (&p)[TC_CHUNK]) {
 #pragma unroll
-    for (int sh = 1; sh < 8; sh <<= 1) {
-        const long long ok1 = __shfl_xor_sync(0xffffffffu, k1, sh);
-        const long long od2 = __shfl_xor_sync(0xffffffffu, d2, sh);
-        const long long hi = max(k1, ok1);
-        d2 = min(min(d2, od2), hi >> 32);
-        k1 = min(k1, ok1);
+    for (int i = 0; i < TC_CHUNK; ++i) {
+        const int c = FULL ? i : max(min(i, lim - 1), 0);
+        const uint4 b4 = __ldg(reinterpret_cast<const uint4*>(base + c * 128));
+        p[i] = __dp4a(a4.w, b4.w, __dp4a(a4.z, b4.z, __dp4a(a4.y, b4.y, __dp4a(a4.x, b4.x, 0u))));
     }
 }
 
-// A warp finishes 4 query rows at a time, 8 lanes per row: lane = 8 * grp + seg, seg the 16-byte
-// segment of the 128-byte rows that the lane multiplies. Per row:
+// A warp finishes 4 PASSES query rows, 4 at a time with 8 lanes per row: lane = 8 * grp + seg, seg the
+// 16-byte segment of the 128-byte rows that the lane multiplies; lane 8 * grp + t owns the row of pass t.
 //   1. the K best chunks over the column splits (value descending, chunk ascending; one split's
-//      records are already in that order);
+//      records are already in that order: the owner reads them before the first pass);
 //   2. the exact distances of the re-ranked chunks' 16 columns each: 16 independent 16-byte loads
 //      and dp4a per lane, then a transposed butterfly over seg (8 + 4 + 2 shuffles) leaves lane seg
-//      the whole dots of columns 2 seg, 2 seg + 1; top-2 over the row's lanes;
-//   3. (lane seg 0) the certificate and the float32 ratio test of the reference: BF16, the best
-//      chunk's tensor-core maximum must equal the exact best (the values are exact) and the next
+//      the whole dots of columns 2 seg, 2 seg + 1; top-2 over the row's lanes, of 32-bit keys (a squared
+//      distance of byte rows is below 2^23, the column among the re-ranked ones takes five bits);
+//   3. (the owners, after the passes) the certificate and the float32 ratio test of the reference: BF16,
+//      the best chunk's tensor-core maximum must equal the exact best (the values are exact) and the next
 //      chunk's maximum is the exact best outside it; E4M3, the rounding bound must settle the
 //      decision. Unsettled rows go to k_tc_exact_rows.
-template <int K>
-__global__ void __launch_bounds__(256) k_tc_finish(const TcPair* __restrict__ pairs, const Cand* __restrict__ part,
-                                                   float ratio, int prec, int32_t* __restrict__ flagged,
+// Bound by the latency of the chunk rows (L2) and by instruction issue. Against 64-bit keys, a certificate by
+// one lane in eight after each pass, predicated loads with 64-bit addresses, target norms read after the
+// dots and candidate records read in every pass: 124 -> 55 us (BF16, 262 000 rows, 537 MB of chunk rows),
+// 152 -> 75 us (E4M3, 215 000 rows, 880 MB). Four blocks per SM cost E4M3 ten registers and gain 8 us.
+template <int PREC, int PASSES>
+__global__ void __launch_bounds__(256, 4) k_tc_finish(const TcPair* __restrict__ pairs, const Cand* __restrict__ part,
+                                                   float ratio, int32_t* __restrict__ flagged,
                                                    int* __restrict__ n_flagged, float* __restrict__ err_stat) {
+    constexpr int K = TcTraits<PREC>::TOPK;
+    static_assert(K == 2 && PASSES <= 8, "two records are one 16-byte load; eight lanes own the rows of a group");
+    constexpr int nre = PREC == FSB_PREC_BF16 ? 1 : K;   // chunks re-ranked
     __shared__ float s_mx, s_sum;
     __shared__ int s_n;
     if (threadIdx.x == 0) {
@@ -698,28 +732,33 @@ __global__ void __launch_bounds__(256) k_tc_finish(const TcPair* __restrict__ pa
     __syncthreads();
     const TcPair& P = pairs[blockIdx.y];
     const int lane = threadIdx.x & 31, seg = lane & 7, grp = lane >> 3;
-    const int nre = prec == FSB_PREC_BF16 ? 1 : K;
     const bool h4 = seg & 4, h2 = seg & 2, h1 = seg & 1;
-    ErrAcc acc;
-    const int wq = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (4 * FIN_PASSES);
-    for (int pass = 0; pass < FIN_PASSES; ++pass) {
+    const int n_q = P.na, n_b = P.nb, splits = P.splits;
+    const int wq = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (4 * PASSES);
+    const int own = wq + 4 * seg + grp;
+    const bool owner = seg < PASSES && own < n_q;
+    float sv[K] = {-INFINITY, -INFINITY};   // of the owned row
+    int sc[K] = {-1, -1};
+    if (splits == 1 && owner) {
+        const int4 c = *reinterpret_cast<const int4*>(part + P.part0 + (size_t)own * K);
+        sv[0] = __int_as_float(c.x);
+        sc[0] = c.y;
+        sv[1] = __int_as_float(c.z);
+        sc[1] = c.w;
+    }
+    uint32_t own1 = ~0u, own2 = ~0u;
+#pragma unroll 1
+    for (int pass = 0; pass < PASSES; ++pass) {
         const int q0 = wq + 4 * pass;
-        if (q0 >= P.na) break;   // warp-uniform
-        const int qr = q0 + grp;
-        const bool live = qr < P.na;
-        const int q = live ? qr : P.na - 1;   // dead groups repeat a live row and write nothing
+        if (q0 >= n_q) break;   // warp-uniform
+        const int q = min(q0 + grp, n_q - 1);   // groups past the end repeat a row and keep nothing
         // 1. the K best chunks
-        float sv[K];
-        int sc[K];
-        if (P.splits == 1) {
+        int ch[K];
+        if (splits == 1) {
 #pragma unroll
-            for (int k = 0; k < K; ++k) {
-                const Cand c = part[P.part0 + (size_t)q * K + k];
-                sv[k] = c.v;
-                sc[k] = c.j;
-            }
+            for (int k = 0; k < K; ++k) ch[k] = __shfl_sync(0xffffffffu, sc[k], (lane & 24) | pass);
         } else {
-            const int ne = P.splits * K;   // <= 32: at most 4 records per lane
+            const int ne = splits * K;   // <= 32: at most 4 records per lane
             Cand e[4];
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
@@ -746,44 +785,32 @@ __global__ void __launch_bounds__(256) k_tc_finish(const TcPair* __restrict__ pa
                         bc = oc;
                     }
                 }
-                sv[k] = bv;
-                sc[k] = bc == INT_MAX ? -1 : bc;
+                ch[k] = bc == INT_MAX ? -1 : bc;
+                if (seg == pass) {
+                    sv[k] = bv;
+                    sc[k] = ch[k];
+                }
 #pragma unroll
                 for (int t = 0; t < 4; ++t)
                     if (e[t].j == bc && bc != INT_MAX) e[t] = Cand{-INFINITY, INT_MAX};
             }
         }
-        const long long na = P.nA[q];
-        double inv_s = 1.0, eps = 0.0;
-        if (prec == FSB_PREC_FP8) {
-            const float4 rs = reinterpret_cast<const float4*>(P.rowsc)[q];
-            const double bl = P.bmax[0], be = P.bmax[1];
-            inv_s = rs.y;
-            eps = (double)rs.z * be + (double)rs.w * bl + (double)rs.w * be + (double)rs.z * bl * (1.0 / 512.0) +
-                  4.0;
-        }
         // 2. exact distances of the re-ranked chunks
+        const int na = __ldg(P.nA + q);
         const uint4 a4 = __ldg(reinterpret_cast<const uint4*>(P.a + (size_t)q * 128) + seg);
-        long long k1 = LLONG_MAX, d2 = NO_D;
+        uint32_t k1 = ~0u, k2 = ~0u;
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            if (k >= nre) break;   // warp-uniform
-            const int jc = sc[k] < 0 ? P.nb : sc[k] * TC_CHUNK;   // an empty chunk: no valid column
+        for (int k = 0; k < nre; ++k) {
+            const bool any = ch[k] >= 0 && ch[k] * TC_CHUNK < n_b;   // an empty chunk: no valid column
+            const int jc = any ? ch[k] * TC_CHUNK : 0, lim = any ? min(n_b - jc, TC_CHUNK) : 0;
+            const uint8_t* base = P.b + (size_t)jc * 128 + seg * 16;
+            const int c0 = 2 * seg;   // this lane's columns after the butterfly
+            const int n0 = c0 < lim ? __ldg(P.nB + jc + c0) : 0, n1 = c0 + 1 < lim ? __ldg(P.nB + jc + c0 + 1) : 0;
             uint32_t p[TC_CHUNK];
-#pragma unroll
-            for (int i = 0; i < TC_CHUNK; ++i) {
-                const int j = jc + i;
-                uint32_t dot = 0;
-                if (j < P.nb) {
-                    const uint4 b4 = __ldg(reinterpret_cast<const uint4*>(P.b + (size_t)j * 128) + seg);
-                    dot = __dp4a(a4.x, b4.x, dot);
-                    dot = __dp4a(a4.y, b4.y, dot);
-                    dot = __dp4a(a4.z, b4.z, dot);
-                    dot = __dp4a(a4.w, b4.w, dot);
-                }
-                p[i] = dot;
-            }
+            if (__all_sync(0xffffffffu, lim == TC_CHUNK)) chunk_dots<true>(a4, base, lim, p);
+            else chunk_dots<false>(a4, base, lim, p);
             constexpr int C2 = TC_CHUNK / 2, C4 = TC_CHUNK / 4, C8 = TC_CHUNK / 8;
+            static_assert(C8 == 2, "two columns per lane");
 #pragma unroll
             for (int t = 0; t < C2; ++t)
                 p[t] = (h4 ? p[t + C2] : p[t]) + __shfl_xor_sync(0xffffffffu, h4 ? p[t] : p[t + C2], 4);
@@ -793,35 +820,51 @@ __global__ void __launch_bounds__(256) k_tc_finish(const TcPair* __restrict__ pa
 #pragma unroll
             for (int t = 0; t < C8; ++t)
                 p[t] = (h1 ? p[t + C8] : p[t]) + __shfl_xor_sync(0xffffffffu, h1 ? p[t] : p[t + C8], 1);
-#pragma unroll
-            for (int t = 0; t < C8; ++t) {
-                const int j = jc + C8 * seg + t;
-                if (j < P.nb) {
-                    const long long d = na + __ldg(P.nB + j) - 2ll * (long long)p[t];
-                    const long long key = (d << 32) | (unsigned)j;
-                    if (key < k1) {
-                        d2 = min(d2, k1 >> 32);
-                        k1 = key;
-                    } else {
-                        d2 = min(d2, d);
-                    }
-                }
-            }
+            // equal distances order by column: the earlier chunk's columns first
+            const uint32_t at = (nre > 1 && ch[k] > ch[1 - k] ? TC_CHUNK : 0) + c0;
+            const uint32_t x0 = c0 < lim ? (uint32_t)(na + n0 - 2 * (int)p[0]) << 5 | at : ~0u;
+            const uint32_t x1 = c0 + 1 < lim ? (uint32_t)(na + n1 - 2 * (int)p[1]) << 5 | (at + 1) : ~0u;
+            const uint32_t lo = min(x0, x1), hi = max(x0, x1);
+            k2 = min(min(k2, hi), max(k1, lo));
+            k1 = min(k1, lo);
         }
-        group_top2(k1, d2);
-        if (seg != 0 || !live) continue;
-        // 3. certificate and ratio test
-        const int g = P.row0 + q;
-        const bool has1 = k1 != LLONG_MAX;
-        const long long e1 = has1 ? (k1 >> 32) : NO_D;
-        const int j1 = (int)(k1 & 0xffffffffll);
-        long long e2 = d2;
+#pragma unroll
+        for (int sh = 1; sh < 8; sh <<= 1) {
+            const uint32_t o1 = __shfl_xor_sync(0xffffffffu, k1, sh);
+            const uint32_t o2 = __shfl_xor_sync(0xffffffffu, k2, sh);
+            k2 = min(min(k2, o2), max(k1, o1));
+            k1 = min(k1, o1);
+        }
+        if (seg == pass) {
+            own1 = k1;
+            own2 = k2;
+        }
+    }
+    // 3. certificate and ratio test
+    ErrAcc acc;
+    if (owner) {
+        const long long na = P.nA[own];
+        double inv_s = 1.0, eps = 0.0;
+        if (PREC == FSB_PREC_FP8) {
+            const float4 rs = reinterpret_cast<const float4*>(P.rowsc)[own];
+            const double bl = P.bmax[0], be = P.bmax[1];
+            inv_s = rs.y;
+            eps = (double)rs.z * be + (double)rs.w * bl + (double)rs.w * be + (double)rs.z * bl * (1.0 / 512.0) +
+                  4.0;
+        }
+        const int q = own, g = P.row0 + q;
+        const bool has1 = own1 != ~0u;
+        const long long e1 = has1 ? (long long)(own1 >> 5) : NO_D;
+        const bool late = own1 & TC_CHUNK;   // the later of the two re-ranked chunks
+        const int c1 = nre == 1 ? sc[0] : late ? max(sc[0], sc[1]) : min(sc[0], sc[1]);
+        const int j1 = c1 * TC_CHUNK + (int)(own1 & (TC_CHUNK - 1));
+        long long e2 = own2 != ~0u ? (long long)(own2 >> 5) : NO_D;
         bool mismatch = false;
         float err = 0.f;
         if (has1) {
             const double approx = (double)na - 2.0 * (double)sv[0] * inv_s;   // the best chunk's maximum
             err = (float)fabs(approx - (double)e1);
-            if (prec == FSB_PREC_BF16) {
+            if (PREC == FSB_PREC_BF16) {
                 mismatch = err != 0.f;
                 // BF16 values are exact: the best column outside the first chunk is the second chunk's maximum
                 if (sv[1] > -INFINITY) e2 = min(e2, na - (long long)(2.0 * (double)sv[1]));
@@ -1037,15 +1080,14 @@ int32_t run_match_bf_tc(fsb_ctx* ctx, int n_pairs, const uint8_t* const* d_a, co
     PackSeg* d_segs = reinterpret_cast<PackSeg*>(take(b_segs));
     int32_t* norms = reinterpret_cast<int32_t*>(take(b_norm));
     float* rowsc = reinterpret_cast<float*>(take(b_rowsc));
-    float* bmax = reinterpret_cast<float*>(take(b_bmax));
     int32_t* flagged = reinterpret_cast<int32_t*>(take(b_rowi));
     unsigned long long* keys = reinterpret_cast<unsigned long long*>(take(b_keys));
     int32_t* flag = reinterpret_cast<int32_t*>(take(b_flag));
     int32_t* pos = reinterpret_cast<int32_t*>(take(b_flag));
     void* scan_tmp = take(al(tb_scan));
     int* small = reinterpret_cast<int*>(take(256));   // [0] abort, [1] flagged rows, [2..4] error statistics
-    FSB_CUDA(cudaMemsetAsync(small, 0, 64, s));
-    if (fp8) FSB_CUDA(cudaMemsetAsync(bmax, 0, (size_t)n_pairs * 8, s));
+    float* bmax = reinterpret_cast<float*>(take(b_bmax));
+    FSB_CUDA(cudaMemsetAsync(small, 0, 256 + (size_t)n_pairs * 8, s));   // and bmax
     std::vector<PackSeg> segs;
     segs.reserve(2 * n_pairs);
     size_t pa = 0, pb = 0, nn = 0, rr = 0;
@@ -1064,17 +1106,18 @@ int32_t run_match_bf_tc(fsb_ctx* ctx, int n_pairs, const uint8_t* const* d_a, co
         max_na = std::max(max_na, P.na);
         max_nb = std::max(max_nb, P.nb);
         segs.push_back(PackSeg{P.a, const_cast<uint8_t*>(P.pa), const_cast<int32_t*>(P.nA), const_cast<float*>(P.rowsc),
-                               nullptr, P.na, pad_a, 0});
+                               nullptr, nullptr, P.na, pad_a, 0});
         segs.push_back(PackSeg{P.b, const_cast<uint8_t*>(P.pb), const_cast<int32_t*>(P.nB), nullptr,
-                               const_cast<float*>(P.bmax), P.nb, pad_b, 1});
+                               const_cast<float*>(P.bmax), P.key, P.nb, pad_b, 1});
         pa += (size_t)pad_a * RB;
         pb += (size_t)pad_b * RB;
         nn += (size_t)P.na + P.nb;
         rr += (size_t)P.na;
     }
-    FSB_CUDA(cudaMemcpyAsync(d_pairs, hp.data(), (size_t)n_pairs * sizeof(TcPair), cudaMemcpyHostToDevice, s));
-    FSB_CUDA(cudaMemcpyAsync(d_segs, segs.data(), segs.size() * sizeof(PackSeg), cudaMemcpyHostToDevice, s));
-    FSB_CUDA(cudaMemsetAsync(keys, 0xff, (size_t)n_keys * 8, s));
+    std::vector<uint8_t> tables(b_pairs + b_segs);   // both tables in one transfer
+    memcpy(tables.data(), hp.data(), (size_t)n_pairs * sizeof(TcPair));
+    memcpy(tables.data() + b_pairs, segs.data(), segs.size() * sizeof(PackSeg));
+    FSB_CUDA(cudaMemcpyAsync(d_pairs, tables.data(), tables.size(), cudaMemcpyHostToDevice, s));
     const dim3 pack_grid(nblk(max_pad, PACK_ROWS), (unsigned)segs.size());
     if (fp8)
         k_tc_pack<FSB_PREC_FP8><<<pack_grid, PACK_T, 0, s>>>(d_segs);
@@ -1089,13 +1132,18 @@ int32_t run_match_bf_tc(fsb_ctx* ctx, int n_pairs, const uint8_t* const* d_a, co
     note_launch(1);
     ctx->stage_end(ST_TC_DENSE);
     float* err_stat = stats ? reinterpret_cast<float*>(small + 2) : nullptr;
-    const dim3 fin_grid(nblk(max_na, 8 * 4 * FIN_PASSES), (unsigned)n_pairs);
-    if (fp8)
-        k_tc_finish<TcTraits<FSB_PREC_FP8>::TOPK><<<fin_grid, 256, 0, s>>>(d_pairs, part, ratio, precision, flagged,
-                                                                           small + 1, err_stat);
-    else
-        k_tc_finish<TcTraits<FSB_PREC_BF16>::TOPK><<<fin_grid, 256, 0, s>>>(d_pairs, part, ratio, precision, flagged,
-                                                                            small + 1, err_stat);
+    // enough rows for every warp slot of the GPU: 16 rows per warp (the certificate at the end by half of the
+    // lanes, records read once), else 4 (a chain of one pass)
+    constexpr int FIN_LONG = 4;
+    auto finish = [&](auto kernel, int passes) {
+        kernel<<<dim3(nblk(max_na, 8 * 4 * passes), (unsigned)n_pairs), 256, 0, s>>>(d_pairs, part, ratio, flagged,
+                                                                                     small + 1, err_stat);
+    };
+    const bool many = rows >= 32 * 4 * FIN_LONG * num_sms;
+    if (fp8 && many) finish(k_tc_finish<FSB_PREC_FP8, FIN_LONG>, FIN_LONG);
+    else if (fp8) finish(k_tc_finish<FSB_PREC_FP8, 1>, 1);
+    else if (many) finish(k_tc_finish<FSB_PREC_BF16, FIN_LONG>, FIN_LONG);
+    else finish(k_tc_finish<FSB_PREC_BF16, 1>, 1);
     // the rows the certificate did not settle (their number is on the device; usually none, and the blocks leave)
     k_tc_exact_rows<<<std::min(rows, 2 * num_sms), 256, 0, s>>>(d_pairs, n_pairs, flagged, small + 1, ratio);
     note_launch(2);
