@@ -21,8 +21,8 @@
 //                shared-memory ring with bulk asynchronous copies (no tensor map, no multicast);
 //                warp 1 issues the MMAs (M=128, N=256) for the two 128-row halves of a 256-row
 //                query block into FP32 accumulators (2 x 256 of the 512 TMEM columns); warps 2-9
-//                read the accumulators with tcgen05.ld (four 32-column loads per wait), a half being
-//                drained while the other is computed, and keep, per query row, the two largest
+//                read the accumulators with tcgen05.ld (64 columns being loaded while 64 are reduced), a
+//                half being drained while the other is computed, and keep, per query row, the two largest
 //                16-column maxima and their chunks. At N = 128 an MMA's operands take the whole
 //                shared-memory read bandwidth (8 KB per 64 cycles); at N = 256 three quarters of it.
 //   k_tc_finish  per query row: the two best chunks over all column splits and the exact integer
@@ -358,7 +358,8 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
                  : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+// 32 columns of the warp's 32 lanes into r[0..31]
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
         "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
@@ -369,7 +370,19 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
           "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
         : "r"(taddr));
 }
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// Waits for the thread's loads from tensor memory; the 64 registers are operands, so that nothing that
+// reads them moves before the wait (and work on other registers may stay between the loads and it).
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[64]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]),
+                   "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]),
+                   "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31]),
+                   "+r"(r[32]), "+r"(r[33]), "+r"(r[34]), "+r"(r[35]), "+r"(r[36]), "+r"(r[37]), "+r"(r[38]), "+r"(r[39]),
+                   "+r"(r[40]), "+r"(r[41]), "+r"(r[42]), "+r"(r[43]), "+r"(r[44]), "+r"(r[45]), "+r"(r[46]), "+r"(r[47]),
+                   "+r"(r[48]), "+r"(r[49]), "+r"(r[50]), "+r"(r[51]), "+r"(r[52]), "+r"(r[53]), "+r"(r[54]), "+r"(r[55]),
+                   "+r"(r[56]), "+r"(r[57]), "+r"(r[58]), "+r"(r[59]), "+r"(r[60]), "+r"(r[61]), "+r"(r[62]), "+r"(r[63]));
+}
 
 __device__ __forceinline__ float max3(float a, float b, float c) {
     float r;
@@ -377,21 +390,38 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
     return r;
 }
 
-// v > t[K-1]: insert keeping t descending; among equal values the earlier chunk stays first
-template <int K>
-__device__ __forceinline__ void top_insert(float (&t)[K], int (&j)[K], float v, int col) {
+// v > t[1]: insert keeping t descending; among equal values the earlier chunk stays first. Selects, no
+// branch: some lane of a warp inserts in about a third of the chunks, and a branch per chunk made the
+// drain of an accumulator a chain of branches.
+__device__ __forceinline__ void top_insert(float (&t)[2], int (&j)[2], float v, int col) {
+    const bool first = v > t[0], second = v > t[1];
+    j[1] = first ? j[0] : second ? col : j[1];
+    j[0] = first ? col : j[0];
+    t[1] = fmaxf(t[1], fminf(t[0], v));
+    t[0] = fmaxf(t[0], v);
+}
+
+// The chunk maxima of 64 columns (the first is column j0 of the job's targets, of which nb exist)
+__device__ __forceinline__ void top_columns(const uint32_t (&r)[64], int j0, int nb, bool edge, float (&tv)[2],
+                                            int (&tj)[2]) {
+    static_assert(TC_CHUNK == 16, "maximum tree");
+    float mx[64 / TC_CHUNK];
 #pragma unroll
-    for (int i = K - 1; i >= 0; --i) {
-        if (v > t[i]) {
-            if (i > 0 && v > t[i - 1]) {
-                t[i] = t[i - 1];
-                j[i] = j[i - 1];
-            } else {
-                t[i] = v;
-                j[i] = col;
-            }
+    for (int ch = 0; ch < 64 / TC_CHUNK; ++ch) {
+        float v[TC_CHUNK];
+#pragma unroll
+        for (int i = 0; i < TC_CHUNK; ++i) v[i] = __uint_as_float(r[ch * TC_CHUNK + i]);
+        if (edge) {   // the last tile of the job (uniform)
+#pragma unroll
+            for (int i = 0; i < TC_CHUNK; ++i)
+                if (j0 + ch * TC_CHUNK + i >= nb) v[i] = -INFINITY;
         }
+        const float a0 = max3(v[0], v[1], v[2]), a1 = max3(v[3], v[4], v[5]), a2 = max3(v[6], v[7], v[8]);
+        const float a3 = max3(v[9], v[10], v[11]), a4 = max3(v[12], v[13], v[14]);
+        mx[ch] = fmaxf(max3(a0, a1, a2), max3(a3, a4, v[15]));
     }
+#pragma unroll
+    for (int ch = 0; ch < 64 / TC_CHUNK; ++ch) top_insert(tv, tj, mx[ch], j0 / TC_CHUNK + ch);
 }
 
 // The item of CTA `cta` in round w: items are in descending length (the pairs are sorted by their
@@ -410,6 +440,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     constexpr int TB = tile_bytes<PREC>(), HB = half_bytes<PREC>();
     constexpr int NST = T::STAGES;
     constexpr int K = T::TOPK;
+    static_assert(K == 2, "top_insert");
     constexpr uint32_t SBO = T::ROW_BYTES * 8;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem =
@@ -583,7 +614,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             const int local = item - P.item0;
             const int rb = local / P.splits, sp = local - rb * P.splits;
             const int t0 = sp * P.tps, t1 = min(P.ntiles, t0 + P.tps);
-            const int q = rb * TC_ROWS + rloc;
+            const int q = rb * TC_ROWS + rloc, nb = P.nb;
             float tv[K];
             int tj[K];
 #pragma unroll
@@ -595,38 +626,30 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                 ok = mbar_wait(acc_full + h, tit & 1, abort_flag);
                 if (!ok) break;
                 tc_fence_after();
+                // 64 columns of the row at a time: the next ones are loaded while these are reduced (128 loaded,
+                // then reduced with a branch per chunk: BF16 781 us against 739 for 16 x 16384^2, E4M3 374
+                // against 328 for 24 pairs, the half's next MMA waiting for the drain);
+                // after the last loads the accumulator is free
                 const uint32_t base = tmem + ((uint32_t)(lq * 32) << 16) + (uint32_t)(h * TC_N);
-#pragma unroll 1
-                for (int c0 = 0; c0 < TC_N; c0 += 128) {
-                    // 128 columns of the row at once (four loads, one wait); after the last ones the
-                    // accumulator is free
-                    uint32_t r[4][32];
+                const int j0 = t * TC_N;
+                const bool edge = j0 + TC_N > nb;
+                constexpr int PIECES = TC_N / 64;
+                uint32_t r[2][64];
+                tmem_ld32(base, r[0]);
+                tmem_ld32(base + 32, r[0] + 32);
+                tmem_wait_ld(r[0]);
 #pragma unroll
-                    for (int ch = 0; ch < 4; ++ch) tmem_ld32(base + c0 + ch * 32, r[ch]);
-                    tmem_wait_ld();
-                    if (c0 + 128 == TC_N) {
+                for (int c = 0; c < PIECES; ++c) {
+                    if (c + 1 < PIECES) {
+                        tmem_ld32(base + (c + 1) * 64, r[(c + 1) & 1]);
+                        tmem_ld32(base + (c + 1) * 64 + 32, r[(c + 1) & 1] + 32);
+                    } else {
                         tc_fence_before();
                         __syncwarp();
                         if (lane == 0) mbar_arrive(acc_empty + h);
                     }
-#pragma unroll
-                    for (int ch = 0; ch < 128 / TC_CHUNK; ++ch) {
-                        const int j0 = t * TC_N + c0 + ch * TC_CHUNK;
-                        float v[TC_CHUNK];
-#pragma unroll
-                        for (int i = 0; i < TC_CHUNK; ++i)
-                            v[i] = __uint_as_float(r[ch / (32 / TC_CHUNK)][ch % (32 / TC_CHUNK) * TC_CHUNK + i]);
-                        if (j0 + TC_CHUNK > P.nb) {
-#pragma unroll
-                            for (int i = 0; i < TC_CHUNK; ++i)
-                                if (j0 + i >= P.nb) v[i] = -INFINITY;
-                        }
-                        static_assert(TC_CHUNK == 16, "maximum tree");
-                        const float a0 = max3(v[0], v[1], v[2]), a1 = max3(v[3], v[4], v[5]), a2 = max3(v[6], v[7], v[8]);
-                        const float a3 = max3(v[9], v[10], v[11]), a4 = max3(v[12], v[13], v[14]);
-                        const float mx = fmaxf(max3(a0, a1, a2), max3(a3, a4, v[15]));
-                        if (mx > tv[K - 1]) top_insert<K>(tv, tj, mx, j0 / TC_CHUNK);
-                    }
+                    top_columns(r[c & 1], j0 + c * 64, nb, edge, tv, tj);
+                    if (c + 1 < PIECES) tmem_wait_ld(r[(c + 1) & 1]);
                 }
             }
             if (!ok) break;
