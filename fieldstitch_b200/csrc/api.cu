@@ -938,6 +938,35 @@ int32_t fsb_sift_features_ex_d(fsb_ctx* ctx, const uint8_t* d_img, int32_t h, in
 
 namespace fsb {
 namespace {
+// the launches of a batch as a graph, for later calls with the same key
+int32_t capture_batch(fsb_ctx* ctx, const BatchCall& bc, const std::vector<char>& key) {
+    auto& x = ctx->xb;
+    if (x.graph.exec) cudaGraphExecDestroy(x.graph.exec);
+    if (x.graph.graph) cudaGraphDestroy(x.graph.graph);
+    x.graph.exec = nullptr;
+    x.graph.graph = nullptr;
+    const long long m0 = launch_mark();
+    FSB_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+    const int32_t st = batch_body(ctx, bc);
+    x.graph.n_kernels = (int)(launch_mark() - m0);
+    note_launch(-x.graph.n_kernels);   // the kernels run (and count) at each replay
+    cudaGraph_t g = nullptr;
+    const cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
+    if (st != FSB_OK) {
+        if (g) cudaGraphDestroy(g);
+        return st;
+    }
+    if (e != cudaSuccess) {
+        if (g) cudaGraphDestroy(g);
+        set_error("capture of the extraction batch failed: %s", cudaGetErrorString(e));
+        return FSB_ERR_CUDA;
+    }
+    x.graph.graph = g;
+    FSB_CUDA(cudaGraphInstantiate(&x.graph.exec, g, 0));
+    x.graph.key = key;
+    return FSB_OK;
+}
+
 // fsb_sift_features_batch_d and, with h_imgs, fsb_sift_features_batch_hd
 int32_t sift_features_batch(fsb_ctx* ctx, int32_t n_img, const uint8_t* const* h_imgs, const uint8_t* const* d_imgs,
                             int32_t h, int32_t w, int32_t stride, const fsb_sift_params* p, const int32_t* nfeats,
@@ -1076,53 +1105,29 @@ int32_t sift_features_batch(fsb_ctx* ctx, int32_t n_img, const uint8_t* const* h
         key_put(key, ws->sort_tmp.bytes);
     }
     // A call with other arguments than the last one is launched directly (about 65 launches an image, queued
-    // faster than they run); capturing and instantiating it costs 3.6 ms per 16 images before any of them
-    // runs: 16 photos of 2640 x 1978 in new buffers 16.9 -> 14.0 ms. The second such call in a row captures
-    // the graph, later ones replay it (13.7 ms).
+    // faster than they run); capturing and instantiating a graph costs 3.6 ms per 16 images before any of
+    // them runs: 16 photos of 2640 x 1978 in new buffers 16.9 -> 14.0 ms. The second such call in a row is
+    // launched directly too, and the graph captured while the GPU works on it; later ones replay it (13.7 ms).
+    BatchCall bc{n_img, d_imgs, h_imgs, h, w, stride, p, nfeats, d_xy, d_resp, d_rootsift, d_counts};
     const bool replay = x.graph.exec && key == x.graph.key;
-    const bool direct = !replay && key != x.last_key;
+    const bool again = !replay && key == x.last_key;
     x.last_key = key;
-    if (direct) {
-        BatchCall bc{n_img, d_imgs, h_imgs, h, w, stride, p, nfeats, d_xy, d_resp, d_rootsift, d_counts};
+    if (replay) {
+        for (int i = 0; h_imgs && i < n_img; ++i)
+            FSB_CUDA(cudaGraphExecMemcpyNodeSetParams1D(x.graph.exec, x.copy_nodes[i], const_cast<uint8_t*>(d_imgs[i]),
+                                                        h_imgs[i], (size_t)h * stride, cudaMemcpyHostToDevice));
+        FSB_CUDA(cudaGraphLaunch(x.graph.exec, s));
+        note_launch(x.graph.n_kernels);
+    } else {
         const int32_t st = batch_body(ctx, bc);
         if (st != FSB_OK) {   // no work left behind on the chains' streams
             for (cudaStream_t c : x.streams) cudaStreamSynchronize(c);
             if (x.upload) cudaStreamSynchronize(x.upload);
             return st;
         }
-    } else if (!replay) {
-        if (x.graph.exec) cudaGraphExecDestroy(x.graph.exec);
-        if (x.graph.graph) cudaGraphDestroy(x.graph.graph);
-        x.graph.exec = nullptr;
-        x.graph.graph = nullptr;
-        BatchCall bc{n_img, d_imgs, h_imgs, h, w, stride, p, nfeats, d_xy, d_resp, d_rootsift, d_counts};
-        const long long m0 = launch_mark();
-        FSB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        const int32_t st = batch_body(ctx, bc);
-        x.graph.n_kernels = (int)(launch_mark() - m0);
-        note_launch(-x.graph.n_kernels);   // the kernels run (and count) at each replay
-        cudaGraph_t g = nullptr;
-        const cudaError_t e = cudaStreamEndCapture(s, &g);
-        if (st != FSB_OK) {
-            if (g) cudaGraphDestroy(g);
-            return st;
-        }
-        if (e != cudaSuccess) {
-            if (g) cudaGraphDestroy(g);
-            set_error("capture of the extraction batch failed: %s", cudaGetErrorString(e));
-            return FSB_ERR_CUDA;
-        }
-        x.graph.graph = g;
-        FSB_CUDA(cudaGraphInstantiate(&x.graph.exec, g, 0));
-        x.graph.key = key;
     }
-    if (!direct) {
-        for (int i = 0; h_imgs && i < n_img; ++i)
-            FSB_CUDA(cudaGraphExecMemcpyNodeSetParams1D(x.graph.exec, x.copy_nodes[i], const_cast<uint8_t*>(d_imgs[i]),
-                                                        h_imgs[i], (size_t)h * stride, cudaMemcpyHostToDevice));
-        FSB_CUDA(cudaGraphLaunch(x.graph.exec, s));
-        note_launch(x.graph.n_kernels);
-    }
+    int32_t capture_st = FSB_OK;
+    if (again) capture_st = capture_batch(ctx, bc, key);
     // one wait per batch: the flags say which images (if any) exceeded a capacity
     FSB_TRY(stage_ensure(ctx, (size_t)n_img * 8 + 64));
     uint32_t* h_status = static_cast<uint32_t*>(ctx->pinned);
@@ -1154,7 +1159,7 @@ int32_t sift_features_batch(fsb_ctx* ctx, int32_t n_img, const uint8_t* const* h
         x.redone += 1;
     }
     if (h_counts) std::memcpy(h_counts, h_cnt, (size_t)n_img * 4);
-    return FSB_OK;
+    return capture_st;
 }
 }  // namespace
 }  // namespace fsb
@@ -1280,7 +1285,7 @@ int32_t fsb_pyramid_batch_d(fsb_ctx* ctx, int32_t n_img, const uint8_t* const* d
     }
     FSB_CUDA(cudaGraphLaunch(x.pyr_graph.exec, s));
     note_launch(x.pyr_graph.n_kernels);
-    // the error words of the chains' bounded waits (strip engine)
+    // the error words of the chains' bounded waits (tensor copies of the tiles)
     const int used = chains < n_img ? chains : n_img;
     FSB_TRY(stage_ensure(ctx, (size_t)used * 4 + 64));
     int32_t* h_err = static_cast<int32_t*>(ctx->pinned);

@@ -153,9 +153,9 @@ int32_t fsb_sift_features_ex_d(fsb_ctx* ctx, const uint8_t* d_img, int32_t h, in
 /* fsb_sift_features_d over a batch of n_img same-size images in device memory (the per-photo
    feature step of the reference's GPU worker, app/planesite/features.py:115-129 and 343-378, for a
    batch), with no host wait inside the batch: every count stays on the device and each launch is
-   sized by a capacity fixed for the geometry, so the whole batch is one CUDA graph - `chains`
-   images in flight, each chain with its own stream and workspace - captured on the first call and
-   replayed while the arguments and buffers are unchanged. Image i: d_imgs[i] (h x w, row pitch
+   sized by a capacity fixed for the geometry: `chains` images in flight, each chain with its own
+   stream and workspace. A call with new arguments or buffers is launched directly, the second equal
+   call in a row captures a CUDA graph, later equal calls replay it. Image i: d_imgs[i] (h x w, row pitch
    stride), nfeats[i] features; outputs d_xy[i] (nfeat*2 float32), d_resp[i] (nfeat float32,
    nullable array), d_rootsift[i] (nfeat*128 uint8); d_counts (device, n_img int32) receives the
    feature counts, h_counts (host, nullable) too. The first call for a geometry runs image 0 by
@@ -167,7 +167,7 @@ int32_t fsb_sift_features_batch_d(fsb_ctx* ctx, int32_t n_img, const uint8_t* co
                                   float* const* d_resp, uint8_t* const* d_rootsift, int32_t* d_counts,
                                   int32_t* h_counts, int32_t chains);
 /* fsb_sift_features_batch_d from host images: h_imgs[i] (page-locked host memory, h rows of
-   `stride` bytes) is uploaded into d_imgs[i] by the same graph, on a copy stream in image order,
+   `stride` bytes) is uploaded into d_imgs[i] by the same batch, on a copy stream in image order,
    and image i's extraction waits for its own upload only, so the uploads of later images overlap
    the extraction of earlier ones. The graph is keyed like fsb_sift_features_batch_d's (device
    buffers, not host addresses): a later call with other host buffers replays it with the uploads
@@ -207,8 +207,7 @@ int32_t fsb_match_guided_d(fsb_ctx* ctx, const double* d_pred, const uint8_t* d_
    data in device memory): pair p matches d_a[p] (na[p] queries, predicted positions d_pred[p])
    against d_b[p] (nb[p] targets at d_bxy[p], frame w_b[p] x h_b[p]) and writes n_out[p] pairs
    into d_q[p], d_t[p]. All pairs share one set of launches (one grid build, one guided kernel
-   over every query of every pair, one batched _unique), issued as a CUDA graph that is captured
-   on the first call and replayed while the pair table and the context's scratch are unchanged.
+   over every query of every pair, one batched _unique).
    Replaces a loop over matching._guided (app/planesite/matching.py:113-152); results are
    identical to per-pair calls. */
 int32_t fsb_match_guided_batch_d(fsb_ctx* ctx, int32_t n_pairs, const double* const* d_pred,
