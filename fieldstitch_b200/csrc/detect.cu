@@ -89,9 +89,11 @@ __device__ __forceinline__ void ex_cp_async8(float2* dst, const float* src) {
 // 27-neighbourhood - ties count - and is beyond the threshold, as scipy's maximum_filter / minimum_filter
 // test in the reference (gsift.py:293-319). Candidates of a row are appended with one atomic.
 //
-// Bound by instruction issue (max / min on the ALU pipe at half rate; HBM, 557 MB, would allow 85 us). Two
-// columns per lane share a row's addresses, copies, loop and half of its shuffles, and a smaller window
-// (the layers are reduced first) leaves the registers for it. 2640 x 1978: 181 -> 138 us.
+// Bound by latency at 28 warps per SM (the copies' wait, shuffles, an atomic per row with candidates; issue
+// 31 %; HBM, 557 MB, would allow 85 us). Two columns per lane share a row's addresses, copies, loop and half
+// of its shuffles, and a smaller window (the layers are reduced first) leaves the registers for it.
+// 2640 x 1978: 181 -> 138 us. Candidates collected in shared memory and appended by one atomic per 192 of
+// them cost 30 us (less L1 left for the copies).
 __global__ void __launch_bounds__(EX_T, EX_BLOCKS) k_extrema(const float* __restrict__ DF, DetectConsts k, ExTiles tl,
                                                   uint32_t* __restrict__ cand, uint32_t* counter, uint32_t cap) {
     __shared__ float2 ex_ring[EX_DEPTH * 5 * EX_T];

@@ -949,8 +949,8 @@ int32_t launch_group_t(GroupArgs a, cudaStream_t s) {
 
 // The group with tiles for small octaves: 32 x 16 while they all fit on the GPU at once, else 64 x 16. An
 // octave of 240 x 320 is 24 tiles of 128 x 32 - 24 SMs, each six passes over 13 000 pixels of input,
-// 17 us - or 150 tiles of 32 x 16 with 5 000 pixels each. 320 x 240: the groups 18.7 and 14.7 us a launch, now 10.9 and
-// 9.6; the whole pyramid 147 -> 117 us.
+// 17 us - or 150 tiles of 32 x 16 with 5 000 pixels each. 320 x 240: the groups 18.7 and 14.7 us a
+// launch, now 10.9 and 9.6; the whole pyramid 147 -> 117 us.
 template <int G>
 int32_t launch_group_small(const GroupArgs& a, cudaStream_t s) {
     const long long small = (long long)((a.C + 31) / 32) * ((a.R + 15) / 16);

@@ -119,10 +119,10 @@ def sift_gpu_batch(images, nfeats, streams=4, contrast=0.015, edge=12.0, exact=F
 def sift_gpu_batch_d(images, nfeats, out_xy, out_u8, out_resp=None, chains=16, contrast=0.015, edge=12.0,
                      exact=False, device=0, host_images=None):
     """Batched feature extraction on device data with no host wait inside the batch
-    (fsb_sift_features_batch_d: one CUDA graph, `chains` images in flight). images: same-size
+    (fsb_sift_features_batch_d: `chains` images in flight, a CUDA graph once the call repeats). images: same-size
     uint8 CUDA tensors; nfeats: one cap per image; out_xy[i] (>= nfeat, 2) float32, out_u8[i]
     (>= nfeat, 128) uint8 and optionally out_resp[i] CUDA tensors. With host_images (page-locked
-    host arrays or CPU tensors, one per image, rows as long as the device images'), the graph
+    host arrays or CPU tensors, one per image, rows as long as the device images'), the batch
     uploads host_images[i] into images[i] itself, overlapping the uploads with the extraction
     (fsb_sift_features_batch_hd). Returns the feature counts (host list); equal to sift_gpu_u8 /
     fsb_sift_features_d image by image."""
@@ -180,9 +180,9 @@ _BATCH_BUFS = {}
 
 
 def sift_gpu_u8_batch(images, nfeats, chains=16, contrast=0.015, edge=12.0, exact=False, device=0):
-    """sift_gpu_u8 of many same-size host images as one sync-free batch: one CUDA graph extracts
-    them all (fsb_sift_features_batch_d; images in page-locked memory are uploaded by the graph
-    itself, overlapping the extraction: fsb_sift_features_batch_hd) and the results come back. Returns [(xy float32 (n,2), RootSIFT
+    """sift_gpu_u8 of many same-size host images as one sync-free batch
+    (fsb_sift_features_batch_d; images in page-locked memory are uploaded by the batch itself,
+    overlapping the extraction: fsb_sift_features_batch_hd). Returns [(xy float32 (n,2), RootSIFT
     uint8 (n,128), resp float32 (n,))], equal to sift_gpu_u8 image by image. The device buffers are
     kept between calls of the same shape, so a repeated batch replays its graph."""
     import torch

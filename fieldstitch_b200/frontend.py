@@ -4,10 +4,10 @@ every pair, with the features kept in device memory between the two stages.
 In the reference, the feature workers write one npz file per photo (features._save,
 app/planesite/features.py:74-86) and the pair workers read them back (matching._get,
 app/planesite/matching.py:48-64) before guided matching (matching._guided, matching.py:113-152).
-``extract_and_match`` does the same work for a batch: one CUDA graph extracts every image
-(features.sift_gpu_batch_d; images in page-locked memory are uploaded by that graph, each
+``extract_and_match`` does the same work for a batch: one sync-free batch extracts every image
+(features.sift_gpu_batch_d; images in page-locked memory are uploaded by that batch, each
 image's extraction starting once its own upload is done), every pair's prior prediction is
-projected on the device, one CUDA graph matches every pair (matching.guided_from_pred_batch_d),
+projected on the device, one set of launches matches every pair (matching.guided_from_pred_batch_d),
 and the match lists come back in one copy. The features come back too when asked for (one copy
 per kind).
 """

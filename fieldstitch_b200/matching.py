@@ -91,7 +91,7 @@ def ratio_match_bf_batch_d(a_list, b_list, ratio, precision="bf16", device=0, ou
 
 
 def guided_from_pred_batch_d(problems, radius, kc, ratio, device=0, out=None):
-    """Many ``guided_from_pred`` problems in one call on device-resident data, as one CUDA graph.
+    """Many ``guided_from_pred`` problems in one call on device-resident data, as one set of launches.
 
     ``problems[p]`` = (pred float64 (na,2), a uint8 (na,128), b_xy float64 (nb,2), b uint8 (nb,128),
     (w_b, h_b)), CUDA tensors on ``device``. ``out[p]`` (optional, reused across calls): a pair of
