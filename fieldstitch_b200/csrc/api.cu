@@ -938,33 +938,35 @@ int32_t fsb_sift_features_ex_d(fsb_ctx* ctx, const uint8_t* d_img, int32_t h, in
 
 namespace fsb {
 namespace {
-// the launches of a batch as a graph, for later calls with the same key
-int32_t capture_batch(fsb_ctx* ctx, const BatchCall& bc, const std::vector<char>& key) {
+// The launches of a batch as a graph, for later calls with the same key. The graph is a cache: the call's own
+// work is done without it, so a failed capture leaves no graph and no error, and its key is not tried again.
+void capture_batch(fsb_ctx* ctx, const BatchCall& bc, const std::vector<char>& key) {
     auto& x = ctx->xb;
+    if (key == x.no_graph) return;
     if (x.graph.exec) cudaGraphExecDestroy(x.graph.exec);
     if (x.graph.graph) cudaGraphDestroy(x.graph.graph);
     x.graph.exec = nullptr;
     x.graph.graph = nullptr;
     const long long m0 = launch_mark();
-    FSB_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-    const int32_t st = batch_body(ctx, bc);
+    cudaGraph_t g = nullptr;
+    cudaGraphExec_t e = nullptr;
+    bool ok = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+    if (ok) {
+        ok = batch_body(ctx, bc) == FSB_OK;
+        ok = cudaStreamEndCapture(ctx->stream, &g) == cudaSuccess && ok;
+    }
     x.graph.n_kernels = (int)(launch_mark() - m0);
     note_launch(-x.graph.n_kernels);   // the kernels run (and count) at each replay
-    cudaGraph_t g = nullptr;
-    const cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
-    if (st != FSB_OK) {
+    ok = ok && cudaGraphInstantiate(&e, g, 0) == cudaSuccess;
+    if (!ok) {
         if (g) cudaGraphDestroy(g);
-        return st;
-    }
-    if (e != cudaSuccess) {
-        if (g) cudaGraphDestroy(g);
-        set_error("capture of the extraction batch failed: %s", cudaGetErrorString(e));
-        return FSB_ERR_CUDA;
+        cudaGetLastError();
+        x.no_graph = key;
+        return;
     }
     x.graph.graph = g;
-    FSB_CUDA(cudaGraphInstantiate(&x.graph.exec, g, 0));
+    x.graph.exec = e;
     x.graph.key = key;
-    return FSB_OK;
 }
 
 // fsb_sift_features_batch_d and, with h_imgs, fsb_sift_features_batch_hd
@@ -1126,8 +1128,7 @@ int32_t sift_features_batch(fsb_ctx* ctx, int32_t n_img, const uint8_t* const* h
             return st;
         }
     }
-    int32_t capture_st = FSB_OK;
-    if (again) capture_st = capture_batch(ctx, bc, key);
+    if (again) capture_batch(ctx, bc, key);
     // one wait per batch: the flags say which images (if any) exceeded a capacity
     FSB_TRY(stage_ensure(ctx, (size_t)n_img * 8 + 64));
     uint32_t* h_status = static_cast<uint32_t*>(ctx->pinned);
@@ -1159,7 +1160,7 @@ int32_t sift_features_batch(fsb_ctx* ctx, int32_t n_img, const uint8_t* const* h
         x.redone += 1;
     }
     if (h_counts) std::memcpy(h_counts, h_cnt, (size_t)n_img * 4);
-    return capture_st;
+    return FSB_OK;
 }
 }  // namespace
 }  // namespace fsb

@@ -186,6 +186,7 @@ struct fsb_ctx {
         std::vector<cudaGraphNode_t> copy_nodes;  // the upload of image i in the captured graph
         fsb::BatchGraph graph;
         std::vector<char> last_key;   // the arguments of the latest call
+        std::vector<char> no_graph;   // arguments whose capture failed
         fsb::BatchGraph pyr_graph;   // fsb_pyramid_batch_d
         int pyr_h = 0, pyr_w = 0;     // geometry whose pyramid ran once outside a capture (autotuned)
         fsb::DevBuf status;

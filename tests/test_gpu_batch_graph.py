@@ -1,0 +1,91 @@
+"""The graph of a batched extraction is a cache: a call whose work is done returns its results whether or
+not a graph could be made from it. The capture is made to fail on the host: a preloaded
+cudaGraphInstantiate that returns an error stands before the CUDA runtime's."""
+import os
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+SHIM = r"""
+#define _GNU_SOURCE
+#include <dlfcn.h>
+static int calls, fail;
+int shim_calls(void) { return calls; }
+void shim_fail(int on) { fail = on; }
+int cudaGraphInstantiate(void** exec, void* graph, unsigned long long flags) {
+    int (*real)(void**, void*, unsigned long long) = dlsym(RTLD_NEXT, "cudaGraphInstantiate");
+    if (!real) {
+        void* rt = dlopen("libcudart.so.12", RTLD_NOW | RTLD_NOLOAD);
+        if (rt) real = dlsym(rt, "cudaGraphInstantiate");
+    }
+    ++calls;
+    if (fail || !real) return 2; /* out of memory */
+    return real(exec, graph, flags);
+}
+"""
+
+BODY = """
+import ctypes, sys
+import numpy as np, torch
+import fieldstitch_b200 as F
+from fieldstitch_b200 import synth
+shim = ctypes.CDLL(sys.argv[1])
+dev = torch.device("cuda", 0)
+
+
+class Batch:
+    def __init__(self, imgs, nfeats):
+        self.nf = nfeats
+        self.want = [F.features.sift_gpu_u8(im, nf) for im, nf in zip(imgs, nfeats)]
+        self.img = [torch.from_numpy(im).to(dev) for im in imgs]
+        m = max(nfeats)
+        self.xy = [torch.zeros((m, 2), device=dev) for _ in imgs]
+        self.u8 = [torch.zeros((m, 128), dtype=torch.uint8, device=dev) for _ in imgs]
+        self.rs = [torch.zeros(m, device=dev) for _ in imgs]
+
+    def call(self, host=None):
+        for t in self.xy + self.u8 + self.rs:
+            t.zero_()
+        n = F.features.sift_gpu_batch_d(self.img, self.nf, self.xy, self.u8, self.rs, chains=2, host_images=host)
+        for k, (wxy, wu8, wrs) in enumerate(self.want):
+            assert n[k] == len(wxy) > 0
+            np.testing.assert_array_equal(self.xy[k][:n[k]].cpu().numpy(), wxy)
+            np.testing.assert_array_equal(self.u8[k][:n[k]].cpu().numpy(), wu8)
+            np.testing.assert_array_equal(self.rs[k][:n[k]].cpu().numpy(), wrs)
+
+"""
+
+
+def _run(tmp_path, body):
+    src, so, prog = tmp_path / "shim.c", tmp_path / "shim.so", tmp_path / "prog.py"
+    src.write_text(SHIM)
+    subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(so), str(src), "-ldl"], check=True)
+    prog.write_text(BODY + textwrap.dedent(body))
+    env = dict(os.environ, LD_PRELOAD=str(so), PYTHONPATH=ROOT + os.pathsep + os.environ.get("PYTHONPATH", ""))
+    r = subprocess.run([sys.executable, str(prog), str(so)], env=env, capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_failed_capture_is_no_failed_call(tmp_path):
+    _run(tmp_path, """
+    b = Batch([synth.synth_image(240, 320, 40 + k) for k in range(3)], [600, 200, 900])
+    shim.shim_fail(1)
+    for _ in range(5):
+        b.call()
+    tried = shim.shim_calls()
+    assert tried > 0           # the preloaded function was reached
+    for _ in range(3):
+        b.call()
+    assert shim.shim_calls() == tried   # what failed is not tried at every call
+    shim.shim_fail(0)
+    c = Batch([synth.synth_image(200, 300, 50 + k) for k in range(3)], [600, 200, 900])
+    for _ in range(4):
+        c.call()
+    assert shim.shim_calls() > tried    # another size gets its graph
+    """)
