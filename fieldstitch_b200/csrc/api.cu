@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <string>
 
@@ -79,7 +80,7 @@ static int32_t prepare_workspace(Workspace& ws, int h, int w) {
     if (ws.cap_cand < 65536) ws.cap_cand = 65536;
     if (ws.cap_cand < sum / 64) ws.cap_cand = sum / 64;
     FSB_TRY(ws.cand.ensure(ws.cap_cand * 4));
-    FSB_TRY(ws.counters.ensure(64));
+    FSB_TRY(ws.counters.ensure(64 + sizeof(ImageSlot)));
     return FSB_OK;
 }
 
@@ -345,12 +346,18 @@ static int32_t matches_out(fsb_ctx* ctx, const int64_t* dq, int cap, int64_t* q,
 
 // selected keypoints -> describe inputs (tx..tly) and optional interleaved xy / response outputs
 // d_n (nullable): the selection count on the device, n a capacity
-__global__ void k_take(const int32_t* __restrict__ sel, int n, const int* __restrict__ d_n, const float* x,
+// slot (nullable): the outputs' addresses are read there
+__global__ void k_take(const int32_t* __restrict__ sel, int n, const int* __restrict__ d_n,
+                       const ImageSlot* __restrict__ slot, const float* x,
                        const float* y, const float* sz, const float* an, const float* rs, const int32_t* oc,
                        const int32_t* ly, float* ox, float* oy, float* osz, float* oan, float* ors, int32_t* ooc,
                        int32_t* oly, float* oxy, float* oresp) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (d_n) n = min(*d_n, n);
+    if (slot) {
+        oxy = slot->xy;
+        oresp = slot->resp;
+    }
     if (i >= n) return;
     const int k = sel[i];
     ox[i] = x[k]; oy[i] = y[k]; osz[i] = sz[k]; oan[i] = an[k]; ors[i] = rs[k]; ooc[i] = oc[k]; oly[i] = ly[k];
@@ -380,7 +387,7 @@ static int32_t features_dev(fsb_ctx* ctx, Workspace& ws, int nfeat, bool exact, 
     float* trs = tan_ + n_sel;
     int32_t* toc = reinterpret_cast<int32_t*>(trs + n_sel);
     int32_t* tly = toc + n_sel;
-    k_take<<<(n_sel + 255) / 256, 256, 0, s>>>(sel, n_sel, nullptr, ws.kx.as<float>(), ws.ky.as<float>(),
+    k_take<<<(n_sel + 255) / 256, 256, 0, s>>>(sel, n_sel, nullptr, nullptr, ws.kx.as<float>(), ws.ky.as<float>(),
                                                ws.ksize.as<float>(), ws.kangle.as<float>(), ws.kresp.as<float>(),
                                                ws.koct.as<int32_t>(), ws.klayer.as<int32_t>(), tx, ty, tsz, tan_,
                                                trs, toc, tly, d_xy, d_resp);
@@ -464,20 +471,29 @@ void fsb_ctx::stage_release() {
 
 using namespace fsb;
 
-// ---- sync-free batched extraction: one CUDA graph per batch
+// ---- sync-free batched extraction: chains of images, a CUDA graph per chain
 namespace fsb {
 namespace {
+constexpr int MAX_CHAINS = 32;
+struct SlotFill {
+    ImageSlot* at[MAX_CHAINS];
+    ImageSlot v[MAX_CHAINS];
+};
+__global__ void k_image_slots(const __grid_constant__ SlotFill f, int n) {
+    if ((int)threadIdx.x < n) *f.at[threadIdx.x] = f.v[threadIdx.x];
+}
+
 // per image after its chain ran: the feature count and the flags (ASYNC_*, 8 = pyramid timeout)
-__global__ void k_batch_status(const uint32_t* cnt, int32_t* count, uint32_t* status) {
+__global__ void k_batch_status(const uint32_t* cnt, const ImageSlot* slot) {
     if (threadIdx.x != 0) return;
-    *count = (int32_t)cnt[6];
-    *status = cnt[7] | (cnt[PYR_ERR_WORD] ? 8u : 0u);
+    *slot->count = (int32_t)cnt[6];
+    *slot->status = cnt[7] | (cnt[PYR_ERR_WORD] ? 8u : 0u);
 }
 
 struct BatchCall {
     int n_img;
     const uint8_t* const* imgs;
-    const uint8_t* const* h_imgs;   // page-locked host images uploaded by the graph, or null
+    const uint8_t* const* h_imgs;   // page-locked host images to upload, or null
     int h, w, stride;
     const fsb_sift_params* p;
     const int32_t* nfeats;
@@ -487,13 +503,67 @@ struct BatchCall {
     int32_t* d_counts;
 };
 
-// the stream work of the batch (captured): image i on chain i mod chains
-int32_t batch_body(fsb_ctx* ctx, const BatchCall& b) {
+// Everything of an image once its slot is filled.
+int32_t chain_body(fsb_ctx* ctx, Workspace& ws, const BatchCall& b, cudaStream_t s) {
+    const AsyncCaps& caps = ctx->xb.caps;
+    const bool exact = (b.p->flags & FSB_SIFT_EXACT_BLUR) != 0;
+    FSB_TRY(run_pyramid_base(ws, nullptr, b.stride, exact, s, ws.slot()));
+    FSB_TRY(run_octaves(ws, exact, s, nullptr, nullptr));
+    FSB_TRY(run_detect_async(ws, b.p->contrast, b.p->edge, caps, exact, s));
+    const int nf = caps.nfeat;
+    float* tx = ws.take.as<float>();
+    float* ty = tx + nf;
+    float* tsz = ty + nf;
+    float* tan_ = tsz + nf;
+    float* trs = tan_ + nf;
+    int32_t* toc = reinterpret_cast<int32_t*>(trs + nf);
+    int32_t* tly = toc + nf;
+    int32_t* sel = tly + nf;
+    FSB_TRY(spread_async(ws, caps, sel, s));
+    const int* d_nsel = reinterpret_cast<const int*>(ws.counters.as<uint32_t>() + 6);
+    k_take<<<(nf + 255) / 256, 256, 0, s>>>(sel, nf, d_nsel, ws.slot(), ws.kx.as<float>(), ws.ky.as<float>(),
+                                           ws.ksize.as<float>(), ws.kangle.as<float>(), ws.kresp.as<float>(),
+                                           ws.koct.as<int32_t>(), ws.klayer.as<int32_t>(), tx, ty, tsz, tan_, trs,
+                                           toc, tly, nullptr, nullptr);
+    FSB_TRY(run_describe_dev(ws, nf, d_nsel, tx, ty, tsz, tan_, toc, tly, exact, s));
+    k_batch_status<<<1, 32, 0, s>>>(ws.counters.as<uint32_t>(), ws.slot());
+    note_launch(2);
+    FSB_CUDA(cudaGetLastError());
+    return FSB_OK;
+}
+
+// the chain's graph for a key (then its first one), or null
+fsb_ctx::ChainGraphs::Kept* find_graph(fsb_ctx::ChainGraphs& gs, const std::vector<char>& key) {
+    for (size_t k = 0; k < gs.kept.size(); ++k)
+        if (gs.kept[k].key == key) {
+            if (k) std::rotate(gs.kept.begin(), gs.kept.begin() + k, gs.kept.begin() + k + 1);
+            return &gs.kept[0];
+        }
+    return nullptr;
+}
+
+// the stream work of the batch: image i on chain i mod chains, keys[c] what chain c's graph depends on
+int32_t batch_body(fsb_ctx* ctx, const BatchCall& b, const std::vector<std::vector<char>>& keys) {
     auto& x = ctx->xb;
     const int chains = (int)x.streams.size();
-    const bool exact = (b.p->flags & FSB_SIFT_EXACT_BLUR) != 0;
+    // the slots of images i0 .. i0 + n - 1 (of as many chains) filled on stream s
+    auto fill = [&](int i0, int n, cudaStream_t s) -> int32_t {
+        SlotFill f{};
+        for (int k = 0; k < n; ++k) {
+            const int i = i0 + k;
+            const uint32_t max_kp = (uint32_t)std::max(1, std::min((int)((double)b.nfeats[i] * 2.2), x.caps.kp));
+            f.at[k] = x.ws[i % chains]->slot();
+            f.v[k] = ImageSlot{b.imgs[i], b.xy[i], b.resp ? b.resp[i] : nullptr, b.u8[i], b.d_counts + i,
+                               x.status.as<uint32_t>() + i, max_kp, b.nfeats[i]};
+        }
+        k_image_slots<<<1, MAX_CHAINS, 0, s>>>(f, n);
+        note_launch();
+        FSB_CUDA(cudaGetLastError());
+        return FSB_OK;
+    };
+    const int used = std::min(b.n_img, chains);
+    FSB_TRY(fill(0, used, ctx->stream));
     FSB_CUDA(cudaEventRecord(x.fork, ctx->stream));
-    for (int c = 0; c < chains; ++c) FSB_CUDA(cudaStreamWaitEvent(x.streams[c], x.fork, 0));
     if (b.h_imgs) {
         // the uploads on their own stream, in image order: image i's chain waits for image i only,
         // so later uploads overlap the extraction of earlier images
@@ -502,58 +572,26 @@ int32_t batch_body(fsb_ctx* ctx, const BatchCall& b) {
         for (int i = 0; i < b.n_img; ++i) {
             FSB_CUDA(cudaMemcpyAsync(const_cast<uint8_t*>(b.imgs[i]), b.h_imgs[i], bytes, cudaMemcpyHostToDevice,
                                      x.upload));
-            cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-            const cudaGraphNode_t* deps = nullptr;
-            size_t nd = 0;
-            FSB_CUDA(cudaStreamGetCaptureInfo(x.upload, &cs, nullptr, nullptr, &deps, &nd));
-            if (cs == cudaStreamCaptureStatusActive) {
-                if (nd != 1) {
-                    set_error("capture of the image uploads: unexpected capture state");
-                    return FSB_ERR_CUDA;
-                }
-                // (a direct launch leaves the nodes of the graph that is kept)
-                x.copy_nodes.resize(b.n_img);
-                x.copy_nodes[i] = deps[0];
-            }
             FSB_CUDA(cudaEventRecord(x.uploaded[i], x.upload));
         }
     }
-    uint32_t* status = x.status.as<uint32_t>();
     for (int i = 0; i < b.n_img; ++i) {
         const int c = i % chains;
         cudaStream_t s = x.streams[c];
-        Workspace& ws = *x.ws[c];
-        const int nfeat = b.nfeats[i];
+        if (i < used) FSB_CUDA(cudaStreamWaitEvent(s, x.fork, 0));
         if (b.h_imgs) FSB_CUDA(cudaStreamWaitEvent(s, x.uploaded[i], 0));
-        FSB_TRY(run_pyramid(ws, b.imgs[i], b.stride, exact, s, nullptr, nullptr));
-        FSB_TRY(run_detect_async(ws, b.p->contrast, b.p->edge, x.caps, (int)((double)nfeat * 2.2), exact, s));
-        const int nf = x.caps.nfeat;
-        float* tx = ws.take.as<float>();
-        float* ty = tx + nf;
-        float* tsz = ty + nf;
-        float* tan_ = tsz + nf;
-        float* trs = tan_ + nf;
-        int32_t* toc = reinterpret_cast<int32_t*>(trs + nf);
-        int32_t* tly = toc + nf;
-        int32_t* sel = tly + nf;
-        FSB_TRY(spread_async(ws, x.caps, nfeat, sel, s));
-        const int* d_nsel = reinterpret_cast<const int*>(ws.counters.as<uint32_t>() + 6);
-        k_take<<<(nf + 255) / 256, 256, 0, s>>>(sel, nf, d_nsel, ws.kx.as<float>(), ws.ky.as<float>(),
-                                               ws.ksize.as<float>(), ws.kangle.as<float>(), ws.kresp.as<float>(),
-                                               ws.koct.as<int32_t>(), ws.klayer.as<int32_t>(), tx, ty, tsz, tan_, trs,
-                                               toc, tly, b.xy[i], b.resp ? b.resp[i] : nullptr);
-        FSB_TRY(run_describe_dev(ws, nf, d_nsel, tx, ty, tsz, tan_, toc, tly, nullptr, b.u8[i], exact, s));
-        k_batch_status<<<1, 32, 0, s>>>(ws.counters.as<uint32_t>(), b.d_counts + i, status + i);
-        note_launch(2);
-        FSB_CUDA(cudaGetLastError());
+        if (i >= used) FSB_TRY(fill(i, 1, s));
+        if (auto* g = find_graph(x.graphs[c], keys[c])) {
+            FSB_CUDA(cudaGraphLaunch(g->exec, s));
+            note_launch(g->n_kernels);
+            g->uses += 1;
+        } else {
+            FSB_TRY(chain_body(ctx, *x.ws[c], b, s));
+        }
     }
-    for (int c = 0; c < chains; ++c) {
+    for (int c = 0; c < used; ++c) {
         FSB_CUDA(cudaEventRecord(x.join[c], x.streams[c]));
         FSB_CUDA(cudaStreamWaitEvent(ctx->stream, x.join[c], 0));
-    }
-    if (b.h_imgs) {   // the upload stream rejoins too (its last node precedes every chain anyway)
-        FSB_CUDA(cudaEventRecord(x.uploaded[b.n_img - 1], x.upload));
-        FSB_CUDA(cudaStreamWaitEvent(ctx->stream, x.uploaded[b.n_img - 1], 0));
     }
     return FSB_OK;
 }
@@ -626,8 +664,11 @@ int32_t fsb_destroy(fsb_ctx* ctx) {
         auto& x = ctx->xb;
         for (cudaStream_t cs : x.streams) cudaStreamSynchronize(cs);
         if (x.upload) cudaStreamSynchronize(x.upload);
-        if (x.graph.exec) cudaGraphExecDestroy(x.graph.exec);
-        if (x.graph.graph) cudaGraphDestroy(x.graph.graph);
+        for (auto& gs : x.graphs)
+            for (auto& g : gs.kept) {
+                cudaGraphExecDestroy(g.exec);
+                cudaGraphDestroy(g.graph);
+            }
         if (x.pyr_graph.exec) cudaGraphExecDestroy(x.pyr_graph.exec);
         if (x.pyr_graph.graph) cudaGraphDestroy(x.pyr_graph.graph);
         for (Workspace* w : x.ws) {
@@ -938,35 +979,36 @@ int32_t fsb_sift_features_ex_d(fsb_ctx* ctx, const uint8_t* d_img, int32_t h, in
 
 namespace fsb {
 namespace {
-// The launches of a batch as a graph, for later calls with the same key. The graph is a cache: the call's own
-// work is done without it, so a failed capture leaves no graph and no error, and its key is not tried again.
-void capture_batch(fsb_ctx* ctx, const BatchCall& bc, const std::vector<char>& key) {
-    auto& x = ctx->xb;
-    if (key == x.no_graph) return;
-    if (x.graph.exec) cudaGraphExecDestroy(x.graph.exec);
-    if (x.graph.graph) cudaGraphDestroy(x.graph.graph);
-    x.graph.exec = nullptr;
-    x.graph.graph = nullptr;
+// What chain c runs for an image as a graph, for later images with the same key. The graph is a cache: the call's
+// own work is queued without it, so a failed capture leaves no graph and no error, and its key is not tried
+// again. Nothing of it runs here, and the workspace is only named.
+void capture_chain(fsb_ctx* ctx, int c, const BatchCall& b, const std::vector<char>& key) {
+    auto& gs = ctx->xb.graphs[c];
+    cudaStream_t s = ctx->xb.streams[c];
+    fsb_ctx::ChainGraphs::Kept g;
     const long long m0 = launch_mark();
-    cudaGraph_t g = nullptr;
-    cudaGraphExec_t e = nullptr;
-    bool ok = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+    bool ok = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
     if (ok) {
-        ok = batch_body(ctx, bc) == FSB_OK;
-        ok = cudaStreamEndCapture(ctx->stream, &g) == cudaSuccess && ok;
+        ok = chain_body(ctx, *ctx->xb.ws[c], b, s) == FSB_OK;
+        ok = cudaStreamEndCapture(s, &g.graph) == cudaSuccess && ok;
     }
-    x.graph.n_kernels = (int)(launch_mark() - m0);
-    note_launch(-x.graph.n_kernels);   // the kernels run (and count) at each replay
-    ok = ok && cudaGraphInstantiate(&e, g, 0) == cudaSuccess;
+    g.n_kernels = (int)(launch_mark() - m0);
+    note_launch(-g.n_kernels);   // the kernels run (and count) at each replay
+    ok = ok && cudaGraphInstantiate(&g.exec, g.graph, 0) == cudaSuccess;
     if (!ok) {
-        if (g) cudaGraphDestroy(g);
+        if (g.graph) cudaGraphDestroy(g.graph);
         cudaGetLastError();
-        x.no_graph = key;
+        gs.failed = key;
         return;
     }
-    x.graph.graph = g;
-    x.graph.exec = e;
-    x.graph.key = key;
+    if (cudaGraphUpload(g.exec, s) != cudaSuccess) cudaGetLastError();   // else the first launch uploads it
+    g.key = key;
+    if ((int)gs.kept.size() == gs.KEEP) {
+        cudaGraphExecDestroy(gs.kept.back().exec);
+        cudaGraphDestroy(gs.kept.back().graph);
+        gs.kept.pop_back();
+    }
+    gs.kept.insert(gs.kept.begin(), g);
 }
 
 // fsb_sift_features_batch_d and, with h_imgs, fsb_sift_features_batch_hd
@@ -980,7 +1022,7 @@ int32_t sift_features_batch(fsb_ctx* ctx, int32_t n_img, const uint8_t* const* h
     FSB_ARG(d_imgs && nfeats && d_xy && d_rootsift && d_counts, "null array");
     FSB_ARG(h > 0 && w > 0 && stride >= w, "bad image size or stride");
     FSB_ARG(h <= 32768 && w <= 32768, "image larger than 32768 pixels on a side");
-    FSB_ARG(chains >= 1 && chains <= 32, "chains must be 1..32");
+    FSB_ARG(chains >= 1 && chains <= MAX_CHAINS, "chains must be 1..32");
     int nf_max = 0;
     for (int i = 0; i < n_img; ++i) {
         FSB_ARG(nfeats[i] >= 0 && nfeats[i] <= (1 << 24), "nfeat out of range");
@@ -999,7 +1041,7 @@ int32_t sift_features_batch(fsb_ctx* ctx, int32_t n_img, const uint8_t* const* h
     auto& x = ctx->xb;
     cudaStream_t s = ctx->stream;
     const bool timing = ctx->timing;
-    ctx->timing = false;   // stage events are not captured
+    ctx->timing = false;   // no stage events inside a batch
     struct Restore {
         fsb_ctx* c;
         bool t;
@@ -1036,6 +1078,7 @@ int32_t sift_features_batch(fsb_ctx* ctx, int32_t n_img, const uint8_t* const* h
         x.streams.push_back(cs);
         x.join.push_back(ev);
         x.ws.push_back(new Workspace());
+        x.graphs.emplace_back();
     }
     if (!x.fork) FSB_CUDA(cudaEventCreateWithFlags(&x.fork, cudaEventDisableTiming));
     if (h_imgs) {
@@ -1060,7 +1103,7 @@ int32_t sift_features_batch(fsb_ctx* ctx, int32_t n_img, const uint8_t* const* h
         caps.rank = (uint32_t)(2 * caps.kp + 32);
         x.caps = caps;
     }
-    // the streams the capture uses are the first `chains`; the others idle
+    // the streams the batch uses are the first `chains`; the others idle
     std::vector<cudaStream_t> all_streams = x.streams;
     std::vector<cudaEvent_t> all_join = x.join;
     std::vector<Workspace*> all_ws = x.ws;
@@ -1079,56 +1122,55 @@ int32_t sift_features_batch(fsb_ctx* ctx, int32_t n_img, const uint8_t* const* h
         FSB_TRY(prepare_async(*ws, x.caps, s));
     }
     FSB_TRY(x.status.ensure((size_t)n_img * 4 + 64));
-    // the captured graph is replayed while every argument and buffer address is unchanged
-    std::vector<char> key;
-    key_put(key, n_img);
-    key_put(key, h_imgs != nullptr);   // the uploads' sources are set per launch, not keyed
-    key_put(key, h);
-    key_put(key, w);
-    key_put(key, stride);
-    key_put(key, chains);
-    key_put(key, *p);
-    key_put(key, x.caps);
-    key_put(key, d_counts);
-    key_put(key, x.status.p);
-    for (int i = 0; i < n_img; ++i) {
-        key_put(key, d_imgs[i]);
-        key_put(key, nfeats[i]);
-        key_put(key, d_xy[i]);
-        key_put(key, d_resp ? d_resp[i] : nullptr);
-        key_put(key, d_rootsift[i]);
+    // A chain's graphs depend on the size and stride, the thresholds, the capacities, the workspace's buffers and
+    // the settings that choose the pyramid's kernels; a caller's buffers and caps are read from the image's slot.
+    // So one is captured once per size, in the call that first meets it (a call that also tunes the pyramid and
+    // allocates the workspaces), after that call's own launches are queued. A chain keeps KEEP of them; a further
+    // one takes the place of the one unused for longest, but where that one was hardly replayed - thresholds that
+    // differ at every call - only once it repeats in the next call.
+    // Directly launched, an image is about 65 launches, 200 us of the host: more than a photo of 480 x 640 takes
+    // the GPU beside 15 others. Its graph is one launch, about 15 us, and 0.2 ms to capture. One graph of the
+    // whole call that held the caller's buffers replayed 1 to 5 % faster (a launch instead of one per image),
+    // but each new set of buffers was launched directly and its second call paid for the next capture. First,
+    // second, third, fourth call with new buffers, 16 photos of 480 x 640: 3.1, 6.1, 2.1, 1.95 ms, now 2.0 each;
+    // of 2640 x 1978: 14.7, 14.6, 14.0, 13.9, now 14.0 each.
+    BatchCall bc{n_img, d_imgs, h_imgs, h, w, stride, p, nfeats, d_xy, d_resp, d_rootsift, d_counts};
+    std::vector<char> key0;
+    key_put(key0, h);
+    key_put(key0, w);
+    key_put(key0, stride);
+    key_put(key0, *p);
+    key_put(key0, x.caps);
+    for (const char* name : {"FSB_PYRAMID", "FSB_LAYER_VARIANT", "FSB_AUTOTUNE"}) {
+        const char* v = std::getenv(name);
+        if (v) key0.insert(key0.end(), v, v + std::strlen(v));
+        key0.push_back(0);
     }
-    for (Workspace* ws : x.ws) {
+    const int used = std::min(n_img, chains);
+    std::vector<std::vector<char>> keys(chains);
+    for (int c = 0; c < used; ++c) {
+        keys[c] = key0;
+        const Workspace* ws = x.ws[c];
         const void* ptrs[] = {ws->dog.p, ws->grad.p, ws->plane[0].p, ws->plane[1].p, ws->plane[2].p,
                               ws->next_base.p, ws->cand.p, ws->refined.p, ws->oriented.p, ws->keys_a.p, ws->keys_b.p,
                               ws->vals_a.p, ws->sort_tmp.p, ws->counters.p, ws->kx.p, ws->ky.p, ws->ksize.p,
                               ws->kangle.p, ws->kresp.p, ws->koct.p, ws->klayer.p, ws->spread.p, ws->take.p};
-        for (const void* q : ptrs) key_put(key, q);
-        key_put(key, ws->sort_tmp.bytes);
+        for (const void* q : ptrs) key_put(keys[c], q);
+        key_put(keys[c], ws->sort_tmp.bytes);
     }
-    // A call with other arguments than the last one is launched directly (about 65 launches an image, queued
-    // faster than they run); capturing and instantiating a graph costs 3.6 ms per 16 images before any of
-    // them runs: 16 photos of 2640 x 1978 in new buffers 16.9 -> 14.0 ms. The second such call in a row is
-    // launched directly too, and the graph captured while the GPU works on it; later ones replay it (13.7 ms).
-    BatchCall bc{n_img, d_imgs, h_imgs, h, w, stride, p, nfeats, d_xy, d_resp, d_rootsift, d_counts};
-    const bool replay = x.graph.exec && key == x.graph.key;
-    const bool again = !replay && key == x.last_key;
-    x.last_key = key;
-    if (replay) {
-        for (int i = 0; h_imgs && i < n_img; ++i)
-            FSB_CUDA(cudaGraphExecMemcpyNodeSetParams1D(x.graph.exec, x.copy_nodes[i], const_cast<uint8_t*>(d_imgs[i]),
-                                                        h_imgs[i], (size_t)h * stride, cudaMemcpyHostToDevice));
-        FSB_CUDA(cudaGraphLaunch(x.graph.exec, s));
-        note_launch(x.graph.n_kernels);
-    } else {
-        const int32_t st = batch_body(ctx, bc);
-        if (st != FSB_OK) {   // no work left behind on the chains' streams
-            for (cudaStream_t c : x.streams) cudaStreamSynchronize(c);
-            if (x.upload) cudaStreamSynchronize(x.upload);
-            return st;
-        }
+    const int32_t st = batch_body(ctx, bc, keys);
+    if (st != FSB_OK) {   // no work left behind on the chains' streams
+        for (cudaStream_t c : x.streams) cudaStreamSynchronize(c);
+        if (x.upload) cudaStreamSynchronize(x.upload);
+        return st;
     }
-    if (again) capture_batch(ctx, bc, key);
+    for (int c = 0; c < used; ++c) {
+        auto& gs = x.graphs[c];
+        const bool repeat = keys[c] == gs.seen;
+        gs.seen = keys[c];
+        if (keys[c] == gs.failed || find_graph(gs, keys[c])) continue;
+        if (repeat || (int)gs.kept.size() < gs.KEEP || gs.kept.back().uses >= 2) capture_chain(ctx, c, bc, keys[c]);
+    }
     // one wait per batch: the flags say which images (if any) exceeded a capacity
     FSB_TRY(stage_ensure(ctx, (size_t)n_img * 8 + 64));
     uint32_t* h_status = static_cast<uint32_t*>(ctx->pinned);
@@ -1207,6 +1249,7 @@ int32_t fsb_pyramid_batch_d(fsb_ctx* ctx, int32_t n_img, const uint8_t* const* d
         x.streams.push_back(cs);
         x.join.push_back(ev);
         x.ws.push_back(new Workspace());
+        x.graphs.emplace_back();
     }
     if (!x.fork) FSB_CUDA(cudaEventCreateWithFlags(&x.fork, cudaEventDisableTiming));
     for (int c = 0; c < chains; ++c)

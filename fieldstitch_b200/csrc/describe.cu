@@ -270,7 +270,8 @@ __global__ void __launch_bounds__(DW * 32) k_describe(const float2* __restrict__
                                                       const float* __restrict__ kx,
                                                       const float* __restrict__ ky, const float* __restrict__ ks,
                                                       const float* __restrict__ ka, const int32_t* __restrict__ ko,
-                                                      const int32_t* __restrict__ kl, float* __restrict__ desc,
+                                                      const int32_t* __restrict__ kl,
+                                                      const ImageSlot* __restrict__ slot, float* __restrict__ desc,
                                                       uint8_t* __restrict__ u8) {
     typedef typename std::conditional<EXACT, double, float>::type Acc;
     __shared__ Acc s_acc[DW][4 * NB][32];
@@ -280,6 +281,7 @@ __global__ void __launch_bounds__(DW * 32) k_describe(const float2* __restrict__
     Acc (*acc)[32] = s_acc[wid];
     const int Rq = lane / 5 - 1, Cq = lane % 5 - 1;
     if (d_n) n = min(*d_n, n);   // the count on the device, n a capacity
+    if (slot) u8 = slot->u8;
     for (int k = blockIdx.x * DW + wid; k < n; k += gridDim.x * DW) {
         for (int b = 0; b < 4 * NB; ++b) acc[b][lane] = (Acc)0;
         // keypoint geometry in float64 as the reference's host code computes it (gsift.py:490-501)
@@ -481,11 +483,11 @@ int32_t run_describe_mode(const Workspace& ws, int n, const float* d_x, const fl
     if (exact)
         k_describe<true><<<grid, DW * 32, 0, s>>>(ws.grad.as<float2>(), ws.g, n, nullptr, d_x, d_y,
                                                   d_size,
-                                                  d_angle, d_oct, d_layer, d_desc, d_u8);
+                                                  d_angle, d_oct, d_layer, nullptr, d_desc, d_u8);
     else
         k_describe<false><<<grid, DW * 32, 0, s>>>(ws.grad.as<float2>(), ws.g, n, nullptr, d_x, d_y,
                                                    d_size,
-                                                   d_angle, d_oct, d_layer, d_desc, d_u8);
+                                                   d_angle, d_oct, d_layer, nullptr, d_desc, d_u8);
     note_launch();
     FSB_CUDA(cudaGetLastError());
     return FSB_OK;
@@ -509,19 +511,19 @@ int32_t run_orient_dev(const Workspace& ws, const Refined* ref, const uint32_t* 
     return FSB_OK;
 }
 
-// Descriptors of *d_n keypoints (read on the device; at most cap), grid sized for cap.
+// RootSIFT of *d_n keypoints (read on the device; at most cap) to the slot's output, grid sized for cap.
 int32_t run_describe_dev(const Workspace& ws, int cap, const int* d_n, const float* d_x, const float* d_y,
                          const float* d_size, const float* d_angle, const int32_t* d_oct, const int32_t* d_layer,
-                         float* d_desc, uint8_t* d_u8, bool exact, cudaStream_t s) {
+                         bool exact, cudaStream_t s) {
     if (cap <= 0) return FSB_OK;
     const unsigned nb = blocks(cap, DW);
     const unsigned grid = nb;
     if (exact)
         k_describe<true><<<grid, DW * 32, 0, s>>>(ws.grad.as<float2>(), ws.g, cap, d_n, d_x, d_y,
-                                                  d_size, d_angle, d_oct, d_layer, d_desc, d_u8);
+                                                  d_size, d_angle, d_oct, d_layer, ws.slot(), nullptr, nullptr);
     else
         k_describe<false><<<grid, DW * 32, 0, s>>>(ws.grad.as<float2>(), ws.g, cap, d_n, d_x, d_y,
-                                                   d_size, d_angle, d_oct, d_layer, d_desc, d_u8);
+                                                   d_size, d_angle, d_oct, d_layer, ws.slot(), nullptr, nullptr);
     note_launch();
     FSB_CUDA(cudaGetLastError());
     return FSB_OK;

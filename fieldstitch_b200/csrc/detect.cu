@@ -456,6 +456,7 @@ __global__ void k_gather_ranked(const Oriented* __restrict__ slots, const uint32
 //   * the stable response sort of features.py:126 orders the selection by (response descending,
 //     selection position): index order, except inside a run of equal responses, where the
 //     selection positions decide.
+// slot (nullable): the feature cap is read there instead.
 // The input is split into chunks of `ch` elements (a multiple of 1024; at most 64 chunks), one
 // 1024-thread block each, one element per thread per step: k_sp_hist counts cells per chunk;
 // k_sp_pos ranks elements in their cells (per-warp multi-split by __match_any_sync, warps in
@@ -494,10 +495,12 @@ __global__ void __launch_bounds__(SP_T) k_sp_hist(const float* __restrict__ x, c
 
 __global__ void __launch_bounds__(SP_T) k_sp_pos(const float* __restrict__ x, const float* __restrict__ y, int n,
                                                  const int* __restrict__ d_n, float W, float H, int ch, int nch,
-                                                 const int* __restrict__ hist, int cap, int nfeat,
-                                                 int* __restrict__ pos, int* __restrict__ grp_sel,
+                                                 const int* __restrict__ hist, const ImageSlot* __restrict__ slot,
+                                                 int nfeat, int* __restrict__ pos, int* __restrict__ grp_sel,
                                                  int* __restrict__ chunk_sel) {
     if (d_n) n = min(*d_n, n);
+    if (slot) nfeat = slot->nfeat;
+    const int cap = (nfeat + SP_CELLS - 1) / SP_CELLS;
     __shared__ int run[SP_CELLS];          // elements of the cell before the current step (all chunks)
     __shared__ int start0[SP_CELLS];       // first selection position of the cell's group-0 elements
     __shared__ int wc[SP_NW][SP_CELLS];    // per warp and cell: count, then the warp's base
@@ -610,11 +613,13 @@ __global__ void __launch_bounds__(SP_T) k_sp_pos(const float* __restrict__ x, co
 // d_n (nullable): the keypoint count on the device, n a capacity; at most nfeat keypoints are
 // all selected, in their own order (features.py:39-40 returns range(n)), as k_iota does
 __global__ void __launch_bounds__(256) k_sp_place(const float* __restrict__ resp, int n, const int* __restrict__ d_n,
-                                                  int nfeat, int ch, const int* __restrict__ pos,
+                                                  const ImageSlot* __restrict__ slot, int nfeat, int ch,
+                                                  const int* __restrict__ pos,
                                                   const int* __restrict__ grp_sel, const int* __restrict__ chunk_sel,
                                                   bool by_position, int32_t* __restrict__ sel) {
     const int lane = threadIdx.x & 31;
     const int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;   // 32-element group
+    if (slot) nfeat = slot->nfeat;
     if (d_n) {
         n = min(*d_n, n);
         if (n <= nfeat) {
@@ -810,10 +815,9 @@ int32_t spread_dev(fsb_ctx* ctx, const float* d_x, const float* d_y, const float
     int* chunk_sel = hist + (size_t)nch * SP_CELLS;
     int* grp_sel = chunk_sel + nch;
     int* pos = grp_sel + ngrp;
-    const int cap = (nfeat + SP_CELLS - 1) / SP_CELLS;
     k_sp_hist<<<nch, SP_T, 0, s>>>(d_x, d_y, n, nullptr, W, H, ch, hist);
-    k_sp_pos<<<nch, SP_T, 0, s>>>(d_x, d_y, n, nullptr, W, H, ch, nch, hist, cap, nfeat, pos, grp_sel, chunk_sel);
-    k_sp_place<<<blocks((long long)ngrp * 32, 256), 256, 0, s>>>(d_resp, n, nullptr, nfeat, ch, pos, grp_sel,
+    k_sp_pos<<<nch, SP_T, 0, s>>>(d_x, d_y, n, nullptr, W, H, ch, nch, hist, nullptr, nfeat, pos, grp_sel, chunk_sel);
+    k_sp_place<<<blocks((long long)ngrp * 32, 256), 256, 0, s>>>(d_resp, n, nullptr, nullptr, nfeat, ch, pos, grp_sel,
                                                                    chunk_sel, by_position, d_sel);
     note_launch(3);
     FSB_CUDA(cudaGetLastError());
@@ -833,15 +837,17 @@ int32_t run_spread(const Workspace& ws, int nfeat, int32_t* d_sel_out, int* n_se
 // the same outputs as run_detect, each launch sized by a capacity fixed beforehand and reading its
 // count from ws.counters. Status words (uint32) of ws.counters: [0] candidates, [1] refined,
 // [2] orientation peaks, [3] / [4] the current orientation pass's rank range, [5] keypoints kept,
-// [6] features selected, [7] flags (ASYNC_*). A flagged image must be redone by the host-driven path.
+// [6] features selected, [7] flags (ASYNC_*). The image's own caps are read from ws.slot(). A flagged image must
+// be redone by the host-driven path.
 namespace fsb {
 namespace {
 
 // orientation pass `pass`: the next rank range, as run_detect's loop forms it (empty once the cap
 // is met or every refined extremum is oriented)
-__global__ void k_orient_range(uint32_t* cnt, int pass, uint32_t max_kp, uint32_t cap_ref, uint32_t cap_rank) {
+__global__ void k_orient_range(uint32_t* cnt, const ImageSlot* slot, int pass, uint32_t cap_ref, uint32_t cap_rank) {
     if (threadIdx.x != 0) return;
     const uint32_t n_ref = min(cnt[1], cap_ref), total = cnt[2], k1 = pass == 0 ? 0u : cnt[4];
+    const uint32_t max_kp = slot->max_kp;
     if (pass > 0 && (total >= max_kp || k1 >= n_ref)) {
         cnt[3] = k1;
         return;
@@ -855,9 +861,9 @@ __global__ void k_orient_range(uint32_t* cnt, int pass, uint32_t max_kp, uint32_
 }
 
 // after the passes: keypoints kept and the overflow / incomplete flags
-__global__ void k_detect_finish(uint32_t* cnt, uint32_t max_kp, uint32_t cap_cand, uint32_t cap_ref) {
+__global__ void k_detect_finish(uint32_t* cnt, const ImageSlot* slot, uint32_t cap_cand, uint32_t cap_ref) {
     if (threadIdx.x != 0) return;
-    const uint32_t n_ref = min(cnt[1], cap_ref), total = cnt[2], k1 = cnt[4];
+    const uint32_t n_ref = min(cnt[1], cap_ref), total = cnt[2], k1 = cnt[4], max_kp = slot->max_kp;
     uint32_t flags = cnt[7];
     if (cnt[0] > cap_cand) flags |= ASYNC_CAND_OVERFLOW;
     if (cnt[1] > cap_ref) flags |= ASYNC_REF_OVERFLOW;
@@ -867,10 +873,10 @@ __global__ void k_detect_finish(uint32_t* cnt, uint32_t max_kp, uint32_t cap_can
 }
 
 // features selected: none below 10 keypoints (features.py:121-122), else min(n, nfeat)
-__global__ void k_select_count(uint32_t* cnt, int nfeat) {
+__global__ void k_select_count(uint32_t* cnt, const ImageSlot* slot) {
     if (threadIdx.x != 0) return;
     const uint32_t n = cnt[5];
-    cnt[6] = n < 10u ? 0u : min(n, (uint32_t)nfeat);
+    cnt[6] = n < 10u ? 0u : min(n, (uint32_t)slot->nfeat);
 }
 
 }  // namespace
@@ -921,9 +927,7 @@ int32_t prepare_async(Workspace& ws, const AsyncCaps& c, cudaStream_t s) {
     return FSB_OK;
 }
 
-int32_t run_detect_async(Workspace& ws, double contrast, double edge, const AsyncCaps& c, int max_kp, bool exact,
-                         cudaStream_t s) {
-    const uint32_t mk = (uint32_t)std::max(1, std::min(max_kp, c.kp));
+int32_t run_detect_async(Workspace& ws, double contrast, double edge, const AsyncCaps& c, bool exact, cudaStream_t s) {
     const Geometry& g = ws.g;
     const DetectConsts k = make_consts(g, contrast, edge);
     uint32_t* cnt = ws.counters.as<uint32_t>();
@@ -947,11 +951,11 @@ int32_t run_detect_async(Workspace& ws, double contrast, double edge, const Asyn
     FSB_CUDA(cudaMemsetAsync(rcnt, 0, (size_t)c.rank * 4, s));
     Oriented* slots = ws.oriented.as<Oriented>();
     for (int pass = 0; pass < ASYNC_ORIENT_PASSES; ++pass) {
-        k_orient_range<<<1, 32, 0, s>>>(cnt, pass, mk, c.ref, c.rank);
+        k_orient_range<<<1, 32, 0, s>>>(cnt, ws.slot(), pass, c.ref, c.rank);
         FSB_TRY(run_orient_dev(ws, ws.refined.as<Refined>(), order, (uint32_t)c.kp, cnt + 3, slots, rcnt, cnt + 2,
                                exact, s));
     }
-    k_detect_finish<<<1, 32, 0, s>>>(cnt, mk, c.cand, c.ref);
+    k_detect_finish<<<1, 32, 0, s>>>(cnt, ws.slot(), c.cand, c.ref);
     tb = ws.sort_tmp.bytes;
     FSB_CUDA(cub::DeviceScan::ExclusiveSum(ws.sort_tmp.p, tb, rcnt, rpos, (int)c.rank, s));
     k_gather_ranked<<<blocks(c.rank, 256), 256, 0, s>>>(slots, rcnt, rpos, ws.refined.as<Refined>(), c.rank, 0, cnt + 4,
@@ -963,10 +967,10 @@ int32_t run_detect_async(Workspace& ws, double contrast, double edge, const Asyn
     return FSB_OK;
 }
 
-int32_t spread_async(Workspace& ws, const AsyncCaps& c, int nfeat, int32_t* d_sel, cudaStream_t s) {
+int32_t spread_async(Workspace& ws, const AsyncCaps& c, int32_t* d_sel, cudaStream_t s) {
     uint32_t* cnt = ws.counters.as<uint32_t>();
-    k_select_count<<<1, 32, 0, s>>>(cnt, nfeat);
-    if (nfeat <= 0) return FSB_OK;
+    const ImageSlot* slot = ws.slot();
+    k_select_count<<<1, 32, 0, s>>>(cnt, slot);
     const int* d_n = reinterpret_cast<const int*>(cnt + 5);
     const int n = c.kp;
     const int ch = (int)(1024 * (((long long)n + 65535) / 65536));
@@ -976,12 +980,11 @@ int32_t spread_async(Workspace& ws, const AsyncCaps& c, int nfeat, int32_t* d_se
     int* chunk_sel = hist + (size_t)nch * SP_CELLS;
     int* grp_sel = chunk_sel + nch;
     int* pos = grp_sel + ngrp;
-    const int cap = (nfeat + SP_CELLS - 1) / SP_CELLS;
     const float W = (float)ws.g.w, H = (float)ws.g.h;
     k_sp_hist<<<nch, SP_T, 0, s>>>(ws.kx.as<float>(), ws.ky.as<float>(), n, d_n, W, H, ch, hist);
-    k_sp_pos<<<nch, SP_T, 0, s>>>(ws.kx.as<float>(), ws.ky.as<float>(), n, d_n, W, H, ch, nch, hist, cap, nfeat, pos,
+    k_sp_pos<<<nch, SP_T, 0, s>>>(ws.kx.as<float>(), ws.ky.as<float>(), n, d_n, W, H, ch, nch, hist, slot, 0, pos,
                                   grp_sel, chunk_sel);
-    k_sp_place<<<blocks((long long)ngrp * 32, 256), 256, 0, s>>>(ws.kresp.as<float>(), n, d_n, nfeat, ch, pos, grp_sel,
+    k_sp_place<<<blocks((long long)ngrp * 32, 256), 256, 0, s>>>(ws.kresp.as<float>(), n, d_n, slot, 0, ch, pos, grp_sel,
                                                                    chunk_sel, false, d_sel);
     note_launch(4);
     FSB_CUDA(cudaGetLastError());

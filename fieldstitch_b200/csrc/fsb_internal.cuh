@@ -121,6 +121,18 @@ struct AsyncCaps {
     int kp, nfeat;              // keypoint cap (largest max_kp of the batch), features selected
 };
 
+// What of an image of a batch is the caller's: in device memory beside the chain's counters, so that the launches
+// of a captured chain serve every image and every call.
+struct ImageSlot {
+    const uint8_t* img;
+    float *xy, *resp;        // outputs; resp may be null
+    uint8_t* u8;
+    int32_t* count;          // features written
+    uint32_t* status;        // flags (ASYNC_*, 8: a copy of the pyramid timed out)
+    uint32_t max_kp;         // keypoint cap
+    int32_t nfeat;           // feature cap
+};
+
 // Outcome of one tensor-core dense match (all pairs of the call).
 struct TcStats {
     long long rows = 0;            // query rows
@@ -129,7 +141,7 @@ struct TcStats {
     float mean_abs_err = 0.f;      // and its mean
 };
 
-// A captured batch graph and the exact inputs it was captured for.
+// A captured graph and everything that its launches depend on.
 struct BatchGraph {
     std::vector<char> key;
     cudaGraph_t graph = nullptr;
@@ -147,7 +159,8 @@ struct Workspace {
     DevBuf cand, refined, oriented;
     DevBuf keys_a, keys_b, vals_a, vals_b, sort_tmp;
     DevBuf spread, take;         // sync-free extraction: spread scratch, selected keypoint fields
-    DevBuf counters;             // [0] candidates, [1] refined, [2] oriented
+    DevBuf counters;             // [0] candidates, [1] refined, [2] oriented; the image slot after 64 bytes
+    ImageSlot* slot() const { return reinterpret_cast<ImageSlot*>(static_cast<char*>(counters.p) + 64); }
     size_t cap_cand = 0, cap_ref = 0;
     // sorted, capped keypoints (structure of arrays)
     DevBuf kx, ky, ksize, kangle, kresp, koct, klayer;
@@ -175,18 +188,23 @@ struct fsb_ctx {
     fsb::DevBuf s_gb;      // guided matching scratch
     fsb::TcStats tc_stats{};                      // of the last tensor-core dense match
     // sync-free batched extraction (fsb_sift_features_batch_d): chains of images, each with its own
-    // stream and workspace, captured as one CUDA graph and replayed while the call is unchanged
+    // stream, workspace and graph
+    struct ChainGraphs {
+        struct Kept : fsb::BatchGraph {
+            int uses = 0;                    // images replayed
+        };
+        std::vector<Kept> kept;              // the latest used first, at most KEEP
+        std::vector<char> seen, failed;      // keys: the latest one that ran, one whose capture failed
+        static constexpr int KEEP = 4;
+    };
     struct ExtractBatch {
         std::vector<cudaStream_t> streams;
+        std::vector<ChainGraphs> graphs;
         std::vector<fsb::Workspace*> ws;
         std::vector<cudaEvent_t> join;
         cudaEvent_t fork = nullptr;
         cudaStream_t upload = nullptr;            // host-image batches: the uploads, in image order
-        std::vector<cudaEvent_t> uploaded;        // image i on the device (captured edges)
-        std::vector<cudaGraphNode_t> copy_nodes;  // the upload of image i in the captured graph
-        fsb::BatchGraph graph;
-        std::vector<char> last_key;   // the arguments of the latest call
-        std::vector<char> no_graph;   // arguments whose capture failed
+        std::vector<cudaEvent_t> uploaded;        // image i on the device
         fsb::BatchGraph pyr_graph;   // fsb_pyramid_batch_d
         int pyr_h = 0, pyr_w = 0;     // geometry whose pyramid ran once outside a capture (autotuned)
         fsb::DevBuf status;
@@ -227,13 +245,19 @@ int32_t upload_taps();
 // side / ev (2 MAXO events) may be null: then every octave runs on s alone
 int32_t run_pyramid(Workspace& ws, const uint8_t* d_img, int img_stride, bool exact, cudaStream_t s,
                     cudaStream_t side = nullptr, cudaEvent_t* ev = nullptr);
+// its two parts: the octave-0 base of an image, and everything from that base on (no caller's address)
+// (slot: the image's address is read there, d_img is unused)
+int32_t run_pyramid_base(Workspace& ws, const uint8_t* d_img, int img_stride, bool exact, cudaStream_t s,
+                         const ImageSlot* slot = nullptr);
+int32_t run_octaves(Workspace& ws, bool exact, cudaStream_t s, cudaStream_t side, cudaEvent_t* ev);
 // octave.cu
 int32_t upload_octave_taps(const float* taps, int stride, const int* counts);
 int layer_tile_variants();
 int layer_tile_height(int variant);
 int32_t launch_layer_fast(int layer, const float* src, int R, int C, int P, float* dst, float* dog, float2* grad,
                           float* down, int down_pitch, int variant, int* err, cudaStream_t s);
-int32_t launch_base_fast(const uint8_t* img, int stride, int ih, int iw, int P, float* dst, int variant, cudaStream_t s);
+int32_t launch_base_fast(const uint8_t* img, const ImageSlot* slot, int stride, int ih, int iw, int P, float* dst,
+                         int variant, cudaStream_t s);
 int32_t launch_group_lower(const float* src, int R, int C, int P, float* dog, float2* grad, float* l3, float* down,
                            int down_pitch, bool small, cudaStream_t s);
 int32_t launch_group_upper(const float* src, int R, int C, int P, float* dog3, bool small, cudaStream_t s);
@@ -260,16 +284,15 @@ constexpr uint32_t ASYNC_CAND_OVERFLOW = 1, ASYNC_REF_OVERFLOW = 2, ASYNC_ORIENT
 constexpr int ASYNC_ORIENT_PASSES = 3;
 int32_t async_caps(const Workspace& ws, int max_kp, int nfeat, AsyncCaps* c);
 int32_t prepare_async(Workspace& ws, const AsyncCaps& c, cudaStream_t s);
-// max_kp (<= c.kp) is this image's keypoint cap
-int32_t run_detect_async(Workspace& ws, double contrast, double edge, const AsyncCaps& c, int max_kp, bool exact,
-                         cudaStream_t s);
-int32_t spread_async(Workspace& ws, const AsyncCaps& c, int nfeat, int32_t* d_sel, cudaStream_t s);
+// the keypoint and feature caps (max_kp 1 .. c.kp, nfeat <= c.nfeat) and the outputs are those of ws.slot()
+int32_t run_detect_async(Workspace& ws, double contrast, double edge, const AsyncCaps& c, bool exact, cudaStream_t s);
+int32_t spread_async(Workspace& ws, const AsyncCaps& c, int32_t* d_sel, cudaStream_t s);
 int32_t run_orient_dev(const Workspace& ws, const Refined* ref, const uint32_t* order, uint32_t max_ranks,
                        const uint32_t* d_range, Oriented* slots, uint32_t* cnt, uint32_t* d_total, bool exact,
                        cudaStream_t s);
 int32_t run_describe_dev(const Workspace& ws, int cap, const int* d_n, const float* d_x, const float* d_y,
                          const float* d_size, const float* d_angle, const int32_t* d_oct, const int32_t* d_layer,
-                         float* d_desc, uint8_t* d_u8, bool exact, cudaStream_t s);
+                         bool exact, cudaStream_t s);
 int32_t spread_dev(fsb_ctx* ctx, const float* d_x, const float* d_y, const float* d_resp, int n, float W, float H,
                    int nfeat, bool by_position, int32_t* d_sel, int* n_sel, cudaStream_t s);
 

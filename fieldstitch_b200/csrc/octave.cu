@@ -230,6 +230,7 @@ constexpr int LT2_W = LX + 34;   // row-pair tile pitch (float2): 16 bytes past 
 struct LayerArgs {
     const float* src;   // L_{I-1}, R x C
     const uint8_t* img; // base: uint8 image ih x iw, row pitch img_stride
+    const ImageSlot* slot;   // base: the image's address is read here (null: img)
     int img_stride, ih, iw;
     int R, C, P;        // octave rows, columns, row pitch of every plane
     float* dst;         // L_I or null
@@ -465,6 +466,7 @@ __global__ void __launch_bounds__(LNT, r <= 10 ? 4 : 3) k_layer(const __grid_con
         float* vcs = reinterpret_cast<float*>(cns + LIN_C);
         int* box = reinterpret_cast<int*>(vcs + IH * VCW);   // source row min / max, column min / max
         float* ps = s_in;
+        const uint8_t* const img = a.slot ? a.slot->img : a.img;
         if (tid < 4) box[tid] = (tid & 1) ? -1 : 0x7fffffff;
         __syncthreads();
         for (int i0 = 0; i0 < IH + LIN_C; i0 += LNT) {
@@ -505,7 +507,7 @@ __global__ void __launch_bounds__(LNT, r <= 10 ? 4 : 3) k_layer(const __grid_con
         const float sc = (float)(1.0 / 255.0);
         if (nsr <= SRW && nsx <= VCW) {
             for (int row = tid >> 5; row < nsr; row += LNT / 32) {
-                const uint8_t* src = a.img + (size_t)(sy0 + row) * a.img_stride + sx0;
+                const uint8_t* src = img + (size_t)(sy0 + row) * a.img_stride + sx0;
                 for (int k = tid & 31; k < nsx; k += 32) ps[row * VCW + k] = __fmul_rn((float)__ldg(src + k), sc);
             }
             __syncthreads();
@@ -556,8 +558,8 @@ __global__ void __launch_bounds__(LNT, r <= 10 ? 4 : 3) k_layer(const __grid_con
         } else {
             for (int i = tid; i < IH * LIN_C; i += LNT) {
                 const int row = i / LIN_C, col = i - row * LIN_C;
-                const uint8_t* r0 = a.img + (size_t)ry[row] * a.img_stride;
-                const uint8_t* r1 = a.img + (size_t)rn[row] * a.img_stride;
+                const uint8_t* r0 = img + (size_t)ry[row] * a.img_stride;
+                const uint8_t* r1 = img + (size_t)rn[row] * a.img_stride;
                 const int ix = cxs[col], nx = cns[col];
                 const float vc = __fadd_rn(__fmul_rn(0.75f, __fmul_rn((float)__ldg(r0 + ix), sc)),
                                            __fmul_rn(0.25f, __fmul_rn((float)__ldg(r1 + ix), sc)));
@@ -1024,9 +1026,11 @@ int32_t launch_group_upper(const float* src, int R, int C, int P, float* dog3, b
 }
 
 // The float32 octave-0 base: blur (tap set 0, radius 5) of the 2x upsampled uint8 image.
-int32_t launch_base_fast(const uint8_t* img, int stride, int ih, int iw, int P, float* dst, int variant, cudaStream_t s) {
+int32_t launch_base_fast(const uint8_t* img, const ImageSlot* slot, int stride, int ih, int iw, int P, float* dst,
+                         int variant, cudaStream_t s) {
     LayerArgs a{};
     a.img = img;
+    a.slot = slot;
     a.img_stride = stride;
     a.ih = ih;
     a.iw = iw;

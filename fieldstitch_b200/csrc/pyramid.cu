@@ -109,6 +109,7 @@ __device__ __forceinline__ int mirror(int p, int n) {
 struct BlurArgs {
     const float* src;          // previous gauss layer (layer launches)
     const uint8_t* img;        // uint8 input (base launch)
+    const ImageSlot* slot;     // its address is read here (null: img)
     int img_stride, ih, iw;
     int rows, cols, pitch;     // pitch: of every plane of the octave
     float* dst;                // this layer, or null
@@ -121,13 +122,13 @@ struct BlurArgs {
 // Bilinear 2x upsample sample of the uint8 image at (Y, X) of the 2h x 2w grid, float32 with the
 // reference's rounding: a = u8 * float(1/255); t = 0.75 a[iy] + 0.25 a[ny] (rows first), then the
 // same along columns (gsift.py:90-102, 160).
-__device__ __forceinline__ float up2_sample(const BlurArgs& a, int Y, int X) {
+__device__ __forceinline__ float up2_sample(const BlurArgs& a, const uint8_t* img, int Y, int X) {
     const float s = (float)(1.0 / 255.0);
     const int iy = Y >> 1, ix = X >> 1;
     const int ny = (Y & 1) ? min(iy + 1, a.ih - 1) : max(iy - 1, 0);
     const int nx = (X & 1) ? min(ix + 1, a.iw - 1) : max(ix - 1, 0);
-    const uint8_t* r0 = a.img + (size_t)iy * a.img_stride;
-    const uint8_t* r1 = a.img + (size_t)ny * a.img_stride;
+    const uint8_t* r0 = img + (size_t)iy * a.img_stride;
+    const uint8_t* r1 = img + (size_t)ny * a.img_stride;
     const float p00 = __fmul_rn((float)r0[ix], s), p10 = __fmul_rn((float)r1[ix], s);
     const float p01 = __fmul_rn((float)r0[nx], s), p11 = __fmul_rn((float)r1[nx], s);
     const float vc = __fadd_rn(__fmul_rn(0.75f, p00), __fmul_rn(0.25f, p10));
@@ -161,10 +162,11 @@ __global__ void __launch_bounds__(NT) k_blur(BlurArgs a) {
     __shared__ float s_in[IH * SW];
     __shared__ float s_mid[TY * SW];
     const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
+    const uint8_t* const img = !BASE ? nullptr : a.slot ? a.slot->img : a.img;
     for (int i = threadIdx.x; i < IH * IW; i += NT) {
         const int yy = i / IW, xx = i - yy * IW;
         const int gy = mirror(y0 + yy - RAD, a.rows), gx = mirror(x0 + xx - RAD, a.cols);
-        s_in[yy * SW + xx] = BASE ? up2_sample(a, gy, gx) : __ldg(a.src + (size_t)gy * a.pitch + gx);
+        s_in[yy * SW + xx] = BASE ? up2_sample(a, img, gy, gx) : __ldg(a.src + (size_t)gy * a.pitch + gx);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < TY * IW; i += NT) {
@@ -225,13 +227,14 @@ int32_t run_layer_call(void* p, int v) {
 }
 struct BaseCall {
     const uint8_t* img;
+    const ImageSlot* slot;
     int stride, h, w, P;
     float* dst;
     cudaStream_t s;
 };
 int32_t run_base_call(void* p, int v) {
     const BaseCall* c = static_cast<const BaseCall*>(p);
-    return launch_base_fast(c->img, c->stride, c->h, c->w, c->P, c->dst, v == 1 ? 2 : 0, c->s);   // heights 32, 64
+    return launch_base_fast(c->img, c->slot, c->stride, c->h, c->w, c->P, c->dst, v == 1 ? 2 : 0, c->s);   // heights 32, 64
 }
 // one tuned per-layer launch: the tile height is chosen per (layer, octave size);
 // FSB_LAYER_VARIANT=k (read on every call) runs variant k everywhere instead, so each variant can
@@ -311,32 +314,48 @@ int32_t run_octave_call(void* p, int v) {
 }
 }  // namespace
 
-int32_t run_pyramid(Workspace& ws, const uint8_t* d_img, int img_stride, bool exact, cudaStream_t s, cudaStream_t side,
-                    cudaEvent_t* ev) {
+// The octave-0 base (the blurred 2x upsample) of an image into plane 0, and a cleared error word. slot
+// (nullable): the image's address is read there when the kernel runs, d_img is unused.
+int32_t run_pyramid_base(Workspace& ws, const uint8_t* d_img, int img_stride, bool exact, cudaStream_t s,
+                         const ImageSlot* slot) {
     const Geometry& g = ws.g;
-    float* P[3] = {ws.plane[0].as<float>(), ws.plane[1].as<float>(), ws.plane[2].as<float>()};
-    int* err = ws.counters.as<int>() + PYR_ERR_WORD;
-    FSB_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
-    float* DF = ws.dog.as<float>();
-    float2* GRAD = ws.grad.as<float2>();
+    float* base = ws.plane[0].as<float>();
+    FSB_CUDA(cudaMemsetAsync(ws.counters.as<int>() + PYR_ERR_WORD, 0, sizeof(int), s));
+    if (!exact) {
+        BaseCall bc{d_img, slot, img_stride, g.h, g.w, g.P[0], base, s};
+        char key[64];
+        std::snprintf(key, sizeof(key), "k_base_%dx%d", g.h, g.w);
+        int v = 0;
+        return autotune(key, 2, run_base_call, &bc, s, &v);
+    }
     BlurArgs a{};
     a.img = d_img;
+    a.slot = slot;
     a.img_stride = img_stride;
     a.ih = g.h;
     a.iw = g.w;
     a.rows = g.R[0];
     a.cols = g.C[0];
     a.pitch = g.P[0];
-    a.dst = P[0];
-    if (exact) {
-        launch<0, 5, true>(exact, a, s);
-    } else {
-        BaseCall bc{d_img, img_stride, g.h, g.w, g.P[0], P[0], s};
-        char key[64];
-        std::snprintf(key, sizeof(key), "k_base_%dx%d", g.h, g.w);
-        int v = 0;
-        FSB_TRY(autotune(key, 2, run_base_call, &bc, s, &v));
-    }
+    a.dst = base;
+    launch<0, 5, true>(exact, a, s);
+    FSB_CUDA(cudaGetLastError());
+    return FSB_OK;
+}
+
+int32_t run_pyramid(Workspace& ws, const uint8_t* d_img, int img_stride, bool exact, cudaStream_t s, cudaStream_t side,
+                    cudaEvent_t* ev) {
+    FSB_TRY(run_pyramid_base(ws, d_img, img_stride, exact, s));
+    return run_octaves(ws, exact, s, side, ev);
+}
+
+// Every octave from the base in plane 0 (which they overwrite).
+int32_t run_octaves(Workspace& ws, bool exact, cudaStream_t s, cudaStream_t side, cudaEvent_t* ev) {
+    const Geometry& g = ws.g;
+    float* P[3] = {ws.plane[0].as<float>(), ws.plane[1].as<float>(), ws.plane[2].as<float>()};
+    int* err = ws.counters.as<int>() + PYR_ERR_WORD;
+    float* DF = ws.dog.as<float>();
+    float2* GRAD = ws.grad.as<float2>();
     const Engine eng = exact ? Engine::Layer : pyramid_engine();
     if (!exact) {
         // octave o reads its base from P[0] (o = 0) or one half of next_base and writes the next

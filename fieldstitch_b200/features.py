@@ -119,7 +119,7 @@ def sift_gpu_batch(images, nfeats, streams=4, contrast=0.015, edge=12.0, exact=F
 def sift_gpu_batch_d(images, nfeats, out_xy, out_u8, out_resp=None, chains=16, contrast=0.015, edge=12.0,
                      exact=False, device=0, host_images=None):
     """Batched feature extraction on device data with no host wait inside the batch
-    (fsb_sift_features_batch_d: `chains` images in flight, a CUDA graph once the call repeats). images: same-size
+    (fsb_sift_features_batch_d: `chains` images in flight, replayed as CUDA graphs from the size's second call on). images: same-size
     uint8 CUDA tensors; nfeats: one cap per image; out_xy[i] (>= nfeat, 2) float32, out_u8[i]
     (>= nfeat, 128) uint8 and optionally out_resp[i] CUDA tensors. With host_images (page-locked
     host arrays or CPU tensors, one per image, rows as long as the device images'), the batch
@@ -167,7 +167,7 @@ def sift_gpu_batch_d(images, nfeats, out_xy, out_u8, out_resp=None, chains=16, c
 
 
 def _all_pinned(images):
-    """True when every image is a host array in page-locked memory (the graph can upload it)."""
+    """True when every image is a host array in page-locked memory (the batch can upload it)."""
     import torch
     for im in images:
         a = np.asarray(im)
@@ -184,7 +184,7 @@ def sift_gpu_u8_batch(images, nfeats, chains=16, contrast=0.015, edge=12.0, exac
     (fsb_sift_features_batch_d; images in page-locked memory are uploaded by the batch itself,
     overlapping the extraction: fsb_sift_features_batch_hd). Returns [(xy float32 (n,2), RootSIFT
     uint8 (n,128), resp float32 (n,))], equal to sift_gpu_u8 image by image. The device buffers are
-    kept between calls of the same shape, so a repeated batch replays its graph."""
+    kept between calls of the same shape, so no call but the first allocates them."""
     import torch
     n = len(images)
     if n == 0:
@@ -202,7 +202,7 @@ def sift_gpu_u8_batch(images, nfeats, chains=16, contrast=0.015, edge=12.0, exac
                             "rs": torch.empty((n, nmax), dtype=torch.float32, device=dev)}
     b = _BATCH_BUFS[key]
     host = None
-    if _all_pinned(images):   # the graph uploads them, overlapping the extraction
+    if _all_pinned(images):   # the batch uploads them, overlapping the extraction
         host = [np.asarray(im) for im in images]
     else:
         for i, im in enumerate(images):

@@ -43,7 +43,7 @@ def extract_and_match(images, nfeats, pairs, priors, radius, kc=16, ratio=0.85, 
     """Features of every image and guided matches of every pair.
 
     images: same-size uint8 host arrays (page-locked ones are uploaded inside the extraction
-    graph, overlapping the extraction of the images before them); nfeats: one
+    batch, overlapping the extraction of the images before them); nfeats: one
     keypoint cap per image (features.sift_gpu's nfeat); pairs: list of (i, j) image indices;
     priors: one 3x3 homography per pair mapping image i pixels to image j pixels (the GNSS /
     gimbal prior of matching._predict in homography form); offsets: optional per-pair float32
@@ -60,7 +60,7 @@ def extract_and_match(images, nfeats, pairs, priors, radius, kc=16, ratio=0.85, 
     nmax = max(1, max(int(v) for v in nf))
     b = _buffers(n_img, h, w, nmax, max(P, 1), device)
     host = None
-    if features._all_pinned(images):   # uploaded by the extraction graph, overlapping the extraction
+    if features._all_pinned(images):   # uploaded by the extraction batch, overlapping the extraction
         host = [np.asarray(im) for im in images]
     else:
         for i, im in enumerate(images):

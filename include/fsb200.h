@@ -154,8 +154,8 @@ int32_t fsb_sift_features_ex_d(fsb_ctx* ctx, const uint8_t* d_img, int32_t h, in
    feature step of the reference's GPU worker, app/planesite/features.py:115-129 and 343-378, for a
    batch), with no host wait inside the batch: every count stays on the device and each launch is
    sized by a capacity fixed for the geometry: `chains` images in flight, each chain with its own
-   stream and workspace. A call with new arguments or buffers is launched directly, the second equal
-   call in a row captures a CUDA graph, later equal calls replay it. Image i: d_imgs[i] (h x w, row pitch
+   stream and workspace, and a CUDA graph that the first call of a size captures once its own work is
+   queued; later calls replay it whatever their buffers, caps and number of images. Image i: d_imgs[i] (h x w, row pitch
    stride), nfeats[i] features; outputs d_xy[i] (nfeat*2 float32), d_resp[i] (nfeat float32,
    nullable array), d_rootsift[i] (nfeat*128 uint8); d_counts (device, n_img int32) receives the
    feature counts, h_counts (host, nullable) too. The first call for a geometry runs image 0 by
@@ -169,9 +169,7 @@ int32_t fsb_sift_features_batch_d(fsb_ctx* ctx, int32_t n_img, const uint8_t* co
 /* fsb_sift_features_batch_d from host images: h_imgs[i] (page-locked host memory, h rows of
    `stride` bytes) is uploaded into d_imgs[i] by the same batch, on a copy stream in image order,
    and image i's extraction waits for its own upload only, so the uploads of later images overlap
-   the extraction of earlier ones. The graph is keyed like fsb_sift_features_batch_d's (device
-   buffers, not host addresses): a later call with other host buffers replays it with the uploads
-   re-pointed. Pageable host memory is rejected (FSB_ERR_ARG). The end-to-end form of the
+   the extraction of earlier ones. Pageable host memory is rejected (FSB_ERR_ARG). The end-to-end form of the
    reference's per-photo worker loop (app/planesite/features.py:115-129 over a spawn queue). */
 int32_t fsb_sift_features_batch_hd(fsb_ctx* ctx, int32_t n_img, const uint8_t* const* h_imgs,
                                    uint8_t* const* d_imgs, int32_t h, int32_t w, int32_t stride,

@@ -89,3 +89,47 @@ def test_failed_capture_is_no_failed_call(tmp_path):
         c.call()
     assert shim.shim_calls() > tried    # another size gets its graph
     """)
+
+
+@pytest.mark.parametrize("hw", [(240, 320), (101, 333)])
+def test_graphs_are_made_once_per_size(tmp_path, hw):
+    """What a batch keeps for later calls is made by the first call of a size: a second call with the same
+    buffers, calls with other buffers, smaller caps, fewer images and page-locked uploads make no more of it,
+    and every one of them returns the per-image results. A few thresholds that take turns have a graph each;
+    one beyond the number kept takes the place of one that was replayed, else none until it repeats."""
+    _run(tmp_path, """
+    H, W = %d, %d
+    imgs = [synth.synth_image(H, W, 60 + k) for k in range(6)]
+    nf = [600, 200, 900, 50, 900, 20]
+    a, b = Batch(imgs[:5], nf[:5]), Batch(imgs[1:], nf[1:])
+    a.call()
+    made = shim.shim_calls()
+    assert made > 0
+    for _ in range(3):
+        a.call()
+    for _ in range(2):
+        b.call()
+    few = Batch(imgs[:3], [100, 700, 30])
+    few.call()
+    a.call([torch.from_numpy(im).pin_memory() for im in imgs[:5]])
+    a.call()
+    assert shim.shim_calls() == made, (made, shim.shim_calls())
+    def at(contrast, k=0):
+        want = F.features.sift_gpu_u8(imgs[k], nf[k], contrast=contrast)
+        n = F.features.sift_gpu_batch_d(a.img, nf[:5], a.xy, a.u8, a.rs, chains=2, contrast=contrast)
+        assert n[k] == len(want[0])
+        np.testing.assert_array_equal(a.u8[k][:n[k]].cpu().numpy(), want[1])
+        return shim.shim_calls()
+    for contrast in (0.03, 0.02, 0.01):
+        two = at(contrast)
+    assert two == made + 3 * 2              # one per chain and threshold
+    for contrast in (0.03, 0.02, 0.01, 0.015, 0.03):
+        assert at(contrast) == two          # kept
+    for k, contrast in enumerate((0.031, 0.032, 0.033, 0.034)):
+        assert at(contrast) == two + 2 * (k + 1)   # in the place of the four above
+    for contrast in (0.035, 0.036):
+        assert at(contrast) == two + 8      # none of those was replayed
+    assert at(0.036) == two + 10
+    assert at(0.036) == two + 10
+    assert at(0.034) == two + 10            # kept all the while
+    """ % hw)
