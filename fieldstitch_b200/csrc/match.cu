@@ -361,7 +361,6 @@ __device__ __forceinline__ int cell_of(double v, double o, double cs, int n) {
 }
 
 constexpr int G_WARPS = 4, G_CAND = 512;
-constexpr int G_QUERIES = 16;   // queries of a block (four per warp)
 
 // One pair of a guided batch (an array in device memory, or one by value).
 struct GPair {
@@ -456,7 +455,8 @@ __global__ void __launch_bounds__(G_WARPS * 32) k_gb_guided(const __grid_constan
                                                             const int32_t* __restrict__ start,
                                                             const int32_t* __restrict__ items,
                                                             const double2* __restrict__ pos, double radius, int kc,
-                                                            float ratio, unsigned long long* __restrict__ key,
+                                                            float ratio, int per_block,
+                                                            unsigned long long* __restrict__ key,
                                                             int32_t* __restrict__ c_t, float* __restrict__ c_b12,
                                                             int* __restrict__ overflow) {
     __shared__ double s_cd[G_WARPS][G_CAND];
@@ -467,8 +467,8 @@ __global__ void __launch_bounds__(G_WARPS * 32) k_gb_guided(const __grid_constan
     int32_t* ci = s_ci[wid];
     const unsigned lt = (1u << lane) - 1u;
     const bool wide = (reinterpret_cast<uintptr_t>(P.a) & 15) == 0;
-    const int q1 = min(P.na, (int)(blockIdx.x + 1) * G_QUERIES);
-    for (int q = blockIdx.x * G_QUERIES + wid; q < q1; q += G_WARPS) {
+    const int q1 = min(P.na, (int)(blockIdx.x + 1) * per_block);
+    for (int q = blockIdx.x * per_block + wid; q < q1; q += G_WARPS) {
         const double px = P.pred[2 * (size_t)q], py = P.pred[2 * (size_t)q + 1];
         Top2 best{INFINITY, INFINITY, -1};
         if (px > -radius && px < P.wb + radius && py > -radius && py < P.hb + radius) {
@@ -916,8 +916,13 @@ int32_t run_match_guided_batch(fsb_ctx* ctx, int n_pairs, const double* const* d
     FSB_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb, count, start, (int)(cells + 1), s));
     k_gb_fill<<<dim3(blocks(max_nb, 256), py), 256, 0, s>>>(hp[0], tab, cell, start, cursor, gitems, pos);
     if (!c_t) FSB_CUDA(cudaMemsetAsync(keys, 0xff, (size_t)items * 8, s));
-    k_gb_guided<<<dim3(blocks(max_na, G_QUERIES), py), G_WARPS * 32, 0, s>>>(hp[0], tab, start, gitems, pos, radius, kc,
-                                                                           ratio, keys, c_t, c_b12, overflow);
+    // Queries of a block of four warps. One per warp: the chains of dependent reads of up to 5 300 queries run at
+    // once (one pair of 2000 x 2000, a radius of 400: 179 us with four per warp, one after another, 117 with one;
+    // 9000 x 9000: 480 and 307). From about 150 000 queries on the GPU is full either way and fewer, longer blocks
+    // are faster (16 pairs of 9000 and a radius of 40: 344 and 343 us; of 14 000: 434 and 456; of 30 000: 955 and 1018).
+    const int per_block = rows <= 150000 ? G_WARPS : 4 * G_WARPS;
+    k_gb_guided<<<dim3(blocks(max_na, per_block), py), G_WARPS * 32, 0, s>>>(
+        hp[0], tab, start, gitems, pos, radius, kc, ratio, per_block, keys, c_t, c_b12, overflow);
     note_launch(4);
     FSB_CUDA(cudaGetLastError());
     if (!c_t) {
