@@ -853,21 +853,25 @@ int32_t fsb_state_atlas(fsb_state* st, int32_t which, float* out, int64_t n_floa
     }
     FSB_TRY(use_device(st->ctx));
     fsb_ctx* ctx = st->ctx;
-    if (!want) return FSB_OK;
-    FSB_TRY(ctx->s_misc.ensure((size_t)want * 4));
+    // packed in pieces of whole rows through at most 16 MB of scratch (the atlases of a 2640 x 1978 photo are
+    // 560 and 330 MB), one copy each
+    const int64_t piece = std::max<int64_t>((int64_t)4 << 20, g.C[0]);
+    FSB_TRY(ctx->s_misc.ensure((size_t)std::min(want, piece) * 4));
     float* src = ctx->s_misc.as<float>();
-    int64_t at = 0;
     for (int o = 0; o < g.n_oct; ++o) {
-        const long long rows = (long long)layers * g.R[o], n = rows * g.C[o];
+        const int64_t rows = (int64_t)layers * g.R[o], step = piece / g.C[o];
         const float* plane = which == 0 ? st->ws->dog.as<float>() + g.dog_off[o]
                                         : st->ws->grad.as<float>() + 2 * g.grad_off[o];
-        k_atlas_part<<<(unsigned)std::min<long long>((n + 255) / 256, 148 * 64), 256, 0, ctx->stream>>>(
-            plane, rows, g.C[o], g.P[o], which, src + at);
-        note_launch();
-        FSB_CUDA(cudaGetLastError());
-        at += n;
+        for (int64_t r0 = 0; r0 < rows; r0 += step) {
+            const int64_t nr = std::min(step, rows - r0), n = nr * g.C[o];
+            k_atlas_part<<<(unsigned)std::min<int64_t>((n + 255) / 256, 148 * 64), 256, 0, ctx->stream>>>(
+                plane + r0 * g.P[o] * (which == 0 ? 1 : 2), nr, g.C[o], g.P[o], which, src);
+            note_launch();
+            FSB_CUDA(cudaGetLastError());
+            FSB_CUDA(cudaMemcpyAsync(out, src, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream));
+            out += n;
+        }
     }
-    FSB_CUDA(cudaMemcpyAsync(out, src, (size_t)want * 4, cudaMemcpyDeviceToHost, ctx->stream));
     FSB_CUDA(cudaStreamSynchronize(ctx->stream));
     return FSB_OK;
 }
