@@ -48,6 +48,7 @@
 #include <vector>
 
 #include "fsb_internal.cuh"
+#include "tc_chunk.cuh"
 #include "unique.cuh"
 
 namespace fsb {
@@ -58,7 +59,6 @@ inline unsigned nblk(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 constexpr int TC_THREADS = 320;      // producer warp, MMA warp, 8 epilogue warps
 constexpr int TC_ROWS = 256;         // query rows per work item (two M=128 halves)
 constexpr int TC_N = 256;            // target rows per tile (MMA N)
-constexpr int TC_CHUNK = 16;         // columns per candidate chunk
 constexpr int TC_MAX_SPLITS = 8;
 constexpr long long TC_TIMEOUT_CYCLES = 4000000000ll;   // about two seconds at full clock
 
@@ -824,8 +824,7 @@ __global__ void __launch_bounds__(256, 4) k_tc_finish(const TcPair* __restrict__
         uint32_t k1 = ~0u, k2 = ~0u;
 #pragma unroll
         for (int k = 0; k < nre; ++k) {
-            const bool any = ch[k] >= 0 && ch[k] * TC_CHUNK < n_b;   // an empty chunk: no valid column
-            const int jc = any ? ch[k] * TC_CHUNK : 0, lim = any ? min(n_b - jc, TC_CHUNK) : 0;
+            const int lim = chunk_columns(ch[k], n_b), jc = lim ? ch[k] * TC_CHUNK : 0;   // none of an empty chunk
             const uint8_t* base = P.b + (size_t)jc * 128 + seg * 16;
             const int c0 = 2 * seg;   // this lane's columns after the butterfly
             const int n0 = c0 < lim ? __ldg(P.nB + jc + c0) : 0, n1 = c0 + 1 < lim ? __ldg(P.nB + jc + c0 + 1) : 0;
