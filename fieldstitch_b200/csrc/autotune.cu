@@ -8,7 +8,8 @@
 // inside a real call leaves that call's outputs as they would have been. A variant may itself call
 // autotune() for its own launches (the lock is never held while a variant runs).
 //   FSB_AUTOTUNE=0          always variant 0 (no timing)
-//   FSB_AUTOTUNE_FILE=path  choices are read from and appended to `path` ("key variant" lines)
+//   FSB_AUTOTUNE_FILE=path  choices are read from and appended to `path` ("key variant" lines, the key with the
+//                           device and the version of the variants)
 #include <cstdlib>
 #include <cstring>
 #include <fstream>
@@ -57,10 +58,14 @@ std::string device_tag(int dev) {
     return name;
 }
 
+// The version of the variants' numbering, part of every key: a choice kept in a file by a library whose
+// variants meant something else is not taken. To be raised with any change of a variant's meaning.
+constexpr const char* VARIANTS = "v2/";
+
 std::string full_key(const char* key) {
     int dev = 0;
     cudaGetDevice(&dev);
-    return device_tag(dev) + key;
+    return device_tag(dev) + VARIANTS + key;
 }
 
 }  // namespace
