@@ -255,13 +255,16 @@ int32_t tuned_layer(int layer, const float* src, int R, int C, int P, float* dst
 
 // FSB_PYRAMID selects the float32 octave engine (all are bit-identical): unset, the autotuner picks
 // per octave size between the per-layer kernels (variant 0, also with FSB_AUTOTUNE=0) and the
-// fused layer groups on large (1) or small (2) tiles; "layer" / "group" / "group_small" force one,
-// other values choose as unset. Read on every call.
+// fused layer groups on large (1) or small (2) tiles; "layer" / "group" / "group_small" force one.
+// "strip" and "fused", the names of two fused engines that the groups took the place of, force the
+// groups too, so that a setting that asked for a fused engine still gets one. Other values choose as
+// unset. Read on every call.
 enum class Engine { Auto, Group, GroupSmall, Layer };
 static Engine pyramid_engine() {
     const char* e = std::getenv("FSB_PYRAMID");
     if (e && std::strcmp(e, "layer") == 0) return Engine::Layer;
-    if (e && std::strcmp(e, "group") == 0) return Engine::Group;
+    for (const char* name : {"group", "strip", "fused"})
+        if (e && std::strcmp(e, name) == 0) return Engine::Group;
     if (e && std::strcmp(e, "group_small") == 0) return Engine::GroupSmall;
     return Engine::Auto;
 }
