@@ -102,6 +102,12 @@ static void give_back(fsb_ctx* ctx, Workspace* w) {
     ctx->pool.push_back(w);
 }
 
+static int32_t state_alive(const fsb_state* st) {
+    if (st->ctx) return FSB_OK;
+    set_error("the state's context was destroyed");
+    return FSB_ERR_STATE;
+}
+
 static int32_t use_device(fsb_ctx* ctx) {
     FSB_CUDA(cudaSetDevice(ctx->device));
     return FSB_OK;
@@ -656,6 +662,12 @@ int32_t fsb_destroy(fsb_ctx* ctx) {
         delete w;
     }
     ctx->pool.clear();
+    for (fsb_state* st : ctx->states) {   // what is left of them is freed by fsb_state_free
+        st->ws->release();
+        delete st->ws;
+        st->ws = nullptr;
+        st->ctx = nullptr;
+    }
     DevBuf* all[] = {&ctx->s_u8a, &ctx->s_u8b, &ctx->s_f32a, &ctx->s_f32b, &ctx->s_i32, &ctx->s_i64,
                      &ctx->s_u64, &ctx->s_misc, &ctx->s_misc2, &ctx->s_host_stage, &ctx->s_cub,
                      &ctx->s_tc_pack, &ctx->s_tc_part, &ctx->s_tc_aux, &ctx->s_count, &ctx->s_gb};
@@ -768,7 +780,7 @@ int32_t fsb_detect(fsb_ctx* ctx, const uint8_t* img, int32_t h, int32_t w, int32
     s->ws = ws;
     s->magic = STATE_MAGIC;
     s->exact = (p->flags & FSB_SIFT_EXACT_BLUR) != 0;
-    ctx->live_states++;
+    ctx->states.push_back(s);
     *state = s;
     *n_kp = ws->n_kp;
     return FSB_OK;
@@ -777,6 +789,7 @@ int32_t fsb_detect(fsb_ctx* ctx, const uint8_t* img, int32_t h, int32_t w, int32
 int32_t fsb_state_keypoints(fsb_state* st, float* x, float* y, float* size, float* angle, float* response,
                             int32_t* octave, int32_t* layer) {
     FSB_ARG(st && st->magic == STATE_MAGIC, "invalid state");
+    FSB_TRY(state_alive(st));
     fsb_ctx* ctx = st->ctx;
     FSB_TRY(use_device(ctx));
     const Workspace& ws = *st->ws;
@@ -830,6 +843,7 @@ int32_t fsb_describe(fsb_ctx* ctx, fsb_state* st, int32_t n, const float* x, con
 
 int32_t fsb_state_geometry(fsb_state* st, int32_t* n_oct, int32_t* rows, int32_t* cols) {
     FSB_ARG(st && st->magic == STATE_MAGIC, "invalid state");
+    FSB_TRY(state_alive(st));
     const Geometry& g = st->ws->g;
     if (n_oct) *n_oct = g.n_oct;
     for (int o = 0; o < g.n_oct; ++o) {
@@ -842,6 +856,7 @@ int32_t fsb_state_geometry(fsb_state* st, int32_t* n_oct, int32_t* rows, int32_t
 int32_t fsb_state_atlas(fsb_state* st, int32_t which, float* out, int64_t n_floats) {
     FSB_ARG(st && st->magic == STATE_MAGIC, "invalid state");
     FSB_ARG(out && which >= 0 && which <= 2, "bad atlas request");
+    FSB_TRY(state_alive(st));
     const Geometry& g = st->ws->g;
     const int layers = which == 0 ? 5 : 3;
     int64_t want = 0;
@@ -879,11 +894,12 @@ int32_t fsb_state_atlas(fsb_state* st, int32_t which, float* out, int64_t n_floa
 int32_t fsb_state_free(fsb_state* st) {
     if (!st) return FSB_OK;
     FSB_ARG(st->magic == STATE_MAGIC, "invalid state (double free?)");
-    fsb_ctx* ctx = st->ctx;
     st->magic = 0;
-    cudaSetDevice(ctx->device);
-    give_back(ctx, st->ws);
-    ctx->live_states--;
+    if (fsb_ctx* ctx = st->ctx) {
+        cudaSetDevice(ctx->device);
+        give_back(ctx, st->ws);
+        ctx->states.erase(std::find(ctx->states.begin(), ctx->states.end(), st));
+    }
     delete st;
     return FSB_OK;
 }

@@ -179,7 +179,7 @@ struct fsb_ctx {
     void* jpeg_handle = nullptr;                  // nvJPEG decoder of this context (created on first use)
     void* jpeg_state = nullptr;
     std::vector<fsb::Workspace*> pool;   // idle workspaces
-    int live_states = 0;
+    std::vector<struct fsb_state*> states;   // alive; fsb_destroy leaves them without a context
     // scratch for description and matching (grown on demand)
     fsb::DevBuf s_u8a, s_u8b, s_f32a, s_f32b, s_i32, s_i64, s_u64, s_misc, s_misc2, s_host_stage;
     fsb::DevBuf s_cub;   // CUB temporary storage (one primitive at a time)

@@ -56,6 +56,8 @@ const char* fsb_last_error(void);
 /* Creates a context on CUDA device `device` (the CuPy device/stream the reference's GPU worker
    uses, app/planesite/features.py:258-267). Fails with FSB_ERR_UNSUPPORTED unless sm_100. */
 int32_t fsb_create(int32_t device, fsb_ctx** out);
+/* Frees the context and its states' device memory. A state that is still alive is then only good for
+   fsb_state_free; other calls on it return FSB_ERR_STATE. */
 int32_t fsb_destroy(fsb_ctx* ctx);
 /* Waits, for at most timeout_ms, for the context's stream; FSB_ERR_TIMEOUT if it did not drain. */
 int32_t fsb_sync(fsb_ctx* ctx, int32_t timeout_ms);
