@@ -1,10 +1,12 @@
 // Candidate chunks of the tensor-core matcher: runs of TC_CHUNK targets.
 #pragma once
 
+#ifndef FSB_HD
 #ifdef __CUDACC__
 #define FSB_HD __host__ __device__ __forceinline__
 #else
 #define FSB_HD inline
+#endif
 #endif
 
 namespace fsb {
