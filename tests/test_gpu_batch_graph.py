@@ -133,3 +133,42 @@ def test_graphs_are_made_once_per_size(tmp_path, hw):
     assert at(0.036) == two + 10
     assert at(0.034) == two + 10            # kept all the while
     """ % hw)
+
+
+@pytest.mark.parametrize("exact", [False, True])
+def test_slots_carry_every_call_s_own_arguments(exact):
+    """More images than chains, other caps and outputs at each call (none for the responses, a cap of zero among
+    them), padded rows, both pyramids: the launches kept from the first call take all of it from the slots."""
+    import numpy as np
+    import torch
+    import fieldstitch_b200 as F
+    from fieldstitch_b200 import synth
+    dev = torch.device("cuda", 0)
+    h, w = 150, 203
+    imgs = [synth.synth_image(h, w, 80 + k) for k in range(7)]
+    for call in range(4):
+        rng = np.random.default_rng(call)
+        pick = [int(k) for k in rng.permutation(7)[:5 + call % 3]]
+        caps = [int(rng.integers(1, 900)) for _ in pick]
+        caps[call % len(caps)] = 0
+        pitch = w if call < 2 else w + 5   # another row pitch: graphs of its own
+        d = [torch.zeros((h, pitch), dtype=torch.uint8, device=dev)[:, :w] for _ in pick]
+        for t, k in zip(d, pick):
+            t.copy_(torch.from_numpy(imgs[k]))
+        xy = [torch.full((1000, 2), -7.0, device=dev) for _ in pick]
+        u8 = [torch.full((1000, 128), 9, dtype=torch.uint8, device=dev) for _ in pick]
+        rs = [torch.full((1000,), -7.0, device=dev) for _ in pick] if call % 2 else None
+        n = F.features.sift_gpu_batch_d(d, caps, xy, u8, rs, chains=3, exact=exact)
+        for i, (k, cap) in enumerate(zip(pick, caps)):
+            if cap == 0:
+                assert n[i] == 0
+            else:
+                wxy, wu8, wrs = F.features.sift_gpu_u8(imgs[k], cap, exact=exact)
+                assert n[i] == len(wxy)
+                np.testing.assert_array_equal(xy[i][:n[i]].cpu().numpy(), wxy)
+                np.testing.assert_array_equal(u8[i][:n[i]].cpu().numpy(), wu8)
+                if rs is not None:
+                    np.testing.assert_array_equal(rs[i][:n[i]].cpu().numpy(), wrs)
+            # nothing behind the image's own rows
+            assert (xy[i][n[i]:] == -7.0).all() and (u8[i][n[i]:] == 9).all()
+            assert rs is None or (rs[i][n[i]:] == -7.0).all()
