@@ -15,7 +15,7 @@ value  : pairs/s with the images resident in HBM (device-pointer C ABI, fsb_*_d)
 e2e    : the same pairs through the public host API (features.sift_gpu_u8 + matching
          guided_from_pred) with host buffers, copies included.
 roofline: the pyramid (dominant stage): the step's images through the pyramid stage alone as one
-         graph with the extraction graph's images in flight (fsb_pyramid_batch_d), CUDA events on its
+         graph with the extraction batch's images in flight (fsb_pyramid_batch_d), CUDA events on its
          stream; beside it the same for one image at a time on one stream; algorithmic bytes per
          image = H*W + 44 * (sum of octave pixels).
 --impl reference: the reference's CPU implementation of the path (OpenCV SIFT as
@@ -61,9 +61,9 @@ def parse():
     p.add_argument("--no-cpu", action="store_true")
     p.add_argument("--streams", type=int, default=6, help="host threads, each with its own context/stream")
     p.add_argument("--extract", default="graph", choices=["graph", "threads"],
-                   help="graph: every image of a step in one sync-free batch (one CUDA graph); threads: "
+                   help="graph: every image of a step in one sync-free batch (CUDA graphs); threads: "
                         "fsb_sift_features_d per image on --streams host threads")
-    p.add_argument("--chains", type=int, default=16, help="images in flight inside the extraction graph")
+    p.add_argument("--chains", type=int, default=16, help="images in flight inside the extraction batch")
     p.add_argument("--sweep-pairs", type=int, default=256, help="dense precision sweep: pairs per batch (0: skip)")
     p.add_argument("--sweep-n", type=int, default=16384, help="dense precision sweep: descriptors per image")
     p.add_argument("--plain-pairs", type=int, default=16,
@@ -471,7 +471,7 @@ def synthetic_flight(args, local):
 
     Batched path: every frame extracted once (sift_gpu sequence, nfeat 7000, the "accurate" preset)
     on args.streams contexts, the prior projections, then every pair's guided match in one
-    fsb_match_guided_batch_d call (a CUDA graph). Plain path: one context, frames then pairs one
+    fsb_match_guided_batch_d call. Plain path: one context, frames then pairs one
     after another (host waits after every call). Both from frames resident in HBM; device events and
     the host clock, the larger. The learned filter is trained on the first pairs' candidates (labels:
     the plain pipeline's RANSAC) and replaces the ratio test on every pair."""
@@ -570,7 +570,7 @@ def synthetic_flight(args, local):
         return max(e0.elapsed_time(e1), (time.perf_counter() - w0) * 1000.0), out
 
     streams = [torch.cuda.ExternalStream(c.stream()) for c in ctxs + [mctx]]
-    batched()   # warm-up: workspaces, autotuning of the frame geometry, the match graph's capture
+    batched()   # warm-up: workspaces, autotuning of the frame geometry
     torch.cuda.synchronize()
     ms_batched, _ = clocked(batched, streams)
     got = [(q_b[p, :counts[p]].clone(), t_b[p, :counts[p]].clone()) for p in range(P)]
@@ -687,7 +687,7 @@ def synthetic_flight(args, local):
                         % (n, w, h, args.flight_lines, args.flight_lines, P, KC, RADIUS, RATIO),
             "frames": n, "pairs": P, "generate_s": gen_s,
             "batched": {"ms": ms_batched, "pairs_per_s": P / (ms_batched / 1000.0), "streams": S,
-                        "path": "frames extracted once on %d contexts + projections + one guided-batch graph" % S},
+                        "path": "frames extracted once on %d contexts + projections + one guided batch" % S},
             "plain_fp32": {"ms": ms_plain, "pairs_per_s": P / (ms_plain / 1000.0),
                            "path": "one context, frames then pairs one call at a time"},
             "batched_over_plain": ms_plain / ms_batched,
@@ -809,7 +809,7 @@ def run_fsb(args):
     m_cnt = Iv()
 
     def match_batch():
-        """Every pair's guided match in one call (one CUDA graph, replayed from the second step)."""
+        """Every pair's guided match in one call (one set of launches)."""
         _lib.check(mctx.lib.fsb_match_guided_batch_d(
             mctx.handle, NPs, Pv(*[b["pred"].data_ptr() for b in pb]), Pv(*[b["u8"][0].data_ptr() for b in pb]),
             Iv(*[b["n"][0] for b in pb]), Pv(*[b["bxy"].data_ptr() for b in pb]),
@@ -819,7 +819,7 @@ def run_fsb(args):
         return sum(m_cnt[i] for i in range(NPs))
 
     # the step's extraction as one sync-free batch: every image in one fsb_sift_features_batch_d call
-    # (one CUDA graph, args.chains images in flight), then every pair's prior projections queued
+    # (args.chains images in flight), then every pair's prior projections queued
     # with one call on the match context
     ectx = _lib.Context(local)
     estream = torch.cuda.ExternalStream(ectx.stream())
@@ -971,8 +971,8 @@ def run_fsb(args):
         e_off = [noise[i].astype(np.float32) for i in range(len(pairs))]
 
         def e2e_step_batch():
-            """frontend.extract_and_match: the step's host images to the device, one graph extracting
-            every image, the priors projected on the device, one graph matching every pair, the match
+            """frontend.extract_and_match: the step's host images to the device, one batch extracting
+            every image, the priors projected on the device, one batch matching every pair, the match
             lists back to the host."""
             res = F.frontend.extract_and_match(x_imgs, e_nfs, e_pairs, e_priors, RADIUS, KC, RATIO, offsets=e_off,
                                                chains=args.chains, device=local)
@@ -1003,8 +1003,8 @@ def run_fsb(args):
         ms_e2e = max_over_ranks(ms_e2e, dist, dev)
         e2e = {"value": job_rate(world, args.pairs, ms_e2e), "unit": "pairs/s", "h2d_bytes_per_step": int(h2d),
                "d2h_bytes_per_step": int(d2h), "ms_per_step": ms_e2e, "steps": ksteps,
-               "api": ("frontend.extract_and_match: host images in, one graph for every image, priors projected "
-                       "on the device, one graph for every pair, match lists out" if args.extract == "graph" else
+               "api": ("frontend.extract_and_match: host images in, one batch for every image, priors projected "
+                       "on the device, one batch for every pair, match lists out" if args.extract == "graph" else
                        "features.sift_gpu_u8 + matching.guided_from_pred, %d host threads" % args.streams),
                "host_inputs": ("images in pinned host memory, the prior homographies and their errors in host "
                                "memory; the features stay on the device between extraction and matching"
@@ -1012,7 +1012,7 @@ def run_fsb(args):
                                "images in pinned host memory; keypoints / descriptors between the two calls in "
                                "the numpy arrays the API returns")}
 
-    # ---- roofline of the dominant stage (pyramid), in the configuration the extraction graph runs
+    # ---- roofline of the dominant stage (pyramid), in the configuration the extraction batch runs
     # it: the pyramids of the step's images alone as one graph (fsb_pyramid_batch_d, args.chains
     # images in flight), CUDA events on the extraction context's stream around 3 replays
     def pyr_batch():
@@ -1052,7 +1052,7 @@ def run_fsb(args):
             "algorithmic_bytes": alg, "ms_per_launch_group": pyr_batch_ms,
             "measured": ("CUDA events on the extraction stream around %d replays of the pyramid stage of the step's "
                          "%d images as one graph (fsb_pyramid_batch_d, %d in flight: the configuration of the "
-                         "extraction graph); time per image" % (pyr_reps, NI, args.chains)),
+                         "extraction batch); time per image" % (pyr_reps, NI, args.chains)),
             "one_stream": {"achieved": ach_one, "frac": (ach_one / pk) if ach_one else None,
                            "ms_per_launch_group": per_img_ms,
                            "measured": "CUDA events on the library stream, one image at a time on one stream, "
@@ -1111,12 +1111,12 @@ def run_fsb(args):
                 "warmup": args.warmup, "ms_per_step": ms_step, "higher_is_better": True, "scaling": "weak",
                 "vs_baseline": None, "dtype": "f32", "data": "synthetic (seeded)",
                 "config": config(args, {"host_streams": args.streams, "extraction": (
-                                            "every image of a step in one fsb_sift_features_batch_d call (one CUDA "
-                                            "graph, %d images in flight, no host wait inside)" % args.chains
+                                            "every image of a step in one fsb_sift_features_batch_d call (a CUDA graph "
+                                            "per image, %d images in flight, no host wait inside)" % args.chains
                                             if args.extract == "graph" else
                                             "fsb_sift_features_d per image on %d host threads" % args.streams),
                                         "matching": "every pair of a step in one fsb_match_guided_batch_d call "
-                                                    "(one CUDA graph, captured once, replayed each step)"}),
+                                                    "(one set of launches)"}),
                 "clocks": clk, "e2e": e2e, "gpu_launches": int(launches), "roofline": roof, "cpu_baseline": cpu,
                 "parity_checked": parity["parity_checked"], "parity": parity,
                 "matches_per_step": matches / args.steps, "plain_single_stream": plain,

@@ -92,7 +92,9 @@ __device__ __forceinline__ void ex_cp_async8(float2* dst, const float* src) {
 // Bound by latency at 28 warps per SM (the copies' wait, shuffles, an atomic per row with candidates; issue
 // 31 %; HBM, 557 MB, would allow 85 us). Two columns per lane share a row's addresses, copies, loop and half
 // of its shuffles, and a smaller window (the layers are reduced first) leaves the registers for it.
-// 2640 x 1978: 181 -> 138 us. Candidates collected in shared memory and appended by one atomic per 192 of
+// 2640 x 1978, the kernel alone from cold caches: 188-191 us whatever the photo, now 145 with 77 000 warp rows that
+// hold a candidate, 167 with 86 000, 180 with 101 000 (the append); the stage with its wait, on photos of 94 000 to
+// 112 000 candidates, 220 -> 166. Candidates collected in shared memory and appended by one atomic per 192 of
 // them cost 30 us (less L1 left for the copies).
 __global__ void __launch_bounds__(EX_T, EX_BLOCKS) k_extrema(const float* __restrict__ DF, DetectConsts k, ExTiles tl,
                                                   uint32_t* __restrict__ cand, uint32_t* counter, uint32_t cap) {

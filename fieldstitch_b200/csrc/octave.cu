@@ -182,7 +182,7 @@ EncodeTiledFn encode_tiled() {
 
 
 // bounded waits on a shared-memory mbarrier (TMA completion)
-constexpr long long TSTRIP_TIMEOUT = 2000000000ll;   // cycles (about a second) for one TMA copy
+constexpr long long TILE_TIMEOUT = 2000000000ll;   // cycles (about a second) for one TMA copy
 
 __device__ __forceinline__ uint32_t s_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -203,7 +203,7 @@ __device__ __forceinline__ bool s_mbar_wait(uint64_t* b, uint32_t parity) {
     bool ok = s_mbar_test(b, parity);
     if (!ok) {
         const long long t0 = clock64();
-        while (!(ok = s_mbar_test(b, parity)) && clock64() - t0 < TSTRIP_TIMEOUT) {
+        while (!(ok = s_mbar_test(b, parity)) && clock64() - t0 < TILE_TIMEOUT) {
         }
     }
     return ok;
@@ -212,7 +212,7 @@ __device__ __forceinline__ bool s_mbar_wait(uint64_t* b, uint32_t parity) {
 // ------------------------------------------------------------------------------------------------
 // Per-layer tiled kernels (float32 path), 128 x 32 outputs per CTA:
 //   k_layer<I, RAD(I), false>  L_I of one octave from L_{I-1}: the same pair blurs and gradient as
-//                              the fused kernel (bit-identical results), DoG, gradient of L_{I-1},
+//                              the layer groups (bit-identical results), DoG, gradient of L_{I-1},
 //                              L_{I-1}[::2, ::2]
 //   k_layer<0, 5, true>        the octave-0 base: the 2x bilinear upsample of the uint8 image
 //                              (the reference's float32 rounding, gsift.py:90-102) computed while the

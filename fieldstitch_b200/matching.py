@@ -138,7 +138,7 @@ def match_guided_batch(problems, radius, kc=None, ratio=0.85, device=0):
     """Batched guided matching on host arrays: ``problems[p]`` = (pred (na,2), a_desc (na,128),
     b_xy (nb,2), b_desc (nb,128), (w_b, h_b)) as ``guided_from_pred`` takes them (descriptors uint8
     or their float32 values). The data go to the device in one copy per kind into buffers kept
-    between calls with the same sizes (so a repeated batch replays its graph), every pair runs in
+    between calls with the same sizes, every pair runs in
     one ``guided_from_pred_batch_d`` call and the results come back in one copy; returns [(q, t)]
     int64 numpy arrays per pair, each equal to ``guided_from_pred`` on that pair."""
     import torch

@@ -33,7 +33,7 @@ extern "C" {
 #define FSB_PREC_FP32 0 /* CUDA-core distances (exact 32-bit values): the plain path */
 #define FSB_PREC_BF16 1 /* tcgen05 BF16 x BF16 -> FP32 (exact for uint8 rows), exact integer re-rank */
 #define FSB_PREC_FP8 2  /* tcgen05 E4M3 (per-row power-of-two scale) -> FP32, exact integer re-rank of
-                           the best 4 x 32 columns, certified ratio test, exact fallback rows */
+                           the best two chunks of 16 columns, certified ratio test, exact fallback rows */
 
 typedef struct fsb_ctx fsb_ctx;
 typedef struct fsb_state fsb_state;
