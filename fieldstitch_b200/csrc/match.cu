@@ -286,13 +286,42 @@ int bf_place(const BfPlan& pl, BfPair& p, int item0) {
     p.item0 = item0;
     return item0 + p.splits * ((p.na + bm - 1) / bm);
 }
+
+// The id of the current CUDA context, never given twice in a process (a context made after cudaDeviceReset
+// gets the old one's handle); 0 if it cannot be queried. By the runtime's driver entry points, so that the
+// library needs no link against libcuda.
+unsigned long long context_id() {
+    typedef int (*CtxGetCurrent)(void**);
+    typedef int (*CtxGetId)(void*, unsigned long long*);
+    auto entry = [](const char* name) {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q{};
+        return cudaGetDriverEntryPoint(name, &f, cudaEnableDefault, &q) == cudaSuccess &&
+                       q == cudaDriverEntryPointSuccess ? f : nullptr;
+    };
+    static const CtxGetCurrent get = reinterpret_cast<CtxGetCurrent>(entry("cuCtxGetCurrent"));
+    static const CtxGetId id_of = reinterpret_cast<CtxGetId>(entry("cuCtxGetId"));
+    void* c = nullptr;
+    unsigned long long id = 0;
+    if (!get || !id_of || get(&c) != 0 || !c || id_of(c, &id) != 0) return 0;
+    return id;
+}
+
 int32_t launch_bf(const BfPlan& pl, const BfPair& one, const BfPair* tab, int n, cudaStream_t s) {
-    static std::atomic<int> a2[64], a4[64];
+    static_assert(bf_smem<2>() <= 48 * 1024, "needs no attribute");
     if (pl.wr == 4) {
-        FSB_TRY(smem_attr((const void*)k_bf_exact<4>, bf_smem<4>(), a4));
+        // the attribute belongs to the context: set again in one made after cudaDeviceReset
+        static std::atomic<unsigned long long> set[64];
+        int dev = 0;
+        FSB_CUDA(cudaGetDevice(&dev));
+        const unsigned long long id = context_id();
+        if (id == 0 || dev >= 64 || set[dev].load(std::memory_order_acquire) != id) {
+            FSB_CUDA(cudaFuncSetAttribute((const void*)k_bf_exact<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          bf_smem<4>()));
+            if (dev < 64) set[dev].store(id, std::memory_order_release);
+        }
         k_bf_exact<4><<<pl.items, 256, bf_smem<4>(), s>>>(one, tab, n);
     } else {
-        FSB_TRY(smem_attr((const void*)k_bf_exact<2>, bf_smem<2>(), a2));
         k_bf_exact<2><<<pl.items, 128, bf_smem<2>(), s>>>(one, tab, n);
     }
     note_launch();
@@ -981,27 +1010,10 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratch
 
 std::mutex g_noalloc_mu;
 void* g_noalloc_addr[256] = {};
-void* g_noalloc_ctx[256] = {};   // the CUDA context the cached address belongs to
-
-// The current CUDA context (driver-level handle), through the runtime's driver entry point so the
-// library needs no link against libcuda; null if it cannot be queried.
-void* current_context() {
-    typedef int (*CtxGetCurrent)(void**);
-    static CtxGetCurrent fn = [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q{};
-        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            f = nullptr;
-        return reinterpret_cast<CtxGetCurrent>(f);
-    }();
-    void* c = nullptr;
-    if (fn == nullptr || fn(&c) != 0) return nullptr;
-    return c;
-}
+unsigned long long g_noalloc_ctx[256] = {};   // the id of the CUDA context the cached address belongs to
 
 // Device address of g_noalloc_scratch in the current device's current context. It is looked up
-// on the first call in a context and cached with that context's handle; a different context on
+// on the first call in a context and cached with that context's id; a different context on
 // the same device (the module loaded again after cudaDeviceReset, or a driver-API context other
 // than the primary one) looks it up again.
 int32_t noalloc_scratch(void** out) {
@@ -1011,9 +1023,9 @@ int32_t noalloc_scratch(void** out) {
         set_error("device ordinal %d out of range", dev);
         return FSB_ERR_ARG;
     }
-    void* ctx = current_context();
+    const unsigned long long ctx = context_id();
     std::lock_guard<std::mutex> lk(g_noalloc_mu);
-    if (!g_noalloc_addr[dev] || ctx == nullptr || ctx != g_noalloc_ctx[dev]) {
+    if (!g_noalloc_addr[dev] || ctx == 0 || ctx != g_noalloc_ctx[dev]) {
         void* p = nullptr;
         const cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
         if (e != cudaSuccess || p == nullptr) {
