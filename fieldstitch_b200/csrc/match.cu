@@ -947,9 +947,10 @@ int32_t run_match_guided_batch(fsb_ctx* ctx, int n_pairs, const double* const* d
     if (!c_t) FSB_CUDA(cudaMemsetAsync(keys, 0xff, (size_t)items * 8, s));
     // Queries of a block of four warps. One per warp: the chains of dependent reads of up to 5 300 queries run at
     // once (one pair of 2000 x 2000, a radius of 400: 179 us with four per warp, one after another, 117 with one;
-    // 9000 x 9000: 480 and 307). From about 150 000 queries on the GPU is full either way and fewer, longer blocks
-    // are faster (16 pairs of 9000 and a radius of 40: 344 and 343 us; of 14 000: 434 and 456; of 30 000: 955 and 1018).
-    const int per_block = rows <= 150000 ? G_WARPS : 4 * G_WARPS;
+    // 9000 x 9000: 480 and 307). Photos' pairs of 7000, a radius of 100: 28 000 queries 206 and 192 us, 56 000 295 and
+    // 287, 112 000 454 and 464; a radius of 40: 208 each at 56 000, 377 and 397 at 192 000. Full either way, the GPU
+    // is faster with fewer and longer blocks.
+    const int per_block = rows <= 64000 ? G_WARPS : 4 * G_WARPS;
     k_gb_guided<<<dim3(blocks(max_na, per_block), py), G_WARPS * 32, 0, s>>>(
         hp[0], tab, start, gitems, pos, radius, kc, ratio, per_block, keys, c_t, c_b12, overflow);
     note_launch(4);

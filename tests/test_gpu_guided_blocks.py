@@ -1,4 +1,4 @@
-"""The guided matcher's blocks hold one query per warp up to 150 000 queries of a call and four beyond: both
+"""The guided matcher's blocks hold one query per warp up to 64 000 queries of a call and four beyond: both
 give the per-pair results (whose calls hold one) across that line, with ragged last blocks, and a call of
 few queries spreads them over the GPU instead of queueing them behind one another."""
 import time
@@ -21,7 +21,7 @@ def _problem(na, nb, seed):
     return pred, a, bxy, b, (W, H)
 
 
-@pytest.mark.parametrize("nas", [(60000, 60000, 29999, 1), (60000, 60000, 29999, 2), (140001, 3, 10003)])
+@pytest.mark.parametrize("nas", [(30000, 30000, 3999, 1), (30000, 30000, 3999, 2), (64001, 3, 10003)])
 @pytest.mark.parametrize("kc", [0, 16])
 def test_batches_across_the_line_equal_single_pairs(nas, kc):
     import torch
